@@ -42,6 +42,21 @@ __device__ __forceinline__ double rcp_nr(double x) {
 // correctly rounded divide) for the FP64-pipe bound loops; b = 0 gives NaN.
 __device__ __forceinline__ double qdiv(double a, double b) { return a * rcp_nr(b); }
 
+// rinv = 1 / sqrt(x) and r = sqrt(x) for normal x in [2^-960, 2^960): the estimate y
+// of the PTX instruction rsqrt.approx.ftz.f64 and Householder's third-order step
+// y (1 + c), c = e/2 + 3 e^2 / 8 with e = 1 - x y^2; r is the same step on x y.
+// Each within about one ulp, in six FP64 instructions; a correctly rounded root
+// and then a reciprocal take four times that, in one dependent chain.
+__device__ __forceinline__ void sqrt_pair(double x, double &r, double &rinv) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double h = x * y;
+  const double e = fma(-h, y, 1.0);
+  const double c = fma(0.375, e, 0.5) * e;
+  rinv = fma(y, c, y);
+  r = fma(h, c, h);
+}
+
 // (value, index) argmax with "first index wins" ties -- Fortran MAXLOC order.
 struct ArgMax {
   double v;

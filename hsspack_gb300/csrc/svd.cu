@@ -20,6 +20,7 @@
 #include "hss_block.cuh"
 #include "hss_common.cuh"
 #include "hss_kernels.h"
+#include "hss_leaf.cuh"
 #include "hss_svdprep.cuh"
 
 namespace hss {
@@ -27,13 +28,44 @@ namespace hss {
 constexpr int SVD_LEAF_MAX = 32;
 
 // ------------------------------------------------------------- leaves -----
-// One thread per leaf: the r x (r + sqre) upper bidiagonal rows a .. a + r - 1
+// G lanes per leaf: the r x (r + sqre) upper bidiagonal rows a .. a + r - 1
 // (diag d[a + i], superdiag e[a + i]; with sqre the extra entry e[a + r - 1] sits
 // in column a + r) by the Golub-Kahan implicit-shift QR SVD (Golub & Kahan
 // 1965; Golub & Van Loan, Alg. 8.6.2), U and V accumulated as products of
 // rotations (the role of DLASDQ at SRC/mdlasd0.f90).  The extra column is first
 // chased out by column rotations, leaving its null vector in V(:, r).  Results
 // sorted ascending into slots a .. a + r - 1 (U, V, Dp, perm) and V slot a + r.
+//
+// Bound and layout as the tridiagonal leaves (leaf.cu): a serial chain of
+// rotations at one FP64 warp instruction per 64 cycles.  Each lane carries its
+// own copy of the bidiagonal and its rows of U and V, one pass of the flat
+// loop is one pair of rotations for every lane, and the zero tests run as the
+// sweep goes: bit i of `ez` says E(i) = 0, of `dz` D(i) = 0.  Leaf stage, one
+// thread per leaf before -> now: n = 1001 (64 leaves of 15 rows) 5.12 -> 0.57 ms,
+// n = 16384 (1024 of 15) 5.52 -> 0.92 ms.
+
+// Rotation taking (y, z) to (t, 0): t = hypot(y, z), cs = y / t, sn = z / t.
+__device__ __forceinline__ void plane_rotation(double y, double z, double &t, double &cs,
+                                               double &sn) {
+  const double x = fma(y, y, z * z);
+  const int hx = __double2hiint(x);
+  if (hx >= 0x03f00000 && hx < 0x7bf00000) {  // 2^-960 <= x < 2^960
+    double rinv;
+    sqrt_pair(x, t, rinv);
+    cs = y * rinv;
+    sn = z * rinv;
+  } else {
+    t = hypot(y, z);
+    cs = t == 0.0 ? 1.0 : y / t;
+    sn = t == 0.0 ? 0.0 : z / t;
+  }
+}
+
+static size_t svd_leaf_smem(int rmax, int R) {
+  return (size_t)(2 * rmax + (2 * rmax + 1) * R) * 32 * sizeof(double);
+}
+
+template <int G, int R>
 __global__ void __launch_bounds__(32)
 k_svd_leaf(int nleaf, const int *__restrict__ lstart, const int *__restrict__ lsize,
            const int *__restrict__ lsqre, int rmax, const double *__restrict__ d,
@@ -41,159 +73,245 @@ k_svd_leaf(int nleaf, const int *__restrict__ lstart, const int *__restrict__ ls
            double *__restrict__ V, long long ldv, double *__restrict__ Dp, int *__restrict__ perm,
            int *__restrict__ status) {
   extern __shared__ double lsm[];
-  const int lane = threadIdx.x, LW = blockDim.x;
-  const int leaf = blockIdx.x * LW + lane;
-  const int cmax = rmax + 1;
-  double *Ds = lsm, *Es = lsm + rmax * LW, *Us = lsm + 2 * rmax * LW,
-         *Vs = lsm + (2 * rmax + rmax * rmax) * LW;
-#define DD(i) Ds[(i) * LW + lane]
-#define EE(i) Es[(i) * LW + lane]
-#define UU(r_, c_) Us[((r_) * rmax + (c_)) * LW + lane]
-#define VV(r_, c_) Vs[((r_) * cmax + (c_)) * LW + lane]
-  if (leaf >= nleaf) return;
-  const int a = lstart[leaf], r = lsize[leaf], sq = lsqre[leaf], c = r + sq;
+  constexpr int LPW = 32 / G;
+  const int lane = threadIdx.x, q = lane / G, g0 = lane % G;
+  const int leaf = blockIdx.x * LPW + q;
+  double *D = lsm + lane;           // D[i * 32]
+  double *E = D + rmax * 32;        // E[i * 32]
+  double *Us = E + rmax * 32;       // Us[(c * R + t) * 32]: row g0 + G t, column c
+  double *Vs = Us + rmax * R * 32;  // likewise, rmax + 1 columns
+  // after the iteration: rk[c * 64] rank of column c, rk[c * 64 + 1] scratch
+  int *rk = (int *)(lsm + rmax * 32 + q * G);
+  int a = 0, r = 0, sq = 0;
+  if (leaf < nleaf) {
+    a = lstart[leaf];
+    r = lsize[leaf];
+    sq = lsqre[leaf];
+  }
+  const int c = r + sq;
+  int rows = c;  // rows per lane of the CTA's largest leaf
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) rows = max(rows, __shfl_xor_sync(HSS_FULL, rows, o));
+  rows = (rows + G - 1) / G;
+  // columns i, j of X <- (cs x_i + sn x_j, cs x_j - sn x_i)
+  auto rotate = [&](double *X, int i, int j, double cs, double sn) {
+    for (int t = 0; t < rows; ++t) {
+      const double xi = X[(i * R + t) * 32], xj = X[(j * R + t) * 32];
+      X[(i * R + t) * 32] = cs * xi + sn * xj;
+      X[(j * R + t) * 32] = cs * xj - sn * xi;
+    }
+  };
+  unsigned ez = 0, dz = 0;
+  auto scan = [&]() {  // negligible E to zero, both masks
+    ez = r > 0 ? 1u << (r - 1) : 0u;
+    dz = 0;
+    for (int i = 0; i < r; ++i) {
+      if (i + 1 < r) {
+        const double ei = E[i * 32];
+        if (ei == 0.0 || negligible(ei, D[i * 32], D[(i + 1) * 32])) {
+          E[i * 32] = 0.0;
+          ez |= 1u << i;
+        }
+      }
+      if (D[i * 32] == 0.0) dz |= 1u << i;
+    }
+  };
   for (int i = 0; i < r; ++i) {
-    DD(i) = d[a + i];
-    EE(i) = (i < r - 1 + sq) ? e[a + i] : 0.0;
-    for (int j = 0; j < r; ++j) UU(i, j) = (i == j) ? 1.0 : 0.0;
+    D[i * 32] = d[a + i];
+    E[i * 32] = (i < r - 1 + sq) ? e[a + i] : 0.0;
+#pragma unroll
+    for (int t = 0; t < R; ++t) Us[(i * R + t) * 32] = (g0 + G * t == i) ? 1.0 : 0.0;
   }
   for (int i = 0; i < c; ++i)
-    for (int j = 0; j < c; ++j) VV(i, j) = (i == j) ? 1.0 : 0.0;
-  if (sq) {  // chase the extra column's entry up and out: column r becomes zero
-    double f = EE(r - 1);
-    EE(r - 1) = 0.0;
+#pragma unroll
+    for (int t = 0; t < R; ++t) Vs[(i * R + t) * 32] = (g0 + G * t == i) ? 1.0 : 0.0;
+  if (sq && r > 0) {  // chase the extra column's entry up and out: column r becomes zero
+    double f = E[(r - 1) * 32];
+    E[(r - 1) * 32] = 0.0;
     for (int i = r - 1; i >= 0; --i) {
-      const double t = hypot(DD(i), f);
-      const double cs = t == 0.0 ? 1.0 : DD(i) / t, sn = t == 0.0 ? 0.0 : f / t;
-      DD(i) = t;
-      for (int q = 0; q < c; ++q) {
-        const double vi = VV(q, i), vr = VV(q, r);
-        VV(q, i) = cs * vi + sn * vr;
-        VV(q, r) = -sn * vi + cs * vr;
+      double t, cs, sn;
+      plane_rotation(D[i * 32], f, t, cs, sn);
+      D[i * 32] = t;
+      rotate(Vs, i, r, cs, sn);
+      if (i > 0) {
+        const double ei = E[(i - 1) * 32];
+        f = -sn * ei;
+        E[(i - 1) * 32] = cs * ei;
       }
-      if (i > 0) { f = -sn * EE(i - 1); EE(i - 1) = cs * EE(i - 1); }
     }
   }
-  int iter = 0, bad = 0;
+  scan();
+  int iter = 0, bad = 0, lo = 0, hi = 0, k = 0;
+  bool done = r == 0, sweeping = false;
+  double y = 0.0, z = 0.0, dk = 0.0, ek = 0.0, dprev = 0.0;
+  double uc[R], vc[R];  // this lane's rows of column k
   while (true) {
-    for (int i = 0; i + 1 < r; ++i)
-      if (fabs(EE(i)) <= HSS_EPS * (fabs(DD(i)) + fabs(DD(i + 1)))) EE(i) = 0.0;
-    int hi = r - 1;
-    while (hi > 0 && EE(hi - 1) == 0.0) --hi;
-    if (hi == 0) break;
-    int lo = hi - 1;
-    while (lo > 0 && EE(lo - 1) != 0.0) --lo;
-    if (++iter > 30 * r * r) { bad = 1; break; }
-    int zi = -1;
-    for (int i = lo; i < hi; ++i)
-      if (DD(i) == 0.0) { zi = i; break; }
-    if (zi < 0 && DD(hi) == 0.0) {  // zero at the bottom: chase E(hi-1) out by columns
-      double f = EE(hi - 1);
-      EE(hi - 1) = 0.0;
-      for (int k = hi - 1; k >= lo; --k) {
-        const double t = hypot(DD(k), f);
-        const double cs = DD(k) / t, sn = f / t;
-        DD(k) = t;
-        for (int q = 0; q < c; ++q) {
-          const double vk = VV(q, k), vh = VV(q, hi);
-          VV(q, k) = cs * vk + sn * vh;
-          VV(q, hi) = -sn * vk + cs * vh;
+    const unsigned work = __ballot_sync(HSS_FULL, !done), idle = __ballot_sync(HSS_FULL, !done && !sweeping);
+    if (!work) break;
+    if (4 * __popc(idle) >= __popc(work) && !done && !sweeping) {
+      const unsigned open = ~ez & ((1u << (r - 1)) - 1u);
+      if (!open) {
+        done = true;
+      } else {
+        hi = 32 - __clz(open);  // E(hi - 1) is the last nonzero one
+        const unsigned zb = ez & ((1u << (hi - 1)) - 1u);
+        lo = zb ? 32 - __clz(zb) : 0;
+        const unsigned dzb = dz & (0xffffffffu << lo) & ((1u << hi) - 1u);
+        if (++iter > 30 * r * r) {
+          bad = 1;
+          done = true;
+        } else if (dzb) {  // zero inside: chase row zi's superdiagonal out by rows
+          const int zi = __ffs(dzb) - 1;
+          double f = E[zi * 32];
+          E[zi * 32] = 0.0;
+          for (int j = zi + 1; j <= hi; ++j) {
+            double t, cs, sn;
+            plane_rotation(D[j * 32], f, t, cs, sn);
+            D[j * 32] = t;
+            rotate(Us, j, zi, cs, sn);
+            if (j < hi) {
+              const double ej = E[j * 32];
+              f = -sn * ej;
+              E[j * 32] = cs * ej;
+            }
+          }
+          scan();
+        } else if (dz >> hi & 1u) {  // zero at the bottom: chase E(hi-1) out by columns
+          double f = E[(hi - 1) * 32];
+          E[(hi - 1) * 32] = 0.0;
+          for (int j = hi - 1; j >= lo; --j) {
+            double t, cs, sn;
+            plane_rotation(D[j * 32], f, t, cs, sn);
+            D[j * 32] = t;
+            rotate(Vs, j, hi, cs, sn);
+            if (j > lo) {
+              const double ej = E[(j - 1) * 32];
+              f = -sn * ej;
+              E[(j - 1) * 32] = cs * ej;
+            }
+          }
+          scan();
+        } else {
+          // Wilkinson shift t22 - tq from the trailing 2 x 2 of B^T B of the block.
+          // Any shift keeps the iteration backward stable; tq only steers it, so it
+          // is an FP32 number unless its operands leave FP32's range.
+          const double d1 = D[(hi - 1) * 32], d2 = D[hi * 32], e1 = E[(hi - 1) * 32];
+          const double e0 = hi - 1 > lo ? E[(hi - 2) * 32] : 0.0;
+          const double t11 = fma(d1, d1, e0 * e0), t12 = d1 * e1, t22 = fma(d2, d2, e1 * e1);
+          const double dd = 0.5 * (t11 - t22);
+          const float tf = (float)t12, df = (float)dd;
+          double tq;
+          if (fabsf(tf) > 1e-15f && fabsf(tf) < 1e15f && fabsf(df) < 1e15f) {
+            tq = (double)__fdividef(tf * tf, df + copysignf(sqrtf(fmaf(df, df, tf * tf)), df));
+          } else if (dd == 0.0 && t12 == 0.0) {
+            tq = 0.0;
+          } else {
+            tq = t12 * t12 / (dd + copysign(hypot(dd, t12), dd != 0.0 ? dd : 1.0));
+          }
+          dk = D[lo * 32];
+          ek = E[lo * 32];
+          y = fma(dk, dk, tq - t22);
+          z = dk * ek;
+          k = lo;
+          dprev = 0.0;
+#pragma unroll
+          for (int t = 0; t < R; ++t) {
+            uc[t] = Us[(lo * R + t) * 32];
+            vc[t] = Vs[(lo * R + t) * 32];
+          }
+          sweeping = true;
         }
-        if (k > lo) { f = -sn * EE(k - 1); EE(k - 1) = cs * EE(k - 1); }
       }
-      continue;
     }
-    if (zi >= 0) {  // zero inside: chase row zi's superdiagonal out by rows
-      double f = EE(zi);
-      EE(zi) = 0.0;
-      for (int k = zi + 1; k <= hi; ++k) {
-        const double t = hypot(DD(k), f);
-        const double cs = DD(k) / t, sn = f / t;
-        DD(k) = t;
-        for (int q = 0; q < r; ++q) {
-          const double uk = UU(q, k), ui = UU(q, zi);
-          UU(q, k) = cs * uk + sn * ui;
-          UU(q, zi) = -sn * uk + cs * ui;
+    if (sweeping) {  // columns k, k + 1 by the right, then rows k, k + 1 by the left
+      double d1 = D[(k + 1) * 32];
+      double t, cs, sn;
+      plane_rotation(y, z, t, cs, sn);
+      const double eprev = t;  // E(k - 1)
+      const double d0 = cs * dk + sn * ek, e0 = cs * ek - sn * dk;
+      const double bl = sn * d1;
+      d1 *= cs;
+#pragma unroll
+      for (int j = 0; j < R; ++j) {
+        if (R > 4 && j >= rows) break;
+        const double x = Vs[((k + 1) * R + j) * 32];
+        Vs[(k * R + j) * 32] = cs * vc[j] + sn * x;
+        vc[j] = cs * x - sn * vc[j];
+      }
+      plane_rotation(d0, bl, t, cs, sn);
+      D[k * 32] = t;
+      dz = t == 0.0 ? dz | 1u << k : dz & ~(1u << k);
+      if (k > lo) {
+        const bool ng = negligible(eprev, dprev, t);
+        E[(k - 1) * 32] = ng ? 0.0 : eprev;
+        ez = ng ? ez | 1u << (k - 1) : ez;
+      }
+      dprev = t;
+      const double ekn = cs * e0 + sn * d1, d1n = cs * d1 - sn * e0;
+#pragma unroll
+      for (int j = 0; j < R; ++j) {
+        if (R > 4 && j >= rows) break;
+        const double x = Us[((k + 1) * R + j) * 32];
+        Us[(k * R + j) * 32] = cs * uc[j] + sn * x;
+        uc[j] = cs * x - sn * uc[j];
+      }
+      if (k + 1 < hi) {
+        ek = E[(k + 1) * 32];
+        y = ekn;
+        z = sn * ek;
+        ek *= cs;
+        dk = d1n;
+        ++k;
+      } else {  // end of the sweep
+        D[hi * 32] = d1n;
+        dz = d1n == 0.0 ? dz | 1u << hi : dz & ~(1u << hi);
+        const bool ng = ekn == 0.0 || negligible(ekn, t, d1n);
+        E[k * 32] = ng ? 0.0 : ekn;
+        ez = ng ? ez | 1u << k : ez;
+#pragma unroll
+        for (int j = 0; j < R; ++j) {
+          Us[(hi * R + j) * 32] = uc[j];
+          Vs[(hi * R + j) * 32] = vc[j];
         }
-        if (k < hi) { f = -sn * EE(k); EE(k) = cs * EE(k); }
+        sweeping = false;
       }
-      continue;
-    }
-    // Wilkinson shift from the trailing 2 x 2 of B^T B of the block
-    const int mm = hi;
-    const double t11 = DD(mm - 1) * DD(mm - 1) + (mm - 1 > lo ? EE(mm - 2) * EE(mm - 2) : 0.0);
-    const double t12 = DD(mm - 1) * EE(mm - 1);
-    const double t22 = DD(mm) * DD(mm) + EE(mm - 1) * EE(mm - 1);
-    const double dd = 0.5 * (t11 - t22);
-    double mu;
-    if (dd == 0.0 && t12 == 0.0) mu = t22;
-    else mu = t22 - t12 * t12 / (dd + copysign(hypot(dd, t12), dd != 0.0 ? dd : 1.0));
-    double y = DD(lo) * DD(lo) - mu, z = DD(lo) * EE(lo), bulge = 0.0;
-    for (int k = lo; k < hi; ++k) {
-      double t = hypot(y, z);
-      double cs = t == 0.0 ? 1.0 : y / t, sn = t == 0.0 ? 0.0 : z / t;
-      if (k > lo) EE(k - 1) = t;
-      {
-        const double dk = DD(k), ek = EE(k);
-        DD(k) = cs * dk + sn * ek;
-        EE(k) = -sn * dk + cs * ek;
-      }
-      const double bl = sn * DD(k + 1);
-      DD(k + 1) = cs * DD(k + 1);
-      for (int q = 0; q < c; ++q) {
-        const double vk = VV(q, k), vk1 = VV(q, k + 1);
-        VV(q, k) = cs * vk + sn * vk1;
-        VV(q, k + 1) = -sn * vk + cs * vk1;
-      }
-      y = DD(k);
-      z = bl;
-      t = hypot(y, z);
-      cs = t == 0.0 ? 1.0 : y / t;
-      sn = t == 0.0 ? 0.0 : z / t;
-      DD(k) = t;
-      {
-        const double ek = EE(k), dk1 = DD(k + 1);
-        EE(k) = cs * ek + sn * dk1;
-        DD(k + 1) = -sn * ek + cs * dk1;
-      }
-      if (k + 1 < hi) { bulge = sn * EE(k + 1); EE(k + 1) = cs * EE(k + 1); }
-      for (int q = 0; q < r; ++q) {
-        const double uk = UU(q, k), uk1 = UU(q, k + 1);
-        UU(q, k) = cs * uk + sn * uk1;
-        UU(q, k + 1) = -sn * uk + cs * uk1;
-      }
-      if (k < hi - 1) { y = EE(k); z = bulge; }
     }
   }
+  // ascending by |D| (a negative one turns its column of V): ranks, each lane
+  // those of its own columns
+  __syncwarp();
+  unsigned neg = 0;
   for (int i = 0; i < r; ++i)
-    if (DD(i) < 0.0) {
-      DD(i) = -DD(i);
-      for (int q = 0; q < c; ++q) VV(q, i) = -VV(q, i);
+    if (D[i * 32] < 0.0) {
+      neg |= 1u << i;
+      D[i * 32] = -D[i * 32];
     }
-  for (int i = 0; i + 1 < r; ++i) {  // ascending, moving the columns along
-    int k = i;
-    double pmin = DD(i);
-    for (int j = i + 1; j < r; ++j)
-      if (DD(j) < pmin) { k = j; pmin = DD(j); }
-    if (k != i) {
-      DD(k) = DD(i);
-      DD(i) = pmin;
-      for (int q = 0; q < r; ++q) { const double t = UU(q, i); UU(q, i) = UU(q, k); UU(q, k) = t; }
-      for (int q = 0; q < c; ++q) { const double t = VV(q, i); VV(q, i) = VV(q, k); VV(q, k) = t; }
-    }
+  if (leaf_ranks<G>(r, D, rk, g0)) leaf_ranks_ties(r, D, rk);
+  __syncwarp();
+  for (int i = g0; i < r; i += G) {
+    Dp[a + rk[i * 64]] = D[i * 32];
+    perm[a + i] = a + i;
   }
-  for (int j = 0; j < r; ++j) {
-    for (int q = 0; q < r; ++q) U[(long long)(a + j) * ldu + a + q] = UU(q, j);
-    Dp[a + j] = DD(j);
-    perm[a + j] = a + j;
-  }
-  for (int j = 0; j < c; ++j)
-    for (int q = 0; q < c; ++q) V[(long long)(a + j) * ldv + a + q] = VV(q, j);
   if (bad) atomicMax(status, HSS_LEAF_NOCONV);
-#undef DD
-#undef EE
-#undef UU
-#undef VV
+  // write the blocks: lanes over the entries, one leaf at a time (coalesced)
+  const double *Uw = lsm + (size_t)rmax * 64, *Vw = Uw + (size_t)rmax * R * 32;
+  const int *rw = (const int *)(lsm + (size_t)rmax * 32);
+  for (int l = 0; l < LPW; ++l) {
+    const int a2 = __shfl_sync(HSS_FULL, a, l * G), r2 = __shfl_sync(HSS_FULL, r, l * G),
+              c2 = __shfl_sync(HSS_FULL, c, l * G);
+    const unsigned n2 = __shfl_sync(HSS_FULL, neg, l * G);
+    for (int x = lane; x < r2 * r2; x += 32) {
+      const int j = x / r2, i = x - j * r2;
+      U[(long long)(a2 + rw[j * 64 + 2 * l * G]) * ldu + a2 + i] =
+          Uw[(j * R + i / G) * 32 + l * G + i % G];
+    }
+    for (int x = lane; x < c2 * c2; x += 32) {
+      const int j = x / c2, i = x - j * c2;
+      const int to = j < r2 ? rw[j * 64 + 2 * l * G] : j;
+      const double v = Vw[(j * R + i / G) * 32 + l * G + i % G];
+      V[(long long)(a2 + to) * ldv + a2 + i] = j < r2 && (n2 >> j & 1u) ? -v : v;
+    }
+  }
 }
 
 // ------------------------------------------------------------ deflation ---
@@ -442,23 +560,44 @@ void launch_rows_rotate_back(int n, int ncols, const double *cs, const double *s
   if (n > 1 && ncols > 0) k_rows_rotate_back<<<(ncols + 127) / 128, 128, 0, st>>>(n, ncols, cs, sn, A, lda);
 }
 
+template <int G, int R>
+static void svd_leaf_launch(int nleaf, const int *lstart, const int *lsize, const int *lsqre,
+                            int rmax, const double *d, const double *e, double *U, long long ldu,
+                            double *V, long long ldv, double *Dp, int *perm, int *status,
+                            cudaStream_t st) {
+  const size_t smem = svd_leaf_smem(rmax, R);
+  static size_t attr = 48 * 1024;
+  if (smem > attr) {
+    cudaFuncSetAttribute(k_svd_leaf<G, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    attr = smem;
+  }
+  k_svd_leaf<G, R><<<(nleaf * G + 31) / 32, 32, smem, st>>>(nleaf, lstart, lsize, lsqre, rmax, d, e,
+                                                            U, ldu, V, ldv, Dp, perm, status);
+}
+
 void launch_svd_leaf(int nleaf, const int *lstart, const int *lsize, const int *lsqre, int rmax,
                      const double *d, const double *e, double *U, long long ldu, double *V,
                      long long ldv, double *Dp, int *perm, int *status, cudaStream_t st) {
   if (nleaf <= 0) return;
   rmax = std::max(1, std::min(rmax, SVD_LEAF_MAX));
-  const size_t per = (size_t)(2 * rmax + rmax * rmax + (rmax + 1) * (rmax + 1)) * sizeof(double);
-  int lw = 32;
-  while (lw > 8 && (nleaf + lw - 1) / lw < 2 * 148) lw /= 2;
-  while (lw > 1 && per * lw > 200 * 1024) lw /= 2;
-  const size_t smem = per * lw;
-  static size_t attr = 0;
-  if (smem > 48 * 1024 && smem > attr) {
-    cudaFuncSetAttribute(k_svd_leaf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    attr = smem;
-  }
-  k_svd_leaf<<<(nleaf + lw - 1) / lw, lw, smem, st>>>(nleaf, lstart, lsize, lsqre, rmax, d, e, U,
-                                                       ldu, V, ldv, Dp, perm, status);
+  // two blocks of vectors (shared memory): at most 8 rows of each per lane
+  int G = leaf_lanes(nleaf, rmax + 1);
+  while (G < 32 && (G < 2 || (rmax + G) / G > 8)) G *= 2;
+  const int R = (rmax + G) / G;  // ceil((rmax + 1) / G)
+#define SVDL_ARGS nleaf, lstart, lsize, lsqre, rmax, d, e, U, ldu, V, ldv, Dp, perm, status, st
+#define SVDL_TRY(g, r) if (G == g && R <= r) return svd_leaf_launch<g, r>(SVDL_ARGS)
+  SVDL_TRY(2, 4);
+  SVDL_TRY(2, 8);
+  SVDL_TRY(4, 4);
+  SVDL_TRY(4, 8);
+  SVDL_TRY(8, 2);
+  SVDL_TRY(8, 5);
+  SVDL_TRY(16, 1);
+  SVDL_TRY(16, 3);
+  SVDL_TRY(32, 1);
+  svd_leaf_launch<32, 2>(SVDL_ARGS);  // rmax + 1 <= 33 rows
+#undef SVDL_TRY
+#undef SVDL_ARGS
 }
 
 static int svd_threads(int maxn) {
