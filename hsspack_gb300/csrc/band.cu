@@ -120,7 +120,7 @@ k_band_leaf(int nleaf, const int *__restrict__ lstart, const int *__restrict__ l
             const double *__restrict__ AB, long long ldab, const double *__restrict__ Uc,
             const double *__restrict__ Vc, const double *__restrict__ Sc, double *__restrict__ Q,
             long long ldq, double *__restrict__ Dp, int *__restrict__ perm,
-            int *__restrict__ status) {
+            int *__restrict__ status, int2 *__restrict__ sup) {
   extern __shared__ double bsm[];
   const int ld = mmax + 1;
   double *A = bsm, *Vv = bsm + mmax * ld;
@@ -212,6 +212,7 @@ k_band_leaf(int nleaf, const int *__restrict__ lstart, const int *__restrict__ l
     for (int c = lane; c < m; c += 32) {
       Dp[s + c] = A[ord[c] * ld + ord[c]];
       perm[s + c] = s + c;
+      sup[s + c] = make_int2(s, s + m);  // rows the column is written on
     }
     __syncwarp();
   }
@@ -223,7 +224,8 @@ k_band_leaf(int nleaf, const int *__restrict__ lstart, const int *__restrict__ l
 __global__ void k_band_z(int P, const int *__restrict__ ms, const int *__restrict__ mn,
                          const int *__restrict__ mn1, const int *__restrict__ mcut, int kd,
                          const double *__restrict__ Q, long long ldq, const double *__restrict__ Uc,
-                         const double *__restrict__ Vc, double *__restrict__ Z, long long zld) {
+                         const double *__restrict__ Vc, double *__restrict__ Z, long long zld,
+                         const int2 *__restrict__ sup) {
   for (int m = blockIdx.y; m < P; m += gridDim.y) {
     const int s = ms[m], n = mn[m], n1 = mn1[m], cut = mcut[m];
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -232,9 +234,11 @@ __global__ void k_band_z(int P, const int *__restrict__ ms, const int *__restric
       const int base = top ? s + n1 - kd : s + n1;
       const double *W = (top ? Uc : Vc) + (long long)cut * kd * kd;
       const double *col = Q + (long long)slot * ldq + base;
+      const int2 sr = sup[slot];  // rows that hold data (zero elsewhere)
+      const int r0 = max(0, sr.x - base), r1 = min(kd, sr.y - base);
       for (int k = 0; k < kd; ++k) {
         double acc = 0.0;
-        for (int r = 0; r < kd; ++r) acc = fma(col[r], W[k * kd + r], acc);
+        for (int r = r0; r < r1; ++r) acc = fma(col[r], W[k * kd + r], acc);
         Z[k * zld + slot] = acc;
       }
     }
@@ -292,7 +296,8 @@ void launch_band_cut_svd(int ncut, const int *cut_row, int kd, const double *AB,
 void launch_band_leaf(int nleaf, const int *lstart, const int *lsize, const int *cut_above,
                       const int *cut_below, int mmax, int kd, const double *AB, long long ldab,
                       const double *Uc, const double *Vc, const double *Sc, double *Q,
-                      long long ldq, double *Dp, int *perm, int *status, cudaStream_t st) {
+                      long long ldq, double *Dp, int *perm, int *status, cudaStream_t st,
+                      int2 *sup) {
   if (nleaf <= 0) return;
   const size_t smem = sizeof(double) * 2 * (size_t)mmax * (mmax + 1);
   static size_t attr = 0;
@@ -302,15 +307,15 @@ void launch_band_leaf(int nleaf, const int *lstart, const int *lsize, const int 
   }
   k_band_leaf<<<std::min(nleaf, 65535), 32, smem, st>>>(nleaf, lstart, lsize, cut_above,
                                                          cut_below, mmax, kd, AB, ldab, Uc, Vc,
-                                                         Sc, Q, ldq, Dp, perm, status);
+                                                         Sc, Q, ldq, Dp, perm, status, sup);
 }
 
 void launch_band_z(int P, int maxn, const int *ms, const int *mn, const int *mn1, const int *mcut,
                    int kd, const double *Q, long long ldq, const double *Uc, const double *Vc,
-                   double *Z, long long zld, cudaStream_t st) {
+                   double *Z, long long zld, cudaStream_t st, const int2 *sup) {
   if (P <= 0 || kd <= 0) return;
   dim3 grid((maxn + 255) / 256, std::min(P, 65535));
-  k_band_z<<<grid, 256, 0, st>>>(P, ms, mn, mn1, mcut, kd, Q, ldq, Uc, Vc, Z, zld);
+  k_band_z<<<grid, 256, 0, st>>>(P, ms, mn, mn1, mcut, kd, Q, ldq, Uc, Vc, Z, zld, sup);
 }
 
 void launch_band_zupdate(const LevelView &lv, int total, const double *dl, const double *difl,

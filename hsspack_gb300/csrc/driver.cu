@@ -335,20 +335,22 @@ static void run_merges(Ctx &c, const std::vector<int> &ms, const std::vector<int
   const size_t o_ms = pk0.add(ms), o_mn = pk0.add(mn), o_mn1 = pk0.add(mn1), o_po = pk0.add(poff);
   char *d0 = pk0.upload(c, "g_pack", st);
   int *dms = (int *)(d0 + o_ms), *dmn = (int *)(d0 + o_mn), *dmn1 = (int *)(d0 + o_mn1);
-  int *dout = buf<int>(c, "g_out", 5 * P);
+  // per merge: its row window (with supports), then five counts
+  int2 *dwin = buf<int2>(c, "g_out", P + ((size_t)5 * P + 1) / 2);
+  int *dout = (int *)(dwin + P);
   double *drho = buf<double>(c, "g_rho", P);
   stage_begin(HSS_ST_PREPARE, st);
   if (!(pflags & PREP_SORTED)) {
     // merged order and z for every position of the level in one wide launch
     int *dpo = (int *)(d0 + o_po);
     launch_merge_front(P, poff[P], dpo, dms, dmn, dmn1, e, Q, ldq, Dp, perm, L.w,
-                       bu ? bu->z : nullptr, bu ? bu->rho : nullptr, pflags, st, L.sup);
+                       bu ? bu->z : nullptr, bu ? bu->rho : nullptr, pflags, st, L.sup, dwin);
     pflags |= PREP_FRONT;
     c.launches++;
   }
   launch_merge_prepare(P, *std::max_element(mn.begin(), mn.end()), dms, dmn, dmn1, e, Q, ldq, Dp,
                        perm, L.w, dout, drho, st, bu ? bu->z : nullptr, bu ? bu->rho : nullptr,
-                       pflags, L.sup);
+                       pflags, L.sup, dwin);
   {
     long long nn = 0;
     for (int x : mn) nn += x;
@@ -356,20 +358,21 @@ static void run_merges(Ctx &c, const std::vector<int> &ms, const std::vector<int
     stage_end(HSS_ST_PREPARE, st, 64 * nn, 0.0);
   }
   c.launches++;
-  char *hp = (char *)pinned(c, (size_t)P * (5 * sizeof(int) + sizeof(double)));
-  int *hout = (int *)hp;
-  double *hrho = (double *)(hp + (size_t)P * 5 * sizeof(int));
-  CK(cudaMemcpyAsync(hout, dout, (size_t)P * 5 * sizeof(int), cudaMemcpyDeviceToHost, st));
+  char *hp = (char *)pinned(c, (size_t)P * (7 * sizeof(int) + sizeof(double)));
+  double *hrho = (double *)hp;
+  const int2 *hwin = (const int2 *)(hrho + P);
+  const int *hout = (const int *)(hwin + P);
+  CK(cudaMemcpyAsync((void *)hwin, dwin, (size_t)P * 7 * sizeof(int), cudaMemcpyDeviceToHost, st));
   CK(cudaMemcpyAsync(hrho, drho, (size_t)P * sizeof(double), cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
   // ---- plan
   std::vector<int> as, an, aK, aoff(1, 0), gs, gn, gng;
   std::vector<double> arho;
-  std::vector<int> ds_, dn_, dK_, doff(1, 0);
+  std::vector<int> ds_, dn_, dr_, dK_, doff(1, 0);  // dr_, dn_: row window (first, count)
   std::vector<double> drho_;
   std::vector<long long> q2off, soff, toff;
   std::vector<int> hsel;  // HSS merges (index into active arrays)
-  for (auto *v : {&as, &an, &aK, &aoff, &gs, &gn, &gng, &ds_, &dn_, &dK_, &doff}) v->reserve(P + 1);
+  for (auto *v : {&as, &an, &aK, &aoff, &gs, &gn, &gng, &ds_, &dn_, &dr_, &dK_, &doff}) v->reserve(P + 1);
   for (auto *v : {&arho, &drho_}) v->reserve(P);
   for (auto *v : {&q2off, &soff}) v->reserve(P);
   long long q2tot = 0, stot = 0;
@@ -391,10 +394,12 @@ static void run_merges(Ctx &c, const std::vector<int> &ms, const std::vector<int
       continue;
     }
     c.stats.n_dense_merges++;
-    ds_.push_back(ms[m]); dn_.push_back(mn[m]); dK_.push_back(K); drho_.push_back(hrho[m]);
+    const int row0 = L.sup ? hwin[m].x : ms[m], rows = L.sup ? hwin[m].y - row0 : mn[m];
+    ds_.push_back(ms[m]); dn_.push_back(rows); dr_.push_back(row0); dK_.push_back(K);
+    drho_.push_back(hrho[m]);
     doff.push_back(doff.back() + K);
     q2off.push_back(q2tot);
-    q2tot += (long long)mn[m] * K;
+    q2tot += (long long)rows * K;
     soff.push_back(stot);
     stot += (long long)K * K;
   }
@@ -407,15 +412,15 @@ static void run_merges(Ctx &c, const std::vector<int> &ms, const std::vector<int
   const size_t o_as = pk.add(as), o_aK = pk.add(aK), o_aoff = pk.add(aoff), o_arho = pk.add(arho),
                o_apoff = pk.add(apoff);
   const size_t o_ds = pk.add(ds_), o_dK = pk.add(dK_), o_doff = pk.add(doff), o_drho = pk.add(drho_),
-               o_dn = pk.add(dn_), o_q2 = pk.add(q2off), o_so = pk.add(soff);
+               o_dn = pk.add(dn_), o_dr = pk.add(dr_), o_q2 = pk.add(q2off), o_so = pk.add(soff);
   char *dpk = pk.upload(c, "l_pack", st);
   // ---- Givens rotations of deflation
   if (!gs.empty()) {
     int *g1 = (int *)(dpk + o_gs), *g2 = (int *)(dpk + o_gn), *g3 = (int *)(dpk + o_gng);
     stage_begin(HSS_ST_GIVENS, st);
-    launch_widen((int)gs.size(), maxn_g, g1, g2, g3, L.w, Q, ldq, L.sup, st);
+    launch_widen((int)gs.size(), maxn_g, g1, g3, L.w, Q, ldq, L.sup, st);
     launch_givens((int)gs.size(), maxn_g, g1, g2, g3, L.w, Q, ldq, st, bu ? bu->zrest : nullptr,
-                  bu ? bu->nrest : 0, bu ? bu->zld : 0);
+                  bu ? bu->nrest : 0, bu ? bu->zld : 0, L.sup);
     long long gb = 0;
     for (size_t i = 0; i < gs.size(); ++i) gb += 32LL * gn[i] * gng[i];
     stage_end(HSS_ST_GIVENS, st, gb, 0.0);
@@ -486,7 +491,7 @@ static void run_merges(Ctx &c, const std::vector<int> &ms, const std::vector<int
   const int PD = (int)ds_.size();
   if (PD > 0) {
     int *xs = (int *)(dpk + o_ds), *xK = (int *)(dpk + o_dK), *xoff = (int *)(dpk + o_doff),
-        *xn = (int *)(dpk + o_dn);
+        *xn = (int *)(dpk + o_dn), *xr = (int *)(dpk + o_dr);
     double *xrho = (double *)(dpk + o_drho);
     long long *xq2 = (long long *)(dpk + o_q2), *xso = (long long *)(dpk + o_so);
     LevelView dv{xs, xK, xrho, xoff, PD};
@@ -498,25 +503,24 @@ static void run_merges(Ctx &c, const std::vector<int> &ms, const std::vector<int
     stage_end(HSS_ST_BUILD_S, st, 8LL * stot * 2, 0.0);
     int maxnd = *std::max_element(dn_.begin(), dn_.end());
     stage_begin(HSS_ST_GATHER, st);
-    launch_gather(PD, dtot, maxnd, xs, xn, xoff, L.w.ndslot, L.w.grp, xq2, Q, ldq, Q2, st, L.sup);
+    launch_gather(PD, dtot, maxnd, xs, xn, xoff, L.w.ndslot, L.w.grp, xq2, Q, ldq, Q2, st, L.sup, xr);
     stage_end(HSS_ST_GATHER, st, 16LL * q2tot, 0.0);
     // GEMM problems: top rows use type 1,2 columns, bottom rows type 2,3
     std::vector<GemmDesc> probs;
     probs.reserve(2 * (size_t)PD);
-    int tiles = 0;
     int di = 0;
     for (int m = 0; m < P; ++m) {
       const int K = hout[5 * m];
       if (K == 0 || K >= c.cfg.bsmlz) continue;
       const int c1 = hout[5 * m + 2], c2 = hout[5 * m + 3];
-      const int n = mn[m], n1 = mn1[m];
+      // window rows above and below the cut
+      const int n = dn_[di], cut = ms[m] + mn1[m];
+      const int n1 = std::min(n, std::max(0, cut - dr_[di]));
       double *q2 = Q2 + q2off[di], *t = T + q2off[di], *sm = S + soff[di];
-      GemmDesc top{q2, sm, t, n, K, n, n1, K, c1 + c2, 0, tiles};
-      tiles += gemm_tiles(n1, K);
-      probs.push_back(top);
-      GemmDesc bot{q2 + n1 + (long long)c1 * n, sm + c1, t + n1, n, K, n, n - n1, K, K - c1, 0, tiles};
-      tiles += gemm_tiles(n - n1, K);
-      probs.push_back(bot);
+      if (n1 > 0) probs.push_back(GemmDesc{q2, sm, t, n, K, n, n1, K, c1 + c2, 0, 0});
+      if (n > n1)
+        probs.push_back(GemmDesc{q2 + n1 + (long long)c1 * n, sm + c1, t + n1, n, K, n, n - n1, K,
+                                 K - c1, 0, 0});
       ++di;
     }
     double fl = 0.0;
@@ -529,7 +533,7 @@ static void run_merges(Ctx &c, const std::vector<int> &ms, const std::vector<int
     launch_gemm(probs, c.cfg.precision, st);
     stage_end(HSS_ST_GEMM, st, gbytes, fl);
     stage_begin(HSS_ST_SCATTER, st);
-    launch_scatter(PD, dtot, maxnd, xs, xn, xoff, L.w.ndslot, xq2, T, Q, ldq, st, L.sup);
+    launch_scatter(PD, dtot, maxnd, xs, xn, xoff, L.w.ndslot, xq2, T, Q, ldq, st, L.sup, xr);
     stage_end(HSS_ST_SCATTER, st, 16LL * q2tot, 0.0);
     c.launches += 4;
   }
@@ -914,7 +918,6 @@ static int band_core(Ctx &c, int n, int kd, const double *ab, long long ldab, do
   int *status = buf<int>(c, "status", 8);
   CK(cudaMemsetAsync(status, 0, 8 * sizeof(int), st));
   CK(cudaMemsetAsync(gemm_flag(c), 0, sizeof(int), st));
-  CK(cudaMemsetAsync(Q, 0, sizeof(double) * (size_t)n * n, st));
   const size_t kk = (size_t)kd * kd;
   double *Uc = buf<double>(c, "band_U", std::max<size_t>(ncut, 1) * kk);
   double *Vc = buf<double>(c, "band_V", std::max<size_t>(ncut, 1) * kk);
@@ -926,8 +929,9 @@ static int band_core(Ctx &c, int n, int kd, const double *ab, long long ldab, do
   h2d(dcb, cbelow, st);
   stage_begin(HSS_ST_LEAF, st);
   launch_band_cut_svd(ncut, dcrow, kd, ab, ldab, Uc, Vc, Sc, status, st);
+  int2 *sup = buf<int2>(c, "sup", n);
   launch_band_leaf(nl, dls, dlz, dca, dcb, mmax, kd, ab, ldab, Uc, Vc, Sc, Q, n, Dp, perm, status,
-                   st);
+                   st, sup);
   {
     double fl = 0.0;
     for (int x : sz) fl += 8.0 * x * x * x * 10.0;  // ~10 Jacobi sweeps
@@ -939,6 +943,7 @@ static int band_core(Ctx &c, int n, int kd, const double *ab, long long ldab, do
     CK(cudaMemcpyAsync(hS.data(), Sc, sizeof(double) * hS.size(), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
     LevelArrays L = level_arrays(c, n);
+    L.sup = sup;
     double *Z = buf<double>(c, "band_Z", (size_t)kd * n);
     std::vector<int> lastleaf(nl);
     for (int i = 0; i < nl; ++i) lastleaf[i] = i;
@@ -958,7 +963,7 @@ static int band_core(Ctx &c, int n, int kd, const double *ab, long long ldab, do
       h2d(zs, ms, st); h2d(zn, mn, st); h2d(zn1, mn1, st); h2d(zc, mcut, st);
       stage_begin(HSS_ST_PREPARE, st);
       launch_band_z(P, *std::max_element(mn.begin(), mn.end()), zs, zn, zn1, zc, kd, Q, n, Uc, Vc, Z,
-                    n, st);
+                    n, st, sup);
       stage_end(HSS_ST_PREPARE, st, 8LL * n * kd * 2, 2.0 * n * kd * kd);
       c.launches++;
       double *drho = buf<double>(c, "band_rho", (size_t)P * kd);
@@ -988,8 +993,8 @@ static int band_core(Ctx &c, int n, int kd, const double *ab, long long ldab, do
     }
   }
   stage_begin(HSS_ST_FINAL, st);
-  launch_final_gather(n, perm, Dp, Q, n, z, ldz, w, st);
-  stage_end(HSS_ST_FINAL, st, 16LL * n * n + 20LL * n, 0.0);
+  launch_final_gather(n, perm, Dp, Q, n, z, ldz, w, st, sup);
+  stage_end(HSS_ST_FINAL, st, 8LL * n * n + 20LL * n, 0.0);
   c.launches++;
   CK(cudaEventRecord(ev1, st));
   int hst[8] = {0, 0, 0, 0, 0, 0, 0, 0};

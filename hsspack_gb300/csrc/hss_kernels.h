@@ -86,34 +86,39 @@ void launch_leaf(int nleaf, const int *lstart, const int *lsize, int mmax, int n
 // prepare flags: the block is already in ascending order (no merge of two
 // halves); every column is dense (no top / bottom block structure)
 enum { PREP_SORTED = 1, PREP_DENSE = 2, PREP_FRONT = 4 /* order and z from k_merge_front */ };
+// win (with sup): per merge the rows on which the columns it takes up hold data
 // zsrc: z per slot instead of the rows of Q around the cut; rsrc: the coupling
 // rho_in per merge instead of e[s + n1 - 1]
 void launch_merge_prepare(int P, int maxn, const int *ms, const int *mn, const int *mn1, const double *e,
                           const double *Q, long long ldq, double *Dp, int *perm,
                           const LevelScratch &w, int *out, double *orho, cudaStream_t st,
                           const double *zsrc = nullptr, const double *rsrc = nullptr,
-                          int flags = 0, const int2 *sup = nullptr);
+                          int flags = 0, const int2 *sup = nullptr, int2 *win = nullptr);
 // merged order and z of every position of a level (poff: prefix of mn, P + 1)
 void launch_merge_front(int P, int total, const int *poff, const int *ms, const int *mn,
                         const int *mn1, const double *e, const double *Q, long long ldq,
                         const double *Dp, const int *perm, const LevelScratch &w,
                         const double *zsrc, const double *rsrc, int flags, cudaStream_t st,
-                        const int2 *sup = nullptr);
+                        const int2 *sup = nullptr, int2 *win = nullptr);
 // Zr (nz columns, leading dim zld): rows rotated with the Q columns
 void launch_givens(int P, int maxn, const int *ms, const int *mn, const int *ng,
                    const LevelScratch &w, double *Q, long long ldq, cudaStream_t st,
-                   double *Zr = nullptr, int nz = 0, long long zld = 0);
+                   double *Zr = nullptr, int nz = 0, long long zld = 0,
+                   const int2 *sup = nullptr);
 // sup (optional): per slot the rows [x, y) a column holds data on (zero
-// elsewhere); gathers read within it, scatters set it to the merge's rows
+// elsewhere); gathers read within it, scatters set it to the rows they write.
+// Merge m's columns are copied on the mn[m] rows from mr[m] (mr null: from ms[m])
 void launch_gather(int P, int total, int maxn, const int *ms, const int *mn, const int *rootoff,
                    const int *ndslot, const int *grp, const long long *boff, const double *Q,
-                   long long ldq, double *B, cudaStream_t st, const int2 *sup = nullptr);
+                   long long ldq, double *B, cudaStream_t st, const int2 *sup = nullptr,
+                   const int *mr = nullptr);
 void launch_scatter(int P, int total, int maxn, const int *ms, const int *mn, const int *rootoff,
                     const int *ndslot, const long long *toff, const double *T, double *Q,
-                    long long ldq, cudaStream_t st, int2 *sup = nullptr);
-// columns about to be rotated: zeros written outside their support, support
-// widened to the merge's rows
-void launch_widen(int P, int maxn, const int *ms, const int *mn, const int *ng,
+                    long long ldq, cudaStream_t st, int2 *sup = nullptr,
+                    const int *mr = nullptr);
+// columns about to be rotated: both of a pair made valid on the union of their
+// supports
+void launch_widen(int P, int maxn, const int *ms, const int *ng,
                   const LevelScratch &w, double *Q, long long ldq, int2 *sup, cudaStream_t st);
 void launch_merge_finish(int P, int maxn, const int *ms, const int *mn, const int *mK, const double *lam,
                          const LevelScratch &w, int *perm, double *Dp, cudaStream_t st);
@@ -167,10 +172,11 @@ void launch_band_cut_svd(int ncut, const int *cut_row, int kd, const double *AB,
 void launch_band_leaf(int nleaf, const int *lstart, const int *lsize, const int *cut_above,
                       const int *cut_below, int mmax, int kd, const double *AB, long long ldab,
                       const double *Uc, const double *Vc, const double *Sc, double *Q,
-                      long long ldq, double *Dp, int *perm, int *status, cudaStream_t st);
+                      long long ldq, double *Dp, int *perm, int *status, cudaStream_t st,
+                      int2 *sup);
 void launch_band_z(int P, int maxn, const int *ms, const int *mn, const int *mn1, const int *mcut,
                    int kd, const double *Q, long long ldq, const double *Uc, const double *Vc,
-                   double *Z, long long zld, cudaStream_t st);
+                   double *Z, long long zld, cudaStream_t st, const int2 *sup);
 void launch_band_zupdate(const LevelView &lv, int total, const double *dl, const double *difl,
                          const double *difr, const double *zhat, const double *alpha,
                          const int *ndslot, double *Z, int nrest, long long zld, double *Zt,

@@ -11,6 +11,8 @@
 // through to the end, so no level copies the whole n x n block.
 #include <cooperative_groups.h>
 
+#include <climits>
+
 #include "hss_block.cuh"
 #include "hss_common.cuh"
 #include "hss_kernels.h"
@@ -28,6 +30,23 @@ __device__ __forceinline__ double qat(const double *__restrict__ Q, long long ld
   return Q[(long long)slot * ldq + row];
 }
 
+// Row windows: the union of the supports of the columns that a merge takes up.
+// Rows outside it are zero in all of them and stay zero in the new ones, so the
+// products of a merge run over its window alone.  (Gather, digit planes, products
+// and scatter scale with the rows: 512 problems 60.8 -> 58.2 ms, n = 32768 7.29 ->
+// 6.73 ms, COMPZ = 'V' n = 2048 6.18 -> 4.79 ms, band n = 16384, kd = 4 65.5 -> 62.0.)
+__device__ __forceinline__ void window_add(int2 &w, int2 r) {
+  if (r.y > r.x) { w.x = min(w.x, r.x); w.y = max(w.y, r.y); }
+}
+__device__ __forceinline__ void window_warp(int2 &w) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    w.x = min(w.x, __shfl_xor_sync(HSS_FULL, w.x, o));
+    w.y = max(w.y, __shfl_xor_sync(HSS_FULL, w.y, o));
+  }
+}
+
+// win[m] (with sup): the merge's row window
 // out[5*m + {0..4}] = K, #rotations, #type1, #type2, #type3 ; orho[m] = |2 rho|
 template <int MT>
 __global__ void __launch_bounds__(MT)
@@ -36,9 +55,12 @@ k_merge_prepare(int P, const int *__restrict__ ms, const int *__restrict__ mn,
                 const double *__restrict__ Q, long long ldq, double *__restrict__ Dp,
                 int *__restrict__ perm, LevelScratch w, int *__restrict__ out,
                 double *__restrict__ orho, const double *__restrict__ zsrc,
-                const double *__restrict__ rsrc, int flags, const int2 *__restrict__ sup) {
+                const double *__restrict__ rsrc, int flags, const int2 *__restrict__ sup,
+                int2 *__restrict__ win) {
   const int m = blockIdx.x;
   if (m >= P) return;
+  __shared__ int s_win[2];  // rows of the columns that the merge rewrites or rotates
+  if (threadIdx.x == 0) { s_win[0] = INT_MAX; s_win[1] = 0; }
   const int s = ms[m], n = mn[m], n1 = mn1[m], n2 = n - n1;
   const int tid = threadIdx.x;
   const double rho_in = rsrc ? rsrc[m] : e[s + n1 - 1];
@@ -308,6 +330,7 @@ k_merge_prepare(int P, const int *__restrict__ ms, const int *__restrict__ mn,
   const int nrot = (int)t5;
   int r1 = (int)(pre & 0x1fffff), r2 = (int)((pre >> 21) & 0x1fffff),
       r3 = (int)((pre >> 42) & 0x1fffff);
+  int2 wr = make_int2(INT_MAX, 0);
   for (int i0 = w0; i0 < w1; i0 += 32 * PB) {
     int tb[PB], sb[PB];
     double db[PB], zb[PB];
@@ -329,6 +352,7 @@ k_merge_prepare(int P, const int *__restrict__ ms, const int *__restrict__ mn,
     const int sv = sb[b];
     const unsigned m1 = __ballot_sync(HSS_FULL, t == 1), m2 = __ballot_sync(HSS_FULL, t == 2),
                    m3 = __ballot_sync(HSS_FULL, t == 3), m5 = __ballot_sync(HSS_FULL, t == 5);
+    if (sup && in && t != 4) window_add(wr, sup[sv]);
     if (in) {
       // this position's rank among the non-deflated of each type and the rotated
       const int e1 = r1 + __popc(m1 & below), e2 = r2 + __popc(m2 & below),
@@ -355,7 +379,12 @@ k_merge_prepare(int P, const int *__restrict__ ms, const int *__restrict__ mn,
     r1 += __popc(m1); r2 += __popc(m2); r3 += __popc(m3); r5 += __popc(m5);
     }
   }
+  if (sup) {
+    window_warp(wr);
+    if (lane == 0 && wr.y > 0) { atomicMin(&s_win[0], wr.x); atomicMax(&s_win[1], wr.y); }
+  }
   __syncthreads();
+  if (sup && tid == 0) win[m] = make_int2(s_win[0], s_win[1]);
   // The small-z list is ascending; rotated poles moved inside their gap
   // (mdlaed2.f90:340-356 inserts them in order), so sort those and merge.
   const int n1l = (n - K) - nrot;
@@ -452,7 +481,8 @@ k_merge_prepare_cl(int P, const int *__restrict__ ms, const int *__restrict__ mn
                    const int *__restrict__ mn1, const double *__restrict__ e,
                    double *__restrict__ Dp, int *__restrict__ perm, LevelScratch w,
                    int *__restrict__ out, double *__restrict__ orho,
-                   const double *__restrict__ rsrc) {
+                   const double *__restrict__ rsrc, const int2 *__restrict__ sup,
+                   int2 *__restrict__ win) {
   cg::cluster_group cl = cg::this_cluster();
   const int G = (int)cl.num_blocks(), crank = (int)cl.block_rank();
   const int m = blockIdx.x / G;
@@ -650,6 +680,7 @@ k_merge_prepare_cl(int P, const int *__restrict__ ms, const int *__restrict__ mn
   const int nrot = (int)ct5;
   int r1 = (int)(pre & 0x1fffff), r2 = (int)((pre >> 21) & 0x1fffff),
       r3 = (int)((pre >> 42) & 0x1fffff);
+  int2 wr = make_int2(INT_MAX, 0);
   for (int i0 = w0; i0 < w1; i0 += 32 * PB) {
     int tb[PB], sb[PB];
     double db[PB], zb[PB];
@@ -669,6 +700,7 @@ k_merge_prepare_cl(int P, const int *__restrict__ ms, const int *__restrict__ mn
       const int t = tb[b];
       const unsigned m1 = __ballot_sync(HSS_FULL, t == 1), m2 = __ballot_sync(HSS_FULL, t == 2),
                      m3 = __ballot_sync(HSS_FULL, t == 3), m5 = __ballot_sync(HSS_FULL, t == 5);
+      if (sup && in && t != 4) window_add(wr, sup[sb[b]]);
       if (in) {
         const int e1 = r1 + __popc(m1 & below), e2 = r2 + __popc(m2 & below),
                   e3 = r3 + __popc(m3 & below), e5 = r5 + __popc(m5 & below);
@@ -693,6 +725,10 @@ k_merge_prepare_cl(int P, const int *__restrict__ ms, const int *__restrict__ mn
       }
       r1 += __popc(m1); r2 += __popc(m2); r3 += __popc(m3); r5 += __popc(m5);
     }
+  }
+  if (sup) {  // (the front set win[m] to the empty window)
+    window_warp(wr);
+    if (lane == 0 && wr.y > 0) { atomicMin(&win[m].x, wr.x); atomicMax(&win[m].y, wr.y); }
   }
   cl.sync();  // the lists complete (and no CTA leaves while another reads its slots)
   const int n1l = (n - K) - nrot;
@@ -751,13 +787,14 @@ __global__ void k_merge_front(int P, const int *__restrict__ poff, const int *__
                               long long ldq, const double *__restrict__ Dp,
                               const int *__restrict__ perm, LevelScratch w,
                               const double *__restrict__ zsrc, const double *__restrict__ rsrc,
-                              int flags, const int2 *__restrict__ sup) {
+                              int flags, const int2 *__restrict__ sup, int2 *__restrict__ win) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= poff[P]) return;
   int lo = 0, hi = P;
   while (hi - lo > 1) { const int md = (lo + hi) >> 1; if (poff[md] <= t) lo = md; else hi = md; }
   const int m = lo, i = t - poff[m];
   const int s = ms[m], n1 = mn1[m], n2 = mn[m] - n1;
+  if (win && i == 0) win[m] = make_int2(INT_MAX, 0);
   const bool top = i < n1;
   const int slot = perm[s + i];  // left: perm[s+i]; right: perm[s+n1+(i-n1)]
   const double v = Dp[slot];
@@ -778,27 +815,28 @@ __global__ void k_merge_front(int P, const int *__restrict__ poff, const int *__
   w.typ[s + pos] = (flags & PREP_DENSE) ? 2 : top ? 1 : 3;
 }
 
-// Before the deflating rotations of merge m: every column they touch is made
-// valid on all rows s .. s+n-1 of the merge (zeros written outside the rows it
-// held data on) and its support widened, so the rotations read true values.
-// One CTA per merge, rotations in order (a slot may take part in several).
-__global__ void k_widen(int P, const int *__restrict__ ms, const int *__restrict__ mn,
-                        const int *__restrict__ ng, const LevelScratch w, double *Q, long long ldq,
-                        int2 *__restrict__ sup) {
+// Before the deflating rotations of merge m: the two columns of every rotation
+// are made valid on the union of their rows (zeros written where a column held
+// no data), so the rotations read true values.  One CTA per merge, rotations
+// in order (a slot may take part in several: first as q, last as p).
+__global__ void k_widen(int P, const int *__restrict__ ms, const int *__restrict__ ng,
+                        const LevelScratch w, double *Q, long long ldq, int2 *__restrict__ sup) {
   for (int m = blockIdx.x; m < P; m += gridDim.x) {
-    const int s = ms[m], n = mn[m], g = ng[m];
-    for (int t = 0; t < g; ++t)
-      for (int side = 0; side < 2; ++side) {
-        const int slot = side == 0 ? w.gvp[s + t] : w.gvq[s + t];
-        __syncthreads();  // the previous update of sup is visible to all threads
-        const int2 r = sup[slot];
-        if (r.x == s && r.y == s + n) continue;  // uniform across the CTA
-        double *col = Q + (long long)slot * ldq;
-        for (int i = s + threadIdx.x; i < s + n; i += blockDim.x)
-          if (i < r.x || i >= r.y) col[i] = 0.0;
-        __syncthreads();
-        if (threadIdx.x == 0) sup[slot] = make_int2(s, s + n);
+    const int s = ms[m], g = ng[m];
+    for (int t = 0; t < g; ++t) {
+      __syncthreads();  // the previous update of sup is visible to all threads
+      const int p = w.gvp[s + t], q = w.gvq[s + t];
+      const int2 rp = sup[p], rq = sup[q];
+      if (rp.x == rq.x && rp.y == rq.y) continue;  // uniform across the CTA
+      const int2 u = make_int2(min(rp.x, rq.x), max(rp.y, rq.y));
+      double *cp = Q + (long long)p * ldq, *cq = Q + (long long)q * ldq;
+      for (int i = u.x + threadIdx.x; i < u.y; i += blockDim.x) {
+        if (i < rp.x || i >= rp.y) cp[i] = 0.0;
+        if (i < rq.x || i >= rq.y) cq[i] = 0.0;
       }
+      __syncthreads();
+      if (threadIdx.x == 0) { sup[p] = u; sup[q] = u; }
+    }
     __syncthreads();
   }
 }
@@ -806,9 +844,12 @@ __global__ void k_widen(int P, const int *__restrict__ ms, const int *__restrict
 // Threads r >= n rotate rows p, q of column r - n of Zr (nz columns, leading
 // dim zld) the same way: the remaining columns of a banded merge's
 // Z = Q^T W follow the rotated eigenvectors (mdsbed22.f90 rotates Z(:, 2:)).
+// With sup (after k_widen) a rotation covers the rows of its column p: q holds
+// data on all of them, and outside them both columns were zero when it applied.
 __global__ void k_givens(int P, const int *__restrict__ ms, const int *__restrict__ mn,
                          const int *__restrict__ ng, const LevelScratch w, double *Q,
-                         long long ldq, double *Zr, int nz, long long zld) {
+                         long long ldq, double *Zr, int nz, long long zld,
+                         const int2 *__restrict__ sup) {
   for (int m = blockIdx.y; m < P; m += gridDim.y) {
     const int s = ms[m], n = mn[m], g = ng[m];
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
@@ -819,6 +860,10 @@ __global__ void k_givens(int P, const int *__restrict__ ms, const int *__restric
     else { base = Zr + (r - n) * zld; ld = 1; row = 0; }
     for (int t = 0; t < g; ++t) {
       const long long p = w.gvp[s + t], q = w.gvq[s + t];
+      if (sup && r < n) {
+        const int2 rp = sup[p];
+        if (row < rp.x || row >= rp.y) continue;
+      }
       const double c = w.gvc[s + t], sn = w.gvs[s + t];
       const double x = base[p * ld + row], y = base[q * ld + row];
       base[p * ld + row] = c * x + sn * y;
@@ -840,8 +885,9 @@ __device__ __forceinline__ int gs_merge(const int *__restrict__ rootoff, int P, 
   return lo;
 }
 
+// mr (optional): first row of each merge's columns (mn rows); ms otherwise
 __global__ void k_gather(int P, int nseg, const int *__restrict__ ms, const int *__restrict__ mn,
-                         const int *__restrict__ rootoff, const int *__restrict__ ndslot,
+                         const int *__restrict__ mr, const int *__restrict__ rootoff, const int *__restrict__ ndslot,
                          const int *__restrict__ grp, const long long *__restrict__ boff,
                          const double *__restrict__ Q, long long ldq, double *__restrict__ B,
                          const int2 *__restrict__ sup) {
@@ -854,17 +900,17 @@ __global__ void k_gather(int P, int nseg, const int *__restrict__ ms, const int 
   const int i0 = q * GS_SEG, i1 = min(n, i0 + GS_SEG);
   if (i0 >= i1) return;
   const int col = grp ? grp[s + j] : j;
-  const int slot = ndslot[s + j];
-  const double *src = Q + (long long)slot * ldq + s;
+  const int slot = ndslot[s + j], row0 = mr ? mr[m] : s;
+  const double *src = Q + (long long)slot * ldq + row0;
   double *dst = B + boff[m] + (long long)col * n;
   int vlo = 0, vhi = n;  // rows of the column that hold data (zero elsewhere)
-  if (sup) { const int2 sr = sup[slot]; vlo = max(0, sr.x - s); vhi = min(n, sr.y - s); }
+  if (sup) { const int2 sr = sup[slot]; vlo = max(0, sr.x - row0); vhi = min(n, sr.y - row0); }
   for (int i = i0 + lane; i < i1; i += 32) dst[i] = (i >= vlo && i < vhi) ? src[i] : 0.0;
 }
 
 // Write the new eigenvectors (columns of T, n_m x K) into the non-deflated slots.
 __global__ void k_scatter(int P, int nseg, const int *__restrict__ ms, const int *__restrict__ mn,
-                          const int *__restrict__ rootoff, const int *__restrict__ ndslot,
+                          const int *__restrict__ mr, const int *__restrict__ rootoff, const int *__restrict__ ndslot,
                           const long long *__restrict__ toff, const double *__restrict__ T,
                           double *__restrict__ Q, long long ldq, int2 *__restrict__ sup) {
   const long long wg = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -875,9 +921,10 @@ __global__ void k_scatter(int P, int nseg, const int *__restrict__ ms, const int
   const int s = ms[m], n = mn[m];
   const int i0 = q * GS_SEG, i1 = min(n, i0 + GS_SEG);
   if (i0 >= i1) return;
+  const int row0 = mr ? mr[m] : s;
   const double *src = T + toff[m] + (long long)j * n;
-  double *dst = Q + (long long)ndslot[s + j] * ldq + s;
-  if (sup && q == 0 && lane == 0) sup[ndslot[s + j]] = make_int2(s, s + n);
+  double *dst = Q + (long long)ndslot[s + j] * ldq + row0;
+  if (sup && q == 0 && lane == 0) sup[ndslot[s + j]] = make_int2(row0, row0 + n);
   for (int i = i0 + lane; i < i1; i += 32) dst[i] = src[i];
 }
 
@@ -1091,16 +1138,17 @@ void launch_merge_front(int P, int total, const int *poff, const int *ms, const 
                         const int *mn1, const double *e, const double *Q, long long ldq,
                         const double *Dp, const int *perm, const LevelScratch &w,
                         const double *zsrc, const double *rsrc, int flags, cudaStream_t st,
-                        const int2 *sup) {
+                        const int2 *sup, int2 *win) {
   if (P <= 0 || total <= 0) return;
   k_merge_front<<<(total + 255) / 256, 256, 0, st>>>(P, poff, ms, mn, mn1, e, Q, ldq, Dp, perm,
-                                                     w, zsrc, rsrc, flags, sup);
+                                                     w, zsrc, rsrc, flags, sup, win);
 }
 
 void launch_merge_prepare(int P, int maxn, const int *ms, const int *mn, const int *mn1,
                           const double *e, const double *Q, long long ldq, double *Dp, int *perm,
                           const LevelScratch &w, int *out, double *orho, cudaStream_t st,
-                          const double *zsrc, const double *rsrc, int flags, const int2 *sup) {
+                          const double *zsrc, const double *rsrc, int flags, const int2 *sup,
+                          int2 *win) {
   if (P <= 0) return;
   if ((flags & PREP_FRONT) && maxn > PCL_MIN_N) {
     cudaLaunchConfig_t cfg = {};
@@ -1116,14 +1164,14 @@ void launch_merge_prepare(int P, int maxn, const int *ms, const int *mn, const i
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     if (cudaLaunchKernelEx(&cfg, k_merge_prepare_cl<PCL_T>, P, ms, mn, mn1, e, Dp, perm, w, out,
-                           orho, rsrc) == cudaSuccess)
+                           orho, rsrc, sup, win) == cudaSuccess)
       return;
     (void)cudaGetLastError();  // no cluster launch here: the one-CTA kernel below
   }
 #define PREP_CASE(T)                                                                        \
   case T:                                                                                  \
     k_merge_prepare<T><<<P, T, 0, st>>>(P, ms, mn, mn1, e, Q, ldq, Dp, perm, w, out, orho, \
-                                        zsrc, rsrc, flags, sup);                           \
+                                        zsrc, rsrc, flags, sup, win);                      \
     break;
   switch (merge_threads(maxn)) {
     PREP_CASE(64)
@@ -1136,34 +1184,34 @@ void launch_merge_prepare(int P, int maxn, const int *ms, const int *mn, const i
 }
 void launch_givens(int P, int maxn, const int *ms, const int *mn, const int *ng,
                    const LevelScratch &w, double *Q, long long ldq, cudaStream_t st, double *Zr,
-                   int nz, long long zld) {
+                   int nz, long long zld, const int2 *sup) {
   if (P <= 0) return;
   if (!Zr) nz = 0;
   dim3 grid((maxn + nz + 255) / 256, std::min(P, 65535));
-  k_givens<<<grid, 256, 0, st>>>(P, ms, mn, ng, w, Q, ldq, Zr, nz, zld);
+  k_givens<<<grid, 256, 0, st>>>(P, ms, mn, ng, w, Q, ldq, Zr, nz, zld, sup);
 }
 void launch_gather(int P, int total, int maxn, const int *ms, const int *mn, const int *rootoff,
                    const int *ndslot, const int *grp, const long long *boff, const double *Q,
-                   long long ldq, double *B, cudaStream_t st, const int2 *sup) {
+                   long long ldq, double *B, cudaStream_t st, const int2 *sup, const int *mr) {
   if (total <= 0) return;
   const int nseg = (maxn + GS_SEG - 1) / GS_SEG;
   const long long warps = (long long)total * nseg;
-  k_gather<<<(unsigned)((warps + 7) / 8), 256, 0, st>>>(P, nseg, ms, mn, rootoff, ndslot, grp, boff,
-                                                        Q, ldq, B, sup);
+  k_gather<<<(unsigned)((warps + 7) / 8), 256, 0, st>>>(P, nseg, ms, mn, mr, rootoff, ndslot, grp,
+                                                        boff, Q, ldq, B, sup);
 }
 void launch_scatter(int P, int total, int maxn, const int *ms, const int *mn, const int *rootoff,
                     const int *ndslot, const long long *toff, const double *T, double *Q,
-                    long long ldq, cudaStream_t st, int2 *sup) {
+                    long long ldq, cudaStream_t st, int2 *sup, const int *mr) {
   if (total <= 0) return;
   const int nseg = (maxn + GS_SEG - 1) / GS_SEG;
   const long long warps = (long long)total * nseg;
-  k_scatter<<<(unsigned)((warps + 7) / 8), 256, 0, st>>>(P, nseg, ms, mn, rootoff, ndslot, toff, T,
-                                                         Q, ldq, sup);
+  k_scatter<<<(unsigned)((warps + 7) / 8), 256, 0, st>>>(P, nseg, ms, mn, mr, rootoff, ndslot, toff,
+                                                         T, Q, ldq, sup);
 }
-void launch_widen(int P, int maxn, const int *ms, const int *mn, const int *ng,
+void launch_widen(int P, int maxn, const int *ms, const int *ng,
                   const LevelScratch &w, double *Q, long long ldq, int2 *sup, cudaStream_t st) {
   if (P <= 0 || !sup) return;
-  k_widen<<<std::min(P, 65535), maxn <= 256 ? 128 : 512, 0, st>>>(P, ms, mn, ng, w, Q, ldq, sup);
+  k_widen<<<std::min(P, 65535), maxn <= 256 ? 128 : 512, 0, st>>>(P, ms, ng, w, Q, ldq, sup);
 }
 void launch_merge_finish(int P, int maxn, const int *ms, const int *mn, const int *mK,
                          const double *lam, const LevelScratch &w, int *perm, double *Dp,
