@@ -35,6 +35,7 @@
 #include <cuda_bf16.h>
 #include <stdint.h>
 
+#include <algorithm>
 #include <vector>
 
 #include "hss_common.cuh"
@@ -78,21 +79,51 @@ __device__ __forceinline__ long long scaled_int(double x, int e) {
   return b < 0 ? -q : q;
 }
 
-// BF16 bit pattern of an integer |d| <= 128 (exact)
-__device__ __forceinline__ uint32_t bf16_of_int(int d) {
-  const uint32_t a = (uint32_t)(d < 0 ? -d : d);
-  const int e = 31 - __clz((int)(a | 1u));  // a in [2^e, 2^(e+1)), e <= 7
-  const uint32_t bits = (d < 0 ? 0x8000u : 0u) | ((uint32_t)(e + 127) << 7) | ((a << (7 - e)) & 0x7Fu);
-  return a ? bits : 0u;
+// The SP digits of q (|q| <= 2^60) as FP32 numbers: d_s = round(q_s / 2^{53 - 8s}), ties
+// up, q_{s+1} = q_s - d_s 2^{53 - 8s}, -128 <= d_s <= 128.  They are the bytes of q >> 5
+// read as signed numbers, each plus the top bit of the byte below it (the last:
+// of the five bits dropped), the first being all bits above the sixth byte.  A
+// byte with its top bit flipped is the signed value + 128; put into the low
+// mantissa bits of 2^23, plus that carry, minus 2^23 + 128, it is the digit.  A
+// digit has at most 8 significant bits: its BF16 pattern is the upper half of f.
+__device__ __forceinline__ void digits(long long q, float (&f)[SP]) {
+  const long long x = q >> 5;
+  const unsigned long long c = (((unsigned long long)x >> 7) & 0x010101010101ull) << 8 |
+                               ((unsigned long long)q >> 4 & 1ull);
+  const uint32_t clo = (uint32_t)c, chi = (uint32_t)(c >> 32);
+  const uint32_t xlo = (uint32_t)x ^ 0x80808080u, xhi = (uint32_t)(x >> 32) ^ 0x8080u;
+  const float b = 8388608.f + 128.f;
+  // above byte 5: a signed number of at most 128 (with its carry) in magnitude
+  const int top = ((int)xhi >> 16) + (int)__byte_perm(chi, 0u, 0x4442u);
+  f[0] = __uint_as_float(0x4B000000u + (uint32_t)(top + 128)) - b;
+#pragma unroll
+  for (int s = 1; s < SP; ++s) {
+    const uint32_t sel = (uint32_t)(s < 3 ? 2 - s : SP - 1 - s);  // byte of its word
+    const uint32_t v = __byte_perm(s < 3 ? xhi : xlo, 0x4B000000u, 0x7440u | sel) +
+                       __byte_perm(s < 3 ? chi : clo, 0u, 0x4440u | sel);
+    f[s] = __uint_as_float(v) - b;
+  }
 }
 
-// the value of an FP32 that holds an exact integer below 2^31 in magnitude
-__device__ __forceinline__ int int_of_float(float v) {
-  const int f = __float_as_int(v);
-  const int E = ((f >> 23) & 0xFF) - 127;
-  const int M = (f & 0x7FFFFF) | 0x800000;
-  const int a = E < 0 ? 0 : (E >= 23 ? M << (E - 23) : M >> (23 - E));
-  return f < 0 ? -a : a;
+// BF16 patterns of two such numbers, the first in the lower half
+__device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
+  return __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632u);
+}
+
+// the digits of 8 consecutive elements, per plane as a 16-byte core-matrix row
+template <class Load>
+__device__ __forceinline__ void digits8(int e, uint4 (&row)[SP], Load x) {
+  uint32_t pk[SP][4];
+#pragma unroll
+  for (int c = 0; c < 8; c += 2) {
+    float f0[SP], f1[SP];
+    digits(scaled_int(x(c), e), f0);
+    digits(scaled_int(x(c + 1), e), f1);
+#pragma unroll
+    for (int s = 0; s < SP; ++s) pk[s][c >> 1] = pack_bf16(f0[s], f1[s]);
+  }
+#pragma unroll
+  for (int s = 0; s < SP; ++s) row[s] = make_uint4(pk[s][0], pk[s][1], pk[s][2], pk[s][3]);
 }
 
 // (H + 2^-32 L) 2^e rounded to the nearest double (ties to even), from the
@@ -138,18 +169,6 @@ __device__ __forceinline__ double exact_double(long long H, long long L, int e) 
   const unsigned long long bits = (neg ? 0x8000000000000000ull : 0ull) |
                                   ((unsigned long long)be << 52) | (mant & 0xFFFFFFFFFFFFFull);
   return __longlong_as_double((long long)bits);
-}
-
-// the SP digits of q (|q| <= 2^60): d_s = round(q_s / 2^{53 - 8s}), |d_s| <= 128
-__device__ __forceinline__ void split_digits(double x, int e, __nv_bfloat16 *dig) {
-  long long q = scaled_int(x, e);
-#pragma unroll
-  for (int s = 0; s < SP; ++s) {
-    const int sh = 53 - 8 * s;
-    const long long d = (q + (1ll << (sh - 1))) >> sh;
-    q -= d * (1ll << sh);
-    dig[s] = __ushort_as_bfloat16((unsigned short)bf16_of_int((int)d));
-  }
 }
 
 // frexp exponent of the largest |x| from its bit pattern (0 for zero)
@@ -250,20 +269,14 @@ k_split_a(const SplitProb *__restrict__ probs, int nprob) {
     char *tile = (char *)P.dst + ((long long)tm * P.ktiles + kt) * SP * ATILE;
     const int r = u % TM, k8 = u / TM;
     const int gr = tm * TM + r;
-    __align__(16) __nv_bfloat16 dg[SP][8];
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
+    uint4 row[SP];
+    digits8(sexp[r], row, [&](int c) {
       const int gk = kt * TK + k8 * 8 + c;
-      const double x = (gr < P.rows && gk < P.inner) ? P.src[(long long)gk * P.ld + gr] : 0.0;
-      __nv_bfloat16 d[SP];
-      split_digits(x, sexp[r], d);
-#pragma unroll
-      for (int s = 0; s < SP; ++s) dg[s][c] = d[s];
-    }
+      return (gr < P.rows && gk < P.inner) ? P.src[(long long)gk * P.ld + gr] : 0.0;
+    });
 #pragma unroll
     for (int s = 0; s < SP; ++s)
-      *reinterpret_cast<uint4 *>(tile + s * ATILE + tile_off(r, k8 * 8, TM)) =
-          *reinterpret_cast<uint4 *>(dg[s]);
+      *reinterpret_cast<uint4 *>(tile + s * ATILE + tile_off(r, k8 * 8, TM)) = row[s];
   }
 }
 
@@ -340,20 +353,14 @@ k_split_b(const SplitProb *__restrict__ probs, int nprob) {
     char *tile = (char *)P.dst + ((long long)tn * P.ktiles + kt) * SP * BTILE;
     const int c = u / (TK / 8), k8 = u % (TK / 8);
     const int gc = tn * TN + c;
-    __align__(16) __nv_bfloat16 dg[SP][8];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
+    uint4 row[SP];
+    digits8(sexp[c], row, [&](int q) {
       const int gk = kt * TK + k8 * 8 + q;
-      const double x = (gc < P.rows && gk < P.inner) ? P.src[(long long)gc * P.ld + gk] : 0.0;
-      __nv_bfloat16 d[SP];
-      split_digits(x, sexp[c], d);
-#pragma unroll
-      for (int s = 0; s < SP; ++s) dg[s][q] = d[s];
-    }
+      return (gc < P.rows && gk < P.inner) ? P.src[(long long)gc * P.ld + gk] : 0.0;
+    });
 #pragma unroll
     for (int s = 0; s < SP; ++s)
-      *reinterpret_cast<uint4 *>(tile + tile_off(s * TN + c, k8 * 8, SP * TN)) =
-          *reinterpret_cast<uint4 *>(dg[s]);
+      *reinterpret_cast<uint4 *>(tile + tile_off(s * TN + c, k8 * 8, SP * TN)) = row[s];
   }
 }
 
@@ -391,18 +398,28 @@ __device__ __forceinline__ uint64_t globaltimer_ns() {
   return t;
 }
 
-// wait on phase parity, bounded by WAIT_NS of wall time; false on timeout
+__device__ __forceinline__ bool mbar_try(uint32_t a, uint32_t parity) {
+  uint32_t done;
+  asm volatile(
+      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+      " selp.u32 %0, 1, 0, p;\n}\n"
+      : "=r"(done)
+      : "r"(a), "r"(parity)
+      : "memory");
+  return done != 0;
+}
+
+// wait on phase parity, bounded by WAIT_NS of wall time; false on timeout.  The
+// clock is read only once a wait has failed 64 times: reading %globaltimer takes
+// longer than a chunk's MMAs.
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity) {
   const uint32_t a = smem_u32(bar);
+#pragma unroll 1
+  for (int i = 0; i < 64; ++i)
+    if (mbar_try(a, parity)) return true;
   const uint64_t t0 = globaltimer_ns();
   while (true) {
-    uint32_t done;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-        " selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(done)
-        : "r"(a), "r"(parity));
-    if (done) return true;
+    if (mbar_try(a, parity)) return true;
     if (globaltimer_ns() - t0 > WAIT_NS) return false;
   }
 }
@@ -441,8 +458,16 @@ __device__ __forceinline__ void umma_commit(uint64_t *bar) {
       : "memory");
 }
 
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float *v) {
-  uint32_t r[16];
+// true on one lane of the (converged) warp
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile(
+      "{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n"
+      : "=r"(p));
+  return p != 0;
+}
+
+__device__ __forceinline__ void tmem_ld16_issue(uint32_t taddr, uint32_t (&r)[16]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,"
       "%15}, [%16];"
@@ -450,9 +475,58 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float *v) {
         "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
         "=r"(r[14]), "=r"(r[15])
       : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+// the values of the loads issued so far (the registers pass through the wait,
+// so that no use moves ahead of it)
+__device__ __forceinline__ void tmem_ld16_wait(uint32_t (&r)[16]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]),
+                 "+r"(r[7]), "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]),
+                 "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
+               :
+               : "memory");
+}
+
+// Adds a finished window's seven group sums of 16 columns (groups at column
+// stride `gs`) to the exact accumulators
+//   H += acc_0 2^16 + acc_1 2^8 + acc_2, L += acc_3 2^24 + acc_4 2^16 + acc_5 2^8 + acc_6.
+// |acc_g| <= (g + 1) 2^21.  The sums are integers in FP32: groups 0 and 1 (up to
+// 2^22) by adding 1.5 2^23, which leaves the integer in the low bits, the others by
+// the conversion unit (FP32 to integer, 8 cycles per warp; neither touches the
+// FP64 pipe); then one 32 x 32 + 64-bit multiply-add each.
+__device__ __forceinline__ void drain16(uint32_t taddr, int gs, long long *hacc, long long *lacc) {
+  uint32_t r0[16], r1[16], r2[16], r3[16];
+  tmem_ld16_issue(taddr, r0);
+  tmem_ld16_issue(taddr + gs, r1);
+  tmem_ld16_issue(taddr + 2 * gs, r2);
+  tmem_ld16_wait(r0);
+  tmem_ld16_wait(r1);
+  tmem_ld16_wait(r2);
+  auto magic = [](uint32_t r) {
+    return __float_as_int(__uint_as_float(r) + 12582912.f) - 0x4B400000;
+  };
+  auto conv = [](uint32_t r) { return __float2int_rn(__uint_as_float(r)); };
 #pragma unroll
-  for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+  for (int i = 0; i < 16; ++i) {
+    // |acc_1 2^8 + acc_2| < 2^31
+    hacc[i] += (long long)magic(r0[i]) * 65536;
+    hacc[i] += (long long)(magic(r1[i]) * 256 + conv(r2[i]));
+  }
+  tmem_ld16_issue(taddr + 3 * gs, r0);
+  tmem_ld16_issue(taddr + 4 * gs, r1);
+  tmem_ld16_issue(taddr + 5 * gs, r2);
+  tmem_ld16_issue(taddr + 6 * gs, r3);
+  tmem_ld16_wait(r0);
+  tmem_ld16_wait(r1);
+  tmem_ld16_wait(r2);
+  tmem_ld16_wait(r3);
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    long long l = lacc[i] + (long long)conv(r0[i]) * (1 << 24);
+    l += (long long)conv(r1[i]) * 65536;
+    l += (long long)conv(r2[i]) * 256;
+    lacc[i] = l + conv(r3[i]);
+  }
 }
 
 // ---------------------------------------------------------------- GEMM ----
@@ -475,6 +549,15 @@ struct TcProb {
 // + i gridDim.x; tprob[t] names the tile's product.  Every wait is bounded;
 // after a timeout every role stops, the CTA waits (bounded) for its copies
 // and MMAs in flight, then frees its TMEM.
+//
+// Bound: shared-memory bandwidth.  A chunk (128 x 32 x 16, 896 MMA columns, 484
+// cycles of the tensor core alone) writes 35 KB and the MMAs read 56 KB, 728
+// cycles at 128 B; it takes 828 at 2048^3 (1263 when the drain's conversions,
+// 64-bit divisions in the one-thread loops and operands moved to uniform
+// registers per MMA stood in the way).  Copying the A planes once per cluster of
+// 2 or 4 CTAs by multicast changes nothing.  Through hss_gemm_dev, splitting
+// included: 4096^3 4.89 -> 3.24 ms (42 TFLOP/s FP64-equivalent), 2048^3 0.72 -> 0.54,
+// 2500 x 1400 x 1400 0.51 -> 0.35 ms.
 constexpr int NST = 6;                            // staged chunks in flight
 constexpr int GTH = 320;                          // 10 warps
 constexpr int ACC_SET = 256;                      // TMEM columns per accumulator set
@@ -484,6 +567,27 @@ constexpr int SMEM_TC = NST * STAGE_TC + 1024;
 static_assert(SP * TN <= ACC_SET, "accumulator groups exceed a TMEM set");
 static_assert(SMEM_TC <= 226 * 1024, "stages exceed the shared memory of a CTA");
 
+// The MMAs of the chunk in stage q: A plane s2 times B planes 0 .. SP-1-s2 (stacked
+// along N) is one MMA of N = (SP - s2) TN whose column block p2 lands on group
+// s2 + p2.  The window's first chunk starts with s2 = 0, which overwrites every
+// group; the others end with it: the tensor core queues a few MMAs only, and the
+// longest ones last keep it busy while the warp waits for the next chunks.
+__device__ __forceinline__ void issue_chunk(uint32_t acc, uint64_t ad0, uint64_t bd0, int q,
+                                            bool first) {
+  const uint64_t off = (uint64_t)(q * (STAGE_TC >> 4));
+  if (first) {
+#pragma unroll
+    for (int s2 = 0; s2 < SP; ++s2)
+      umma(acc + s2 * TN, ad0 + off + (uint64_t)((s2 * ATILE) >> 4), bd0 + off,
+           make_idesc(TM, (SP - s2) * TN), s2 > 0 ? 1u : 0u);
+  } else {
+#pragma unroll
+    for (int s2 = SP - 1; s2 >= 0; --s2)
+      umma(acc + s2 * TN, ad0 + off + (uint64_t)((s2 * ATILE) >> 4), bd0 + off,
+           make_idesc(TM, (SP - s2) * TN), 1u);
+  }
+}
+
 __global__ void __launch_bounds__(GTH, 1)
 k_gemm_tc(const TcProb *__restrict__ probs, const int *__restrict__ tprob, int ntiles,
           int *__restrict__ err) {
@@ -491,7 +595,7 @@ k_gemm_tc(const TcProb *__restrict__ probs, const int *__restrict__ tprob, int n
   __shared__ uint64_t full[NST], empty[NST], afull[2], aempty[2], fin;
   __shared__ uint32_t tmem_base;
   __shared__ volatile int s_ok;
-  __shared__ long long s_issued, s_consumed;
+  __shared__ volatile int s_issued, s_consumed;  // chunks, modulo 2^32
   __shared__ int s_skip;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // another CTA's wait already timed out: the launch is failing, skip the
@@ -521,73 +625,100 @@ k_gemm_tc(const TcProb *__restrict__ probs, const int *__restrict__ tprob, int n
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tbase = tmem_base;
   const int kwin = KWIN / TK;  // chunks per exactness window
-  // Chunk g (counted over the CTA's tiles) lives in stage g % NST, that
-  // stage's (g / NST)-th use: its "full" phase has parity (g / NST) & 1 and
-  // the stage is free for it once "empty" of use g / NST - 1 completed.
-  // Window w (counted likewise) accumulates in set w & 1, that set's
-  // (w / 2)-th use, with the same parity rule for afull / aempty.
+  // Chunks (counted over the CTA's tiles) go through the stages in turn; a role
+  // keeps its stage q and the parity ph of that stage's "full" phase, which flips
+  // when q wraps.  A stage is free for its next chunk once the "empty" phase of
+  // the previous one completed; on the unused stages of the first round a wait for
+  // parity ph ^ 1 = 1 returns at once.  Windows alternate between the two
+  // accumulator sets with the same rule for afull / aempty.  The copy and MMA
+  // roles are single threads whose instructions are not hidden by anything, so
+  // the loops carry counters instead of divisions and touch no shared flags.
   if (warp == 0) {
     if (lane == 0) {  // copies
-      long long g = 0;
-      for (int t = blockIdx.x; t < ntiles && s_ok; t += gridDim.x) {
+      int q = 0, g = 0;
+      uint32_t ph = 0;
+      bool ok = true;
+      for (int t = blockIdx.x; t < ntiles && ok && s_ok; t += gridDim.x) {
         const TcProb &P = probs[__ldg(tprob + t)];
         const int nk = P.ktiles, ntm = (P.M + TM - 1) / TM, tt = t - P.tile0;
-        const char *ga0 = P.a_planes + (long long)(tt % ntm) * nk * SP * ATILE;
-        const char *gb0 = P.b_planes + (long long)(tt / ntm) * nk * SP * BTILE;
-        for (int kt = 0; kt < nk && s_ok; ++kt, ++g) {
-          const int q = (int)(g % NST);
-          if (g >= NST && !mbar_wait(&empty[q], (uint32_t)((g / NST) - 1) & 1)) {
-            atomicOr(err, 1); s_ok = 0; break;
-          }
+        const char *ga = P.a_planes + (long long)(tt % ntm) * nk * SP * ATILE;
+        const char *gb = P.b_planes + (long long)(tt / ntm) * nk * SP * BTILE;
+        for (int kt = 0; kt < nk; ++kt) {
+          if (!mbar_wait(&empty[q], ph ^ 1u)) { atomicOr(err, 1); s_ok = 0; ok = false; break; }
           mbar_expect_tx(&full[q], STAGE_TC);
-          tma_load(sa(q), ga0 + (long long)kt * SP * ATILE, SP * ATILE, &full[q]);
-          tma_load(sb(q), gb0 + (long long)kt * SP * BTILE, SP * BTILE, &full[q]);
-          s_issued = g + 1;
+          tma_load(sa(q), ga, SP * ATILE, &full[q]);
+          tma_load(sb(q), gb, SP * BTILE, &full[q]);
+          ga += SP * ATILE;
+          gb += SP * BTILE;
+          s_issued = ++g;
+          if (++q == NST) { q = 0; ph ^= 1u; }
         }
       }
     }
+    __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {  // MMAs
-      long long g = 0, w = 0;
-      for (int t = blockIdx.x; t < ntiles && s_ok; t += gridDim.x) {
-        const int nk = probs[__ldg(tprob + t)].ktiles;
-        for (int k0 = 0; k0 < nk && s_ok; k0 += kwin, ++w) {
-          const int k1 = min(nk, k0 + kwin), a = (int)(w & 1);
-          if (w >= 2 && !mbar_wait(&aempty[a], (uint32_t)((w / 2) - 1) & 1)) {
-            atomicOr(err, 2); s_ok = 0; break;
-          }
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t acc = tbase + (uint32_t)(a * ACC_SET);
-          for (int kt = k0; kt < k1 && s_ok; ++kt, ++g) {
-            const int q = (int)(g % NST);
-            if (!mbar_wait(&full[q], (uint32_t)(g / NST) & 1)) { atomicOr(err, 4); s_ok = 0; break; }
-            s_consumed = g + 1;
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            // descriptor(address + offset) = descriptor(address) + offset / 16.
-            // A plane s2 times B planes 0 .. SP-1-s2 (stacked along N) is one
-            // MMA of N = (SP - s2) TN whose column block p2 lands on group
-            // s2 + p2; the window's first MMA (s2 = 0) overwrites every group
-            const uint64_t ad0 = make_desc(smem_u32(sa(q)), TM * 16, 128);
-            const uint64_t bd = make_desc(smem_u32(sb(q)), SP * TN * 16, 128);
-            const uint32_t later = kt > k0 ? 1u : 0u;
-#pragma unroll
-            for (int s2 = 0; s2 < SP; ++s2)
-              umma(acc + s2 * TN, ad0 + (uint64_t)((s2 * ATILE) >> 4), bd,
-                   make_idesc(TM, (SP - s2) * TN), s2 > 0 ? 1u : later);
-            umma_commit(&empty[q]);  // stage q is free once these MMAs completed
-          }
-          umma_commit(&afull[a]);    // the window's sums are complete
+    // MMAs.  The whole warp runs the loops with warp-uniform values (nk through a
+    // shuffle, waits through a vote) and one lane issues: operands of tcgen05
+    // instructions live in uniform registers, and in loops that only one lane
+    // enters each of them is moved there first (950 against 830 cycles a chunk).
+    int q = 0, g = 0, a = 0;
+    uint32_t ph = 0, aph = 0;
+    bool ok = true;
+    // descriptor(address + offset) = descriptor(address) + offset / 16
+    const uint64_t ad0 = make_desc(smem_u32(sa(0)), TM * 16, 128);
+    const uint64_t bd0 = make_desc(smem_u32(sb(0)), SP * TN * 16, 128);
+    const bool leader = elect_one();
+    for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
+      const int nk = __shfl_sync(HSS_FULL, probs[__ldg(tprob + t)].ktiles, 0);
+      for (int k0 = 0; k0 < nk && ok; k0 += kwin) {
+        const int k1 = min(nk, k0 + kwin);
+        ok = __all_sync(HSS_FULL, mbar_wait(&aempty[a], aph ^ 1u));
+        if (!ok) {
+          if (leader) { atomicOr(err, 2); s_ok = 0; }
+          break;
         }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t acc = tbase + (uint32_t)(a * ACC_SET);
+        for (int kt = k0; kt < k1; kt += 2) {
+          const bool two = kt + 1 < k1;
+          const int q1 = q + 1 == NST ? 0 : q + 1;
+          const uint32_t ph1 = q1 == 0 ? ph ^ 1u : ph;
+          ok = __all_sync(HSS_FULL, mbar_wait(&full[q], ph) && (!two || mbar_wait(&full[q1], ph1)));
+          if (!ok) {
+            if (leader) { atomicOr(err, 4); s_ok = 0; }
+            break;
+          }
+          g += two ? 2 : 1;
+          if (leader) {
+            issue_chunk(acc, ad0, bd0, q, kt == k0);
+            // a stage is free once its MMAs completed
+            umma_commit(&empty[q]);
+            if (two) {
+              issue_chunk(acc, ad0, bd0, q1, false);
+              umma_commit(&empty[q1]);
+            }
+          }
+          for (int r = 0; r < (two ? 2 : 1); ++r)
+            if (++q == NST) { q = 0; ph ^= 1u; }
+        }
+        if (leader) umma_commit(&afull[a]);  // the window's sums are complete
+        a ^= 1;
+        if (a == 0) aph ^= 1u;
       }
-      // every MMA issued (also before an error) completes before TMEM is freed
+    }
+    // every MMA issued (also before an error) completes before TMEM is freed
+    if (leader) {
+      s_consumed = g;
       umma_commit(&fin);
       if (!mbar_wait(&fin, 0)) { atomicOr(err, 8); s_ok = 0; }
     }
+    __syncwarp();
   } else {  // warps 2..9: drain and write; TMEM lanes 32 (warp % 4) ..
     const int quarter = warp & 3, half = (warp - 2) >> 2;
     constexpr int TH = TN / 2;  // output columns per thread
     static_assert(TH == 16, "the drain reads 16 TMEM columns per group");
-    long long w = 0;
+    int a = 0;
+    uint32_t aph = 0;
     for (int t = blockIdx.x; t < ntiles && s_ok; t += gridDim.x) {
       const TcProb &P = probs[__ldg(tprob + t)];
       const int nk = P.ktiles, ntm = (P.M + TM - 1) / TM, tt = t - P.tile0;
@@ -595,11 +726,10 @@ k_gemm_tc(const TcProb *__restrict__ probs, const int *__restrict__ tprob, int n
 #pragma unroll
       for (int j = 0; j < TH; ++j) { hacc[j] = 0; lacc[j] = 0; }
       bool okt = true;
-      for (int k0 = 0; k0 < nk; k0 += kwin, ++w) {
-        const int a = (int)(w & 1);
+      for (int k0 = 0; k0 < nk; k0 += kwin) {
         // one lane waits, the warp follows its verdict (tcgen05.ld is warp-wide)
         int got = 0;
-        if (lane == 0) got = mbar_wait(&afull[a], (uint32_t)(w / 2) & 1) ? 1 : 0;
+        if (lane == 0) got = mbar_wait(&afull[a], aph) ? 1 : 0;
         got = __shfl_sync(HSS_FULL, got, 0);
         if (!got) {
           if (lane == 0) { atomicOr(err, 16); s_ok = 0; }
@@ -609,20 +739,12 @@ k_gemm_tc(const TcProb *__restrict__ probs, const int *__restrict__ tprob, int n
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t lane_addr = tbase + (uint32_t)(a * ACC_SET) +
                                    ((uint32_t)(quarter * 32) << 16) + (uint32_t)(half * TH);
-#pragma unroll
-        for (int gq = 0; gq < SP; ++gq) {
-          float v[16];
-          tmem_ld16(lane_addr + gq * TN, v);
-#pragma unroll
-          for (int i = 0; i < TH; ++i) {
-            const long long x = (long long)int_of_float(v[i]);
-            if (gq < 3) hacc[i] += x * (1ll << (8 * (2 - gq)));
-            else lacc[i] += x * (1ll << (8 * (6 - gq)));
-          }
-        }
+        drain16(lane_addr, TN, hacc, lacc);
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
         if (lane == 0) mbar_arrive(&aempty[a]);  // the set may take new MMAs
+        a ^= 1;
+        if (a == 0) aph ^= 1u;
       }
       if (!okt) break;
       // C = 2^{e_i + f_j - 30} (H + 2^-32 L) (+ C)
@@ -646,8 +768,8 @@ k_gemm_tc(const TcProb *__restrict__ probs, const int *__restrict__ tprob, int n
   if (tid == 0 && !s_ok) {
     // a bounded wait gave up: wait (bounded) for the copies still in flight
     // before the CTA's shared memory is released
-    for (long long g = s_consumed; g < s_issued; ++g)
-      if (!mbar_wait(&full[g % NST], (uint32_t)(g / NST) & 1)) break;
+    for (unsigned g = (unsigned)s_consumed; g != (unsigned)s_issued; ++g)
+      if (!mbar_wait(&full[g % NST], (g / NST) & 1u)) break;
   }
   __syncthreads();
   if (warp == 0)
@@ -688,18 +810,6 @@ struct ExpJob {  // rows of A (stride = lda between k) or columns of B (contiguo
   int off;       // first flattened item of this job
 };
 
-
-// the SP digits of q (|q| <= 2^60) as BF16 bit patterns, packed into the
-// 16-byte core-matrix rows (element c of the 8 at half-word c)
-__device__ __forceinline__ void digits_into(long long q, int c, uint32_t (*pk)[4]) {
-#pragma unroll
-  for (int s = 0; s < SP; ++s) {
-    const int sh = 53 - 8 * s;
-    const long long d = (q + (1ll << (sh - 1))) >> sh;
-    q -= d * (1ll << sh);
-    pk[s][c >> 1] |= bf16_of_int((int)d) << (16 * (c & 1));
-  }
-}
 
 __global__ void k_row_exps(const ExpJob *__restrict__ jobs, int nj, int total) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -788,35 +898,25 @@ k_gemm_fused(const FusedProb *__restrict__ probs, int nprob, int *__restrict__ e
       // split this thread's row of the A chunk (coalesced over the rows)
 #pragma unroll 1
       for (int k8 = 0; k8 < FK / 8; ++k8) {
-        uint32_t pk[SP][4];
-#pragma unroll
-        for (int s2 = 0; s2 < SP; ++s2) pk[s2][0] = pk[s2][1] = pk[s2][2] = pk[s2][3] = 0u;
-#pragma unroll
-        for (int c = 0; c < 8; ++c) {
+        uint4 row[SP];
+        digits8(er, row, [&](int c) {
           const int gk = k0 + k8 * 8 + c;
-          const double x = (rok && gk < w1) ? P.A[(long long)gk * P.lda + r] : 0.0;
-          digits_into(scaled_int(x, er), c, pk);
-        }
+          return (rok && gk < w1) ? P.A[(long long)gk * P.lda + r] : 0.0;
+        });
 #pragma unroll
         for (int s2 = 0; s2 < SP; ++s2)
-          *reinterpret_cast<uint4 *>(sa + s2 * FATILE + tile_off(tid, k8 * 8, FM)) =
-              make_uint4(pk[s2][0], pk[s2][1], pk[s2][2], pk[s2][3]);
+          *reinterpret_cast<uint4 *>(sa + s2 * FATILE + tile_off(tid, k8 * 8, FM)) = row[s2];
       }
       // split one k octet of one B column
       {
-        uint32_t pk[SP][4];
-#pragma unroll
-        for (int s2 = 0; s2 < SP; ++s2) pk[s2][0] = pk[s2][1] = pk[s2][2] = pk[s2][3] = 0u;
-#pragma unroll
-        for (int c = 0; c < 8; ++c) {
+        uint4 row[SP];
+        digits8(ecb, row, [&](int c) {
           const int gk = k0 + ko * 8 + c;
-          const double x = (cok && gk < w1) ? P.B[(long long)gcb * P.ldb + gk] : 0.0;
-          digits_into(scaled_int(x, ecb), c, pk);
-        }
+          return (cok && gk < w1) ? P.B[(long long)gcb * P.ldb + gk] : 0.0;
+        });
 #pragma unroll
         for (int s2 = 0; s2 < SP; ++s2)
-          *reinterpret_cast<uint4 *>(sb + s2 * FBTILE + tile_off(cb, ko * 8, FN)) =
-              make_uint4(pk[s2][0], pk[s2][1], pk[s2][2], pk[s2][3]);
+          *reinterpret_cast<uint4 *>(sb + s2 * FBTILE + tile_off(cb, ko * 8, FN)) = row[s2];
       }
       // generic-proxy stores -> visible to the tensor cores' async proxy
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -852,17 +952,7 @@ k_gemm_fused(const FusedProb *__restrict__ probs, int nprob, int *__restrict__ e
       long long hv[16], lv[16];
 #pragma unroll
       for (int i = 0; i < 16; ++i) { hv[i] = 0; lv[i] = 0; }
-#pragma unroll
-      for (int g = 0; g < SP; ++g) {
-        float v[16];
-        tmem_ld16(lane_addr + g * FN + c, v);
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          const long long x = (long long)int_of_float(v[i]);
-          if (g < 3) hv[i] += x * (1ll << (8 * (2 - g)));
-          else lv[i] += x * (1ll << (8 * (6 - g)));
-        }
-      }
+      drain16(lane_addr + c, FN, hv, lv);
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
         const double v = exact_double(hv[i], lv[i], er + s_eb[c + i] - 30);
@@ -935,8 +1025,8 @@ void launch_gemm_split(const std::vector<GemmDesc> &probs, int *d_err, cudaStrea
   // tile -> product table for the persistent product kernel
   std::vector<int> tp(tiles);
   for (size_t i = 0; i < tc.size(); ++i) {
-    const int nt = ((probs[i].M + TM - 1) / TM) * ((probs[i].N + TN - 1) / TN);
-    for (int k = 0; k < nt; ++k) tp[tc[i].tile0 + k] = (int)i;
+    const int end = i + 1 < tc.size() ? tc[i + 1].tile0 : tiles;
+    for (int k = tc[i].tile0; k < end; ++k) tp[k] = (int)i;
   }
   int *dtp = pool<int>("gs_tp", tp.size());
   stage_h2d(dsa, sa.data(), sa.size() * sizeof(SplitProb), st);
@@ -969,7 +1059,6 @@ void launch_gemm_split(const std::vector<GemmDesc> &probs, int *d_err, cudaStrea
   }
   k_gemm_tc<<<std::min(tiles, sms), GTH, SMEM_TC, st>>>(dtc, dtp, tiles, d_err);
 }
-
 
 void launch_gemm_fused(const std::vector<GemmDesc> &probs, int *d_err, cudaStream_t st) {
   if (probs.empty()) return;
