@@ -96,15 +96,40 @@ HostTree make_tree(int K, int ni) {
 }
 
 // ------------------------------------------------------- device helpers --
-__device__ __forceinline__ ArgMax block_argmax(ArgMax a, ArgMax *red) {
+// (magnitude, position) of a pivot search.  Magnitudes are compared as integers:
+// the bit pattern of |v| orders as |v| does, and an FP64 comparison holds the
+// FP64 pipe for 64 cycles per warp, a reduction of them (two per merge) for
+// thousands.  key 0: none (a NaN is none too), else bits + 1.
+struct KeyIdx {
+  unsigned long long key;
+  int i;
+};
+__device__ __forceinline__ unsigned long long mag_key(double v) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(v) & 0x7FFFFFFFFFFFFFFFull;
+  return b > 0x7FF0000000000000ull ? 0ull : b + 1ull;
+}
+__device__ __forceinline__ double key_value(unsigned long long k) {  // -1 for none
+  return k ? __longlong_as_double((long long)(k - 1ull)) : -1.0;
+}
+// the larger magnitude, the first position on ties (Fortran MAXLOC order)
+__device__ __forceinline__ void key_take(KeyIdx &a, unsigned long long key, int i) {
+  if (key > a.key || (key && key == a.key && i < a.i)) { a.key = key; a.i = i; }
+}
+__device__ __forceinline__ KeyIdx warp_best(KeyIdx a) {
+  const unsigned hi = (unsigned)(a.key >> 32), lo = (unsigned)a.key;
+  const unsigned mh = __reduce_max_sync(HSS_FULL, hi);
+  const unsigned ml = __reduce_max_sync(HSS_FULL, hi == mh ? lo : 0u);
+  const bool in = hi == mh && lo == ml;
+  const int i = __reduce_min_sync(HSS_FULL, in ? a.i : INT_MAX);
+  return KeyIdx{(unsigned long long)mh << 32 | ml, i};
+}
+__device__ __forceinline__ KeyIdx block_best(KeyIdx a, KeyIdx *red) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  a = warp_argmax(a);
+  a = warp_best(a);
   __syncthreads();
   if (lane == 0) red[w] = a;
   __syncthreads();
-  ArgMax r = red[0];
-  for (int i = 1; i < (int)(blockDim.x >> 5); ++i) r = argmax_merge(r, red[i]);
-  return r;
+  return warp_best(lane < (int)(blockDim.x >> 5) ? red[lane] : KeyIdx{0ull, INT_MAX});
 }
 
 __device__ __forceinline__ double warp_prod(double v) {
@@ -121,32 +146,33 @@ __device__ __forceinline__ double warp_prod(double v) {
 // memory, and swaps of other-side entries done by rank 0 between cluster
 // barriers.  Other-side entries are read through L2 (ld.global.cg) so that a
 // CTA never sees a stale L1 copy of an entry another CTA of the cluster wrote.
-struct ArgMax3 {
-  double v;
-  int i;  // position (first wins on ties)
-  int a;  // auxiliary index carried with the winner
-};
-
 __device__ __forceinline__ void csync(int G) {
   if (G > 1) cg::this_cluster().sync();
   else __syncthreads();
 }
 
-// the cluster-wide best of each CTA's (value, position, aux), identical in every
+// the cluster-wide best of each CTA's (magnitude, position), identical in every
 // CTA; slot: two shared slots used alternately (a slot is rewritten only after
 // the next cluster barrier, by which time every CTA has read it)
-__device__ __forceinline__ ArgMax3 cluster_best(ArgMax3 x, int G, ArgMax3 *slot, int &phase) {
+__device__ __forceinline__ KeyIdx cluster_best(KeyIdx x, int G, KeyIdx *slot, int &phase) {
   if (G == 1) return x;
   cg::cluster_group cl = cg::this_cluster();
+  const int lane = threadIdx.x & 31;
   if (threadIdx.x == 0) slot[phase] = x;
   cl.sync();
-  ArgMax3 r{-1.0, INT_MAX, 0};
-  for (int q = 0; q < G; ++q) {
-    const ArgMax3 y = *cl.map_shared_rank(slot + phase, q);
-    if (y.v > r.v || (y.v == r.v && y.i < r.i)) r = y;
-  }
+  const KeyIdx r = warp_best(lane < G ? *cl.map_shared_rank(slot + phase, lane) : KeyIdx{0ull, INT_MAX});
   phase ^= 1;
   return r;
+}
+
+// |d| as FP32 rounded towards zero by integer operations (a conversion holds the
+// FP64 pipe); 0 below FP32's range, infinity above
+__device__ __forceinline__ float abs_f32(double d) {
+  const unsigned hi = (unsigned)__double2hiint(d) & 0x7fffffffu, lo = (unsigned)__double2loint(d);
+  const int e = (int)(hi >> 20) - 1023 + 127;
+  if (e <= 0) return 0.f;
+  if (e >= 255) return __int_as_float(0x7f800000);
+  return __uint_as_float((unsigned)e << 23 | (hi & 0xfffffu) << 3 | lo >> 29);
 }
 
 // Structured strong RRLU of one node (row or column case).  Node side (length
@@ -163,14 +189,15 @@ template <bool ROW>
 __device__ int rrlu_node(const PoleDiff &P, double *F, double *A, double *Z, double *W, int *PL,
                          int *PQ, double *V, int *PU, int M, int N, double tol, int rmax,
                          int *overflow, int *nswap, double rho, int G, int crank) {
-  __shared__ ArgMax red[HT / 32];
-  __shared__ ArgMax3 cslot[2];
-  __shared__ int s_rk;
+  __shared__ KeyIdx red[HT / 32];
+  __shared__ KeyIdx cslot[2];
+  __shared__ double s_wp[HT / 32 + 1];  // partial products of W[k], and its first factor
   int cphase = 0;
   const int tid = threadIdx.x;
   const int jstep = G * HT, joff = crank * HT;  // this CTA's share of the other side
-  auto Vr = [&](int j) -> double { return __ldcg(V + j); };
-  auto PUr = [&](int j) -> int { return __ldcg(PU + j); };
+  // (G = 1: V and PU may be in shared memory, and no other CTA writes them)
+  auto Vr = [&](int j) -> double { return G > 1 ? __ldcg(V + j) : V[j]; };
+  auto PUr = [&](int j) -> int { return G > 1 ? __ldcg(PU + j) : PU[j]; };
   // row poles: ROW -> F values (old poles); COL -> lam values (index PL)
   auto den = [&](int pl, int pu) -> double {  // C denominator for pole indices
     return ROW ? P.fd(pl, pu) : -P.fd(pu, pl);
@@ -179,59 +206,49 @@ __device__ int rrlu_node(const PoleDiff &P, double *F, double *A, double *Z, dou
     return ROW ? P.fv(F[i], F[j]) : P.dd(PL[i], PL[j]);
   };
   for (int i = tid; i < M; i += HT) { Z[i] = A[i]; PQ[i] = i; }
-  if (tid == 0) s_rk = -1;
   __syncthreads();
   const int mn = min(M, N);
   double Amax = 0.0;
-  auto colmax = [&](int k) -> int {
-    ArgMax a{-1.0, INT_MAX};
-    const int puk = PUr(k);
-    for (int i = k + tid; i < M; i += HT) {
-      const double t = fabs(qdiv(Z[i], den(PL[i], puk)));
-      if (t > a.v) { a.v = t; a.i = i; }
-    }
-    a = block_argmax(a, red);
-    return a.i == INT_MAX ? k : a.i;
-  };
+  // largest |Z_i / den| of column k (rows from k) and |V_j / den| of row k (columns
+  // from k); arg: its position
   auto colmax_v = [&](int k, int &arg) -> double {
-    ArgMax a{-1.0, INT_MAX};
+    KeyIdx a{0ull, INT_MAX};
     const int puk = PUr(k);
-    for (int i = k + tid; i < M; i += HT) {
-      const double t = fabs(qdiv(Z[i], den(PL[i], puk)));
-      if (t > a.v) { a.v = t; a.i = i; }
-    }
-    a = block_argmax(a, red);
+    for (int i = k + tid; i < M; i += HT) key_take(a, mag_key(qdiv(Z[i], den(PL[i], puk))), i);
+    a = block_best(a, red);
     arg = a.i == INT_MAX ? k : a.i;
-    return a.v;
+    return key_value(a.key);
   };
   auto rowmax_v = [&](int k, int &arg) -> double {
-    ArgMax a{-1.0, INT_MAX};
-    for (int j = k + joff + tid; j < N; j += jstep) {
-      const double t = fabs(qdiv(Vr(j), den(PL[k], PUr(j))));
-      if (t > a.v) { a.v = t; a.i = j; }
-    }
-    a = block_argmax(a, red);
-    const ArgMax3 c = cluster_best(ArgMax3{a.v, a.i, 0}, G, cslot, cphase);
-    arg = c.i == INT_MAX ? k : c.i;
-    return c.v;
+    KeyIdx a{0ull, INT_MAX};
+    const int plk = PL[k];
+    for (int j = k + joff + tid; j < N; j += jstep) key_take(a, mag_key(qdiv(Vr(j), den(plk, PUr(j)))), j);
+    a = cluster_best(block_best(a, red), G, cslot, cphase);
+    arg = a.i == INT_MAX ? k : a.i;
+    return key_value(a.key);
   };
   auto swap_row = [&](int a, int b) {
     __syncthreads();
-    if (tid == 0 && a != b) {
-      double t; int ti;
-      t = F[a]; F[a] = F[b]; F[b] = t;
-      t = Z[a]; Z[a] = Z[b]; Z[b] = t;
-      t = A[a]; A[a] = A[b]; A[b] = t;
-      ti = PL[a]; PL[a] = PL[b]; PL[b] = ti;
-      ti = PQ[a]; PQ[a] = PQ[b]; PQ[b] = ti;
+    if (tid < 5 && a != b) {  // a thread per array
+      if (tid < 3) {
+        double *x = tid == 0 ? F : tid == 1 ? Z : A;
+        const double t = x[a];
+        x[a] = x[b];
+        x[b] = t;
+      } else {
+        int *x = tid == 3 ? PL : PQ;
+        const int t = x[a];
+        x[a] = x[b];
+        x[b] = t;
+      }
     }
     __syncthreads();
   };
   auto swap_col = [&](int a, int b) {
     csync(G);
-    if (crank == 0 && tid == 0 && a != b) {
-      const double t = Vr(a); V[a] = Vr(b); V[b] = t;
-      const int ti = PUr(a); PU[a] = PUr(b); PU[b] = ti;
+    if (crank == 0 && tid < 2 && a != b) {
+      if (tid == 0) { const double t = Vr(a), u = Vr(b); V[a] = u; V[b] = t; }
+      else { const int t = PUr(a), u = PUr(b); PU[a] = u; PU[b] = t; }
     }
     csync(G);
   };
@@ -240,76 +257,98 @@ __device__ int rrlu_node(const PoleDiff &P, double *F, double *A, double *Z, dou
   // updated entries (the scan step k+1 would start with), unless a strong swap
   // changes the rows or entries in between
   bool have_next = false;
-  ArgMax next_best{-1.0, INT_MAX};
+  KeyIdx next_best{0ull, INT_MAX};
   for (int k = 0; k < mn; ++k) {
     if (k >= rmax) {  // would exceed the generator capacity
       if (tid == 0 && crank == 0) atomicOr(overflow, 1);
       Rk = k;
       break;
     }
+    double aukk = -1.0;  // |pivot|, from the search that settled on it
     {  // Gu's variant of complete pivoting (CauchyPivtEig, :571-680)
       int jl, ju;
       double jkL = colmax_v(k, jl);
       double jkU;
       if (have_next) {  // row k's maximum was found during step k-1's update pass
-        const ArgMax3 c = cluster_best(ArgMax3{next_best.v, next_best.i, 0}, G, cslot, cphase);
+        const KeyIdx c = cluster_best(next_best, G, cslot, cphase);
         ju = c.i == INT_MAX ? k : c.i;
-        jkU = c.v;
+        jkU = key_value(c.key);
       } else {
         jkU = rowmax_v(k, ju);
       }
       have_next = false;
       jkL *= fabs(Vr(k));
       jkU *= fabs(Z[k]);
-      const double piv = fabs(Z[k] * Vr(k) / den(PL[k], PUr(k)));
-      if (!(jkL <= piv && jkU <= piv)) {
+      if (jl == k && ju == k) {  // the pivot is the largest of its column and its row
+        aukk = jkU;
+      } else {
         bool fromcol = jkL > jkU;
         for (int guard = 0; guard < 4 * (M + N) + 8; ++guard) {
           if (fromcol) {
             swap_row(k, jl);
-            rowmax_v(k, ju);
-            if (ju == k) break;
+            const double v = rowmax_v(k, ju);
+            if (ju == k) { aukk = v * fabs(Z[k]); break; }
             fromcol = false;
           }
           swap_col(k, ju);
-          jl = colmax(k);
-          if (jl == k) break;
+          const double v = colmax_v(k, jl);
+          if (jl == k) { aukk = v * fabs(Vr(k)); break; }
           fromcol = true;
         }
       }
     }
     __syncthreads();
-    double Ukk = Z[k] * Vr(k) / den(PL[k], PUr(k));
-    Amax = fmax(Amax, fabs(Ukk));
-    if (fabs(Ukk) < tol * Amax) {
+    if (!(aukk >= 0.0)) aukk = fabs(Z[k] * Vr(k) / den(PL[k], PUr(k)));
+    Amax = fmax(Amax, aukk);
+    if (aukk < tol * Amax) {
+      // An upper bound of what is left of the Schur complement first: two FP64
+      // differences and FP32 arithmetic per entry.  Where it is below the tolerance
+      // too (the usual end of a node), the search below could only confirm that.
+      // (|Z|, |V| rounded up, differences down, none to 0 or infinity.)
+      float *ZF = (float *)(W + k);  // rows k .. M - 1; W(k) and on are not set yet
+      auto up_f32 = [](double v) { return fmaxf(abs_f32(v) * 1.000001f, 1.2e-38f); };
+      for (int i = k + tid; i < M; i += HT) ZF[i - k] = up_f32(Z[i]);
+      __syncthreads();
+      float em = 0.f;
+      for (int j = k + joff + tid; j < N; j += jstep) {
+        const int puj = PUr(j);
+        const float vj = up_f32(Vr(j));
+        float cm = 1e-37f;
+        for (int i = k; i < M; ++i)
+          cm = fmaxf(cm, ZF[i - k] / fminf(abs_f32(den(PL[i], puj)), 3e38f));
+        em = fmaxf(em, cm * vj);
+      }
+      KeyIdx e{(unsigned long long)__float_as_uint(em), 0};
+      e = cluster_best(block_best(e, red), G, cslot, cphase);
+      const double bound = (double)__uint_as_float((unsigned)e.key);
+      __syncthreads();
+      if (bound * 1.0001 < tol * Amax) { Rk = k; break; }
       // complete pivoting over the Schur complement (CauchyPivtEig_CP)
-      ArgMax best{-1.0, INT_MAX};
+      KeyIdx best{0ull, INT_MAX};
       int bi_loc = k;
       for (int j = k + joff + tid; j < N; j += jstep) {
-        double cm = -1.0;
-        int a = k;
+        KeyIdx cm{0ull, INT_MAX};
         const int puj = PUr(j);
-        for (int i = k; i < M; ++i) {
-          const double t = fabs(qdiv(Z[i], den(PL[i], puj)));
-          if (t > cm) { cm = t; a = i; }
-        }
-        const double t = fabs(cm * Vr(j));
-        if (t > best.v) { best.v = t; best.i = j; bi_loc = a; }
+        for (int i = k; i < M; ++i) key_take(cm, mag_key(qdiv(Z[i], den(PL[i], puj))), i);
+        const unsigned long long t = mag_key(key_value(cm.key) * Vr(j));
+        if (cm.key && t > best.key) { best.key = t; best.i = j; bi_loc = cm.i; }
       }
+      // the column first, then its row, from the CTA that holds it
       __shared__ int s_bi;
-      ArgMax r = block_argmax(best, red);
-      if (tid == 0 && r.i == INT_MAX) s_bi = k;
+      const KeyIdx r = cluster_best(block_best(best, red), G, cslot, cphase);
+      const int bj = r.i == INT_MAX ? k : r.i;
+      if (tid == 0) s_bi = -1;
       __syncthreads();
-      if (r.i != INT_MAX && best.i == r.i && best.v == r.v) s_bi = bi_loc;
+      if (r.i != INT_MAX && best.i == r.i) s_bi = bi_loc;
       __syncthreads();
-      const ArgMax3 c = cluster_best(ArgMax3{r.v, r.i, s_bi}, G, cslot, cphase);
-      const int bj = c.i == INT_MAX ? k : c.i;
-      const int bi = c.i == INT_MAX ? k : c.a;
+      KeyIdx row{s_bi >= 0 ? 1ull : 0ull, s_bi >= 0 ? s_bi : INT_MAX};
+      row = cluster_best(row, G, cslot, cphase);
+      const int bi = row.i == INT_MAX ? k : row.i;
       swap_row(k, bi);
       swap_col(k, bj);
-      Ukk = Z[k] * Vr(k) / den(PL[k], PUr(k));
-      Amax = fmax(Amax, fabs(Ukk));
-      if (fabs(Ukk) < tol * Amax) { Rk = k; break; }
+      aukk = fabs(Z[k] * Vr(k) / den(PL[k], PUr(k)));
+      Amax = fmax(Amax, aukk);
+      if (aukk < tol * Amax) { Rk = k; break; }
     }
     // Schur-complement generator updates
     const double Fk = ROW ? F[k] : 0.0;
@@ -318,59 +357,58 @@ __device__ int rrlu_node(const PoleDiff &P, double *F, double *A, double *Z, dou
       Z[j] *= qdiv(rowdiff(j, k), den(PL[j], puk));
     const bool fuse = k + 1 < mn && k + 1 < M;
     const int pln = fuse ? PL[k + 1] : 0;
-    ArgMax nb{-1.0, INT_MAX};
+    KeyIdx nb{0ull, INT_MAX};
     for (int j = k + 1 + joff + tid; j < N; j += jstep) {
       const int puj = PUr(j);
       const double vj = Vr(j) * (ROW ? qdiv(P.dd(puj, puk), -P.fd(PL[k], puj))
                                      : qdiv(P.fv(__ldg(P.F + puj), __ldg(P.F + puk)), P.fd(puj, PL[k])));
       V[j] = vj;
-      if (fuse) {  // |C(k+1, j)| / |A(k+1)| of the next step's Schur complement
-        const double t = fabs(qdiv(vj, den(pln, puj)));
-        if (t > nb.v) { nb.v = t; nb.i = j; }
-      }
+      // |C(k+1, j)| / |A(k+1)| of the next step's Schur complement
+      if (fuse) key_take(nb, mag_key(qdiv(vj, den(pln, puj))), j);
     }
-    if (fuse) {
-      next_best = block_argmax(nb, red);
-      have_next = true;
-    }
-    for (int j = tid; j < k; j += HT)
-      W[j] *= ROW ? qdiv(-P.fd(PL[j], puk), P.fv(Fk, F[j]))
-                  : qdiv(P.fd(puk, PL[j]), P.dd(PL[k], PL[j]));
-    if (tid < 32) {  // W[k] = den(k,k)/A[k] * prod_{j<k} ...
+    // W[j], j < k, and the factors of W[k] = den(k,k)/A[k] * prod_{j<k} ..., a thread
+    // per j; the first factor on the last warp meanwhile
+    {
       double pr = 1.0;
-      for (int j = tid; j < k; j += 32) {
+      for (int j = tid; j < k; j += HT) {
         const int puj = PUr(j);
+        W[j] *= ROW ? qdiv(-P.fd(PL[j], puk), P.fv(Fk, F[j]))
+                    : qdiv(P.fd(puk, PL[j]), P.dd(PL[k], PL[j]));
         pr *= ROW ? (-P.fd(PL[k], puj)) / P.fv(F[j], Fk) : P.fd(puj, PL[k]) / P.dd(PL[j], PL[k]);
       }
-      pr = warp_prod(pr);
-      if (tid == 0) W[k] = (den(PL[k], puk) / A[k]) * pr;
+      if ((tid & ~31) < k) {  // warps that hold factors
+        pr = warp_prod(pr);
+        if ((tid & 31) == 0) s_wp[tid >> 5] = pr;
+      }
+      if (tid == HT - 1) s_wp[HT / 32] = den(PL[k], puk) / A[k];
     }
-    csync(G);  // every CTA reads the updated V[k+1] next
+    if (fuse) {
+      next_best = block_best(nb, red);
+      have_next = true;
+    }
+    csync(G);  // every CTA reads the updated V[k+1] next, and s_wp is complete
+    if (tid == 0) {
+      double w = s_wp[HT / 32];
+      for (int q = 0; q < HT / 32 && 32 * q < k; ++q) w *= s_wp[q];
+      W[k] = w;
+    }
     // strong swaps every 10 steps when an interpolation entry exceeds rho
     // (searchMax2Eig[m] with rho = 1.5, CauchyHssEig.f90:98-99; searchMax2 with
     // rho = 1.02 for generic Cauchy matrices, CauchyHss_VP2.f90:70-71)
     if ((k + 1) % 10 == 0) {
       for (int guard = 0; guard < M + 8; ++guard) {
-        ArgMax best{-1.0, INT_MAX};
-        int ii_loc = 0;
-        for (int j = tid; j <= k; j += HT) {
-          double cm = -1.0;
-          int a = k + 1;
-          for (int i = k + 1; i < M; ++i) {
-            const double t = fabs(qdiv(Z[i], rowdiff(i, j)));
-            if (t > cm) { cm = t; a = i; }
-          }
-          const double t = cm * fabs(W[j]);
-          if (t > best.v) { best.v = t; best.i = j; ii_loc = a; }
+        // largest |W_j Z_i / (row pole i - row pole j)|, j <= k < i: lanes over j,
+        // warps over i; the position j 1024 + i orders ties by j, then i
+        __syncthreads();
+        KeyIdx best{0ull, INT_MAX};
+        for (int j = tid & 31; j <= k; j += 32) {
+          const double wj = W[j];
+          for (int i = k + 1 + (tid >> 5); i < M; i += HT / 32)
+            key_take(best, mag_key(qdiv(Z[i], rowdiff(i, j)) * wj), j * 1024 + i);
         }
-        __shared__ int s_jj;
-        ArgMax r = block_argmax(best, red);
-        if (tid == 0) s_jj = (r.i == INT_MAX) ? M : -1;
-        __syncthreads();
-        if (r.i != INT_MAX && best.i == r.i && best.v == r.v) s_jj = ii_loc;
-        __syncthreads();
-        const int ii = r.i == INT_MAX ? 0 : r.i, jj = s_jj;
-        if (!(r.v > rho) || jj >= M) break;
+        const KeyIdx r = block_best(best, red);
+        const int ii = r.i == INT_MAX ? 0 : r.i >> 10, jj = r.i == INT_MAX ? M : r.i & 1023;
+        if (!(key_value(r.key) > rho) || jj >= M) break;
         have_next = false;  // rows and other-side entries change
         if (tid == 0 && crank == 0) atomicAdd(nswap, 1);
         for (int j = k + 1 + joff + tid; j < N; j += jstep) {
@@ -437,6 +475,10 @@ __device__ int rrlu_node(const PoleDiff &P, double *F, double *A, double *Z, dou
 // Row compression of every node of one level: node block row against all
 // other current columns (ComprcauchyEig 'r', :2338-2380).
 constexpr int MMAXS = 512;  // max rows of a node handled in shared memory
+// The other side of a node with a CTA of its own stays in (dynamic) shared memory
+// up to this length: every scan reads it, and from L2 a scan costs its latency.
+constexpr int OSIDE = 2048;
+constexpr size_t OSIDE_SMEM = OSIDE * (sizeof(double) + sizeof(int));
 
 __global__ void __launch_bounds__(HT)
 k_hss_rows(HssDev h, const int *__restrict__ nodes, int nn, double tol, int csz) {
@@ -451,8 +493,10 @@ k_hss_rows(HssDev h, const int *__restrict__ nodes, int nn, double tol, int csz)
   const int c0 = h.lc0[node], nc = h.lc1[node] - c0 + 1;
   const int lca = *h.lca, N = lca - nc;
   if (M > MMAXS) { if (tid == 0) atomicOr(h.flag, 2); return; }
-  double *V = h.oval + (long long)a * h.K;
-  int *PU = h.oidx + (long long)a * h.K;
+  extern __shared__ double oside[];
+  const bool osm = csz == 1 && N <= OSIDE;
+  double *V = osm ? oside : h.oval + (long long)a * h.K;
+  int *PU = osm ? (int *)(oside + OSIDE) : h.oidx + (long long)a * h.K;
   for (int j = crank * HT + tid; j < lca; j += csz * HT) {  // this CTA's share of the copy
     if (j < c0) { V[j] = h.V[j]; PU[j] = h.PU[j]; }
     else if (j > h.lc1[node]) { V[j - nc] = h.V[j]; PU[j - nc] = h.PU[j]; }
@@ -506,8 +550,10 @@ k_hss_cols(HssDev h, const int *__restrict__ nodes, int nn, double tol, int csz)
   const int r0 = h.lr0[node], nr = h.lr1[node] - r0 + 1;
   const int lda = *h.lda, N = lda - nr;
   if (M > MMAXS) { if (tid == 0) atomicOr(h.flag, 2); return; }
-  double *V = h.oval + (long long)a * h.K;
-  int *PU = h.oidx + (long long)a * h.K;
+  extern __shared__ double oside[];
+  const bool osm = csz == 1 && N <= OSIDE;
+  double *V = osm ? oside : h.oval + (long long)a * h.K;
+  int *PU = osm ? (int *)(oside + OSIDE) : h.oidx + (long long)a * h.K;
   for (int j = crank * HT + tid; j < lda; j += csz * HT) {  // this CTA's share of the copy
     if (j < r0) { V[j] = h.U[j]; PU[j] = h.PL[j]; }
     else if (j > h.lr1[node]) { V[j - nr] = h.U[j]; PU[j - nr] = h.PL[j]; }
@@ -662,7 +708,7 @@ static void launch_node_rrlu(void (*kern)(HssDev, const int *, int, double, int)
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(nn * G));
   cfg.blockDim = dim3(HT);
-  cfg.dynamicSmemBytes = 0;
+  cfg.dynamicSmemBytes = G == 1 ? OSIDE_SMEM : 0;
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
