@@ -165,6 +165,26 @@ __device__ __forceinline__ KeyIdx cluster_best(KeyIdx x, int G, KeyIdx *slot, in
   return r;
 }
 
+// A pole with its root: F_i, F_{i+1} and lam_i - F_i, lam_i - F_{i+1}.  The differences
+// of PoleDiff on values that are loaded once (in the scans one of the two poles is
+// fixed, and the other's values serve several differences).
+struct Pole {
+  double F, F1, dl, dr;
+  int i;
+};
+__device__ __forceinline__ Pole load_pole(const PoleDiff &P, int K, int i) {
+  const int n = min(i + 1, K - 1);  // (the last pole has no successor, none is used)
+  return Pole{__ldg(P.F + i), __ldg(P.F + n), __ldg(P.difl + i), __ldg(P.difr + i), i};
+}
+__device__ __forceinline__ double pole_fd(bool sq, const Pole &p, const Pole &q) {  // F_p - lam_q
+  const double lin = p.i <= q.i ? (p.F - q.F) - q.dl : (p.F - q.F1) - q.dr;
+  return sq ? lin * (p.F + (q.F + q.dl)) : lin;
+}
+__device__ __forceinline__ double pole_dd(bool sq, const Pole &p, const Pole &q) {  // lam_p - lam_q
+  const double lin = p.i < q.i ? (p.F1 - q.F) + p.dr - q.dl : (p.F - q.F1) + p.dl - q.dr;
+  return sq ? lin * ((p.F + p.dl) + (q.F + q.dl)) : lin;
+}
+
 // |d| as FP32 rounded towards zero by integer operations (a conversion holds the
 // FP64 pipe); 0 below FP32's range, infinity above
 __device__ __forceinline__ float abs_f32(double d) {
@@ -185,10 +205,15 @@ __device__ __forceinline__ float abs_f32(double d) {
 // Returns Rk; on exit A/PL/F are permuted, Z holds the Schur row generators,
 // W the column generators of the interpolation block, PQ the row permutation.
 // G, crank: the cluster size and this CTA's rank in it (1, 0 without a cluster).
+//
+// Bound: the latency of a pivot step, a chain of scans and reductions with FP64
+// warp instructions of 64 cycles each (12000 to 14000 cycles per step of a short
+// node, 43000 with FP64 comparisons in the reductions).  HSS stage of Cauchy
+// n = 3000 14.3 -> 5.9 ms, of the disordered chain n = 3000 27.8 -> 12.0 ms.
 template <bool ROW>
 __device__ int rrlu_node(const PoleDiff &P, double *F, double *A, double *Z, double *W, int *PL,
                          int *PQ, double *V, int *PU, int M, int N, double tol, int rmax,
-                         int *overflow, int *nswap, double rho, int G, int crank) {
+                         int *overflow, int *nswap, double rho, int G, int crank, int K) {
   __shared__ KeyIdx red[HT / 32];
   __shared__ KeyIdx cslot[2];
   __shared__ double s_wp[HT / 32 + 1];  // partial products of W[k], and its first factor
@@ -202,6 +227,10 @@ __device__ int rrlu_node(const PoleDiff &P, double *F, double *A, double *Z, dou
   auto den = [&](int pl, int pu) -> double {  // C denominator for pole indices
     return ROW ? P.fd(pl, pu) : -P.fd(pu, pl);
   };
+  auto pole = [&](int i) { return load_pole(P, K, i); };
+  auto den_p = [&](const Pole &pl, const Pole &pu) -> double {  // den on loaded poles
+    return ROW ? pole_fd(P.sq, pl, pu) : -pole_fd(P.sq, pu, pl);
+  };
   auto rowdiff = [&](int i, int j) -> double {  // row pole i minus row pole j
     return ROW ? P.fv(F[i], F[j]) : P.dd(PL[i], PL[j]);
   };
@@ -213,16 +242,18 @@ __device__ int rrlu_node(const PoleDiff &P, double *F, double *A, double *Z, dou
   // from k); arg: its position
   auto colmax_v = [&](int k, int &arg) -> double {
     KeyIdx a{0ull, INT_MAX};
-    const int puk = PUr(k);
-    for (int i = k + tid; i < M; i += HT) key_take(a, mag_key(qdiv(Z[i], den(PL[i], puk))), i);
+    const Pole puk = pole(PUr(k));
+    for (int i = k + tid; i < M; i += HT)
+      key_take(a, mag_key(qdiv(Z[i], den_p(pole(PL[i]), puk))), i);
     a = block_best(a, red);
     arg = a.i == INT_MAX ? k : a.i;
     return key_value(a.key);
   };
   auto rowmax_v = [&](int k, int &arg) -> double {
     KeyIdx a{0ull, INT_MAX};
-    const int plk = PL[k];
-    for (int j = k + joff + tid; j < N; j += jstep) key_take(a, mag_key(qdiv(Vr(j), den(plk, PUr(j)))), j);
+    const Pole plk = pole(PL[k]);
+    for (int j = k + joff + tid; j < N; j += jstep)
+      key_take(a, mag_key(qdiv(Vr(j), den_p(plk, pole(PUr(j))))), j);
     a = cluster_best(block_best(a, red), G, cslot, cphase);
     arg = a.i == INT_MAX ? k : a.i;
     return key_value(a.key);
@@ -311,11 +342,15 @@ __device__ int rrlu_node(const PoleDiff &P, double *F, double *A, double *Z, dou
       __syncthreads();
       float em = 0.f;
       for (int j = k + joff + tid; j < N; j += jstep) {
-        const int puj = PUr(j);
+        const Pole puj = pole(PUr(j));
         const float vj = up_f32(Vr(j));
         float cm = 1e-37f;
-        for (int i = k; i < M; ++i)
-          cm = fmaxf(cm, ZF[i - k] / fminf(abs_f32(den(PL[i], puj)), 3e38f));
+#pragma unroll 4
+        for (int i = k; i < M; ++i) {
+          // (ROW: the node's old poles are in shared memory, and no more is used of them)
+          const Pole pli = ROW ? Pole{F[i], 0.0, 0.0, 0.0, PL[i]} : pole(PL[i]);
+          cm = fmaxf(cm, ZF[i - k] / fminf(abs_f32(den_p(pli, puj)), 3e38f));
+        }
         em = fmaxf(em, cm * vj);
       }
       KeyIdx e{(unsigned long long)__float_as_uint(em), 0};
@@ -353,32 +388,36 @@ __device__ int rrlu_node(const PoleDiff &P, double *F, double *A, double *Z, dou
     // Schur-complement generator updates
     const double Fk = ROW ? F[k] : 0.0;
     const int puk = PUr(k);
-    for (int j = k + 1 + tid; j < M; j += HT)
-      Z[j] *= qdiv(rowdiff(j, k), den(PL[j], puk));
+    const Pole puk_p = pole(puk), plk_p = pole(PL[k]);
+    // (the three passes of a step start on different warps, so that short ones run
+    // beside each other: V from warp 0, Z from warp 2, W from warp 4)
+    for (int j = k + 1 + ((tid + HT - 64) & (HT - 1)); j < M; j += HT)
+      Z[j] *= qdiv(rowdiff(j, k), den_p(pole(PL[j]), puk_p));
     const bool fuse = k + 1 < mn && k + 1 < M;
-    const int pln = fuse ? PL[k + 1] : 0;
+    const Pole pln = pole(fuse ? PL[k + 1] : 0);
     KeyIdx nb{0ull, INT_MAX};
     for (int j = k + 1 + joff + tid; j < N; j += jstep) {
-      const int puj = PUr(j);
-      const double vj = Vr(j) * (ROW ? qdiv(P.dd(puj, puk), -P.fd(PL[k], puj))
-                                     : qdiv(P.fv(__ldg(P.F + puj), __ldg(P.F + puk)), P.fd(puj, PL[k])));
+      const Pole puj = pole(PUr(j));
+      const double vj = Vr(j) * (ROW ? qdiv(pole_dd(P.sq, puj, puk_p), -pole_fd(P.sq, plk_p, puj))
+                                     : qdiv(P.fv(puj.F, puk_p.F), pole_fd(P.sq, puj, plk_p)));
       V[j] = vj;
       // |C(k+1, j)| / |A(k+1)| of the next step's Schur complement
-      if (fuse) key_take(nb, mag_key(qdiv(vj, den(pln, puj))), j);
+      if (fuse) key_take(nb, mag_key(qdiv(vj, den_p(pln, puj))), j);
     }
     // W[j], j < k, and the factors of W[k] = den(k,k)/A[k] * prod_{j<k} ..., a thread
     // per j; the first factor on the last warp meanwhile
     {
+      const int tw = (tid + HT / 2) & (HT - 1);
       double pr = 1.0;
-      for (int j = tid; j < k; j += HT) {
+      for (int j = tw; j < k; j += HT) {
         const int puj = PUr(j);
         W[j] *= ROW ? qdiv(-P.fd(PL[j], puk), P.fv(Fk, F[j]))
                     : qdiv(P.fd(puk, PL[j]), P.dd(PL[k], PL[j]));
         pr *= ROW ? (-P.fd(PL[k], puj)) / P.fv(F[j], Fk) : P.fd(puj, PL[k]) / P.dd(PL[j], PL[k]);
       }
-      if ((tid & ~31) < k) {  // warps that hold factors
+      if ((tw & ~31) < k) {  // warps that hold factors
         pr = warp_prod(pr);
-        if ((tid & 31) == 0) s_wp[tid >> 5] = pr;
+        if ((tw & 31) == 0) s_wp[tw >> 5] = pr;
       }
       if (tid == HT - 1) s_wp[HT / 32] = den(PL[k], puk) / A[k];
     }
@@ -480,7 +519,7 @@ constexpr int MMAXS = 512;  // max rows of a node handled in shared memory
 constexpr int OSIDE = 2048;
 constexpr size_t OSIDE_SMEM = OSIDE * (sizeof(double) + sizeof(int));
 
-__global__ void __launch_bounds__(HT)
+__global__ void __launch_bounds__(HT, 2)
 k_hss_rows(HssDev h, const int *__restrict__ nodes, int nn, double tol, int csz) {
   __shared__ double F[MMAXS], A[MMAXS], Z[MMAXS], W[MMAXS];
   __shared__ int PL[MMAXS], PQ[MMAXS], INV[MMAXS];
@@ -510,7 +549,7 @@ k_hss_rows(HssDev h, const int *__restrict__ nodes, int nn, double tol, int csz)
   csync(csz);
   PoleDiff P{h.FF, h.DIFL, h.DIFR, h.sq};
   int Rk = rrlu_node<true>(P, F, A, Z, W, PL, PQ, V, PU, M, N, tol, h.rmax, h.flag, h.flag + 1,
-                           h.rho, csz, crank);
+                           h.rho, csz, crank, h.K);
   if (crank != 0) return;  // rank 0 writes the node's results
   __syncthreads();
   for (int i = tid; i < M; i += HT) { h.U[r0 + i] = A[i]; h.PL[r0 + i] = PL[i]; INV[PQ[i]] = i; }
@@ -537,7 +576,7 @@ k_hss_rows(HssDev h, const int *__restrict__ nodes, int nn, double tol, int csz)
 // Column compression: node block column against all other current rows
 // (ComprcauchyEig 'c', :2382-2430).  The transposed block has the node's
 // roots as row poles.
-__global__ void __launch_bounds__(HT)
+__global__ void __launch_bounds__(HT, 2)
 k_hss_cols(HssDev h, const int *__restrict__ nodes, int nn, double tol, int csz) {
   __shared__ double F[MMAXS], A[MMAXS], Z[MMAXS], W[MMAXS];
   __shared__ int PL[MMAXS], PQ[MMAXS], INV[MMAXS];
@@ -567,7 +606,7 @@ k_hss_cols(HssDev h, const int *__restrict__ nodes, int nn, double tol, int csz)
   csync(csz);
   PoleDiff P{h.FF, h.DIFL, h.DIFR, h.sq};
   int Rk = rrlu_node<false>(P, F, A, Z, W, PL, PQ, V, PU, M, N, tol, h.rmax, h.flag, h.flag + 1,
-                            h.rho, csz, crank);
+                            h.rho, csz, crank, h.K);
   if (crank != 0) return;  // rank 0 writes the node's results
   __syncthreads();
   for (int i = tid; i < M; i += HT) { h.V[c0 + i] = A[i]; h.PU[c0 + i] = PL[i]; INV[PQ[i]] = i; }
@@ -688,23 +727,27 @@ __global__ void k_init_gens(int K, const double *__restrict__ u, const double *_
 
 // --------------------------------------------------------------- host ----
 // CTAs per node of a level (a thread-block cluster): doubled while the level
-// stays within HSS_CLUSTER_CTAS CTAs, up to a portable cluster of 8.  Levels of
-// 8 nodes or fewer run one CTA per node: their other side (the skeletons of the
-// remaining nodes) is short, and the cluster barriers of every pivot step cost
-// more than the split scans save (measured on the 8192-point Cauchy merge).
+// stays within HSS_CLUSTER_CTAS CTAs, up to a portable cluster of 8 (Cauchy
+// n = 3000, 23 leaves: 8.3 ms with at most 152 or 304 CTAs, 9.0 with 100, 10.5 with
+// 40).  Levels of 8 nodes or fewer run one CTA per node where the other side is
+// the skeletons of the remaining nodes: it is short, and the cluster barriers of
+// every pivot step cost more than the split scans save.  Their leaf level, with
+// all K columns on the other side, takes clusters from HSS_CLUSTER_MIN columns (the
+// three merges of the disordered chain n = 3000: 21.5 -> 19.8 ms).
 constexpr int HSS_CLUSTER_MAX = 8;
 constexpr int HSS_CLUSTER_CTAS = 304;  // two CTAs per SM
-static int hss_cluster_size(int nn) {
+constexpr int HSS_CLUSTER_MIN = 1024;
+static int hss_cluster_size(int nn, int other) {
   int G = 1;
-  if (nn <= 8) return 1;
+  if (nn <= 8 && other < HSS_CLUSTER_MIN) return 1;
   while (G < HSS_CLUSTER_MAX && (long long)nn * G * 2 <= HSS_CLUSTER_CTAS) G *= 2;
   return G;
 }
 
 static void launch_node_rrlu(void (*kern)(HssDev, const int *, int, double, int),
-                             const HssDev &h, const int *dn, int nn, double tol,
+                             const HssDev &h, const int *dn, int nn, int other, double tol,
                              cudaStream_t st) {
-  const int G = hss_cluster_size(nn);
+  const int G = hss_cluster_size(nn, other);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(nn * G));
   cfg.blockDim = dim3(HT);
@@ -810,9 +853,11 @@ static int hss_construct(HssPlan &pl, int K, int ni, double tol, const double *F
     snprintf(nm, sizeof nm, "hs_pairs%d", LL);
     int *dpr = up(nm, pairs, st);
     const int nn = (int)nodes.size();
-    launch_node_rrlu(k_hss_rows, h, dn, nn, tol, st);
+    // other side of the rows: all columns on the first (leaf) level; above it and for
+    // the columns the skeletons, whose number only the device knows yet
+    launch_node_rrlu(k_hss_rows, h, dn, nn, LL == t.lvl ? K : 0, tol, st);
     k_hss_compact<<<1, 512, 0, st>>>(h, dn, nn, da, (int)above.size(), dp, 0, 1);
-    launch_node_rrlu(k_hss_cols, h, dn, nn, tol, st);
+    launch_node_rrlu(k_hss_cols, h, dn, nn, 0, tol, st);
     k_hss_compact<<<1, 512, 0, st>>>(h, dn, nn, da, (int)above.size(), dp, (int)parents.size() / 3, 0);
     k_hss_B<<<nn, 256, 0, st>>>(h, dpr, nn);
     launches += 5;
