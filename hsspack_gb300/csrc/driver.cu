@@ -477,16 +477,21 @@ static void run_merges(Ctx &c, const std::vector<int> &ms, const std::vector<int
                 *std::max_element(aK.begin(), aK.end()));
   stage_end(HSS_ST_LOWNER, st, 40LL * total, 5.0 * k2);
   c.launches += 2;
-  if (bu && bu->nrest > 0) {
-    // the remaining Z columns follow the new eigenvectors (mdsbed4.f90:266-268)
+  // the remaining Z columns follow the new eigenvectors (mdsbed4.f90:266-268); the
+  // norms come from the dense blocks, or from a pass of their own with HSS merges
+  const bool zup = bu && bu->nrest > 0;
+  auto zupdate = [&]() {
     double *zt = buf<double>(c, "band_zt", (size_t)bu->nrest * bu->zld);
     stage_begin(HSS_ST_OTHER, st);
-    launch_alpha(lv, total, L.w.dl, L.difl, L.difr, L.zhat, L.alpha, st);
+    if (!hsel.empty()) {
+      launch_alpha(lv, total, L.w.dl, L.difl, L.difr, L.zhat, L.alpha, st);
+      c.launches++;
+    }
     launch_band_zupdate(lv, total, L.w.dl, L.difl, L.difr, L.zhat, L.alpha, L.w.ndslot, bu->zrest,
                         bu->nrest, bu->zld, zt, st);
     stage_end(HSS_ST_OTHER, st, 0, (2.0 + 4.0 * bu->nrest) * k2);
-    c.launches += 3;
-  }
+    c.launches += 2;
+  };
   // ---- dense merges: S, gather, GEMM (block structured), scatter
   const int PD = (int)ds_.size();
   if (PD > 0) {
@@ -499,8 +504,10 @@ static void run_merges(Ctx &c, const std::vector<int> &ms, const std::vector<int
     double *Q2 = buf<double>(c, "Q2", q2tot), *T = buf<double>(c, "T", q2tot);
     double *S = buf<double>(c, "S", stot);
     stage_begin(HSS_ST_BUILD_S, st);
-    launch_build_S(dv, dtot, L.w.dl, L.difl, L.difr, L.zhat, L.w.grp, xso, S, st);
+    launch_build_S(dv, dtot, L.w.dl, L.difl, L.difr, L.zhat, L.w.grp, xso, S, st,
+                   zup && hsel.empty() ? L.alpha : nullptr);
     stage_end(HSS_ST_BUILD_S, st, 8LL * stot * 2, 0.0);
+    if (zup) zupdate();
     int maxnd = *std::max_element(dn_.begin(), dn_.end());
     stage_begin(HSS_ST_GATHER, st);
     launch_gather(PD, dtot, maxnd, xs, xn, xoff, L.w.ndslot, L.w.grp, xq2, Q, ldq, Q2, st, L.sup, xr);
@@ -537,6 +544,7 @@ static void run_merges(Ctx &c, const std::vector<int> &ms, const std::vector<int
     stage_end(HSS_ST_SCATTER, st, 16LL * q2tot, 0.0);
     c.launches += 4;
   }
+  if (PD == 0 && zup) zupdate();
   // ---- HSS merges: one at a time (each has its own HSS tree)
   for (int a : hsel) {
     HssMergeArgs h;

@@ -67,7 +67,8 @@ void launch_alpha(const LevelView &lv, int total, const double *dl, const double
                   bool sq = false);
 void launch_build_S(const LevelView &lv, int total, const double *dl, const double *difl,
                     const double *difr, const double *zhat, const int *grp,
-                    const long long *soff, double *Sws, cudaStream_t st);
+                    const long long *soff, double *Sws, cudaStream_t st,
+                    double *alpha = nullptr);
 void launch_cauchy_eig(int K, const double *F, const double *u, const double *v,
                        const double *difl, const double *difr, double *C, cudaStream_t st,
                        bool sq = false);

@@ -47,19 +47,41 @@ __device__ int svd_prep_chain(int s, int N, double tol, const LevelScratch &w) {
     }
     __syncthreads();
   }
+  // A pair t rotates when d_t - d_{t-1} is within tol, whatever the rotations before it
+  // did (they change z and types only): the pairs that rotate are listed in order
+  // by all threads, and one thread walks the list (z chains from pair to pair).
+  // Walking every pair on that thread took 0.24 ms of a 1400-candidate merge.
+  int *lst = w.l1slot + s;  // free until the deflated lists are written
+  {
+    const int pc = (max(nc - 1, 0) + MT - 1) / MT;
+    const int p0 = min(nc, 1 + tid * pc), p1 = min(nc, p0 + pc);
+    auto close = [&](int t) {
+      const double dp = in_smem ? c_d[t - 1] : w.ds[s + w.cand[s + t - 1]];
+      const double dn = in_smem ? c_d[t] : w.ds[s + w.cand[s + t]];
+      return fabs(dn - dp) <= tol;
+    };
+    int cp = 0;
+    for (int t = p0; t < p1; ++t) cp += close(t);
+    unsigned long long ptot;
+    int pp = (int)block_scan64<MT>((unsigned long long)cp, &ptot);
+    if (cp)
+      for (int t = p0; t < p1; ++t)
+        if (close(t)) lst[pp++] = t;
+    if (tid == 0) s_ng = (int)ptot;
+    __syncthreads();
+  }
   if (tid == 0) {
+    const int nl = s_ng;
     int ng = 0;
-    for (int t = 1; t < nc; ++t) {
-      const int pt = t - 1;
+    for (int a = 0; a < nl; ++a) {
+      const int t = lst[a], pt = t - 1;
       const int pp = w.cand[s + pt], np_ = w.cand[s + t];
       const double zp = in_smem ? c_z[pt] : w.zs[s + pp];
       const double zn = in_smem ? c_z[t] : w.zs[s + np_];
-      const double dp = in_smem ? c_d[pt] : w.ds[s + pp];
-      const double dn = in_smem ? c_d[t] : w.ds[s + np_];
       // the predecessor is the previous candidate: after a rotation the pole
       // rotated into becomes the new JPREV (mdlasd2.f90 loop 100)
       const unsigned char tp = in_smem ? c_t[pt] : w.typ[s + pp];
-      if (fabs(dn - dp) <= tol) {
+      {
         const double tau = hypot(zn, zp);
         const double cg = zn / tau, sg = -zp / tau;
         const unsigned char tn = in_smem ? c_t[t] : w.typ[s + np_];

@@ -581,11 +581,13 @@ __global__ void k_alpha(LevelView lv, const double *__restrict__ dl,
 // (LAPACK DLAED3's S, used at SRC/mdlaed1.f90:198-201): column j holds
 // z_hat_i / (d_i - lam_j) normalised to unit length.  Row i is written at
 // group position grp[s+i] (columns of Q2 grouped by block structure) of a
-// per-merge K x K column-major buffer starting at Sws + soff[m].
+// per-merge K x K column-major buffer starting at Sws + soff[m].  alpha (optional)
+// receives the norms as k_alpha forms them.
 __global__ void k_build_S(LevelView lv, const double *__restrict__ dl,
                           const double *__restrict__ difl, const double *__restrict__ difr,
                           const double *__restrict__ zhat, const int *__restrict__ grp,
-                          const long long *__restrict__ soff, double *__restrict__ Sws) {
+                          const long long *__restrict__ soff, double *__restrict__ Sws,
+                          double *__restrict__ alpha) {
   const int lane = threadIdx.x & 31;
   const int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (r >= __ldg(lv.rootoff + lv.P)) return;
@@ -594,11 +596,17 @@ __global__ void k_build_S(LevelView lv, const double *__restrict__ dl,
   const int s = __ldg(lv.s + m);
   const int K = __ldg(lv.K + m);
   double *S = Sws + __ldg(soff + m) + (long long)j * K;
+  PoleDiff P{dl + s, difl + s, difr + s};
   if (K == 1) {
-    if (lane == 0) S[0] = 1.0;
+    if (lane == 0) {
+      S[0] = 1.0;
+      if (alpha) {
+        const double w = __ldg(zhat + s) * rcp_nr(P.fd(0, 0));
+        alpha[s] = 1.0 / sqrt(w * w);
+      }
+    }
     return;
   }
-  PoleDiff P{dl + s, difl + s, difr + s};
   double acc = 0.0;
   for (int i = lane; i < K; i += HSS_WARP) {
     const double w = __ldg(zhat + s + i) * rcp_nr(P.fd(i, j));
@@ -607,6 +615,7 @@ __global__ void k_build_S(LevelView lv, const double *__restrict__ dl,
   }
   acc = warp_sum(acc);
   const double a = 1.0 / sqrt(acc);
+  if (alpha && lane == 0) alpha[s + j] = a;
   __syncwarp();
   for (int i = lane; i < K; i += HSS_WARP) {
     const int g = __ldg(grp + s + i);
@@ -1091,10 +1100,10 @@ void launch_alpha(const LevelView &lv, int total, const double *dl, const double
 }
 void launch_build_S(const LevelView &lv, int total, const double *dl, const double *difl,
                     const double *difr, const double *zhat, const int *grp,
-                    const long long *soff, double *Sws, cudaStream_t st) {
+                    const long long *soff, double *Sws, cudaStream_t st, double *alpha) {
   if (total <= 0) return;
   const int tb = root_block((long long)total * 32);
-  k_build_S<<<warp_grid(total, tb), tb, 0, st>>>(lv, dl, difl, difr, zhat, grp, soff, Sws);
+  k_build_S<<<warp_grid(total, tb), tb, 0, st>>>(lv, dl, difl, difr, zhat, grp, soff, Sws, alpha);
 }
 void launch_cauchy_eig(int K, const double *F, const double *u, const double *v,
                        const double *difl, const double *difr, double *C, cudaStream_t st, bool sq) {
