@@ -1054,12 +1054,18 @@ __global__ void k_scale(int n, double *x, double a) {
 // HSS products (DHSSVCS), sigma back to scale and the new ascending order.
 // hout: the prepare's 5 ints per merge (pinned); mpos: positions per merge
 // (the arrow's size, the pole first); mN / mM: rows of U / V in its window
-// [ms, ms + mN) / [ms, ms + mM); dms / dpos: ms and mpos on the device.
+// [ms, ms + mN) / [ms, ms + mM); dms / dpos: ms and mpos on the device.  sp (optional): the columns'
+// supports and the merges' row windows, which the dense merges then work on.
+struct SvdSupports {
+  int2 *U, *V;           // per slot
+  const int2 *winU, *winV;  // per merge (host)
+};
 static void svd_merge_tail(Ctx &c, const std::vector<int> &ms, const std::vector<int> &mpos,
                            const std::vector<int> &mN, const std::vector<int> &mM,
                            const int *dms, const int *dpos, const int *hout, const double *dnrm,
                            double *U, double *V, long long ld, double *Dp, int *perm,
-                           LevelArrays &L, int *status, cudaStream_t st) {
+                           LevelArrays &L, int *status, cudaStream_t st,
+                           const SvdSupports *sp = nullptr) {
   const int P = (int)ms.size();
   const int maxPos = *std::max_element(mpos.begin(), mpos.end());
   std::vector<int> aK(P), aoff(P + 1, 0), gs, gN, gM, gng;
@@ -1085,8 +1091,13 @@ static void svd_merge_tail(Ctx &c, const std::vector<int> &ms, const std::vector
         *g4 = buf<int>(c, "sg_g", G);
     h2d(g1, gs, st); h2d(g2, gN, st); h2d(g3, gM, st); h2d(g4, gng, st);
     stage_begin(HSS_ST_GIVENS, st);
-    launch_givens(G, maxNg, g1, g2, g4, L.w, U, ld, st);
-    launch_givens(G, maxMg, g1, g3, g4, L.w, V, ld, st);
+    if (sp) {
+      launch_widen(G, maxNg, g1, g4, L.w, U, ld, sp->U, st);
+      launch_widen(G, maxMg, g1, g4, L.w, V, ld, sp->V, st);
+      c.launches += 2;
+    }
+    launch_givens(G, maxNg, g1, g2, g4, L.w, U, ld, st, nullptr, 0, 0, sp ? sp->U : nullptr);
+    launch_givens(G, maxMg, g1, g3, g4, L.w, V, ld, st, nullptr, 0, 0, sp ? sp->V : nullptr);
     stage_end(HSS_ST_GIVENS, st, 0, 0.0);
     c.launches += 2;
   }
@@ -1125,7 +1136,7 @@ static void svd_merge_tail(Ctx &c, const std::vector<int> &ms, const std::vector
   stage_end(HSS_ST_LOWNER, st, 40LL * total, 8.0 * k2);
   c.launches += 2;
   // ---- dense merges (K < bsmlz): K x K U / V blocks, batched GEMMs
-  std::vector<int> ds_, dN_, dM_, dK_, doff_(1, 0);
+  std::vector<int> ds_, dN_, dM_, rU_, rV_, dK_, doff_(1, 0);  // rU_ / rV_: first rows of U / V
   std::vector<long long> qU, qV, bo;
   long long totU = 0, totV = 0, totB = 0;
   int maxNd = 1, maxMd = 1;
@@ -1133,21 +1144,26 @@ static void svd_merge_tail(Ctx &c, const std::vector<int> &ms, const std::vector
   for (int m = 0; m < P; ++m) {
     const int K = aK[m];
     if (K >= c.cfg.bsmlz) { hsel.push_back(m); continue; }
-    ds_.push_back(ms[m]); dN_.push_back(mN[m]); dM_.push_back(mM[m]); dK_.push_back(K);
+    const int r0U = sp ? sp->winU[m].x : ms[m], nU = sp ? sp->winU[m].y - r0U : mN[m];
+    const int r0V = sp ? sp->winV[m].x : ms[m], nV = sp ? sp->winV[m].y - r0V : mM[m];
+    ds_.push_back(ms[m]); dN_.push_back(nU); dM_.push_back(nV); dK_.push_back(K);
+    rU_.push_back(r0U); rV_.push_back(r0V);
     doff_.push_back(doff_.back() + K);
-    qU.push_back(totU); totU += (long long)mN[m] * K;
-    qV.push_back(totV); totV += (long long)mM[m] * K;
+    qU.push_back(totU); totU += (long long)nU * K;
+    qV.push_back(totV); totV += (long long)nV * K;
     bo.push_back(totB); totB += (long long)K * K;
-    maxNd = std::max(maxNd, mN[m]); maxMd = std::max(maxMd, mM[m]);
+    maxNd = std::max(maxNd, nU); maxMd = std::max(maxMd, nV);
   }
   const int PD = (int)ds_.size();
   if (PD > 0) {
     int *xs = buf<int>(c, "svd_s", PD), *xN = buf<int>(c, "svd_N", PD), *xM = buf<int>(c, "svd_M", PD),
-        *xK = buf<int>(c, "svd_K", PD), *xoff = buf<int>(c, "svd_off", PD + 1);
+        *xK = buf<int>(c, "svd_K", PD), *xoff = buf<int>(c, "svd_off", PD + 1),
+        *xrU = buf<int>(c, "svd_rU", PD), *xrV = buf<int>(c, "svd_rV", PD);
     long long *dqU = buf<long long>(c, "sv_qU", PD), *dqV = buf<long long>(c, "sv_qV", PD),
               *dbo = buf<long long>(c, "sv_bo", PD);
     h2d(xs, ds_, st); h2d(xN, dN_, st); h2d(xM, dM_, st); h2d(xK, dK_, st); h2d(xoff, doff_, st);
-    h2d(dqU, qU, st); h2d(dqV, qV, st); h2d(dbo, bo, st);
+    h2d(dqU, qU, st); h2d(dqV, qV, st); h2d(dbo, bo, st); h2d(xrU, rU_, st); h2d(xrV, rV_, st);
+    int2 *sU = sp ? sp->U : nullptr, *sV = sp ? sp->V : nullptr;
     LevelView dv{xs, xK, vr, xoff, PD};
     const int dtot = doff_.back();
     double *Ub = buf<double>(c, "sv_Ub", totB), *Vb = buf<double>(c, "sv_Vb", totB);
@@ -1157,8 +1173,8 @@ static void svd_merge_tail(Ctx &c, const std::vector<int> &ms, const std::vector
     double *U2 = buf<double>(c, "sv_U2", totU), *TU = buf<double>(c, "sv_TU", totU);
     double *V2 = buf<double>(c, "sv_V2", totV), *TV = buf<double>(c, "sv_TV", totV);
     stage_begin(HSS_ST_GATHER, st);
-    launch_gather(PD, dtot, maxNd, xs, xN, xoff, L.w.ndslot, nullptr, dqU, U, ld, U2, st);
-    launch_gather(PD, dtot, maxMd, xs, xM, xoff, L.w.ndslot, nullptr, dqV, V, ld, V2, st);
+    launch_gather(PD, dtot, maxNd, xs, xN, xoff, L.w.ndslot, nullptr, dqU, U, ld, U2, st, sU, xrU);
+    launch_gather(PD, dtot, maxMd, xs, xM, xoff, L.w.ndslot, nullptr, dqV, V, ld, V2, st, sV, xrV);
     stage_end(HSS_ST_GATHER, st, 16LL * (totU + totV), 0.0);
     std::vector<GemmDesc> probs;
     int tiles = 0;
@@ -1177,8 +1193,8 @@ static void svd_merge_tail(Ctx &c, const std::vector<int> &ms, const std::vector
     launch_gemm(probs, c.cfg.precision, st);
     stage_end(HSS_ST_GEMM, st, gb, fl);
     stage_begin(HSS_ST_SCATTER, st);
-    launch_scatter(PD, dtot, maxNd, xs, xN, xoff, L.w.ndslot, dqU, TU, U, ld, st);
-    launch_scatter(PD, dtot, maxMd, xs, xM, xoff, L.w.ndslot, dqV, TV, V, ld, st);
+    launch_scatter(PD, dtot, maxNd, xs, xN, xoff, L.w.ndslot, dqU, TU, U, ld, st, sU, xrU);
+    launch_scatter(PD, dtot, maxMd, xs, xM, xoff, L.w.ndslot, dqV, TV, V, ld, st, sV, xrV);
     stage_end(HSS_ST_SCATTER, st, 16LL * (totU + totV), 0.0);
     c.launches += 6;
   }
@@ -1190,6 +1206,7 @@ static void svd_merge_tail(Ctx &c, const std::vector<int> &ms, const std::vector
     h.dl = L.w.dl + h.s; h.difl = L.difl + h.s; h.difr = L.difr + h.s; h.zhat = L.zhat + h.s;
     h.ndslot = L.w.ndslot + h.s;
     h.U = U; h.V = V; h.ld = ld;
+    if (sp) { h.supU = sp->U; h.supV = sp->V; }
     int rank = 0;
     c.launches += svd_hss_merge(h, &rank, st);
     c.stats.n_hss_merges++;
@@ -1210,7 +1227,8 @@ static void svd_merge_tail(Ctx &c, const std::vector<int> &ms, const std::vector
 static void run_svd_merges(Ctx &c, const std::vector<int> &ms, const std::vector<int> &mnl,
                            const std::vector<int> &mnr, const std::vector<int> &msq,
                            const double *d, const double *e, double *U, double *V, long long ld,
-                           double *Dp, int *perm, LevelArrays &L, int *status, cudaStream_t st) {
+                           double *Dp, int *perm, LevelArrays &L, int *status, int2 *supU,
+                           int2 *supV, cudaStream_t st) {
   const int P = (int)ms.size();
   if (P == 0) return;
   std::vector<int> mN(P), mM(P);
@@ -1219,21 +1237,25 @@ static void run_svd_merges(Ctx &c, const std::vector<int> &ms, const std::vector
   int *dms = buf<int>(c, "sv_s", P), *dnl = buf<int>(c, "sv_nl", P), *dnr = buf<int>(c, "sv_nr", P),
       *dsq = buf<int>(c, "sv_sq", P), *dN = buf<int>(c, "sv_N", P);
   h2d(dms, ms, st); h2d(dnl, mnl, st); h2d(dnr, mnr, st); h2d(dsq, msq, st); h2d(dN, mN, st);
-  int *dout = buf<int>(c, "g_out", 5 * P);
+  // per merge: the row windows of U and V, then five counts
+  int2 *dwin = buf<int2>(c, "g_out", 2 * (size_t)P + ((size_t)5 * P + 1) / 2);
+  int *dout = (int *)(dwin + 2 * (size_t)P);
   double *dnrm = buf<double>(c, "sv_nrm", P);
   stage_begin(HSS_ST_PREPARE, st);
   launch_svd_prepare(P, maxN, dms, dnl, dnr, dsq, d, e, U, ld, V, ld, Dp, perm, L.w, dout, dnrm,
-                     st);
+                     supU, supV, dwin, dwin + P, st);
   {
     long long nn = 0;
     for (int x : mN) nn += x;
     stage_end(HSS_ST_PREPARE, st, 64 * nn, 0.0);
   }
   c.launches++;
-  int *hout = (int *)pinned(c, (size_t)P * 5 * sizeof(int));
-  CK(cudaMemcpyAsync(hout, dout, (size_t)P * 5 * sizeof(int), cudaMemcpyDeviceToHost, st));
+  const int2 *hwin = (const int2 *)pinned(c, (size_t)P * 9 * sizeof(int));
+  CK(cudaMemcpyAsync((void *)hwin, dwin, (size_t)P * 9 * sizeof(int), cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
-  svd_merge_tail(c, ms, mN, mN, mM, dms, dN, hout, dnrm, U, V, ld, Dp, perm, L, status, st);
+  const SvdSupports sp{supU, supV, hwin, hwin + P};
+  svd_merge_tail(c, ms, mN, mN, mM, dms, dN, (const int *)(hwin + 2 * (size_t)P), dnrm, U, V, ld, Dp,
+                 perm, L, status, st, &sp);
 }
 
 // MDBDSDC('U', COMPQ) (SRC/mdbdsdc.f90:1) of the upper bidiagonal (d, e) in
@@ -1272,8 +1294,8 @@ static int svd_core(Ctx &c, int n, const double *d, const double *e, double *Uo,
   int *status = buf<int>(c, "status", 8);
   CK(cudaMemsetAsync(status, 0, 8 * sizeof(int), st));
   CK(cudaMemsetAsync(gemm_flag(c), 0, sizeof(int), st));
-  CK(cudaMemsetAsync(U, 0, sizeof(double) * (size_t)n * n, st));
-  CK(cudaMemsetAsync(V, 0, sizeof(double) * (size_t)n * n, st));
+  // no zero fill of U and V: every column is tracked with the rows it holds data on
+  int2 *supU = buf<int2>(c, "sup", n), *supV = buf<int2>(c, "sv_sup", n);
   {
     const std::vector<Node> &leaves = lv.back();
     std::vector<int> ls, lz, lq;
@@ -1288,7 +1310,7 @@ static int svd_core(Ctx &c, int n, const double *d, const double *e, double *Uo,
     int *dls = buf<int>(c, "leaf_s", nl), *dlz = buf<int>(c, "leaf_z", nl), *dlq = buf<int>(c, "leaf_q", nl);
     h2d(dls, ls, st); h2d(dlz, lz, st); h2d(dlq, lq, st);
     stage_begin(HSS_ST_LEAF, st);
-    launch_svd_leaf(nl, dls, dlz, dlq, rmax, d, e, U, n, V, n, Dp, perm, status, st);
+    launch_svd_leaf(nl, dls, dlz, dlq, rmax, d, e, U, n, V, n, Dp, perm, status, supU, supV, st);
     stage_end(HSS_ST_LEAF, st, 16LL * n * smlsiz, flops);
     c.launches++;
   }
@@ -1302,17 +1324,17 @@ static int svd_core(Ctx &c, int n, const double *d, const double *e, double *Uo,
       }
       c.stats.n_levels++;
       if (c.cfg.batched) {
-        run_svd_merges(c, ms, mnl, mnr, msq, d, e, U, V, n, Dp, perm, L, status, st);
+        run_svd_merges(c, ms, mnl, mnr, msq, d, e, U, V, n, Dp, perm, L, status, supU, supV, st);
       } else {
         for (size_t m = 0; m < ms.size(); ++m)
           run_svd_merges(c, {ms[m]}, {mnl[m]}, {mnr[m]}, {msq[m]}, d, e, U, V, n, Dp, perm, L,
-                         status, st);
+                         status, supU, supV, st);
       }
     }
   }
   stage_begin(HSS_ST_FINAL, st);
-  launch_svd_outputs(n, perm, Dp, U, n, V, n, Uo, ldu, VT, ldvt, w, vectors, st);
-  stage_end(HSS_ST_FINAL, st, vectors ? 32LL * n * n : 16LL * n, 0.0);
+  launch_svd_outputs(n, perm, Dp, U, n, V, n, Uo, ldu, VT, ldvt, w, vectors, st, supU, supV);
+  stage_end(HSS_ST_FINAL, st, vectors ? 16LL * n * n : 16LL * n, 0.0);
   c.launches += 2;
   CK(cudaEventRecord(ev1, st));
   int hst[8] = {0, 0, 0, 0, 0, 0, 0, 0};

@@ -1029,7 +1029,8 @@ int svd_hss_merge(const SvdHssArgs &a, int *rank, cudaStream_t st) {
     double *Q = side == 0 ? a.V : a.U;
     std::vector<int> hv{a.s, nr, 0, a.K};
     int *dv = up(side == 0 ? "svh_gv0" : "svh_gv1", hv, st);
-    launch_gather(1, a.K, nr, dv, dv + 1, dv + 2, a.ndslot - a.s, nullptr, boff, Q, a.ld, X, st);
+    int2 *sup = side == 0 ? a.supV : a.supU;
+    launch_gather(1, a.K, nr, dv, dv + 1, dv + 2, a.ndslot - a.s, nullptr, boff, Q, a.ld, X, st, sup);
     const double *u = side == 0 ? a.zhat : ud;
     const double *v = side == 0 ? alpha : beta;
     HssPlan pl;
@@ -1049,7 +1050,7 @@ int svd_hss_merge(const SvdHssArgs &a, int *rank, cudaStream_t st) {
       *rank = a.K;
     }
     if (side == 1) launch_svd_rank1(nr, a.K, X, nr, beta, T, nr, st);
-    launch_scatter(1, a.K, nr, dv, dv + 1, dv + 2, a.ndslot - a.s, boff, T, Q, a.ld, st);
+    launch_scatter(1, a.K, nr, dv, dv + 1, dv + 2, a.ndslot - a.s, boff, T, Q, a.ld, st, sup);
     launches += 4;
   }
   return launches + 1;

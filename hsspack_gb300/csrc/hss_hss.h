@@ -43,6 +43,7 @@ struct SvdHssArgs {
   const int *ndslot;
   double *U, *V;
   long long ld;
+  int2 *supU = nullptr, *supV = nullptr;  // rows each column holds data on (nullptr: all)
 };
 int svd_hss_merge(const SvdHssArgs &a, int *rank, cudaStream_t st);
 

@@ -184,13 +184,17 @@ void launch_band_zupdate(const LevelView &lv, int total, const double *dl, const
                          cudaStream_t st);
 
 // svd.cu: bidiagonal SVD divide and conquer
+// supU / supV: per slot the rows its U / V column holds data on (zero elsewhere)
 void launch_svd_leaf(int nleaf, const int *lstart, const int *lsize, const int *lsqre, int rmax,
                      const double *d, const double *e, double *U, long long ldu, double *V,
-                     long long ldv, double *Dp, int *perm, int *status, cudaStream_t st);
+                     long long ldv, double *Dp, int *perm, int *status, int2 *supU, int2 *supV,
+                     cudaStream_t st);
+// winU / winV: per merge the rows on which the columns it takes up hold data
 void launch_svd_prepare(int P, int maxn, const int *ms, const int *mnl, const int *mnr,
                         const int *msq, const double *d, const double *e, double *U,
                         long long ldu, double *V, long long ldv, const double *Dp, const int *perm,
-                        const LevelScratch &w, int *out, double *onrm, cudaStream_t st);
+                        const LevelScratch &w, int *out, double *onrm, int2 *supU, int2 *supV,
+                        int2 *winU, int2 *winV, cudaStream_t st);
 // U / V blocks (K x K per merge at boff); sigma rescaled by onrm
 void launch_svd_vectors(const LevelView &lv, int total, const double *dl, const double *difl,
                         const double *difr, const double *zhat, const long long *boff, double *Ub,
@@ -206,7 +210,8 @@ void launch_svd_rank1(int nrows, int K, const double *X, long long ldx, const do
 // outputs in descending order: Uo (ldu), VT (ldvt), w; only w if !vectors
 void launch_svd_outputs(int n, const int *perm, const double *Dp, const double *Uq,
                         long long ldq, const double *V, long long ldv, double *Uo, long long ldu,
-                        double *VT, long long ldvt, double *w, bool vectors, cudaStream_t st);
+                        double *VT, long long ldvt, double *w, bool vectors, cudaStream_t st,
+                        const int2 *supU = nullptr, const int2 *supV = nullptr);
 void launch_rows_rotate_back(int n, int ncols, const double *cs, const double *sn, double *A,
                              long long lda, cudaStream_t st);
 

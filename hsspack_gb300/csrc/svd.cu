@@ -23,6 +23,8 @@
 #include "hss_leaf.cuh"
 #include "hss_svdprep.cuh"
 
+#include <climits>
+
 namespace hss {
 
 constexpr int SVD_LEAF_MAX = 32;
@@ -71,7 +73,7 @@ k_svd_leaf(int nleaf, const int *__restrict__ lstart, const int *__restrict__ ls
            const int *__restrict__ lsqre, int rmax, const double *__restrict__ d,
            const double *__restrict__ e, double *__restrict__ U, long long ldu,
            double *__restrict__ V, long long ldv, double *__restrict__ Dp, int *__restrict__ perm,
-           int *__restrict__ status) {
+           int *__restrict__ status, int2 *__restrict__ supU, int2 *__restrict__ supV) {
   extern __shared__ double lsm[];
   constexpr int LPW = 32 / G;
   const int lane = threadIdx.x, q = lane / G, g0 = lane % G;
@@ -291,7 +293,10 @@ k_svd_leaf(int nleaf, const int *__restrict__ lstart, const int *__restrict__ ls
   for (int i = g0; i < r; i += G) {
     Dp[a + rk[i * 64]] = D[i * 32];
     perm[a + i] = a + i;
+    supU[a + i] = make_int2(a, a + r);  // rows the columns are written on
+    supV[a + i] = make_int2(a, a + c);
   }
+  if (sq && g0 == 0) supV[a + r] = make_int2(a, a + c);
   if (bad) atomicMax(status, HSS_LEAF_NOCONV);
   // write the blocks: lanes over the entries, one leaf at a time (coalesced)
   const double *Uw = lsm + (size_t)rmax * 64, *Vw = Uw + (size_t)rmax * R * 32;
@@ -329,14 +334,23 @@ k_svd_prepare(int P, const int *__restrict__ ms, const int *__restrict__ mnl,
               const double *__restrict__ dB, const double *__restrict__ eB, double *__restrict__ U,
               long long ldu, double *__restrict__ V, long long ldv, const double *__restrict__ Dp,
               const int *__restrict__ perm, LevelScratch w, int *__restrict__ out,
-              double *__restrict__ onrm) {
+              double *__restrict__ onrm, int2 *__restrict__ supU, int2 *__restrict__ supV,
+              int2 *__restrict__ winU, int2 *__restrict__ winV) {
   const int m = blockIdx.x;
   if (m >= P) return;
   const int s = ms[m], nl = mnl[m], nr = mnr[m], sqre = msq[m];
   const int N = nl + 1 + nr, c = s + nl;
   const int tid = threadIdx.x;
   const double alpha = dB[c], beta = eB[c];
-  if (tid == 0) U[(long long)c * ldu + c] = 1.0;  // the center row's left vector e_c
+  if (tid == 0) {  // the center row's left vector e_c
+    U[(long long)c * ldu + c] = 1.0;
+    supU[c] = make_int2(c, c + 1);
+  }
+  // V(row, slot): zero outside the rows the column holds data on
+  auto vat = [&](int slot, int row) -> double {
+    const int2 r = supV[slot];
+    return row >= r.x && row < r.y ? V[(long long)slot * ldv + row] : 0.0;
+  };
   // ---- scale (MDLASD1) and merge the children's ascending lists (DLAMRG) into
   //      positions 1 .. N-1; position 0 is the center
   double dm = fmax(fabs(alpha), fabs(beta));
@@ -371,12 +385,12 @@ k_svd_prepare(int P, const int *__restrict__ ms, const int *__restrict__ mnl,
   for (int i = tid + 1; i < N; i += MT) {
     const int slot = w.srt[s + i];
     const bool left = slot < c;
-    w.zs[s + i] = left ? an * V[(long long)slot * ldv + c] : bn * V[(long long)slot * ldv + c + 1];
+    w.zs[s + i] = left ? an * vat(slot, c) : bn * vat(slot, c + 1);
     w.typ[s + i] = left ? 1 : 2;
   }
   if (tid == 0) { w.srt[s] = c; w.ds[s] = 0.0; w.typ[s] = 0; }
-  const double z1 = an * V[(long long)c * ldv + c];
-  const double zM = sqre ? bn * V[(long long)(s + N) * ldv + c + 1] : 0.0;
+  const double z1 = an * vat(c, c);
+  const double zM = sqre ? bn * vat(s + N, c + 1) : 0.0;
   __syncthreads();
   const double dmaxn = N > 1 ? w.ds[s + N - 1] : 0.0;
   const double tol = 8.0 * HSS_EPS * fmax(dmaxn, fmax(fabs(an), fabs(bn)));
@@ -390,12 +404,17 @@ k_svd_prepare(int P, const int *__restrict__ ms, const int *__restrict__ mnl,
     if (zz1 <= tol) zz1 = tol;
     else { cg1 = z1 / zz1; sg1 = zM / zz1; }
     // V(:, c) <- cg V(:, c) + sg V(:, s+N);  V(:, s+N) <- -sg V(:, c) + cg V(:, s+N)
-    for (int i = tid; i < N + 1; i += MT) {
-      const long long rr = s + i;
-      const double vc = V[(long long)c * ldv + rr], vn = V[(long long)(s + N) * ldv + rr];
+    // on the union of their rows
+    const int2 rc = supV[c], rn = supV[s + N];
+    const int2 u = make_int2(min(rc.x, rn.x), max(rc.y, rn.y));
+    __syncthreads();
+    for (int rr = u.x + tid; rr < u.y; rr += MT) {
+      const double vc = rr >= rc.x && rr < rc.y ? V[(long long)c * ldv + rr] : 0.0;
+      const double vn = rr >= rn.x && rr < rn.y ? V[(long long)(s + N) * ldv + rr] : 0.0;
       V[(long long)c * ldv + rr] = cg1 * vc + sg1 * vn;
       V[(long long)(s + N) * ldv + rr] = -sg1 * vc + cg1 * vn;
     }
+    if (tid == 0) { supV[c] = u; supV[s + N] = u; }
   } else {
     zz1 = fabs(z1) <= tol ? tol : z1;
   }
@@ -404,6 +423,27 @@ k_svd_prepare(int P, const int *__restrict__ ms, const int *__restrict__ mnl,
   // ---- compact: non-deflated (position 0 first) and the two deflated lists
   svd_prep_compact<MT>(s, N, tol, ng, Dp, w, out + 5 * m);
   if (tid == 0) onrm[m] = nrm;
+  // ---- row windows: the union of the supports of the columns taken up or rotated
+  __shared__ int s_win[4];
+  if (tid < 4) s_win[tid] = tid & 1 ? 0 : INT_MAX;
+  __syncthreads();
+  int2 wu = make_int2(INT_MAX, 0), wv = wu;
+  for (int i = tid; i < N; i += MT) {
+    if (w.typ[s + i] == 4) continue;
+    const int slot = w.srt[s + i];
+    const int2 a = supU[slot], b = supV[slot];
+    wu = make_int2(min(wu.x, a.x), max(wu.y, a.y));
+    wv = make_int2(min(wv.x, b.x), max(wv.y, b.y));
+  }
+  if (wu.y > 0) {
+    atomicMin(&s_win[0], wu.x); atomicMax(&s_win[1], wu.y);
+    atomicMin(&s_win[2], wv.x); atomicMax(&s_win[3], wv.y);
+  }
+  __syncthreads();
+  if (tid == 0) {
+    winU[m] = make_int2(s_win[0], s_win[1]);
+    winV[m] = make_int2(s_win[2], s_win[3]);
+  }
 }
 
 // ------------------------------------------------------- vector blocks ----
@@ -504,13 +544,19 @@ __global__ void k_svd_unscale(LevelView lv, const double *__restrict__ onrm,
 
 // VT(i, :) = V(:, perm(n-1-i))^T (descending singular values): 32 x 32 tiles
 // through shared memory so both the reads of V and the writes of VT coalesce.
+// sup (optional): rows each column holds data on (zero elsewhere).
 __global__ void k_svd_vt(int n, const int *__restrict__ perm, const double *__restrict__ V,
-                         long long ldv, double *__restrict__ VT, long long ldvt) {
+                         long long ldv, double *__restrict__ VT, long long ldvt,
+                         const int2 *__restrict__ sup) {
   __shared__ double tile[32][33];
   const int i0 = blockIdx.x * 32, j0 = blockIdx.y * 32;  // rows i of VT, columns j
   for (int k = threadIdx.y; k < 32; k += blockDim.y) {
     const int i = i0 + k, j = j0 + threadIdx.x;
-    if (i < n && j < n) tile[k][threadIdx.x] = V[(long long)perm[n - 1 - i] * ldv + j];
+    if (i < n && j < n) {
+      const int p = perm[n - 1 - i];
+      const int2 r = sup ? sup[p] : make_int2(0, n);
+      tile[k][threadIdx.x] = j >= r.x && j < r.y ? V[(long long)p * ldv + j] : 0.0;
+    }
   }
   __syncthreads();
   for (int k = threadIdx.y; k < 32; k += blockDim.y) {
@@ -522,11 +568,13 @@ __global__ void k_svd_vt(int n, const int *__restrict__ perm, const double *__re
 // U(:, i) = Uq(:, perm(n-1-i)), w(i) = Dp(perm(n-1-i)) (descending).
 __global__ void k_svd_u(int n, const int *__restrict__ perm, const double *__restrict__ Dp,
                         const double *__restrict__ Uq, long long ldq, double *__restrict__ Uo,
-                        long long ldu, double *__restrict__ w) {
+                        long long ldu, double *__restrict__ w, const int2 *__restrict__ sup) {
   const int col = blockIdx.x;
   if (col >= n) return;
   const long long p = perm[n - 1 - col];
-  for (int i = threadIdx.x; i < n; i += blockDim.x) Uo[(long long)col * ldu + i] = Uq[p * ldq + i];
+  const int2 r = sup ? sup[p] : make_int2(0, n);
+  for (int i = threadIdx.x; i < n; i += blockDim.x)
+    Uo[(long long)col * ldu + i] = i >= r.x && i < r.y ? Uq[p * ldq + i] : 0.0;
   if (threadIdx.x == 0) w[col] = Dp[p];
 }
 
@@ -564,7 +612,7 @@ template <int G, int R>
 static void svd_leaf_launch(int nleaf, const int *lstart, const int *lsize, const int *lsqre,
                             int rmax, const double *d, const double *e, double *U, long long ldu,
                             double *V, long long ldv, double *Dp, int *perm, int *status,
-                            cudaStream_t st) {
+                            int2 *supU, int2 *supV, cudaStream_t st) {
   const size_t smem = svd_leaf_smem(rmax, R);
   static size_t attr = 48 * 1024;
   if (smem > attr) {
@@ -572,19 +620,22 @@ static void svd_leaf_launch(int nleaf, const int *lstart, const int *lsize, cons
     attr = smem;
   }
   k_svd_leaf<G, R><<<(nleaf * G + 31) / 32, 32, smem, st>>>(nleaf, lstart, lsize, lsqre, rmax, d, e,
-                                                            U, ldu, V, ldv, Dp, perm, status);
+                                                            U, ldu, V, ldv, Dp, perm, status,
+                                                            supU, supV);
 }
 
 void launch_svd_leaf(int nleaf, const int *lstart, const int *lsize, const int *lsqre, int rmax,
                      const double *d, const double *e, double *U, long long ldu, double *V,
-                     long long ldv, double *Dp, int *perm, int *status, cudaStream_t st) {
+                     long long ldv, double *Dp, int *perm, int *status, int2 *supU, int2 *supV,
+                     cudaStream_t st) {
   if (nleaf <= 0) return;
   rmax = std::max(1, std::min(rmax, SVD_LEAF_MAX));
   // two blocks of vectors (shared memory): at most 8 rows of each per lane
   int G = leaf_lanes(nleaf, rmax + 1);
   while (G < 32 && (G < 2 || (rmax + G) / G > 8)) G *= 2;
   const int R = (rmax + G) / G;  // ceil((rmax + 1) / G)
-#define SVDL_ARGS nleaf, lstart, lsize, lsqre, rmax, d, e, U, ldu, V, ldv, Dp, perm, status, st
+#define SVDL_ARGS \
+  nleaf, lstart, lsize, lsqre, rmax, d, e, U, ldu, V, ldv, Dp, perm, status, supU, supV, st
 #define SVDL_TRY(g, r) if (G == g && R <= r) return svd_leaf_launch<g, r>(SVDL_ARGS)
   SVDL_TRY(2, 4);
   SVDL_TRY(2, 8);
@@ -607,12 +658,13 @@ static int svd_threads(int maxn) {
 void launch_svd_prepare(int P, int maxn, const int *ms, const int *mnl, const int *mnr,
                         const int *msq, const double *d, const double *e, double *U,
                         long long ldu, double *V, long long ldv, const double *Dp, const int *perm,
-                        const LevelScratch &w, int *out, double *onrm, cudaStream_t st) {
+                        const LevelScratch &w, int *out, double *onrm, int2 *supU, int2 *supV,
+                        int2 *winU, int2 *winV, cudaStream_t st) {
   if (P <= 0) return;
 #define SVDP_CASE(T)                                                                        \
   case T:                                                                                  \
     k_svd_prepare<T><<<P, T, 0, st>>>(P, ms, mnl, mnr, msq, d, e, U, ldu, V, ldv, Dp, perm, \
-                                      w, out, onrm);                                       \
+                                      w, out, onrm, supU, supV, winU, winV);               \
     break;
   switch (svd_threads(maxn)) {
     SVDP_CASE(64)
@@ -638,12 +690,13 @@ void launch_svd_unscale(const LevelView &lv, int total, const double *onrm, doub
 
 void launch_svd_outputs(int n, const int *perm, const double *Dp, const double *Uq,
                         long long ldq, const double *V, long long ldv, double *Uo, long long ldu,
-                        double *VT, long long ldvt, double *w, bool vectors, cudaStream_t st) {
+                        double *VT, long long ldvt, double *w, bool vectors, cudaStream_t st,
+                        const int2 *supU, const int2 *supV) {
   if (n <= 0) return;
   if (vectors) {
-    k_svd_u<<<n, 256, 0, st>>>(n, perm, Dp, Uq, ldq, Uo, ldu, w);
+    k_svd_u<<<n, 256, 0, st>>>(n, perm, Dp, Uq, ldq, Uo, ldu, w, supU);
     dim3 g((n + 31) / 32, (n + 31) / 32);
-    k_svd_vt<<<g, dim3(32, 8), 0, st>>>(n, perm, V, ldv, VT, ldvt);
+    k_svd_vt<<<g, dim3(32, 8), 0, st>>>(n, perm, V, ldv, VT, ldvt, supV);
   } else {
     k_svd_w<<<(n + 255) / 256, 256, 0, st>>>(n, perm, Dp, w);
   }

@@ -50,3 +50,23 @@ def test_tridiagonal_windows(kind, n, cfg):
     if n <= 2600:
         T = torch.diag(dd) + torch.diag(ee[:n - 1], 1) + torch.diag(ee[:n - 1], -1)
         assert float((w - torch.linalg.eigvalsh(T)).abs().max()) <= 1e-13 * tn
+
+
+@pytest.mark.parametrize("kind", ["random", "glued", "mixed"])
+@pytest.mark.parametrize("lower", [False, True])
+@pytest.mark.parametrize("n,cfg", [(700, dict()), (2500, dict(smlsiz=8, precision=1, predictor=2)),
+                                   (1500, dict(bsmlz=60, hss_leaf=64, tol=1e-14))])
+def test_bidiagonal_windows(kind, lower, n, cfg):
+    d, e = _tridiagonal(kind, n, np.random.default_rng(n + 1))
+    d = np.abs(d) + 0.05
+    old = hp.set_config(**cfg)
+    try:
+        s, U, VT = hp.svd_bidiagonal(d, e, lower=lower)
+    finally:
+        hp.restore_config(old)
+    B = np.diag(d) + np.diag(e, -1 if lower else 1)
+    bn = float(np.abs(d).max() + np.abs(e).max())
+    assert np.abs(s - np.linalg.svd(B, compute_uv=False)).max() <= 1e-13 * bn
+    assert np.linalg.norm(B @ VT.T - U * s) / (n * bn) <= 1e-12
+    assert np.linalg.norm(U.T @ U - np.eye(n)) / n <= 1e-12
+    assert np.linalg.norm(VT @ VT.T - np.eye(n)) / n <= 1e-12
