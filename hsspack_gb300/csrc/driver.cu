@@ -504,7 +504,10 @@ static void run_merges(Ctx &c, const std::vector<int> &ms, const std::vector<int
     double *Q2 = buf<double>(c, "Q2", q2tot), *T = buf<double>(c, "T", q2tot);
     double *S = buf<double>(c, "S", stot);
     stage_begin(HSS_ST_BUILD_S, st);
-    launch_build_S(dv, dtot, L.w.dl, L.difl, L.difr, L.zhat, L.w.grp, xso, S, st,
+    // (banded updates keep one order of summation: their small z are rounding noise
+    // of earlier updates and decide signs of vectors)
+    launch_build_S(dv, dtot, L.w.dl, L.difl, L.difr, L.zhat, L.w.grp, xso, S,
+                   *std::max_element(dK_.begin(), dK_.end()), bu != nullptr, st,
                    zup && hsel.empty() ? L.alpha : nullptr);
     stage_end(HSS_ST_BUILD_S, st, 8LL * stot * 2, 0.0);
     if (zup) zupdate();

@@ -93,18 +93,24 @@ int gemm_tiles(int M, int N) { return ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
 
 // Small products (N, K <= 32: the lowest DC levels): one thread per output
 // element, the K-term dot product from L1 (a 64 x 64 tile would be mostly
-// empty).  Problem p owns outputs [eoff[p], eoff[p+1]).
+// empty).  Problem p owns outputs [eoff[p], eoff[p+1]).  A warp finds the problem
+// of its first output together and the lanes walk on from there: a search of
+// its own by every thread (17 dependent loads with a batch's 88000 problems)
+// took longer than the K <= 32 multiply-adds.
 __global__ void __launch_bounds__(256)
 k_gemm_small(int nprob, const GemmDesc *__restrict__ probs, const long long *__restrict__ eoff) {
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= eoff[nprob]) return;
-  int lo = 0, hi = nprob;
-  while (hi - lo > 1) { const int mid = (lo + hi) >> 1; if (eoff[mid] <= idx) lo = mid; else hi = mid; }
+  const long long first = idx - (threadIdx.x & 31), end = __ldg(eoff + nprob);
+  if (first >= end) return;
+  int lo = find_merge_warp(eoff, nprob, first);
+  if (idx >= end) return;
+  while (__ldg(eoff + lo + 1) <= idx) ++lo;
   const GemmDesc P = probs[lo];
-  const long long e = idx - eoff[lo];
-  const int i = (int)(e % P.M), j = (int)(e / P.M);
+  const unsigned e = (unsigned)(idx - __ldg(eoff + lo));  // below M N
+  const int j = (int)(e / (unsigned)P.M), i = (int)(e - (unsigned)j * P.M);
   const double *a = P.A + i, *b = P.B + (long long)j * P.ldb;
   double acc = 0.0;
+#pragma unroll 4
   for (int k = 0; k < P.K; ++k) acc = fma(__ldg(a + (long long)k * P.lda), __ldg(b + k), acc);
   double *c = P.C + (long long)j * P.ldc + i;
   *c = P.beta ? *c + acc : acc;

@@ -65,9 +65,10 @@ void launch_lowner(const LevelView &lv, int total, const double *dl, const doubl
 void launch_alpha(const LevelView &lv, int total, const double *dl, const double *difl,
                   const double *difr, const double *zhat, double *alpha, cudaStream_t st,
                   bool sq = false);
+// fixed: one order of summation whatever the level's sizes (alpha needs it)
 void launch_build_S(const LevelView &lv, int total, const double *dl, const double *difl,
                     const double *difr, const double *zhat, const int *grp,
-                    const long long *soff, double *Sws, cudaStream_t st,
+                    const long long *soff, double *Sws, int maxk, bool fixed, cudaStream_t st,
                     double *alpha = nullptr);
 void launch_cauchy_eig(int K, const double *F, const double *u, const double *v,
                        const double *difl, const double *difr, double *C, cudaStream_t st,

@@ -879,12 +879,6 @@ __global__ void k_givens(int P, const int *__restrict__ ms, const int *__restric
 // hundreds of thousands of blocks that copy a few dozen values each).
 constexpr int GS_SEG = 256;
 
-__device__ __forceinline__ int gs_merge(const int *__restrict__ rootoff, int P, int r) {
-  int lo = 0, hi = P;
-  while (hi - lo > 1) { int mid = (lo + hi) >> 1; if (rootoff[mid] <= r) lo = mid; else hi = mid; }
-  return lo;
-}
-
 // mr (optional): first row of each merge's columns (mn rows); ms otherwise
 __global__ void k_gather(int P, int nseg, const int *__restrict__ ms, const int *__restrict__ mn,
                          const int *__restrict__ mr, const int *__restrict__ rootoff, const int *__restrict__ ndslot,
@@ -895,7 +889,7 @@ __global__ void k_gather(int P, int nseg, const int *__restrict__ ms, const int 
   const int lane = threadIdx.x & 31;
   const int r = (int)(wg / nseg), q = (int)(wg - (long long)r * nseg);
   if (r >= rootoff[P]) return;
-  const int m = gs_merge(rootoff, P, r), j = r - rootoff[m];
+  const int m = find_merge_warp(rootoff, P, r), j = r - rootoff[m];
   const int s = ms[m], n = mn[m];
   const int i0 = q * GS_SEG, i1 = min(n, i0 + GS_SEG);
   if (i0 >= i1) return;
@@ -917,7 +911,7 @@ __global__ void k_scatter(int P, int nseg, const int *__restrict__ ms, const int
   const int lane = threadIdx.x & 31;
   const int r = (int)(wg / nseg), q = (int)(wg - (long long)r * nseg);
   if (r >= rootoff[P]) return;
-  const int m = gs_merge(rootoff, P, r), j = r - rootoff[m];
+  const int m = find_merge_warp(rootoff, P, r), j = r - rootoff[m];
   const int s = ms[m], n = mn[m];
   const int i0 = q * GS_SEG, i1 = min(n, i0 + GS_SEG);
   if (i0 >= i1) return;

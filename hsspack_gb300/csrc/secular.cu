@@ -581,45 +581,60 @@ __global__ void k_alpha(LevelView lv, const double *__restrict__ dl,
 // (LAPACK DLAED3's S, used at SRC/mdlaed1.f90:198-201): column j holds
 // z_hat_i / (d_i - lam_j) normalised to unit length.  Row i is written at
 // group position grp[s+i] (columns of Q2 grouped by block structure) of a
-// per-merge K x K column-major buffer starting at Sws + soff[m].  alpha (optional)
-// receives the norms as k_alpha forms them.
+// per-merge K x K column-major buffer starting at Sws + soff[m].  alpha (optional,
+// L = 32) receives the norms as k_alpha forms them.
+//
+// L lanes per column.  FP64-pipe bound: 8 instructions per term and lane pass,
+// plus a column's reduction and reciprocal root, which a warp pays once however
+// many columns it holds (with a warp per column the 14-root merges at the bottom
+// of a batch spent 27 of 35 instructions there).
+template <int L>
 __global__ void k_build_S(LevelView lv, const double *__restrict__ dl,
                           const double *__restrict__ difl, const double *__restrict__ difr,
                           const double *__restrict__ zhat, const int *__restrict__ grp,
                           const long long *__restrict__ soff, double *__restrict__ Sws,
                           double *__restrict__ alpha) {
-  const int lane = threadIdx.x & 31;
-  const int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (r >= __ldg(lv.rootoff + lv.P)) return;
-  const int m = find_merge(lv.rootoff, lv.P, r);
-  const int j = r - __ldg(lv.rootoff + m);
-  const int s = __ldg(lv.s + m);
-  const int K = __ldg(lv.K + m);
-  double *S = Sws + __ldg(soff + m) + (long long)j * K;
-  PoleDiff P{dl + s, difl + s, difr + s};
-  if (K == 1) {
-    if (lane == 0) {
-      S[0] = 1.0;
-      if (alpha) {
-        const double w = __ldg(zhat + s) * rcp_nr(P.fd(0, 0));
-        alpha[s] = 1.0 / sqrt(w * w);
-      }
-    }
-    return;
+  const int lane = threadIdx.x & 31, gl = lane & (L - 1);
+  const int r = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) / L);
+  const int total = __ldg(lv.rootoff + lv.P);
+  const int r0 = r - lane / L;  // the warp's first column
+  if (r0 >= total) return;
+  int m = find_merge_warp(lv.rootoff, lv.P, r0);
+  const bool valid = r < total;
+  int j = 0, s = 0, K = 0;
+  if (valid) {
+    while (__ldg(lv.rootoff + m + 1) <= r) ++m;
+    j = r - __ldg(lv.rootoff + m);
+    s = __ldg(lv.s + m);
+    K = __ldg(lv.K + m);
   }
+  double *S = Sws + (valid ? __ldg(soff + m) + (long long)j * K : 0ll);
+  PoleDiff P{dl + s, difl + s, difr + s};
   double acc = 0.0;
-  for (int i = lane; i < K; i += HSS_WARP) {
+  for (int i = gl; i < K; i += L) {
     const double w = __ldg(zhat + s + i) * rcp_nr(P.fd(i, j));
     S[__ldg(grp + s + i)] = w;
     acc += w * w;
   }
-  acc = warp_sum(acc);
-  const double a = 1.0 / sqrt(acc);
-  if (alpha && lane == 0) alpha[s + j] = a;
+  acc = group_sum<L>(acc);
+  double a;
+  if (L == 32) {
+    a = 1.0 / sqrt(acc);
+    if (alpha && valid && gl == 0) alpha[s + j] = a;
+  } else {
+    double rt;
+    const int hx = __double2hiint(acc);
+    if (hx >= 0x03f00000 && hx < 0x7bf00000) sqrt_pair(acc, rt, a);  // [2^-960, 2^960)
+    else a = 1.0 / sqrt(acc);
+  }
   __syncwarp();
-  for (int i = lane; i < K; i += HSS_WARP) {
-    const int g = __ldg(grp + s + i);
-    S[g] *= a;
+  if (K == 1) {
+    if (gl == 0) S[0] = 1.0;
+  } else {
+    for (int i = gl; i < K; i += L) {
+      const int g = __ldg(grp + s + i);
+      S[g] *= a;
+    }
   }
 }
 
@@ -1100,10 +1115,20 @@ void launch_alpha(const LevelView &lv, int total, const double *dl, const double
 }
 void launch_build_S(const LevelView &lv, int total, const double *dl, const double *difl,
                     const double *difr, const double *zhat, const int *grp,
-                    const long long *soff, double *Sws, cudaStream_t st, double *alpha) {
+                    const long long *soff, double *Sws, int maxk, bool fixed, cudaStream_t st,
+                    double *alpha) {
   if (total <= 0) return;
-  const int tb = root_block((long long)total * 32);
-  k_build_S<<<warp_grid(total, tb), tb, 0, st>>>(lv, dl, difl, difr, zhat, grp, soff, Sws, alpha);
+  // lanes per column: a group keeps at least two terms per lane, and the level at
+  // least 152 x 512 lanes (512 problems, 32 lanes at every level before: 7.2 ms, now
+  // 3.5 ms).  fixed: 32, whatever the level
+  int L = 32;
+  while (!fixed && L > 4 && (L * 2 > maxk || (long long)total * (L / 2) >= 152LL * 512)) L /= 2;
+  const int tb = root_block((long long)total * L);
+  const unsigned grid = (unsigned)(((long long)total * L + tb - 1) / tb);
+#define BS_CASE(n) \
+  case n: k_build_S<n><<<grid, tb, 0, st>>>(lv, dl, difl, difr, zhat, grp, soff, Sws, alpha); break;
+  switch (L) { BS_CASE(4) BS_CASE(8) BS_CASE(16) BS_CASE(32) }
+#undef BS_CASE
 }
 void launch_cauchy_eig(int K, const double *F, const double *u, const double *v,
                        const double *difl, const double *difr, double *C, cudaStream_t st, bool sq) {
