@@ -185,16 +185,6 @@ __device__ __forceinline__ double pole_dd(bool sq, const Pole &p, const Pole &q)
   return sq ? lin * ((p.F + p.dl) + (q.F + q.dl)) : lin;
 }
 
-// |d| as FP32 rounded towards zero by integer operations (a conversion holds the
-// FP64 pipe); 0 below FP32's range, infinity above
-__device__ __forceinline__ float abs_f32(double d) {
-  const unsigned hi = (unsigned)__double2hiint(d) & 0x7fffffffu, lo = (unsigned)__double2loint(d);
-  const int e = (int)(hi >> 20) - 1023 + 127;
-  if (e <= 0) return 0.f;
-  if (e >= 255) return __int_as_float(0x7f800000);
-  return __uint_as_float((unsigned)e << 23 | (hi & 0xfffffu) << 3 | lo >> 29);
-}
-
 // Structured strong RRLU of one node (row or column case).  Node side (length
 // M) in shared memory, other side (length N) in global scratch.  The scans and
 // generator updates over the N other-side entries are FP64-pipe bound, so their

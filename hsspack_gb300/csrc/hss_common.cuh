@@ -57,24 +57,21 @@ __device__ __forceinline__ void sqrt_pair(double x, double &r, double &rinv) {
   r = fma(h, c, h);
 }
 
-// (value, index) argmax with "first index wins" ties -- Fortran MAXLOC order.
-struct ArgMax {
-  double v;
-  int i;
-};
-__device__ __forceinline__ ArgMax argmax_merge(ArgMax a, ArgMax b) {
-  if (b.v > a.v || (b.v == a.v && b.i < a.i)) return b;
-  return a;
+// |d| as FP32 rounded towards zero by integer operations (a conversion holds the
+// FP64 pipe); 0 below FP32's range, infinity above
+__device__ __forceinline__ float abs_f32(double d) {
+  const unsigned hi = (unsigned)__double2hiint(d) & 0x7fffffffu, lo = (unsigned)__double2loint(d);
+  const int e = (int)(hi >> 20) - 1023 + 127;
+  if (e <= 0) return 0.f;
+  if (e >= 255) return __int_as_float(0x7f800000);
+  return __uint_as_float((unsigned)e << 23 | (hi & 0xfffffu) << 3 | lo >> 29);
 }
-__device__ __forceinline__ ArgMax warp_argmax(ArgMax a) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    ArgMax b;
-    b.v = __shfl_xor_sync(HSS_FULL, a.v, o);
-    b.i = __shfl_xor_sync(HSS_FULL, a.i, o);
-    a = argmax_merge(a, b);
-  }
-  return a;
+
+// a normal FP32 number as FP64, likewise
+__device__ __forceinline__ double f64_of_f32(float f) {
+  const unsigned b = __float_as_uint(f);
+  return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + (896u << 20))),
+                          (int)(b << 29));
 }
 
 // Differences of the old poles F and new roots lam = F + DIFL, formed from

@@ -54,6 +54,7 @@ namespace hss {
 
 constexpr int QR_MAXC = 128;    // largest node dimension (rows of U, rows of V)
 constexpr int QT = 256;         // threads per CTA
+constexpr int QTH = QT + 32;    // and the look-ahead warp of the tall QR
 constexpr int QR_TILE = 25000;  // doubles in the shared QR tile (195 KB)
 constexpr int JAC_SWEEPS = 40;  // one-sided Jacobi sweep limit
 
@@ -68,8 +69,11 @@ struct TallDesc {
 };
 struct QrJob {
   int desc, t0, t1;
-  double *out;  // R (ncol x ncol, upper triangular), leading dim ldo
-  int ldo;
+  double *out;  // R (ncol x ncol, upper triangular): row i, column c at i ros + c ldo
+  int ldo, ros;
+  // > 0: the rows are `tri` upper triangular factors with their rows interleaved, so
+  // column k is zero from row tri (k + 1) on
+  int tri;
 };
 struct BasisJob {
   const double *R;  // r x r upper triangular, leading dim r
@@ -88,7 +92,7 @@ struct CopyDesc {
 
 __host__ __device__ inline int qr_chunk(int r) {
   const int nc = QR_TILE / r - r - 1;
-  return nc > 256 ? 256 : nc;
+  return nc > 512 ? 512 : nc;
 }
 
 __device__ __forceinline__ unsigned group_mask(int gs) {
@@ -109,12 +113,24 @@ __device__ __forceinline__ int group_size(int groups) {
 struct HousePar {
   double beta, tau, scale;
 };
+// (one lane forms it, at a warp's FP64 price: root, reciprocal root and reciprocal
+// from estimates, each within about an ulp)
 __device__ __forceinline__ HousePar house_par(double alpha, double sg) {
   HousePar h{alpha, 0.0, 0.0};
   if (sg > 0.0) {
-    h.beta = -copysign(sqrt(fma(alpha, alpha, sg)), alpha);
-    h.tau = (h.beta - alpha) / h.beta;
-    h.scale = 1.0 / (alpha - h.beta);
+    const double x = fma(alpha, alpha, sg);
+    const int hx = __double2hiint(x);
+    if (hx >= 0x03f00000 && hx < 0x7bf00000) {  // 2^-960 <= x < 2^960
+      double rt, ri;
+      sqrt_pair(x, rt, ri);
+      h.beta = -copysign(rt, alpha);
+      h.tau = (h.beta - alpha) * -copysign(ri, alpha);
+      h.scale = rcp_nr(alpha - h.beta);
+    } else {
+      h.beta = -copysign(sqrt(x), alpha);
+      h.tau = (h.beta - alpha) / h.beta;
+      h.scale = 1.0 / (alpha - h.beta);
+    }
   }
   return h;
 }
@@ -123,52 +139,77 @@ __device__ __forceinline__ HousePar house_par(double alpha, double sg) {
 // so far, rows r..r+na-1 a chunk of the tall matrix; on return rows 0..r-1
 // hold the R factor of both.  Column k's reflector has nonzeros only in row k
 // and the chunk rows (R is triangular), v_k = 1, v_chunk = C(:, k) * scale.
-// Column j > k is updated by a group of gs lanes; the group of column k + 1
-// also forms that column's sum of squares and, on one lane, the next
-// reflector (double-buffered in hp), so one barrier per column.
-__device__ void house_tile(double *S, int LD, int r, int na, HousePar *hp, double *red) {
-  const int tid = threadIdx.x;
+// rows(k): the chunk rows that column k can have nonzeros in (nondecreasing).
+//
+// FP64-pipe bound (2 multiply-adds per entry and step).  The last warp takes
+// column k + 1 alone and forms the next reflector from it; the other 256 threads
+// split the remaining columns into as many row chunks per column as fit, one
+// (column, chunk) pair a thread, the chunks' dot products meeting in `part`.
+// (With power-of-two lane groups per column a third of the threads idled, and the
+// group of column k + 1 worked on while the rest waited.)
+template <class Rows>
+__device__ void house_tile(double *S, int LD, int r, int na, Rows rows, HousePar *hp, double *red,
+                           double *part) {
+  const int tid = threadIdx.x, lane = tid & 31;
   {
     double q = 0.0;
-    for (int i = tid; i < na; i += QT) { const double x = S[r + i]; q = fma(x, x, q); }
+    for (int i = tid; i < rows(0); i += QTH) { const double x = S[r + i]; q = fma(x, x, q); }
     q = warp_sum(q);
-    if ((tid & 31) == 0) red[tid >> 5] = q;
+    if (lane == 0) red[tid >> 5] = q;
     __syncthreads();
     if (tid == 0) {
       double s = 0.0;
-      for (int w = 0; w < QT / 32; ++w) s += red[w];
+      for (int w = 0; w < QTH / 32; ++w) s += red[w];
       hp[0] = house_par(S[0], s);
     }
     __syncthreads();
   }
   for (int k = 0; k < r; ++k) {
     const HousePar h = hp[k & 1];
-    const int left = r - k - 1;
-    if (left > 0) {
-      const int gs = group_size(left);
-      const int grp = tid / gs, ln = tid - grp * gs;
-      if (grp < left) {
-        const unsigned mask = group_mask(gs);
-        double *Sj = S + (k + 1 + grp) * LD;
-        const double *Sk = S + k * LD;
+    const int left = r - k - 1, nk = rows(k);
+    const double *Sk = S + k * LD;
+    double *rk = nullptr, rtw = 0.0;  // this thread's entry of row k, and its change
+    if (tid >= QT) {
+      if (left > 0) {
+        double *Sj = S + (k + 1) * LD;
         if (h.tau != 0.0) {
           double dd = 0.0;
-          for (int i = r + ln; i < r + na; i += gs) dd = fma(Sk[i], Sj[i], dd);
-          dd = group_sum(dd, gs, mask);
+          for (int i = r + lane; i < r + nk; i += 32) dd = fma(Sk[i], Sj[i], dd);
+          dd = warp_sum(dd);
           const double tw = h.tau * fma(h.scale, dd, Sj[k]), tws = tw * h.scale;
-          for (int i = r + ln; i < r + na; i += gs) Sj[i] = fma(-tws, Sk[i], Sj[i]);
-          if (ln == 0) Sj[k] -= tw;
+          for (int i = r + lane; i < r + nk; i += 32) Sj[i] = fma(-tws, Sk[i], Sj[i]);
+          __syncwarp();
+          if (lane == 0) Sj[k] -= tw;
         }
-        if (grp == 0) {
-          double q = 0.0;
-          for (int i = r + ln; i < r + na; i += gs) q = fma(Sj[i], Sj[i], q);
-          q = group_sum(q, gs, mask);
-          // entry (k+1, k+1) is not written during step k
-          if (ln == 0) hp[(k + 1) & 1] = house_par(Sj[k + 1], q);
-        }
+        double q = 0.0;
+        const int n1 = rows(k + 1);
+        for (int i = r + lane; i < r + n1; i += 32) q = fma(Sj[i], Sj[i], q);
+        q = warp_sum(q);
+        // entry (k+1, k+1) is not written during step k
+        if (lane == 0) hp[(k + 1) & 1] = house_par(Sj[k + 1], q);
+      }
+    } else if (left > 1 && h.tau != 0.0) {
+      const int cnt = left - 1, nch = QT / cnt;
+      const int ch = tid / cnt, col = tid - ch * cnt;
+      double *Sj = S + (k + 2 + col) * LD;
+      const bool act = ch < nch;
+      const int i0 = r + nk * ch / nch, i1 = act ? r + nk * (ch + 1) / nch : 0;
+      double dd = 0.0;
+#pragma unroll 4
+      for (int i = i0; i < i1; ++i) dd = fma(Sk[i], Sj[i], dd);
+      if (act) part[ch * cnt + col] = dd;
+      asm volatile("bar.sync 1, %0;" ::"n"(QT) : "memory");
+      if (act) {
+        double s = 0.0;
+        for (int c = 0; c < nch; ++c) s += part[c * cnt + col];
+        const double tw = h.tau * fma(h.scale, s, Sj[k]), tws = tw * h.scale;
+#pragma unroll 4
+        for (int i = i0; i < i1; ++i) Sj[i] = fma(-tws, Sk[i], Sj[i]);
+        if (ch == 0) { rk = Sj + k; rtw = tw; }
       }
     }
     __syncthreads();
+    if (rk) *rk -= rtw;  // (every chunk has read it, and no later step does)
     if (tid == 0) S[k * LD + k] = h.beta;  // nobody reads (k, k) after step k
   }
   __syncthreads();
@@ -176,38 +217,40 @@ __device__ void house_tile(double *S, int LD, int r, int na, HousePar *hp, doubl
 
 // R factor of rows [t0, t1) of a tall matrix (ncol <= QR_MAXC), one CTA per
 // job, tiles of qr_chunk(ncol) rows.
-__global__ void __launch_bounds__(QT)
+__global__ void __launch_bounds__(QTH)
 k_tall_qr(const TallDesc *__restrict__ descs, const QrJob *__restrict__ jobs) {
   extern __shared__ double S[];
   __shared__ HousePar hp[2];
-  __shared__ double red[QT / 32];
+  __shared__ double red[QTH / 32], part[QT];
   const QrJob jb = jobs[blockIdx.x];
   const TallDesc d = descs[jb.desc];
-  const int r = d.ncol, nc = qr_chunk(r), LD = r + nc + 1;
+  const int r = d.ncol, nc = qr_chunk(r), LD = (r + nc) | 1;  // odd: no bank conflicts
   const int tid = threadIdx.x;
-  for (int e = tid; e < LD * r; e += QT) S[e] = 0.0;
+  for (int e = tid; e < LD * r; e += QTH) S[e] = 0.0;
   __syncthreads();
   for (int t = jb.t0; t < jb.t1; t += nc) {
     const int na = min(nc, jb.t1 - t);
     if (d.sc == 1) {  // a tall row is contiguous: lanes along c
-      for (int e = tid; e < na * r; e += QT) {
+      for (int e = tid; e < na * r; e += QTH) {
         const int tt = e / r, c = e - tt * r, v = t + tt;
         const long long ph = v < d.s0 ? v : (long long)v + d.skip;
         S[c * LD + r + tt] = d.base[ph * d.st + c];
       }
     } else {  // a tall column is contiguous: lanes along t
-      for (int e = tid; e < na * r; e += QT) {
+      for (int e = tid; e < na * r; e += QTH) {
         const int c = e / na, tt = e - c * na, v = t + tt;
         const long long ph = v < d.s0 ? v : (long long)v + d.skip;
         S[c * LD + r + tt] = d.base[ph * d.st + (long long)c * d.sc];
       }
     }
     __syncthreads();
-    house_tile(S, LD, r, na, hp, red);
+    const int tri = jb.tri;
+    house_tile(S, LD, r, na,
+               [=](int k) { return tri ? max(0, min(na, tri * (k + 1) - t)) : na; }, hp, red, part);
   }
-  for (int e = tid; e < r * r; e += QT) {
+  for (int e = tid; e < r * r; e += QTH) {
     const int c = e / r, i = e - c * r;
-    jb.out[(long long)c * jb.ldo + i] = i <= c ? S[c * LD + i] : 0.0;
+    jb.out[(long long)c * jb.ldo + (long long)i * jb.ros] = i <= c ? S[c * LD + i] : 0.0;
   }
 }
 
@@ -230,15 +273,28 @@ k_tall_qr(const TallDesc *__restrict__ descs, const QrJob *__restrict__ jobs) {
 //      so few sweeps are needed, on k0 ~ rank rows instead of r.
 //   C. Normalised rows with norm > tol, un-permuted, sorted by decreasing norm.
 // status |= 1 if the sweep limit is reached.
+//
+// Bound: FP64 instructions in a serial chain of steps, one CTA per node and few
+// nodes.  A Jacobi step has three phases, each with all threads on the same kind
+// of work: partial dot products ((pair, chunk) per thread, about one warp per
+// quarter of the SM), one lane per pair forming its rotation (once per step and
+// not once per warp: it costs a warp's FP64 slots whatever lanes it serves), and
+// the rotations.  These are "fast" ones: the rows keep scale factors (actual row
+// = s_t times the stored one, folded in at the start of a sweep), so an entry
+// takes one multiply-add instead of a multiply and a multiply-add.  Angles: an
+// FP32 tangent corrected once in FP64, cosines from an estimate of the reciprocal
+// root, comparisons on bit patterns.
 __global__ void __launch_bounds__(QT)
 k_node_basis(const BasisJob *__restrict__ jobs, double tol, int *status) {
   extern __shared__ double M[];  // column j at M + j * LDM
   __shared__ double cn[QR_MAXC], cref[QR_MAXC], nrm[QR_MAXC];
+  __shared__ double scl[QR_MAXC];  // row scales
+  __shared__ double part[QT], tp[QR_MAXC / 2], tq[QR_MAXC / 2];
   __shared__ int prm[QR_MAXC], pos[QR_MAXC];
   __shared__ HousePar s_h;
   __shared__ int s_piv, s_k;
   const BasisJob jb = jobs[blockIdx.x];
-  const int r = jb.r, LDM = r + 1, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int r = jb.r, LDM = r | 1, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   for (int e = tid; e < r * r; e += QT) {
     const int c = e / r, i = e - c * r;
     M[c * LDM + i] = i <= c ? jb.R[i + (long long)c * r] : 0.0;
@@ -260,10 +316,19 @@ k_node_basis(const BasisJob *__restrict__ jobs, double tol, int *status) {
   int k0 = r;
   for (int k = 0; k < r; ++k) {
     if (wid == 0) {
-      ArgMax am{-1.0, r};
-      for (int j = k + lane; j < r; j += 32) am = argmax_merge(am, ArgMax{cn[j], j});
-      am = warp_argmax(am);
-      if (lane == 0) s_piv = ((double)(r - k) * am.v <= stop2) ? -1 : am.i;
+      // the largest trailing column norm, as integers (a norm is >= 0 but for rounding)
+      unsigned long long key = 0;
+      int at = r;
+      for (int j = k + lane; j < r; j += 32) {
+        const long long b = __double_as_longlong(cn[j]);
+        const unsigned long long v = b < 0 ? 1ull : (unsigned long long)b + 2ull;
+        if (v > key) { key = v; at = j; }
+      }
+      const unsigned hi = (unsigned)(key >> 32), lo = (unsigned)key;
+      const unsigned mh = __reduce_max_sync(HSS_FULL, hi);
+      const unsigned ml = __reduce_max_sync(HSS_FULL, hi == mh ? lo : 0u);
+      const int p = __reduce_min_sync(HSS_FULL, hi == mh && lo == ml ? at : r);
+      if (lane == 0) s_piv = ((double)(r - k) * cn[p] <= stop2) ? -1 : p;
     }
     __syncthreads();
     const int p = s_piv;
@@ -331,71 +396,114 @@ k_node_basis(const BasisJob *__restrict__ jobs, double tol, int *status) {
   __syncthreads();
   // ---- B: one-sided Jacobi on the k0 rows
   const int rp = k0 + (k0 & 1), np = rp / 2;
-  const int gs = group_size(np > 0 ? np : 1);
-  const int grp = tid / gs, ln = tid - grp * gs;
+  const int nch = np > 0 ? max(1, 128 / np) : 1;
+  const int ch = np > 0 ? tid / np : 0, pi = np > 0 ? tid - ch * np : 0;
+  const bool act = np > 0 && ch < nch;
+  const int j0 = r * ch / nch, j1 = act ? r * (ch + 1) / nch : 0;
+  const int gs = group_size(k0 > 0 ? k0 : 1), grp = tid / gs, ln = tid - grp * gs;
   const unsigned mask = group_mask(gs);
   const int ng = QT / gs;
-  const int lead = (tid & 31) & ~(gs - 1);
-  const double jtol = HSS_EPS * (r > 16 ? r : 16);
-  const double frz2 = stop2;
+  const double jtol = HSS_EPS * (r > 16 ? r : 16), jtol2 = jtol * jtol;
+  const long long frzb = __double_as_longlong(stop2);
+  for (int t = tid; t < k0; t += QT) scl[t] = 1.0;
   int conv = k0 < 2;
   for (int sweep = 0; sweep < JAC_SWEEPS && !conv; ++sweep) {
-    for (int t = grp; t < k0; t += ng) {
+    __syncthreads();
+    for (int t = grp; t < k0; t += ng) {  // scales folded in, norms refreshed
+      const double sc = scl[t];
       double a = 0.0;
-      for (int j = ln; j < r; j += gs) { const double u = M[j * LDM + t]; a = fma(u, u, a); }
+      for (int j = ln; j < r; j += gs) {
+        const double u = M[j * LDM + t] * sc;
+        M[j * LDM + t] = u;
+        a = fma(u, u, a);
+      }
       a = group_sum(a, gs, mask);
-      if (ln == 0) nrm[t] = a;
+      if (ln == 0) { nrm[t] = a; scl[t] = 1.0; }
     }
     __syncthreads();
     int rot = 0;
     for (int s = 0; s < rp - 1; ++s) {
-      if (grp < np) {
-        int p, q;
-        if (grp == 0) { p = 0; q = 1 + s % (rp - 1); }
-        else { p = 1 + (s + grp) % (rp - 1); q = 1 + (s - grp + rp - 1) % (rp - 1); }
-        if (p < k0 && q < k0) {
+      int p, q;
+      if (pi == 0) { p = 0; q = 1 + s % (rp - 1); }
+      else { p = 1 + (s + pi) % (rp - 1); q = 1 + (s - pi + rp - 1) % (rp - 1); }
+      const bool pair = act && p < k0 && q < k0;
+      if (pair) {
+        double c = 0.0;
+#pragma unroll 4
+        for (int j = j0; j < j1; ++j) c = fma(M[j * LDM + p], M[j * LDM + q], c);
+        part[tid] = c;
+      }
+      __syncthreads();
+      int go = 0;
+      if (tid < np) {  // (ch = 0: this thread's own pair)
+        double ta = 0.0, tb = 0.0;
+        if (pair) {
           const double a = nrm[p], b = nrm[q];
-          if (a > 0.0 && b > 0.0 && a >= frz2 && b >= frz2) {
-            double c = 0.0;
-            for (int j = ln; j < r; j += gs) c = fma(M[j * LDM + p], M[j * LDM + q], c);
-            c = group_sum(c, gs, mask);
-            double cs = 1.0, sn = 0.0;
-            int go = 0;
-            if (ln == 0 && c != 0.0 && fabs(c) > jtol * sqrt(a * b)) {
-              const double zeta = (b - a) / (2.0 * c);
-              const double t = fabs(zeta) > 1e150
-                                   ? 0.5 / zeta
-                                   : copysign(1.0, zeta) / (fabs(zeta) + sqrt(fma(zeta, zeta, 1.0)));
-              cs = 1.0 / sqrt(fma(t, t, 1.0));
-              sn = cs * t;
+          const long long ab = __double_as_longlong(a), bb = __double_as_longlong(b);
+          if (ab > 0 && bb > 0 && ab >= frzb && bb >= frzb) {  // a, b > 0, >= stop2
+            double c = part[pi];
+            for (int x = 1; x < nch; ++x) c += part[x * np + pi];
+            const double sp = scl[p], sq = scl[q], g = sp * sq;
+            c *= g;
+            if (__double_as_longlong(c * c) > __double_as_longlong(jtol2 * a * b)) {
+              // t of smaller modulus with t^2 + 2 zeta t = 1, zeta = (b - a) / 2c
+              const double x = b - a, zeta = x * rcp_nr(2.0 * c);
+              const float zf = abs_f32(zeta);
+              double t;
+              if (zf < 1e15f) {
+                const float rf = sqrtf(fmaf(zf, zf, 1.f));
+                t = copysign(f64_of_f32(__fdividef(1.f, zf + rf)), zeta);
+                // one Newton step: f(t) / (2 (t + zeta)), t + zeta = +-sqrt(1 + zeta^2)
+                const double f = fma(t, fma(2.0, zeta, t), -1.0);
+                t = fma(-f, copysign(f64_of_f32(__fdividef(0.5f, rf)), zeta), t);
+              } else {
+                t = c * rcp_nr(x);
+              }
+              double rt, cs;
+              sqrt_pair(fma(t, t, 1.0), rt, cs);
               nrm[p] = fma(-t, c, a);
               nrm[q] = fma(t, c, b);
+              const double ti = t * rcp_nr(g);  // t / (s_p s_q)
+              ta = ti * (sq * sq);
+              tb = ti * (sp * sp);
+              scl[p] = sp * cs;
+              scl[q] = sq * cs;
               go = 1;
-            }
-            go = __shfl_sync(mask, go, lead);
-            if (go) {
-              cs = __shfl_sync(mask, cs, lead);
-              sn = __shfl_sync(mask, sn, lead);
-              for (int j = ln; j < r; j += gs) {
-                const double u = M[j * LDM + p], v = M[j * LDM + q];
-                M[j * LDM + p] = fma(cs, u, -sn * v);
-                M[j * LDM + q] = fma(sn, u, cs * v);
-              }
-              rot = 1;
             }
           }
         }
+        tp[pi] = ta;
+        tq[pi] = tb;
       }
-      __syncthreads();
+      if (__syncthreads_or(go)) {
+        rot = 1;
+        if (pair) {
+          const double ta = tp[pi], tb = tq[pi];
+          if (__double_as_longlong(tb) != 0) {
+#pragma unroll 4
+            for (int j = j0; j < j1; ++j) {
+              const double u = M[j * LDM + p], v = M[j * LDM + q];
+              M[j * LDM + p] = fma(-ta, v, u);
+              M[j * LDM + q] = fma(tb, u, v);
+            }
+          }
+        }
+        __syncthreads();
+      }
     }
-    conv = !__syncthreads_or(rot);
+    conv = !rot;  // uniform
   }
   if (!conv && tid == 0) atomicOr(status, 1);
   __syncthreads();
-  // ---- C: norms, order, rank, outputs
+  // ---- C: norms, order, rank, outputs of the actual rows
   for (int t = grp; t < k0; t += ng) {
+    const double sc = scl[t];
     double a = 0.0;
-    for (int j = ln; j < r; j += gs) { const double u = M[j * LDM + t]; a = fma(u, u, a); }
+    for (int j = ln; j < r; j += gs) {
+      const double u = M[j * LDM + t] * sc;
+      M[j * LDM + t] = u;
+      a = fma(u, u, a);
+    }
     a = group_sum(a, gs, mask);
     if (ln == 0) nrm[t] = sqrt(a);
   }
@@ -488,11 +596,20 @@ static std::vector<int> tall_bases(const std::vector<TallDesc> &ds, const std::v
                              QR_MAXC * (QR_MAXC + 1) * (int)sizeof(double)));
     attr = true;
   }
-  // rows per first-pass job: enough jobs for two CTAs per SM, and at least
-  // four times the column count
-  long long tot = 0;
-  for (const auto &d : ds) tot += d.ntot;
-  const long long per0 = std::max<long long>(1, tot / (2LL * sm_count()));
+  // Row ranges per matrix: the number of them with the least rows in sequence, full
+  // waves of CTAs (one per SM) over the ranges, then the stacked factors (whose
+  // interleaved triangles cost a third of their rows)
+  int want = 1;
+  {
+    long long tot = 0, rr = 1, best = LLONG_MAX;
+    for (const auto &d : ds) { tot += d.ntot; rr = std::max<long long>(rr, d.ncol); }
+    const long long avg = (tot + nd - 1) / nd, sms = sm_count();
+    for (int nj = 1; nj <= 64 && avg / nj >= 2 * rr; ++nj) {
+      const long long w1 = (nj * (long long)nd + sms - 1) / sms, w2 = (nd + sms - 1) / sms;
+      const long long cost = w1 * ((avg + nj - 1) / nj) + (nj > 1 ? w2 * (nj * rr / 3 + rr) : 0);
+      if (cost < best) { best = cost; want = nj; }
+    }
+  }
   double *Rfin = pool<double>("m2h_Rfin", (size_t)nd * QR_MAXC * QR_MAXC);
   std::vector<QrJob> j1, j2;
   std::vector<TallDesc> d2;
@@ -501,8 +618,7 @@ static std::vector<int> tall_bases(const std::vector<TallDesc> &ds, const std::v
   long long stot = 0;
   for (int i = 0; i < nd; ++i) {
     const int r = ds[i].ncol;
-    const long long per = std::max<long long>(per0, 4LL * r);
-    njob[i] = (int)std::min<long long>(64, (ds[i].ntot + per - 1) / per);
+    njob[i] = (int)std::max<long long>(1, std::min<long long>(want, ds[i].ntot / (2LL * r)));
     if (njob[i] > 1) { soff[i] = stot; stot += (long long)njob[i] * r * r; }
   }
   double *stk = pool<double>("m2h_Rstack", (size_t)std::max<long long>(stot, 1));
@@ -510,26 +626,26 @@ static std::vector<int> tall_bases(const std::vector<TallDesc> &ds, const std::v
     const int r = ds[i].ncol, nj = njob[i];
     double *fin = Rfin + (size_t)i * QR_MAXC * QR_MAXC;
     if (nj == 1) {
-      j1.push_back({i, 0, ds[i].ntot, fin, r});
+      j1.push_back({i, 0, ds[i].ntot, fin, r, 1, 0});
       continue;
     }
     double *sb = stk + soff[i];
     const int ld = nj * r;
     for (int q = 0; q < nj; ++q) {
       const int a = (int)((long long)ds[i].ntot * q / nj), b = (int)((long long)ds[i].ntot * (q + 1) / nj);
-      j1.push_back({i, a, b, sb + (size_t)q * r, ld});
+      j1.push_back({i, a, b, sb + q, ld, nj, 0});  // row i of factor q at i nj + q
     }
     d2.push_back({sb, 1, (long long)ld, ld, r, INT_MAX, 0});
-    j2.push_back({(int)d2.size() - 1, 0, ld, fin, r});
+    j2.push_back({(int)d2.size() - 1, 0, ld, fin, r, 1, nj});
   }
   TallDesc *dd = upload("m2h_desc", ds, st);
   QrJob *dj = upload("m2h_job1", j1, st);
-  k_tall_qr<<<(unsigned)j1.size(), QT, QR_TILE * sizeof(double), st>>>(dd, dj);
+  k_tall_qr<<<(unsigned)j1.size(), QTH, QR_TILE * sizeof(double), st>>>(dd, dj);
   ++launches;
   if (!j2.empty()) {
     TallDesc *dd2 = upload("m2h_desc2", d2, st);
     QrJob *dj2 = upload("m2h_job2", j2, st);
-    k_tall_qr<<<(unsigned)j2.size(), QT, QR_TILE * sizeof(double), st>>>(dd2, dj2);
+    k_tall_qr<<<(unsigned)j2.size(), QTH, QR_TILE * sizeof(double), st>>>(dd2, dj2);
     ++launches;
   }
   int *drk = pool<int>("m2h_rank", nd + 1);
