@@ -152,6 +152,18 @@ void *pool_get(const char *name, size_t bytes) { return buf<char>(ctx(), name, b
 // error word of the tensor-core products (set by a CTA whose bounded wait
 // timed out; reset at the start of every solve, read with its status)
 static int *gemm_flag(Ctx &c) { return buf<int>(c, "gemm_err", 1); }
+// The word around an entry point's products: a set one makes the product kernel
+// skip its tiles, and fresh device memory holds anything.
+static void gemm_flag_clear(Ctx &c, cudaStream_t st) {
+  CK(cudaMemsetAsync(gemm_flag(c), 0, sizeof(int), st));
+}
+// waits for the stream
+static void gemm_flag_check(Ctx &c, cudaStream_t st) {
+  int err = 0;
+  CK(cudaMemcpyAsync(&err, gemm_flag(c), sizeof(int), cudaMemcpyDeviceToHost, st));
+  CK(cudaStreamSynchronize(st));
+  if (err) throw HssError{"tensor-core product: bounded wait timed out"};
+}
 
 // Host->device parameter uploads (level views, product descriptors).  Small
 // ones stay pageable copies (measured faster: they travel with the command
@@ -2441,9 +2453,10 @@ int hss_dhssevc_dev(int k, int ni, double tol, const double *F, const double *u,
   try {
     int rank = 0;
     float t2[2] = {0.f, 0.f};
+    gemm_flag_clear(c, st);
     hss_dhssevc_core(k, ni, tol, c.cfg.precision, F, u, v, difl, difr, Q, ldq, nrows, &rank, st,
                      t2);
-    CK(cudaStreamSynchronize(st));
+    gemm_flag_check(c, st);
     CK(cudaGetLastError());
     c.stats.max_rank = rank;
     // construction and product times of this call (CUDA events)
@@ -2472,8 +2485,9 @@ int hss_cauchyhssmm_dev(int n, const double *D, const double *F, const double *u
   cudaStream_t st = (cudaStream_t)stream;
   try {
     int rank = 0;
+    gemm_flag_clear(c, st);
     hss_cauchyhssmm_core(n, D, F, u, v, ni, tol, c.cfg.precision, B, ldb, ncb, &rank, times, st);
-    CK(cudaStreamSynchronize(st));
+    gemm_flag_check(c, st);
     CK(cudaGetLastError());
     c.stats.max_rank = rank;
     return 0;
@@ -2510,8 +2524,10 @@ void cauchyhssmm_(const double *D, const double *F, const double *U, const doubl
                          cudaMemcpyHostToDevice, st));
     int rank = 0;
     float t[2] = {0.f, 0.f};
+    gemm_flag_clear(c, st);
     hss_cauchyhssmm_core(n, dv, dv + n, dv + 2 * n, dv + 3 * n, ni, *tol_, c.cfg.precision, dB, n,
                          n, &rank, t, st);
+    gemm_flag_check(c, st);
     CK(cudaMemcpy2DAsync(B, sizeof(double) * ldb, dB, sizeof(double) * n, sizeof(double) * n, n,
                          cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
@@ -2831,8 +2847,9 @@ int hss_dhssmm_dev(int n, const double *A, int lda, double *B, int ldb, int k, d
   cudaStream_t st = (cudaStream_t)stream;
   try {
     int rank = 0;
+    gemm_flag_clear(c, st);
     hss_dhssmm_core(n, A, lda, B, ldb, k, tol, ni, side, c.cfg.precision, &rank, times, st);
-    CK(cudaStreamSynchronize(st));
+    gemm_flag_check(c, st);
     CK(cudaGetLastError());
     c.stats.max_rank = rank;
     return 0;
@@ -2876,7 +2893,9 @@ static void dhssmm_host(int side, const double *A, int lda, int m, int n, double
                          cudaMemcpyHostToDevice, st));
     int rank = 0;
     float t[2] = {0.f, 0.f};
+    gemm_flag_clear(c, st);
     hss_dhssmm_core(n, dA, n, dB, br, k, tol, ni, side, c.cfg.precision, &rank, t, st);
+    gemm_flag_check(c, st);
     CK(cudaMemcpy2DAsync(B, sizeof(double) * ldb, dB, sizeof(double) * br, sizeof(double) * br, bc,
                          cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
