@@ -57,6 +57,33 @@ __device__ __forceinline__ void sqrt_pair(double x, double &r, double &rinv) {
   r = fma(h, c, h);
 }
 
+// Householder reflector of (alpha, tail) with the tail's squared norm sg: beta, tau, and
+// scale with v = [1; tail * scale]
+struct HousePar {
+  double beta, tau, scale;
+};
+// (one lane forms it, at a warp's FP64 price: root, reciprocal root and reciprocal
+// from estimates, each within about an ulp)
+__device__ __forceinline__ HousePar house_par(double alpha, double sg) {
+  HousePar h{alpha, 0.0, 0.0};
+  if (sg > 0.0) {
+    const double x = fma(alpha, alpha, sg);
+    const int hx = __double2hiint(x);
+    if (hx >= 0x03f00000 && hx < 0x7bf00000) {  // 2^-960 <= x < 2^960
+      double rt, ri;
+      sqrt_pair(x, rt, ri);
+      h.beta = -copysign(rt, alpha);
+      h.tau = (h.beta - alpha) * -copysign(ri, alpha);
+      h.scale = rcp_nr(alpha - h.beta);
+    } else {
+      h.beta = -copysign(sqrt(x), alpha);
+      h.tau = (h.beta - alpha) / h.beta;
+      h.scale = 1.0 / (alpha - h.beta);
+    }
+  }
+  return h;
+}
+
 // |d| as FP32 rounded towards zero by integer operations (a conversion holds the
 // FP64 pipe); 0 below FP32's range, infinity above
 __device__ __forceinline__ float abs_f32(double d) {

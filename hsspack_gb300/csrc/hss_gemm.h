@@ -15,6 +15,7 @@ struct GemmDesc {
   int M, N, K;
   int beta;
   int tile0;  // first flattened tile index of this problem
+  int tri;    // 1: B is upper triangular with zeros below (the element kernel skips those)
 };
 
 // one operand of the split-BF16 GEMM: `rows` vectors of length `inner`

@@ -63,55 +63,74 @@ constexpr size_t CH_SLOT = (size_t)CH_MAXM * CH_MAXM;
 // Cholesky D = L L^T of each node's diagonal block (one CTA per node, the block
 // in shared memory); L (lower, m x m) and It = L^{-T} (upper) to the node's
 // scratch slot.  status |= 1 when a pivot is not positive.
+//
+// Bound by the serial chain of m steps, each a few FP64 instructions a warp.  The
+// columns stay unscaled until the end, so a step needs one reciprocal and no root; the
+// trailing triangle is folded into a rectangle, column c's part and column t-1-c's in
+// one row of it, so no thread works above the diagonal.  The inverse runs by columns
+// of L in the upper triangle, (column, row) pairs over all threads; it took a thread per
+// column with a division per entry.  256 nodes of 32 rows: 147 -> 45 us.
 __global__ void __launch_bounds__(CHT)
 k_ch_chol(const ChNode *__restrict__ nd, const double *__restrict__ Ah, long long lda,
           double *__restrict__ Lb, double *__restrict__ Ib, int *__restrict__ status) {
-  extern __shared__ double S[];  // column j at S + j * (m + 1)
-  __shared__ int bad;
+  extern __shared__ double S[];  // column j at S + j * ld: L below, It above the diagonal
+  __shared__ double rd[CH_MAXM];
   const ChNode q = nd[blockIdx.x];
-  const int m = q.m, ld = m + 1, tid = threadIdx.x;
+  const int m = q.m, ld = m | 1, tid = threadIdx.x;
   const double *D = Ah + (long long)q.o * lda + q.o;
   for (int e = tid; e < m * m; e += CHT) {
     const int j = e / m, i = e - j * m;
-    S[j * ld + i] = D[(long long)j * lda + i];
+    S[j * ld + i] = i >= j ? D[(long long)j * lda + i] : 0.0;
   }
-  if (tid == 0) bad = 0;
   __syncthreads();
   for (int j = 0; j < m; ++j) {
-    if (tid == 0) {
-      const double d = S[j * ld + j];
-      if (!(d > 0.0)) { bad = 1; S[j * ld + j] = 1.0; }
-      else S[j * ld + j] = sqrt(d);
+    const double *Sj = S + j * ld;
+    const double d = Sj[j];
+    if (!(d > 0.0)) {
+      if (tid == 0) atomicOr(status, 1);
+      return;
     }
-    __syncthreads();
-    if (bad) break;
-    const double piv = S[j * ld + j];
-    for (int i = j + 1 + tid; i < m; i += CHT) S[j * ld + i] /= piv;
-    __syncthreads();
-    const int t = m - j - 1;
-    for (int e = tid; e < t * t; e += CHT) {
-      const int kk = e / t, ii = e - kk * t;
-      if (ii >= kk) S[(j + 1 + kk) * ld + j + 1 + ii] -= S[j * ld + j + 1 + ii] * S[j * ld + j + 1 + kk];
+    const int hd = __double2hiint(d);  // 2^-960 <= d < 2^960
+    const double di = hd >= 0x03f00000 && hd < 0x7bf00000 ? rcp_nr(d) : 1.0 / d;
+    const int t = m - j - 1, w = t | 1, tot = w * ((t + 1) >> 1);
+    for (int e = tid; e < tot; e += CHT) {
+      int c = e / w, r = e - c * w;
+      if (r >= t - c) {  // column t - c (t odd) or t - 1 - c
+        r -= t - c;
+        c = (t & 1 ? t : t - 1) - c;
+      }
+      const double *u = Sj + j + 1;
+      double *x = S + (j + 1 + c) * ld + j + 1 + c + r;
+      *x = fma(-u[c + r] * di, u[c], *x);
     }
     __syncthreads();
   }
-  if (bad) {
-    if (tid == 0) atomicOr(status, 1);
-    return;
+  for (int j = tid; j < m; j += CHT) {
+    const double r = sqrt(S[j * ld + j]);
+    S[j * ld + j] = r;
+    rd[j] = 1.0 / r;
   }
+  __syncthreads();
   double *L = Lb + (size_t)q.slot * CH_SLOT, *It = Ib + (size_t)q.slot * CH_SLOT;
   for (int e = tid; e < m * m; e += CHT) {
     const int j = e / m, i = e - j * m;
+    if (i > j) S[j * ld + i] *= rd[j];
     L[(long long)j * m + i] = i >= j ? S[j * ld + i] : 0.0;
   }
-  // It(c, i) = L^{-1}(i, c): column c of L^{-1} by forward substitution
-  for (int c = tid; c < m; c += CHT) {
-    for (int i = 0; i < c; ++i) It[c + (long long)i * m] = 0.0;
-    for (int i = c; i < m; ++i) {
-      double s = (i == c) ? 1.0 : 0.0;
-      for (int l = c; l < i; ++l) s -= S[l * ld + i] * It[c + (long long)l * m];
-      It[c + (long long)i * m] = s / S[i * ld + i];
+  __syncthreads();
+  // It(c, i) = L^{-1}(i, c): row l of L^{-1} is final before step l, times rd[l]
+  for (int l = 0; l < m - 1; ++l) {
+    const int tot = (l + 1) * (m - l - 1);
+    for (int e = tid; e < tot; e += CHT) {
+      const int ii = e / (l + 1), c = e - ii * (l + 1), i = l + 1 + ii;
+      const double x = c == l ? rd[l] : S[l * ld + c] * rd[l];
+      S[i * ld + c] = fma(-S[l * ld + i], x, S[i * ld + c]);
     }
+    __syncthreads();
+  }
+  for (int e = tid; e < m * m; e += CHT) {
+    const int i = e / m, c = e - i * m;
+    It[(long long)i * m + c] = c < i ? S[i * ld + c] * rd[i] : c == i ? rd[i] : 0.0;
   }
 }
 
@@ -124,156 +143,165 @@ __global__ void k_ch_zero_own(const ChNode *__restrict__ nd, double *__restrict_
   }
 }
 
-// The QL step of one compressed node (one CTA; m <= 128).  In: L, It = L^{-T}
-// (scratch slot), V1 = the first rk right singular vectors (P, ld m).  Out: Qt
-// and Lt (m x m each, the factor store), W = It V1 Lt22^T (m x rk, scratch).
-//   1. Householder QR of V1 (m x rk); the columns rk .. m-1 of its orthogonal
-//      factor span the complement V2.  Q = [V2 V1].
-//   2. M = L Q in shared memory; QL factorisation M = Qt Lt by Householder
-//      reflectors from the last column up (DGEQL2's order), Qt formed
-//      explicitly.
-__global__ void __launch_bounds__(CHT)
+// One reflector step.  Vector j sits at vec(j), entry i at stride s; the reflector is
+// [1 at pv; v(t0:t1) * scale], its parameters in hp[k & 1].  The last warp takes the
+// vector nxt alone (null: none) and forms the next reflector from it, entry npv and tail
+// nt0:nt1; the other threads take cnt vectors, up to eight threads a vector.
+template <class Vec>
+__device__ void ch_reflect(double *v, double *nxt, int s, int t0, int t1, int pv, int nt0, int nt1,
+                           int npv, HousePar *hp, int k, int cnt, Vec vec, double *part) {
+  const int tid = threadIdx.x, lane = tid & 31;
+  const HousePar h = hp[k & 1];
+  double *pe = nullptr, ptw = 0.0;  // this thread's entry pv, and its change
+  if (tid >= CHT) {
+    if (nxt) {
+      if (h.tau != 0.0) {
+        double d = 0.0;
+        for (int i = t0 + lane; i < t1; i += 32) d = fma(v[i * s], nxt[i * s], d);
+        d = warp_sum(d);
+        const double tw = h.tau * fma(h.scale, d, nxt[pv * s]), tws = tw * h.scale;
+        for (int i = t0 + lane; i < t1; i += 32) nxt[i * s] = fma(-tws, v[i * s], nxt[i * s]);
+        __syncwarp();
+        if (lane == 0) nxt[pv * s] -= tw;
+      }
+      double a = 0.0;
+      for (int i = nt0 + lane; i < nt1; i += 32) { const double x = nxt[i * s]; a = fma(x, x, a); }
+      a = warp_sum(a);
+      if (lane == 0) hp[(k + 1) & 1] = house_par(nxt[npv * s], a);
+    }
+  } else if (cnt > 0 && h.tau != 0.0) {
+    if (cnt > CHT / 2) {
+      for (int j = tid; j < cnt; j += CHT) {
+        double *x = vec(j), d = 0.0;
+        for (int i = t0; i < t1; ++i) d = fma(v[i * s], x[i * s], d);
+        const double tw = h.tau * fma(h.scale, d, x[pv * s]), tws = tw * h.scale;
+        for (int i = t0; i < t1; ++i) x[i * s] = fma(-tws, v[i * s], x[i * s]);
+        x[pv * s] -= tw;
+      }
+    } else {
+      const int nch = min(CHT / cnt, 8), ch = tid / cnt, j = tid - ch * cnt;
+      const bool act = ch < nch;
+      double *x = vec(j), d = 0.0;
+      const int i0 = t0 + (t1 - t0) * ch / nch, i1 = act ? t0 + (t1 - t0) * (ch + 1) / nch : i0;
+      for (int i = i0; i < i1; ++i) d = fma(v[i * s], x[i * s], d);
+      if (act) part[ch * cnt + j] = d;
+      asm volatile("bar.sync 1, %0;" ::"n"(CHT) : "memory");
+      if (act) {
+        d = 0.0;
+        for (int c = 0; c < nch; ++c) d += part[c * cnt + j];
+        const double tw = h.tau * fma(h.scale, d, x[pv * s]), tws = tw * h.scale;
+        for (int i = i0; i < i1; ++i) x[i * s] = fma(-tws, v[i * s], x[i * s]);
+        if (ch == 0) { pe = x + pv * s; ptw = tw; }
+      }
+    }
+  }
+  __syncthreads();
+  if (pe) *pe -= ptw;  // (every chunk has read it, and no later step does)
+  if (tid == 0) v[pv * s] = h.beta;
+}
+
+// The QL step of one compressed node (one CTA; m <= 128).  In: L (scratch slot), V1 =
+// the first rk right singular vectors (P, ld m).  Out: Qt and Lt (m x m each, the
+// factor store), W = L^{-T} V1 Lt22^T up to rounding (m x rk, scratch).
+//   1. QL of L V1 = Qt2 Lt22 (rk reflectors from the last column up, DGEQL2's order),
+//      each applied to L and to the identity as well: they end as Qt^T L = [L1; L2]
+//      and Qt^T.  V2 is not formed: Qt1 spans the complement of L V1, so the rows of
+//      L1 span that of V1.
+//   2. LQ of L1 = Lt11 V2^T by ir reflectors on the right, L2 V2 = Lt21 with it.
+//   3. The eliminated variables' Schur step: W = Qt [-Lt11^{-T} Lt21^T; I].
+// That is m reflector steps (forming V2 first, then the QL of L [V2 V1], and Qt from
+// its reflectors took 2 m + 2 rk, a thread per column: n = 8192 with 32-row leaves
+// 3.08 -> 0.77 ms in all).  Bound by the steps' chains, about 20 FP64 instructions a warp each
+// at m = 32.  L, L V1 and Qt^T sit in shared memory, the last two in global memory
+// (sm = 0) where a level's nodes are too large.
+__global__ void __launch_bounds__(CHT + 32)
 k_ch_node(const ChNode *__restrict__ nd, const double *__restrict__ Lb,
-          const double *__restrict__ Ib, const double *__restrict__ Pb, double *__restrict__ Gb,
-          double *__restrict__ fac, double *__restrict__ Wb) {
-  extern __shared__ double S[];  // M, column j at S + j * (m + 1)
-  __shared__ double tau[CH_MAXM], sc[CH_MAXM], red[CHT / 32];
-  __shared__ double s_beta;
+          const double *__restrict__ Pb, double *__restrict__ Gb, double *__restrict__ fac,
+          double *__restrict__ Wb, int sm) {
+  extern __shared__ double S[];
+  __shared__ double rd[CH_MAXM], part[CHT];
+  __shared__ HousePar hp[2];
   const ChNode q = nd[blockIdx.x];
-  const int m = q.m, rk = q.rk, ir = q.ir, ld = m + 1, tid = threadIdx.x;
-  const int lane = tid & 31, wid = tid >> 5;
+  const int m = q.m, rk = q.rk, ir = q.ir, ld = m | 1, tid = threadIdx.x, lane = tid & 31;
+  constexpr int NT = CHT + 32;
   const size_t so = (size_t)q.slot * CH_SLOT;
-  const double *L = Lb + so, *It = Ib + so, *P = Pb + so;
-  double *G = Gb + 4 * so;          // Householder QR of V1 (m x rk)
-  double *Q = G + CH_SLOT;          // [V2 V1]
-  double *Vq = Q + CH_SLOT;         // QL reflectors (column c: rows 0..c-1)
-  double *Y = Vq + CH_SLOT;         // It V1
+  const double *L = Lb + so, *P = Pb + so;
+  double *A2 = S;                                   // L, then [Lt11; Lt21] (columns < ir)
+  double *T = sm ? S + (size_t)m * ld : Gb + 4 * so;  // I, then Qt^T
+  double *A1 = T + (size_t)m * ld;                  // L V1, then Lt22 under Z
   double *Qt = fac + q.f, *Lt = Qt + (size_t)m * m;
   double *W = Wb + so;
-  for (int e = tid; e < m * rk; e += CHT) G[e] = P[e];
+  for (int e = tid; e < m * m; e += NT) {
+    const int j = e / m, i = e - j * m;
+    A2[j * ld + i] = L[e];
+    T[j * ld + i] = i == j ? 1.0 : 0.0;
+  }
   __syncthreads();
-  // ---- 1. QR of V1: reflector k = [1; G(k+1:m, k) * sc[k]]
+  for (int e = tid; e < m * rk; e += NT) {
+    const int j = e / m, i = e - j * m;
+    double s = 0.0;
+    for (int l = 0; l <= i; ++l) s = fma(A2[l * ld + i], P[(long long)j * m + l], s);
+    A1[j * ld + i] = s;
+  }
+  __syncthreads();
+  // the first reflector of a sequence, by the last warp
+  auto first = [&](const double *v, int s, int t0, int t1, int pv) {
+    if (tid >= CHT) {
+      double a = 0.0;
+      for (int i = t0 + lane; i < t1; i += 32) a = fma(v[i * s], v[i * s], a);
+      a = warp_sum(a);
+      if (lane == 0) hp[0] = house_par(v[pv * s], a);
+    }
+    __syncthreads();
+  };
+  if (rk > 0) first(A1 + (rk - 1) * ld, 1, 0, m - 1, m - 1);
   for (int k = 0; k < rk; ++k) {
-    double a = 0.0;
-    for (int i = k + 1 + tid; i < m; i += CHT) { const double x = G[k * m + i]; a = fma(x, x, a); }
-    a = warp_sum(a);
-    if (lane == 0) red[wid] = a;
-    __syncthreads();
-    if (tid == 0) {
-      double s = 0.0;
-      for (int w = 0; w < CHT / 32; ++w) s += red[w];
-      const double alpha = G[k * m + k];
-      double beta = alpha, t = 0.0, scl = 0.0;
-      if (s > 0.0) {
-        beta = -copysign(sqrt(fma(alpha, alpha, s)), alpha);
-        t = (beta - alpha) / beta;
-        scl = 1.0 / (alpha - beta);
+    const int c = rk - 1 - k, p = ir + c, ca = max(c - 1, 0);
+    ch_reflect(A1 + c * ld, c > 0 ? A1 + (c - 1) * ld : nullptr, 1, 0, p, p, 0, p - 1, p - 1, hp, k,
+               ca + 2 * m,
+               [=](int j) { return j < ca ? A1 + j * ld : j < ca + m ? A2 + (j - ca) * ld : T + (j - ca - m) * ld; },
+               part);
+  }
+  __syncthreads();
+  first(A2, ld, 1, m, 0);
+  for (int k = 0; k < ir; ++k) {
+    const bool la = k + 1 < ir;  // (the rows from ir on form no reflector)
+    const int j0 = la ? k + 2 : k + 1;
+    ch_reflect(A2 + k, la ? A2 + k + 1 : nullptr, ld, k + 1, m, k, k + 2, m, k + 1, hp, k, m - j0,
+               [=](int j) { return A2 + j0 + j; }, part);
+  }
+  __syncthreads();
+  for (int e = tid; e < m * m; e += NT) {
+    const int j = e / m, i = e - j * m;
+    Lt[e] = i < j ? 0.0 : j < ir ? A2[j * ld + i] : A1[(j - ir) * ld + i];
+    Qt[e] = T[i * ld + j];
+  }
+  for (int i = tid; i < ir; i += NT) rd[i] = 1.0 / A2[i * ld + i];
+  // Z = Lt11^{-T} Lt21^T in rows 0 .. ir-1 of A1 (row i times rd[i])
+  for (int e = tid; e < ir * rk; e += NT) {
+    const int j = e / ir, i = e - j * ir;
+    A1[j * ld + i] = A2[i * ld + ir + j];
+  }
+  __syncthreads();
+  if (rk > 0) {
+    const int nch = NT / rk, ch = tid / rk, j = tid - ch * rk;
+    for (int i = ir - 1; i > 0; --i) {
+      if (ch < nch) {
+        const double z = A1[j * ld + i] * rd[i];
+        for (int l = ch; l < i; l += nch) A1[j * ld + l] = fma(-A2[l * ld + i], z, A1[j * ld + l]);
       }
-      tau[k] = t; sc[k] = scl; s_beta = beta;
-    }
-    __syncthreads();
-    const double t = tau[k], scl = sc[k];
-    for (int j = k + 1 + tid; j < rk; j += CHT) {  // columns to the right
-      double w = G[j * m + k];
-      for (int i = k + 1; i < m; ++i) w = fma(G[k * m + i] * scl, G[j * m + i], w);
-      w *= t;
-      G[j * m + k] -= w;
-      for (int i = k + 1; i < m; ++i) G[j * m + i] = fma(-w * scl, G[k * m + i], G[j * m + i]);
-    }
-    __syncthreads();
-    for (int i = k + 1 + tid; i < m; i += CHT) G[k * m + i] *= scl;
-    if (tid == 0) G[k * m + k] = s_beta;
-    __syncthreads();
-  }
-  // ---- complement: Q(:, c) = H_0 ... H_{rk-1} e_{rk + c}, c < ir; Q(:, ir + t) = V1(:, t)
-  for (int c = tid; c < ir; c += CHT) {
-    double *x = Q + (long long)c * m;
-    for (int i = 0; i < m; ++i) x[i] = (i == rk + c) ? 1.0 : 0.0;
-    for (int k = rk - 1; k >= 0; --k) {
-      double w = x[k];
-      for (int i = k + 1; i < m; ++i) w = fma(G[k * m + i], x[i], w);
-      w *= tau[k];
-      x[k] -= w;
-      for (int i = k + 1; i < m; ++i) x[i] = fma(-w, G[k * m + i], x[i]);
+      __syncthreads();
     }
   }
-  for (int e = tid; e < m * rk; e += CHT) Q[(long long)ir * m + e] = P[e];
-  __syncthreads();
-  // ---- 2. M = L Q
-  for (int e = tid; e < m * m; e += CHT) {
-    const int j = e / m, i = e - j * m;
-    double s = 0.0;
-    for (int l = 0; l <= i; ++l) s = fma(L[(long long)l * m + i], Q[(long long)j * m + l], s);
-    S[j * ld + i] = s;
+  for (int e = tid; e < ir * rk; e += NT) {
+    const int j = e / ir, i = e - j * ir;
+    A1[j * ld + i] *= rd[i];
   }
   __syncthreads();
-  // QL: column c, reflector v = [S(0:c-1, c) * sc; 1] acting on rows 0..c
-  for (int c = m - 1; c >= 0; --c) {
-    double a = 0.0;
-    for (int i = tid; i < c; i += CHT) { const double x = S[c * ld + i]; a = fma(x, x, a); }
-    a = warp_sum(a);
-    if (lane == 0) red[wid] = a;
-    __syncthreads();
-    if (tid == 0) {
-      double s = 0.0;
-      for (int w = 0; w < CHT / 32; ++w) s += red[w];
-      const double alpha = S[c * ld + c];
-      double beta = alpha, t = 0.0, scl = 0.0;
-      if (s > 0.0) {
-        beta = -copysign(sqrt(fma(alpha, alpha, s)), alpha);
-        t = (beta - alpha) / beta;
-        scl = 1.0 / (alpha - beta);
-      }
-      tau[c] = t; sc[c] = scl; s_beta = beta;
-    }
-    __syncthreads();
-    const double t = tau[c], scl = sc[c];
-    for (int j = tid; j < c; j += CHT) {  // columns to the left, rows 0..c
-      double w = S[j * ld + c];
-      for (int i = 0; i < c; ++i) w = fma(S[c * ld + i] * scl, S[j * ld + i], w);
-      w *= t;
-      S[j * ld + c] -= w;
-      for (int i = 0; i < c; ++i) S[j * ld + i] = fma(-w * scl, S[c * ld + i], S[j * ld + i]);
-    }
-    __syncthreads();
-    for (int i = tid; i < c; i += CHT) {
-      Vq[(long long)c * m + i] = S[c * ld + i] * scl;
-      S[c * ld + i] = 0.0;
-    }
-    if (tid == 0) S[c * ld + c] = s_beta;
-    __syncthreads();
-  }
-  // Lt = S (lower triangular now)
-  for (int e = tid; e < m * m; e += CHT) {
+  for (int e = tid; e < m * rk; e += NT) {
     const int j = e / m, i = e - j * m;
-    Lt[e] = i >= j ? S[j * ld + i] : 0.0;
-  }
-  // Qt = H_{m-1} ... H_0 (H_0 applied first), column j on thread j
-  for (int j = tid; j < m; j += CHT) {
-    double *x = Qt + (long long)j * m;
-    for (int i = 0; i < m; ++i) x[i] = (i == j) ? 1.0 : 0.0;
-    for (int c = 0; c < m; ++c) {
-      if (tau[c] == 0.0) continue;
-      double w = x[c];
-      for (int i = 0; i < c; ++i) w = fma(Vq[(long long)c * m + i], x[i], w);
-      w *= tau[c];
-      x[c] -= w;
-      for (int i = 0; i < c; ++i) x[i] = fma(-w, Vq[(long long)c * m + i], x[i]);
-    }
-  }
-  // Y = It V1 (It upper triangular)
-  for (int e = tid; e < m * rk; e += CHT) {
-    const int t = e / m, i = e - t * m;
-    double s = 0.0;
-    for (int l = i; l < m; ++l) s = fma(It[(long long)l * m + i], P[(long long)t * m + l], s);
-    Y[(long long)t * m + i] = s;
-  }
-  __syncthreads();
-  // W = Y Lt22^T: W(i, j) = sum_{t <= j} Y(i, t) Lt(ir + j, ir + t)
-  for (int e = tid; e < m * rk; e += CHT) {
-    const int j = e / m, i = e - j * m;
-    double s = 0.0;
-    for (int t = 0; t <= j; ++t) s = fma(Y[(long long)t * m + i], S[(ir + t) * ld + ir + j], s);
+    double s = T[i * ld + ir + j];
+    for (int l = 0; l < ir; ++l) s = fma(-T[i * ld + l], A1[j * ld + l], s);
     W[(long long)j * m + i] = s;
   }
 }
@@ -520,6 +548,7 @@ static void set_smem(const void *fn, size_t bytes) {
 }
 
 constexpr size_t CH_SMEM = (size_t)CH_MAXM * (CH_MAXM + 1) * sizeof(double);
+constexpr size_t CH_NODE_SMEM = 220 * 1024;  // of the 227 KB a CTA can have
 
 // Factor A (n x n, lda; read only), leaves of ni rows (npart's tree), singular
 // values above tol kept, at most ncol per node.  ps = 0: the scaled block
@@ -540,7 +569,7 @@ int hss_chol_factor_core(int n, const double *A, long long lda, int ni, double t
   static bool attr = false;
   if (!attr) {
     set_smem((const void *)k_ch_chol, CH_SMEM);
-    set_smem((const void *)k_ch_node, CH_SMEM);
+    set_smem((const void *)k_ch_node, CH_NODE_SMEM);
     attr = true;
   }
   const size_t nn = (size_t)n * n;
@@ -596,11 +625,14 @@ int hss_chol_factor_core(int n, const double *A, long long lda, int ni, double t
     if (!cand.empty()) {
       ChNode *dc = pool<ChNode>("hc_cand", cand.size());
       stage_h2d(dc, cand.data(), cand.size() * sizeof(ChNode), st);
-      k_ch_chol<<<(unsigned)cand.size(), CHT, CH_SMEM, st>>>(dc, cur, Nc, Lb, Ib, status);
+      int mm = 0;  // the shared memory of the level's largest block: more CTAs per SM
+      for (auto &q : cand) mm = std::max(mm, q.m);
+      k_ch_chol<<<(unsigned)cand.size(), CHT, sizeof(double) * mm * (mm | 1), st>>>(dc, cur, Nc, Lb,
+                                                                                   Ib, status);
       std::vector<GemmDesc> g;  // X(:, I) = Ah(:, I) L^{-T}
       for (auto &q : cand)
         g.push_back(GemmDesc{cur + (long long)q.o * Nc, Ib + (size_t)q.slot * CH_SLOT,
-                             X + (long long)q.o * Nc, Nc, q.m, Nc, Nc, q.m, q.m, 0, 0});
+                             X + (long long)q.o * Nc, Nc, q.m, Nc, Nc, q.m, q.m, 0, 0, 1});
       launch_gemm(g, 0, st);
       k_ch_zero_own<<<(unsigned)cand.size(), 256, 0, st>>>(dc, X, Nc);
       std::vector<const double *> xs;
@@ -666,7 +698,14 @@ int hss_chol_factor_core(int n, const double *A, long long lda, int ni, double t
     if (!comp.empty()) {
       ChNode *dq = pool<ChNode>("hc_comp", comp.size());
       stage_h2d(dq, comp.data(), comp.size() * sizeof(ChNode), st);
-      k_ch_node<<<(unsigned)comp.size(), CHT, CH_SMEM, st>>>(dq, Lb, Ib, Pb, Gb, L.fac, Wb);
+      size_t all = 0, l2 = 0;
+      for (auto &q : comp) {
+        all = std::max(all, sizeof(double) * (q.m | 1) * (2 * q.m + q.rk));
+        l2 = std::max(l2, sizeof(double) * (q.m | 1) * q.m);
+      }
+      const int sm = all <= CH_NODE_SMEM;
+      k_ch_node<<<(unsigned)comp.size(), CHT + 32, sm ? all : l2, st>>>(dq, Lb, Pb, Gb, L.fac, Wb,
+                                                                       sm);
     }
     // congruence Ah' = W^T Ah W: X2 = Ah W, Xt = X2^T, Ah' = Xt W
     {

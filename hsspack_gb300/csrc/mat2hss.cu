@@ -110,31 +110,6 @@ __device__ __forceinline__ int group_size(int groups) {
   return gs;
 }
 
-struct HousePar {
-  double beta, tau, scale;
-};
-// (one lane forms it, at a warp's FP64 price: root, reciprocal root and reciprocal
-// from estimates, each within about an ulp)
-__device__ __forceinline__ HousePar house_par(double alpha, double sg) {
-  HousePar h{alpha, 0.0, 0.0};
-  if (sg > 0.0) {
-    const double x = fma(alpha, alpha, sg);
-    const int hx = __double2hiint(x);
-    if (hx >= 0x03f00000 && hx < 0x7bf00000) {  // 2^-960 <= x < 2^960
-      double rt, ri;
-      sqrt_pair(x, rt, ri);
-      h.beta = -copysign(rt, alpha);
-      h.tau = (h.beta - alpha) * -copysign(ri, alpha);
-      h.scale = rcp_nr(alpha - h.beta);
-    } else {
-      h.beta = -copysign(sqrt(x), alpha);
-      h.tau = (h.beta - alpha) / h.beta;
-      h.scale = 1.0 / (alpha - h.beta);
-    }
-  }
-  return h;
-}
-
 // Householder QR of the tile [R; C]: rows 0..r-1 hold the upper triangular R
 // so far, rows r..r+na-1 a chunk of the tall matrix; on return rows 0..r-1
 // hold the R factor of both.  Column k's reflector has nonzeros only in row k
