@@ -115,8 +115,8 @@ struct PoleDiff {
   const double *__restrict__ difr;
   bool sq = false;
   __device__ __forceinline__ double fd(int p, int q) const {
-    const double lin = p <= q ? (__ldg(F + p) - __ldg(F + q)) - __ldg(difl + q)
-                              : (__ldg(F + p) - __ldg(F + q + 1)) - __ldg(difr + q);
+    // (operands chosen before the subtractions: those take the FP64 pipe either way)
+    const double lin = (__ldg(F + p) - __ldg(F + (p <= q ? q : q + 1))) - __ldg((p <= q ? difl : difr) + q);
     return sq ? lin * (__ldg(F + p) + (__ldg(F + q) + __ldg(difl + q))) : lin;
   }
   // a - b for two pole values (a^2 - b^2 in singular-value mode)

@@ -85,6 +85,28 @@ __device__ __forceinline__ SecSums sec_eval(const double *__restrict__ d,
   return s;
 }
 
+// Comparisons of doubles as integers: a root's step has twenty of them, and each
+// would take as much of the FP64 pipe as a multiply-add.  mag_bits orders |x| (NaN above
+// infinity); less_b is x < y, false for a NaN on either side.
+__device__ __forceinline__ unsigned long long mag_bits(double x) {
+  return (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffull;
+}
+__device__ __forceinline__ bool is_zero(double x) { return mag_bits(x) == 0; }
+__device__ __forceinline__ bool sign_bit(double x) { return __double2hiint(x) < 0; }
+__device__ __forceinline__ bool is_neg(double x) {  // x < 0
+  const unsigned long long u = (unsigned long long)__double_as_longlong(x);
+  return u > 0x8000000000000000ull && u <= 0xfff0000000000000ull;
+}
+__device__ __forceinline__ long long order_bits(double x) {  // -0 and +0 alike
+  const long long m = (long long)mag_bits(x), s = __double_as_longlong(x) >> 63;
+  return (m ^ s) - s;
+}
+__device__ __forceinline__ bool less_b(double x, double y) {
+  constexpr long long inf = 0x7ff0000000000000ll;
+  const long long a = order_bits(x), b = order_bits(y);
+  return a < b && a >= -inf && b <= inf;
+}
+
 // Root of  c + A/(da - t) + B/(db - t) = 0  inside (lo, hi); returns false if
 // neither root of the equivalent quadratic lies there.
 __device__ __forceinline__ bool two_pole_root(double c, double A, double B, double da,
@@ -94,20 +116,20 @@ __device__ __forceinline__ bool two_pole_root(double c, double A, double B, doub
   const double a1 = -(c * (da + db) + A + B);
   const double a0 = c * da * db + A * db + B * da;
   double r1, r2;
-  if (a2 == 0.0) {
-    if (a1 == 0.0) return false;
+  if (is_zero(a2)) {
+    if (is_zero(a1)) return false;
     r1 = r2 = -a0 / a1;
   } else {
     double disc = a1 * a1 - 4.0 * a2 * a0;
-    if (disc < 0.0) disc = 0.0;
+    if (is_neg(disc)) disc = 0.0;
     const double q = -0.5 * (a1 + copysign(sqrt(disc), a1));
     r1 = q / a2;
-    r2 = (q != 0.0) ? a0 / q : r1;
+    r2 = !is_zero(q) ? a0 / q : r1;
   }
-  const bool ok1 = r1 > lo && r1 < hi, ok2 = r2 > lo && r2 < hi;
+  const bool ok1 = less_b(lo, r1) && less_b(r1, hi), ok2 = less_b(lo, r2) && less_b(r2, hi);
   if (ok1 && ok2) {  // both inside: take the one nearer the bracket middle
     const double m = 0.5 * (lo + hi);
-    t = fabs(r1 - m) <= fabs(r2 - m) ? r1 : r2;
+    t = mag_bits(r1 - m) <= mag_bits(r2 - m) ? r1 : r2;
     return true;
   }
   if (ok1) { t = r1; return true; }
@@ -206,44 +228,42 @@ __device__ __forceinline__ void root_step(RootState &r, const SecSums &s) {
     // two-pole model with the far poles frozen at the midpoint value
     const double gl = gap(r, r.jl) - r.tau, gr = gap(r, r.jr) - r.tau;
     const double c = w - zl * (zl / gl) - zr * (zr / gr);
-    double t;
-    if (!r.last) {
-      const double tm = r.tau;
-      if (w >= 0.0) {  // root in (d_j, midpoint]
-        r.lo = 0.0; r.hi = tm;
-        if (!two_pole_root(c, zl * zl, zr * zr, 0.0, r.delta, r.lo, r.hi, t)) t = 0.5 * tm;
-      } else {         // root in (midpoint, d_{j+1}): measure from d_{j+1}
-        r.oi = r.j + 1;
-        r.lo = tm - r.delta; r.hi = 0.0;
-        if (!two_pole_root(c, zl * zl, zr * zr, -r.delta, 0.0, r.lo, r.hi, t)) t = 0.5 * r.lo;
-      }
-    } else {
-      const double tm = r.tau;
-      const double da = gap(r, r.jl);
+    // the bracket and the poles' offsets first, then one solve for all three forms
+    double t, da, db;
+    const double tm = r.tau;
+    if (r.last) {
+      da = gap(r, r.jl); db = 0.0;
       if (w >= 0.0) { r.lo = 0.0; r.hi = tm; }
       else { r.lo = tm; r.hi = r.top * (1.0 + 4.0 * HSS_EPS); }
-      if (!two_pole_root(c, zl * zl, zr * zr, da, 0.0, r.lo, r.hi, t)) t = 0.5 * (r.lo + r.hi);
+    } else if (w >= 0.0) {  // root in (d_j, midpoint]
+      da = 0.0; db = r.delta;
+      r.lo = 0.0; r.hi = tm;
+    } else {                // root in (midpoint, d_{j+1}): measure from d_{j+1}
+      r.oi = r.j + 1;
+      da = -r.delta; db = 0.0;
+      r.lo = tm - r.delta; r.hi = 0.0;
     }
+    if (!two_pole_root(c, zl * zl, zr * zr, da, db, r.lo, r.hi, t)) t = 0.5 * (r.lo + r.hi);
     r.tau = t;
     r.phase = 1;
     return;
   }
   // middle-way step
   const double dw = s.dpsi + s.dphi;
-  if (!(fabs(w) <= 1.7e308) || !(dw <= 1.7e308)) {  // overflow next to a pole: bisect
+  if (mag_bits(w) > mag_bits(1.7e308) || mag_bits(dw) > mag_bits(1.7e308)) {  // overflow next to a pole: bisect
     if (r.iters > 41) { r.status = HSS_SECULAR_NOCONV; r.phase = 2; return; }
     r.learned = false;
     r.tau = 0.5 * (r.lo + r.hi);
     return;
   }
   const double erretm = 8.0 * s.eabs + 2.0 * r.rhoinv + 3.0 * fabs(r.tau) * dw;
-  if (fabs(w) <= HSS_EPS * erretm) { r.phase = 2; return; }
+  if (mag_bits(w) <= mag_bits(HSS_EPS * erretm)) { r.phase = 2; return; }
   if (r.iters > 41) { r.status = HSS_SECULAR_NOCONV; r.phase = 2; return; }
   if (r.learned && r.iters == r.first) {
     // residual check of the learned start: a Newton step across most of the
     // half interval means the start is unusable; restart from the standard guess
     r.learned = false;
-    if (!(fabs(w / dw) <= 0.45 * r.delta)) {
+    if (!(mag_bits(w) <= mag_bits(0.45 * r.delta * dw))) {
       r.fell_back = true;
       r.prew = 0.0;
       r.prel = -1.0;
@@ -254,9 +274,13 @@ __device__ __forceinline__ void root_step(RootState &r, const SecSums &s) {
     }
   }
   // a residual that kept its sign and fell by less than 10x: change the model
-  if (!r.last && w * r.prew > 0.0 && fabs(w) > 0.1 * fabs(r.prew)) r.fw = !r.fw;
+  // (w is not 0 from here on; prew = 0: no previous step)
+  if (!r.last && !is_zero(r.prew) && sign_bit(w) == sign_bit(r.prew) &&
+      mag_bits(w) > mag_bits(0.1 * r.prew))
+    r.fw = !r.fw;
   r.prew = w;
-  if (w < 0.0) r.lo = fmax(r.lo, r.tau); else r.hi = fmin(r.hi, r.tau);
+  if (sign_bit(w)) { if (less_b(r.lo, r.tau)) r.lo = r.tau; }
+  else if (less_b(r.tau, r.hi)) r.hi = r.tau;
   // Two-pole model  c + s_l/(gl - eta) + s_r/(gr - eta)  matching w and dw at
   // eta = 0; cleared of denominators it is  c eta^2 - a eta + b = 0, and only
   // c depends on how dw is shared between the two poles.
@@ -279,23 +303,27 @@ __device__ __forceinline__ void root_step(RootState &r, const SecSums &s) {
     // the root lies beyond both poles (gl, gr < 0): the larger root of the
     // quadratic; c < 0 only from rounding
     c = fabs(c);
-    if (c == 0.0) {
+    if (is_zero(c)) {
       eta = r.hi - r.tau;  // no root beyond the poles: bisect
     } else {
       double disc = a * a - 4.0 * b * c;
       if (disc < 0.0) disc = 0.0;
       eta = (a >= 0.0) ? qdiv(a + sqrt(disc), 2.0 * c) : qdiv(2.0 * b, a - sqrt(disc));
     }
-  } else if (c == 0.0) {
-    eta = (a != 0.0) ? qdiv(b, a) : -qdiv(w, dw);
-  } else {  // the root between the two poles
+  } else if (is_zero(c)) {
+    eta = !is_zero(a) ? qdiv(b, a) : -qdiv(w, dw);
+  } else {  // the root between the two poles, both forms by one root and one divide
     double disc = a * a - 4.0 * b * c;
-    if (disc < 0.0) disc = 0.0;
-    eta = (a <= 0.0) ? qdiv(a - sqrt(disc), 2.0 * c) : qdiv(2.0 * b, a + sqrt(disc));
+    if (is_neg(disc)) disc = 0.0;
+    const bool neg = sign_bit(a) || is_zero(a);
+    const double sq = sqrt(disc), e = a + (neg ? -sq : sq), f = 2.0 * (neg ? c : b);
+    eta = qdiv(neg ? e : f, neg ? f : e);
   }
-  if (w * eta >= 0.0) eta = -qdiv(w, dw);  // model went the wrong way: Newton step
+  const double we = w * eta;
+  if (!is_neg(we) && mag_bits(we) <= mag_bits(HUGE_VAL))
+    eta = -qdiv(w, dw);  // model went the wrong way: Newton step
   double tn = r.tau + eta;
-  const bool bisect = !(tn > r.lo && tn < r.hi);
+  const bool bisect = !(less_b(r.lo, tn) && less_b(tn, r.hi));
   if (bisect) {
     // bisect; geometrically when the bracket spans decades on one side of the
     // origin (roots next to a pole sit many decades below the interval)
@@ -306,13 +334,14 @@ __device__ __forceinline__ void root_step(RootState &r, const SecSums &s) {
   const double step = tn - r.tau;
   r.tau = tn;
   if (!r.last) {  // keep the origin at the pole nearer the iterate
-    if (r.oi == r.j && r.tau > 0.5 * r.delta) {
-      r.oi = r.j + 1; r.tau -= r.delta; r.lo -= r.delta; r.hi -= r.delta;
-    } else if (r.oi == r.j + 1 && r.tau < -0.5 * r.delta) {
-      r.oi = r.j; r.tau += r.delta; r.lo += r.delta; r.hi += r.delta;
+    if (mag_bits(r.tau) > mag_bits(0.5 * r.delta) && sign_bit(r.tau) == (r.oi != r.j)) {
+      const double sh = r.oi == r.j ? -r.delta : r.delta;
+      r.oi = r.oi == r.j ? r.j + 1 : r.j;
+      r.tau += sh; r.lo += sh; r.hi += sh;
     }
   }
-  if (fabs(step) <= 2.0 * HSS_EPS * fabs(r.tau) || r.hi - r.lo <= 2.0 * HSS_EPS * fabs(r.tau)) {
+  const double te = 2.0 * HSS_EPS * fabs(r.tau);
+  if (mag_bits(step) <= mag_bits(te) || !less_b(te, r.hi - r.lo)) {
     r.phase = 2;
     return;
   }
@@ -320,8 +349,9 @@ __device__ __forceinline__ void root_step(RootState &r, const SecSums &s) {
   // distance to the origin pole, and at most 100 x the square of the
   // previous relative step): the new iterate's error is below 1e-18 of that
   // distance, so it is final without another evaluation.
-  const double rel = qdiv(fabs(step), fmax(fabs(r.tau), 1e-300));
-  if (!bisect && r.prel >= 0.0 && rel <= 1e-10 && rel <= 100.0 * r.prel * r.prel) {
+  const double rel = qdiv(fabs(step), mag_bits(r.tau) < mag_bits(1e-300) ? 1e-300 : fabs(r.tau));
+  if (!bisect && !sign_bit(r.prel) && mag_bits(rel) <= mag_bits(1e-10) &&
+      mag_bits(rel) <= mag_bits(100.0 * r.prel * r.prel)) {
     r.phase = 2;
     return;
   }
@@ -333,8 +363,7 @@ __device__ __forceinline__ void root_step(RootState &r, const SecSums &s) {
 template <bool SQ>
 __device__ __forceinline__ void secular_out(RootState &st, int s, double *__restrict__ lam,
                                             double *__restrict__ difl, double *__restrict__ difr,
-                                            int *__restrict__ iters, int *__restrict__ status,
-                                            unsigned long long *__restrict__ itsum) {
+                                            int *__restrict__ iters, int *__restrict__ status) {
   double lm, dfl, dfr;
   if (st.K == 1) {
     const double zz = __ldg(st.z) * __ldg(st.z);
@@ -363,12 +392,23 @@ __device__ __forceinline__ void secular_out(RootState &st, int s, double *__rest
   difl[s + st.j] = dfl;
   difr[s + st.j] = dfr;
   if (iters) iters[s + st.j] = st.iters;
-  if (itsum) {
-    atomicAdd(itsum, (unsigned long long)st.iters);
-    if (st.fell_back) atomicAdd(itsum + 1, 1ull);
-    atomicAdd(itsum + 2, (unsigned long long)st.iters * (unsigned long long)st.K);  // pole terms
-  }
   if (st.status) atomicMax(status, st.status);
+}
+
+// A warp's evaluations, restarts and pole terms (itsum[0..2]), added up first: one
+// atomic per root on the same three words would serialise a level's roots.  All lanes.
+__device__ __forceinline__ void secular_count(unsigned long long *itsum, int it, int fb,
+                                              unsigned long long terms) {
+  if (!itsum) return;
+  it = __reduce_add_sync(HSS_FULL, it);
+  fb = __reduce_add_sync(HSS_FULL, fb);
+  const unsigned lo = __reduce_add_sync(HSS_FULL, (unsigned)(terms & 0xffffffu));
+  const unsigned hi = __reduce_add_sync(HSS_FULL, (unsigned)(terms >> 24));
+  if ((threadIdx.x & 31) == 0) {
+    if (it) atomicAdd(itsum, (unsigned long long)it);
+    if (fb) atomicAdd(itsum + 1, (unsigned long long)fb);
+    if (it) atomicAdd(itsum + 2, ((unsigned long long)hi << 24) + lo);
+  }
 }
 
 // One lane per root with a sequence of roots per lane (wide levels): lane l of
@@ -392,7 +432,8 @@ __device__ __forceinline__ void secular_lanes(const LevelView &lv, const double 
   RootState st;
   st.K = 0; st.j = 0; st.jl = 0; st.oi = 0; st.tau = 0.0; st.phase = 2;
   st.d = dl; st.z = zw;
-  int s = 0;
+  int s = 0, cit = 0, cfb = 0;
+  unsigned long long cterms = 0;
   bool act = false;
   auto next = [&]() {  // the lane's next root that needs the iteration
     act = false;
@@ -407,7 +448,7 @@ __device__ __forceinline__ void secular_lanes(const LevelView &lv, const double 
       st.sq = SQ;
       st.oi = 0;
       if (st.K == 1) {
-        secular_out<SQ>(st, s, lam, difl, difr, iters, status, itsum);
+        secular_out<SQ>(st, s, lam, difl, difr, iters, status);
         continue;
       }
       double zsq = 0.0;  // the last root's bound only
@@ -425,12 +466,16 @@ __device__ __forceinline__ void secular_lanes(const LevelView &lv, const double 
     if (act) {
       root_step(st, sm);
       if (st.phase == 2) {
-        secular_out<SQ>(st, s, lam, difl, difr, iters, status, itsum);
+        secular_out<SQ>(st, s, lam, difl, difr, iters, status);
+        cit += st.iters;
+        cfb += st.fell_back;
+        cterms += (unsigned long long)st.iters * (unsigned long long)st.K;
         r += T;
         next();
       }
     }
   }
+  secular_count(itsum, cit, cfb, cterms);
 }
 
 // ------------------------------------------------------------- kernels -----
@@ -492,7 +537,11 @@ k_secular(LevelView lv, const double *__restrict__ dl, const double *__restrict_
       st.phase = __shfl_sync(HSS_FULL, st.phase, lead);
     }
   }
-  if (valid && gl == 0) secular_out<SQ>(st, s, lam, difl, difr, iters, status, itsum);
+  const bool out = valid && gl == 0;
+  if (out) secular_out<SQ>(st, s, lam, difl, difr, iters, status);
+  const bool cnt = out && st.K > 1;
+  secular_count(itsum, cnt ? st.iters : 0, cnt ? st.fell_back : 0,
+                cnt ? (unsigned long long)st.iters * (unsigned long long)st.K : 0ull);
 }
 
 // Loewner: z_hat_i^2 = prod_j (d_i - lam_j) / prod_{j != i} (d_i - d_j)
@@ -502,6 +551,25 @@ k_secular(LevelView lv, const double *__restrict__ dl, const double *__restrict_
 //   Singular-value mode (sq): z_hat_i^2 = prod_j (sigma_j^2 - d_i^2) /
 // prod_{j != i} (d_j^2 - d_i^2) (the z recomputation of DLASD3 / MDLASD8), every
 // factor formed as a product of a difference and a sum.
+//   frexp and ldexp of ordinary numbers by their exponent bits: the library's calls
+// go through the FP64 pipe, which the factors' two subtractions and two multiplies bind.
+__device__ __forceinline__ double frexp_b(double x, int &e) {  // adds the exponent to e
+  const int hi = __double2hiint(x), E = (hi >> 20) & 0x7ff;
+  if ((unsigned)(E - 1) < 2046u) {
+    e += E - 1022;
+    return __hiloint2double((hi & 0x800fffff) | 0x3fe00000, __double2loint(x));
+  }
+  int k = 0;
+  x = frexp(x, &k);
+  e += k;
+  return x;
+}
+__device__ __forceinline__ double ldexp_b(double x, int e) {
+  const int hi = __double2hiint(x), E = (hi >> 20) & 0x7ff;
+  if ((unsigned)(E - 1) < 2046u && e > -4096 && e < 4096 && (unsigned)(E + e - 1) < 2046u)
+    return __hiloint2double(hi + (e << 20), __double2loint(x));
+  return ldexp(x, e);
+}
 template <int L>
 __global__ void k_lowner(LevelView lv, const double *__restrict__ dl,
                          const double *__restrict__ difl, const double *__restrict__ difr,
@@ -529,29 +597,26 @@ __global__ void k_lowner(LevelView lv, const double *__restrict__ dl,
       den *= sq ? (di - dj) * (di + dj) : (di - dj);
     }
     if (++cnt == 8) {
-      int e;
-      num = frexp(num, &e); en += e;
-      den = frexp(den, &e); ed += e;
+      num = frexp_b(num, en);
+      den = frexp_b(den, ed);
       cnt = 0;
     }
   }
-  {
-    int e;
-    num = frexp(num, &e); en += e;
-    den = frexp(den, &e); ed += e;
-  }
+  num = frexp_b(num, en);
+  den = frexp_b(den, ed);
 #pragma unroll
   for (int ofs = L / 2; ofs > 0; ofs >>= 1) {
     double on = __shfl_xor_sync(HSS_FULL, num, ofs);
     double od = __shfl_xor_sync(HSS_FULL, den, ofs);
     int oen = __shfl_xor_sync(HSS_FULL, en, ofs);
     int oed = __shfl_xor_sync(HSS_FULL, ed, ofs);
-    int e;
-    num = frexp(num * on, &e); en += oen + e;
-    den = frexp(den * od, &e); ed += oed + e;
+    en += oen;
+    ed += oed;
+    num = frexp_b(num * on, en);
+    den = frexp_b(den * od, ed);
   }
   if (valid && gl == 0) {
-    const double q = ldexp(fabs(num / den), en - ed);
+    const double q = ldexp_b(fabs(num / den), en - ed);
     zhat[s + i] = copysign(sqrt(q), __ldg(zw + s + i));
   }
 }
