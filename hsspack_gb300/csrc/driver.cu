@@ -513,21 +513,22 @@ static void run_merges(Ctx &c, const std::vector<int> &ms, const std::vector<int
     long long *xq2 = (long long *)(dpk + o_q2), *xso = (long long *)(dpk + o_so);
     LevelView dv{xs, xK, xrho, xoff, PD};
     const int dtot = doff.back();
-    double *Q2 = buf<double>(c, "Q2", q2tot), *T = buf<double>(c, "T", q2tot);
+    double *Q2 = buf<double>(c, "Q2", q2tot);
     double *S = buf<double>(c, "S", stot);
+    int maxnd = *std::max_element(dn_.begin(), dn_.end());
+    stage_begin(HSS_ST_GATHER, st);
+    launch_gather(PD, dtot, maxnd, xs, xn, xoff, L.w.ndslot, L.w.grp, xq2, Q, ldq, Q2, st, L.sup, xr);
+    stage_end(HSS_ST_GATHER, st, 16LL * q2tot, 0.0);
     stage_begin(HSS_ST_BUILD_S, st);
     // (banded updates keep one order of summation: their small z are rounding noise
     // of earlier updates and decide signs of vectors)
     launch_build_S(dv, dtot, L.w.dl, L.difl, L.difr, L.zhat, L.w.grp, xso, S,
                    *std::max_element(dK_.begin(), dK_.end()), bu != nullptr, st,
-                   zup && hsel.empty() ? L.alpha : nullptr);
+                   zup && hsel.empty() ? L.alpha : nullptr, NewRows{L.sup, xr, xn, L.w.ndslot});
     stage_end(HSS_ST_BUILD_S, st, 8LL * stot * 2, 0.0);
     if (zup) zupdate();
-    int maxnd = *std::max_element(dn_.begin(), dn_.end());
-    stage_begin(HSS_ST_GATHER, st);
-    launch_gather(PD, dtot, maxnd, xs, xn, xoff, L.w.ndslot, L.w.grp, xq2, Q, ldq, Q2, st, L.sup, xr);
-    stage_end(HSS_ST_GATHER, st, 16LL * q2tot, 0.0);
-    // GEMM problems: top rows use type 1,2 columns, bottom rows type 2,3
+    // GEMM problems: top rows use type 1,2 columns, bottom rows type 2,3; the products
+    // go straight into the non-deflated slots' columns (their old ones are in Q2)
     std::vector<GemmDesc> probs;
     probs.reserve(2 * (size_t)PD);
     int di = 0;
@@ -538,11 +539,12 @@ static void run_merges(Ctx &c, const std::vector<int> &ms, const std::vector<int
       // window rows above and below the cut
       const int n = dn_[di], cut = ms[m] + mn1[m];
       const int n1 = std::min(n, std::max(0, cut - dr_[di]));
-      double *q2 = Q2 + q2off[di], *t = T + q2off[di], *sm = S + soff[di];
-      if (n1 > 0) probs.push_back(GemmDesc{q2, sm, t, n, K, n, n1, K, c1 + c2, 0, 0});
+      double *q2 = Q2 + q2off[di], *t = Q + dr_[di], *sm = S + soff[di];
+      const int *slots = L.w.ndslot + ms[m], ld = (int)ldq;
+      if (n1 > 0) probs.push_back(GemmDesc{q2, sm, t, n, K, ld, n1, K, c1 + c2, 0, 0, 0, slots});
       if (n > n1)
-        probs.push_back(GemmDesc{q2 + n1 + (long long)c1 * n, sm + c1, t + n1, n, K, n, n - n1, K,
-                                 K - c1, 0, 0});
+        probs.push_back(GemmDesc{q2 + n1 + (long long)c1 * n, sm + c1, t + n1, n, K, ld, n - n1, K,
+                                 K - c1, 0, 0, 0, slots});
       ++di;
     }
     double fl = 0.0;
@@ -554,10 +556,7 @@ static void run_merges(Ctx &c, const std::vector<int> &ms, const std::vector<int
     stage_begin(HSS_ST_GEMM, st);
     launch_gemm(probs, c.cfg.precision, st);
     stage_end(HSS_ST_GEMM, st, gbytes, fl);
-    stage_begin(HSS_ST_SCATTER, st);
-    launch_scatter(PD, dtot, maxnd, xs, xn, xoff, L.w.ndslot, xq2, T, Q, ldq, st, L.sup, xr);
-    stage_end(HSS_ST_SCATTER, st, 16LL * q2tot, 0.0);
-    c.launches += 4;
+    c.launches += 3;
   }
   if (PD == 0 && zup) zupdate();
   // ---- HSS merges: one at a time (each has its own HSS tree)
@@ -1182,24 +1181,28 @@ static void svd_merge_tail(Ctx &c, const std::vector<int> &ms, const std::vector
     LevelView dv{xs, xK, vr, xoff, PD};
     const int dtot = doff_.back();
     double *Ub = buf<double>(c, "sv_Ub", totB), *Vb = buf<double>(c, "sv_Vb", totB);
-    stage_begin(HSS_ST_BUILD_S, st);
-    launch_svd_vectors(dv, dtot, L.w.dl, L.difl, L.difr, L.zhat, dbo, Ub, Vb, st);
-    stage_end(HSS_ST_BUILD_S, st, 16LL * totB, 20.0 * k2);
-    double *U2 = buf<double>(c, "sv_U2", totU), *TU = buf<double>(c, "sv_TU", totU);
-    double *V2 = buf<double>(c, "sv_V2", totV), *TV = buf<double>(c, "sv_TV", totV);
+    double *U2 = buf<double>(c, "sv_U2", totU), *V2 = buf<double>(c, "sv_V2", totV);
     stage_begin(HSS_ST_GATHER, st);
     launch_gather(PD, dtot, maxNd, xs, xN, xoff, L.w.ndslot, nullptr, dqU, U, ld, U2, st, sU, xrU);
     launch_gather(PD, dtot, maxMd, xs, xM, xoff, L.w.ndslot, nullptr, dqV, V, ld, V2, st, sV, xrV);
     stage_end(HSS_ST_GATHER, st, 16LL * (totU + totV), 0.0);
+    stage_begin(HSS_ST_BUILD_S, st);
+    launch_svd_vectors(dv, dtot, L.w.dl, L.difl, L.difr, L.zhat, dbo, Ub, Vb, st,
+                       NewRows{sU, xrU, xN, L.w.ndslot}, NewRows{sV, xrV, xM, L.w.ndslot});
+    stage_end(HSS_ST_BUILD_S, st, 16LL * totB, 20.0 * k2);
+    // the products go straight into the non-deflated slots' columns
     std::vector<GemmDesc> probs;
     int tiles = 0;
     double fl = 0.0;
     long long gb = 0;
     for (int m = 0; m < PD; ++m) {
       const int K = dK_[m], N = dN_[m], M = dM_[m];
-      probs.push_back(GemmDesc{U2 + qU[m], Ub + bo[m], TU + qU[m], N, K, N, N, K, K, 0, tiles});
+      const int *slots = L.w.ndslot + ds_[m], ldi = (int)ld;
+      probs.push_back(GemmDesc{U2 + qU[m], Ub + bo[m], U + rU_[m], N, K, ldi, N, K, K, 0, tiles, 0,
+                               slots});
       tiles += gemm_tiles(N, K);
-      probs.push_back(GemmDesc{V2 + qV[m], Vb + bo[m], TV + qV[m], M, K, M, M, K, K, 0, tiles});
+      probs.push_back(GemmDesc{V2 + qV[m], Vb + bo[m], V + rV_[m], M, K, ldi, M, K, K, 0, tiles, 0,
+                               slots});
       tiles += gemm_tiles(M, K);
       fl += 2.0 * (double)(N + M) * K * K;
       gb += 8LL * ((long long)(N + M) * K * 2 + 2LL * K * K);
@@ -1207,11 +1210,7 @@ static void svd_merge_tail(Ctx &c, const std::vector<int> &ms, const std::vector
     stage_begin(HSS_ST_GEMM, st);
     launch_gemm(probs, c.cfg.precision, st);
     stage_end(HSS_ST_GEMM, st, gb, fl);
-    stage_begin(HSS_ST_SCATTER, st);
-    launch_scatter(PD, dtot, maxNd, xs, xN, xoff, L.w.ndslot, dqU, TU, U, ld, st, sU, xrU);
-    launch_scatter(PD, dtot, maxMd, xs, xM, xoff, L.w.ndslot, dqV, TV, V, ld, st, sV, xrV);
-    stage_end(HSS_ST_SCATTER, st, 16LL * (totU + totV), 0.0);
-    c.launches += 6;
+    c.launches += 4;
   }
   // ---- HSS merges (K >= bsmlz): two HSS products each (DHSSVCS)
   for (int m : hsel) {

@@ -79,11 +79,12 @@ k_gemm_f64(int nprob, const GemmDesc *__restrict__ probs) {
   for (int j = 0; j < 4; ++j) {
     const int gc = n0 + ty * 4 + j;
     if (gc >= P.N) continue;
+    const long long cc = P.cmap ? __ldg(P.cmap + gc) : gc;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int gr = m0 + tx * 4 + i;
       if (gr >= P.M) continue;
-      double *c = P.C + (long long)gc * P.ldc + gr;
+      double *c = P.C + cc * P.ldc + gr;
       *c = P.beta ? *c + acc[i][j] : acc[i][j];
     }
   }
@@ -115,7 +116,7 @@ k_gemm_small(int nprob, const GemmDesc *__restrict__ probs, const long long *__r
   const int K = P.tri ? min(P.K, j + 1) : P.K;
 #pragma unroll 4
   for (int k = 0; k < K; ++k) acc = fma(__ldg(a + (long long)k * P.lda), __ldg(b + k), acc);
-  double *c = P.C + (long long)j * P.ldc + i;
+  double *c = P.C + (long long)(P.cmap ? __ldg(P.cmap + j) : j) * P.ldc + i;
   *c = P.beta ? *c + acc : acc;
 }
 

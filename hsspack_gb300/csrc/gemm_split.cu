@@ -537,6 +537,7 @@ struct TcProb {
   double *C;
   int ldc, M, N, ktiles, beta;
   int tile0;             // first flattened tile index
+  const int *cmap;       // columns of C (GemmDesc)
 };
 
 // Persistent kernel, one CTA per SM: warp 0 (one lane) streams the K chunks
@@ -749,14 +750,17 @@ k_gemm_tc(const TcProb *__restrict__ probs, const int *__restrict__ tprob, int n
       if (!okt) break;
       // C = 2^{e_i + f_j - 30} (H + 2^-32 L) (+ C)
       const int r = (tt % ntm) * TM + quarter * 32 + lane;
-      if (r < P.M) {
-        const int ei = P.ea[r];
+      const int c0 = (tt / ntm) * TN + half * TH;
+      static_assert(TH <= 32, "a lane per column");
+      const int cl = P.cmap && lane < TH && c0 + lane < P.N ? __ldg(P.cmap + c0 + lane) : c0 + lane;
+      const int ei = r < P.M ? P.ea[r] : 0;
 #pragma unroll
-        for (int j = 0; j < TH; ++j) {
-          const int c = (tt / ntm) * TN + half * TH + j;
+      for (int j = 0; j < TH; ++j) {
+        const int c = c0 + j, cc = __shfl_sync(0xffffffffu, cl, j);
+        if (r < P.M) {
           if (c < P.N) {
             const double v = exact_double(hacc[j], lacc[j], ei + P.eb[c] - 30);
-            double *dst = P.C + (long long)c * P.ldc + r;
+            double *dst = P.C + (long long)cc * P.ldc + r;
             *dst = P.beta ? *dst + v : v;
           }
         }
@@ -802,6 +806,7 @@ struct FusedProb {
   const int *ea, *eb;  // row / column exponents (frexp convention)
   int lda, ldb, ldc, M, N, K, beta;
   int tile0;
+  const int *cmap;
 };
 struct ExpJob {  // rows of A (stride = lda between k) or columns of B (contiguous k)
   const double *X;
@@ -968,7 +973,7 @@ k_gemm_fused(const FusedProb *__restrict__ probs, int nprob, int *__restrict__ e
     for (int j = 0; j < FN; ++j) {
       const int c = tn * FN + j;
       if (c < P.N) {
-        double *dst = P.C + (long long)c * P.ldc + r;
+        double *dst = P.C + (long long)(P.cmap ? __ldg(P.cmap + c) : c) * P.ldc + r;
         *dst = P.beta ? *dst + acc[j] : acc[j];
       }
     }
@@ -1004,7 +1009,8 @@ void launch_gemm_split(const std::vector<GemmDesc> &probs, int *d_err, cudaStrea
     wa += (long long)ntm * nkc;
     wb += (long long)ntn * nkc;
     sa.push_back(a); sb.push_back(bb);
-    TcProb t{nullptr, nullptr, nullptr, nullptr, p.C, p.ldc, p.M, p.N, kt, p.beta, tiles};
+    TcProb t{nullptr, nullptr, nullptr, nullptr, p.C, p.ldc, p.M, p.N, kt, p.beta, tiles,
+             p.cmap};
     tiles += ntm * ntn;
     tc.push_back(t);
   }
@@ -1068,7 +1074,8 @@ void launch_gemm_fused(const std::vector<GemmDesc> &probs, int *d_err, cudaStrea
   for (const auto &p : probs) {
     rj.push_back({p.A, p.lda, p.M, p.K, nullptr, rows});
     cj.push_back({p.B, p.ldb, p.N, p.K, nullptr, cols});
-    FusedProb f{p.A, p.B, p.C, nullptr, nullptr, p.lda, p.ldb, p.ldc, p.M, p.N, p.K, p.beta, tiles};
+    FusedProb f{p.A, p.B, p.C, nullptr, nullptr, p.lda, p.ldb, p.ldc, p.M, p.N, p.K, p.beta, tiles,
+                p.cmap};
     fp.push_back(f);
     rows += p.M;
     cols += p.N;

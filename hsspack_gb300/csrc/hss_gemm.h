@@ -16,6 +16,7 @@ struct GemmDesc {
   int beta;
   int tile0;  // first flattened tile index of this problem
   int tri;    // 1: B is upper triangular with zeros below (the element kernel skips those)
+  const int *cmap;  // column j of C is at C + cmap[j] ldc (null: j)
 };
 
 // one operand of the split-BF16 GEMM: `rows` vectors of length `inner`

@@ -36,6 +36,18 @@ struct LevelScratch {
   double *l1val, *l2val;
 };
 
+// Rows that a merge's products write of the non-deflated slots' columns, for the slots'
+// supports (null sup: none kept).  Set once the old columns have been gathered.
+struct NewRows {
+  int2 *sup = nullptr;
+  const int *row0 = nullptr, *rows = nullptr, *ndslot = nullptr;
+#ifdef __CUDACC__
+  __device__ __forceinline__ void set(int m, int pos) const {
+    sup[__ldg(ndslot + pos)] = make_int2(__ldg(row0 + m), __ldg(row0 + m) + __ldg(rows + m));
+  }
+#endif
+};
+
 // secular.cu
 // lane-group width target of the secular kernels (pole terms per lane; 0: 8)
 void set_secular_terms(int t);
@@ -69,7 +81,7 @@ void launch_alpha(const LevelView &lv, int total, const double *dl, const double
 void launch_build_S(const LevelView &lv, int total, const double *dl, const double *difl,
                     const double *difr, const double *zhat, const int *grp,
                     const long long *soff, double *Sws, int maxk, bool fixed, cudaStream_t st,
-                    double *alpha = nullptr);
+                    double *alpha = nullptr, NewRows nr = {});
 void launch_cauchy_eig(int K, const double *F, const double *u, const double *v,
                        const double *difl, const double *difr, double *C, cudaStream_t st,
                        bool sq = false);
@@ -199,7 +211,7 @@ void launch_svd_prepare(int P, int maxn, const int *ms, const int *mnl, const in
 // U / V blocks (K x K per merge at boff); sigma rescaled by onrm
 void launch_svd_vectors(const LevelView &lv, int total, const double *dl, const double *difl,
                         const double *difr, const double *zhat, const long long *boff, double *Ub,
-                        double *Vb, cudaStream_t st);
+                        double *Vb, cudaStream_t st, NewRows nu = {}, NewRows nv = {});
 void launch_svd_unscale(const LevelView &lv, int total, const double *onrm, double *lam,
                         cudaStream_t st);
 // HSS path of one SVD merge: norms and U generator; the row-0 rank-one term

@@ -658,7 +658,7 @@ __global__ void k_build_S(LevelView lv, const double *__restrict__ dl,
                           const double *__restrict__ difl, const double *__restrict__ difr,
                           const double *__restrict__ zhat, const int *__restrict__ grp,
                           const long long *__restrict__ soff, double *__restrict__ Sws,
-                          double *__restrict__ alpha) {
+                          double *__restrict__ alpha, NewRows nr) {
   const int lane = threadIdx.x & 31, gl = lane & (L - 1);
   const int r = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) / L);
   const int total = __ldg(lv.rootoff + lv.P);
@@ -673,6 +673,7 @@ __global__ void k_build_S(LevelView lv, const double *__restrict__ dl,
     s = __ldg(lv.s + m);
     K = __ldg(lv.K + m);
   }
+  if (nr.sup && valid && gl == 0) nr.set(m, s + j);
   double *S = Sws + (valid ? __ldg(soff + m) + (long long)j * K : 0ll);
   PoleDiff P{dl + s, difl + s, difr + s};
   double acc = 0.0;
@@ -1181,7 +1182,7 @@ void launch_alpha(const LevelView &lv, int total, const double *dl, const double
 void launch_build_S(const LevelView &lv, int total, const double *dl, const double *difl,
                     const double *difr, const double *zhat, const int *grp,
                     const long long *soff, double *Sws, int maxk, bool fixed, cudaStream_t st,
-                    double *alpha) {
+                    double *alpha, NewRows nr) {
   if (total <= 0) return;
   // lanes per column: a group keeps at least two terms per lane, and the level at
   // least 152 x 512 lanes (512 problems, 32 lanes at every level before: 7.2 ms, now
@@ -1191,7 +1192,7 @@ void launch_build_S(const LevelView &lv, int total, const double *dl, const doub
   const int tb = root_block((long long)total * L);
   const unsigned grid = (unsigned)(((long long)total * L + tb - 1) / tb);
 #define BS_CASE(n) \
-  case n: k_build_S<n><<<grid, tb, 0, st>>>(lv, dl, difl, difr, zhat, grp, soff, Sws, alpha); break;
+  case n: k_build_S<n><<<grid, tb, 0, st>>>(lv, dl, difl, difr, zhat, grp, soff, Sws, alpha, nr); break;
   switch (L) { BS_CASE(4) BS_CASE(8) BS_CASE(16) BS_CASE(32) }
 #undef BS_CASE
 }

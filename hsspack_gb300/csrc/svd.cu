@@ -453,7 +453,8 @@ k_svd_prepare(int P, const int *__restrict__ ms, const int *__restrict__ mnl,
 __global__ void k_svd_vectors(LevelView lv, const double *__restrict__ dl,
                               const double *__restrict__ difl, const double *__restrict__ difr,
                               const double *__restrict__ zhat, const long long *__restrict__ boff,
-                              double *__restrict__ Ub, double *__restrict__ Vb) {
+                              double *__restrict__ Ub, double *__restrict__ Vb, NewRows nu,
+                              NewRows nv) {
   const int lane = threadIdx.x & 31;
   const int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (r >= __ldg(lv.rootoff + lv.P)) return;
@@ -461,6 +462,8 @@ __global__ void k_svd_vectors(LevelView lv, const double *__restrict__ dl,
   const int j = r - __ldg(lv.rootoff + m);
   const int s = __ldg(lv.s + m);
   const int K = __ldg(lv.K + m);
+  if (nu.sup && lane == 0) nu.set(m, s + j);
+  if (nv.sup && lane == 0) nv.set(m, s + j);
   PoleDiff P{dl + s, difl + s, difr + s, true};
   double *vc = Vb + boff[m] + (long long)j * K, *uc = Ub + boff[m] + (long long)j * K;
   // each entry is formed once (FP64 issue slots are the scarce resource): the
@@ -678,10 +681,10 @@ void launch_svd_prepare(int P, int maxn, const int *ms, const int *mnl, const in
 
 void launch_svd_vectors(const LevelView &lv, int total, const double *dl, const double *difl,
                         const double *difr, const double *zhat, const long long *boff, double *Ub,
-                        double *Vb, cudaStream_t st) {
+                        double *Vb, cudaStream_t st, NewRows nu, NewRows nv) {
   if (total <= 0) return;
   k_svd_vectors<<<(unsigned)(((long long)total * 32 + 255) / 256), 256, 0, st>>>(
-      lv, dl, difl, difr, zhat, boff, Ub, Vb);
+      lv, dl, difl, difr, zhat, boff, Ub, Vb, nu, nv);
 }
 void launch_svd_unscale(const LevelView &lv, int total, const double *onrm, double *lam,
                         cudaStream_t st) {
