@@ -238,6 +238,48 @@ k_tall_qr(const TallDesc *__restrict__ descs, const QrJob *__restrict__ jobs) {
   }
 }
 
+// Tangent of the Jacobi rotation of two rows with squared norms a, b > 0 and product c:
+// the root of smaller modulus of c t^2 + x t - c = 0, x = b - a (t^2 + 2 zeta t = 1 with
+// zeta = x / 2c).  False: c^2 <= jtol2 a b, nothing to rotate.  The test and the first
+// estimate are FP32 on numbers brought to c's exponent by integer operations, and one
+// Newton step in FP64 (whose slope may be FP32's) finishes it: four FP64 instructions
+// where a reciprocal and a comparison in FP64 made it thirteen.  n = 2000, all
+// bases of a DHSSMM: 9.59 -> 9.28 ms.
+__device__ __forceinline__ bool jacobi_tan(double a, double b, double c, double jtol2, double &t) {
+  const int hc = __double2hiint(c), Ec = (hc >> 20) & 0x7ff;
+  const int Ea = __double2hiint(a) >> 20, Eb = __double2hiint(b) >> 20;
+  const double x = b - a;
+  const int hx = __double2hiint(x), Ex = (hx >> 20) & 0x7ff;
+  if (Ea >= 600 && Eb >= 600 && Ea < 1500 && Eb < 1500) {
+    if (Ec < 450) return false;  // (c^2 / (a b) below 2^-300)
+    auto mant = [](double v, int e) {  // |v| as FP32 with the exponent set to e
+      return __int_as_float((e + 127) << 23 | (__double2hiint(v) & 0xfffff) << 3 |
+                            (unsigned)__double2loint(v) >> 29);
+    };
+    const float mc = mant(c, 0);
+    const int D = 2 * Ec - Ea - Eb;
+    if (D < -100 || mc * mc * __int_as_float((D + 127) << 23) <= (float)jtol2 * mant(a, 0) * mant(b, 0))
+      return false;
+    const int dx = Ex - Ec;
+    if (dx < 120) {
+      const float zf = dx < -120 ? 0.f : __fdividef(0.5f * mant(x, dx), mc);
+      const float rf = zf < 1e15f ? sqrtf(fmaf(zf, zf, 1.f)) : zf;
+      const int sg = (hx ^ hc) & 0x80000000;
+      const double t0 = f64_of_f32(__fdividef(1.f, zf + rf));
+      t = __hiloint2double(__double2hiint(t0) | sg, __double2loint(t0));
+      const double f = fma(t, fma(t, c, x), -c);
+      const double w = f64_of_f32(__fdividef(0.5f, rf * mc));  // 1 / |2 c (t + zeta)|, c's sign x's
+      t = fma(f, __hiloint2double((__double2hiint(w) - ((Ec - 1023) << 20)) | (~hx & 0x80000000),
+                                  __double2loint(w)), t);
+      return true;
+    }
+  }
+  if (!(c * c > jtol2 * a * b)) return false;
+  const double zeta = x / (2.0 * c);
+  t = copysign(1.0 / (fabs(zeta) + sqrt(fma(zeta, zeta, 1.0))), zeta);
+  return true;
+}
+
 // Basis of one node from its R factor: the left singular vectors of R^T with
 // singular value > tol, in decreasing order (the left singular vectors of a
 // block row whose transpose has R as QR factor, or the right singular vectors
@@ -272,7 +314,7 @@ __global__ void __launch_bounds__(QT)
 k_node_basis(const BasisJob *__restrict__ jobs, double tol, int *status) {
   extern __shared__ double M[];  // column j at M + j * LDM
   __shared__ double cn[QR_MAXC], cref[QR_MAXC], nrm[QR_MAXC];
-  __shared__ double scl[QR_MAXC];  // row scales
+  __shared__ double scl[QR_MAXC], isc[QR_MAXC];  // row scales, their reciprocals
   __shared__ double part[QT], tp[QR_MAXC / 2], tq[QR_MAXC / 2];
   __shared__ int prm[QR_MAXC], pos[QR_MAXC];
   __shared__ HousePar s_h;
@@ -389,7 +431,7 @@ k_node_basis(const BasisJob *__restrict__ jobs, double tol, int *status) {
   const int ng = QT / gs;
   const double jtol = HSS_EPS * (r > 16 ? r : 16), jtol2 = jtol * jtol;
   const long long frzb = __double_as_longlong(stop2);
-  for (int t = tid; t < k0; t += QT) scl[t] = 1.0;
+  for (int t = tid; t < k0; t += QT) scl[t] = isc[t] = 1.0;
   int conv = k0 < 2;
   for (int sweep = 0; sweep < JAC_SWEEPS && !conv; ++sweep) {
     __syncthreads();
@@ -402,7 +444,7 @@ k_node_basis(const BasisJob *__restrict__ jobs, double tol, int *status) {
         a = fma(u, u, a);
       }
       a = group_sum(a, gs, mask);
-      if (ln == 0) { nrm[t] = a; scl[t] = 1.0; }
+      if (ln == 0) { nrm[t] = a; scl[t] = isc[t] = 1.0; }
     }
     __syncthreads();
     int rot = 0;
@@ -427,31 +469,20 @@ k_node_basis(const BasisJob *__restrict__ jobs, double tol, int *status) {
           if (ab > 0 && bb > 0 && ab >= frzb && bb >= frzb) {  // a, b > 0, >= stop2
             double c = part[pi];
             for (int x = 1; x < nch; ++x) c += part[x * np + pi];
-            const double sp = scl[p], sq = scl[q], g = sp * sq;
-            c *= g;
-            if (__double_as_longlong(c * c) > __double_as_longlong(jtol2 * a * b)) {
-              // t of smaller modulus with t^2 + 2 zeta t = 1, zeta = (b - a) / 2c
-              const double x = b - a, zeta = x * rcp_nr(2.0 * c);
-              const float zf = abs_f32(zeta);
-              double t;
-              if (zf < 1e15f) {
-                const float rf = sqrtf(fmaf(zf, zf, 1.f));
-                t = copysign(f64_of_f32(__fdividef(1.f, zf + rf)), zeta);
-                // one Newton step: f(t) / (2 (t + zeta)), t + zeta = +-sqrt(1 + zeta^2)
-                const double f = fma(t, fma(2.0, zeta, t), -1.0);
-                t = fma(-f, copysign(f64_of_f32(__fdividef(0.5f, rf)), zeta), t);
-              } else {
-                t = c * rcp_nr(x);
-              }
-              double rt, cs;
+            const double sp = scl[p], sq = scl[q];
+            c *= sp * sq;
+            double t, rt, cs;
+            if (jacobi_tan(a, b, c, jtol2, t)) {
               sqrt_pair(fma(t, t, 1.0), rt, cs);
               nrm[p] = fma(-t, c, a);
               nrm[q] = fma(t, c, b);
-              const double ti = t * rcp_nr(g);  // t / (s_p s_q)
-              ta = ti * (sq * sq);
-              tb = ti * (sp * sp);
+              const double ip = isc[p], iq = isc[q];
+              ta = t * (sq * ip);
+              tb = t * (sp * iq);
               scl[p] = sp * cs;
               scl[q] = sq * cs;
+              isc[p] = ip * rt;
+              isc[q] = iq * rt;
               go = 1;
             }
           }
