@@ -426,6 +426,9 @@ k_node_basis(const BasisJob *__restrict__ jobs, double tol, int *status) {
   const int ch = np > 0 ? tid / np : 0, pi = np > 0 ? tid - ch * np : 0;
   const bool act = np > 0 && ch < nch;
   const int j0 = r * ch / nch, j1 = act ? r * (ch + 1) / nch : 0;
+  // the rotations on all threads: twice the loads in flight for the same instructions
+  const int nc2 = np > 0 ? QT / np : 1;
+  const int i0 = ch < nc2 ? r * ch / nc2 : 0, i1 = ch < nc2 ? r * (ch + 1) / nc2 : 0;
   const int gs = group_size(k0 > 0 ? k0 : 1), grp = tid / gs, ln = tid - grp * gs;
   const unsigned mask = group_mask(gs);
   const int ng = QT / gs;
@@ -492,11 +495,11 @@ k_node_basis(const BasisJob *__restrict__ jobs, double tol, int *status) {
       }
       if (__syncthreads_or(go)) {
         rot = 1;
-        if (pair) {
+        if (i1 > i0 && p < k0 && q < k0) {
           const double ta = tp[pi], tb = tq[pi];
           if (__double_as_longlong(tb) != 0) {
 #pragma unroll 4
-            for (int j = j0; j < j1; ++j) {
+            for (int j = i0; j < i1; ++j) {
               const double u = M[j * LDM + p], v = M[j * LDM + q];
               M[j * LDM + p] = fma(-ta, v, u);
               M[j * LDM + q] = fma(tb, u, v);
