@@ -101,6 +101,25 @@ __device__ __forceinline__ double f64_of_f32(float f) {
                           (int)(b << 29));
 }
 
+// (float)d by integer operations, rounded to nearest even as the conversion is (which
+// holds the FP64 pipe); results outside FP32's normal range, but 0, by the conversion
+__device__ __forceinline__ float f32_of_f64(double d) {
+  const unsigned hi = (unsigned)__double2hiint(d), lo = (unsigned)__double2loint(d);
+  const unsigned E = (hi >> 20) & 0x7ffu;
+  if (E - 897u < 254u) {
+    const unsigned u = ((E - 896u) << 23) | ((hi & 0xfffffu) << 3) | (lo >> 29), rem = lo << 3;
+    return __uint_as_float((hi & 0x80000000u) | (u + (rem > 0x80000000u - (u & 1u))));
+  }
+  if (((hi << 1) | lo) == 0) return __uint_as_float(hi);
+  return (float)d;
+}
+// (double)f, 0 included; FP32 subnormals, infinities and NaN by the conversion
+__device__ __forceinline__ double f64_from(float f) {
+  const unsigned e = (__float_as_uint(f) >> 23) & 0xffu;
+  if (e - 1u < 254u) return f64_of_f32(f);
+  return (__float_as_uint(f) << 1) == 0 ? __hiloint2double(__float_as_int(f), 0) : (double)f;
+}
+
 // Differences of the old poles F and new roots lam = F + DIFL, formed from
 // DIFL/DIFR so that no cancellation occurs near the poles
 // (SRC/CauchyHssEig.f90:470-568, computfd / computdd).

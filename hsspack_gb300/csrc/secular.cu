@@ -195,14 +195,14 @@ __device__ __forceinline__ void root_init(RootState &r, float guess, double zsq,
     if (guess != 0.0f && fabsf(guess) <= 0.5f) {  // learned signed distance to the nearer pole
       // the midpoint pass already fixed the half interval (one evaluation)
       const double half = full ? r.delta : 0.5 * r.delta;
-      if (guess > 0.0f) { r.oi = r.j; r.tau = (double)guess * r.delta; r.lo = 0.0; r.hi = half; }
-      else { r.oi = r.j + 1; r.tau = (double)guess * r.delta; r.lo = -half; r.hi = 0.0; }
+      if (guess > 0.0f) { r.oi = r.j; r.tau = f64_from(guess) * r.delta; r.lo = 0.0; r.hi = half; }
+      else { r.oi = r.j + 1; r.tau = f64_from(guess) * r.delta; r.lo = -half; r.hi = 0.0; }
       if (ref.x != 0.0f) {
         // a refined pre-solve: the start tau = x + y exactly (origin as the
         // guess's sign), and z its last step / tau, which counts as the
         // previous step of the quadratic-convergence acceptance
-        r.tau = (double)ref.x + (double)ref.y;
-        r.prel = (double)ref.z;
+        r.tau = f64_from(ref.x) + f64_from(ref.y);
+        r.prel = f64_from(ref.z);
       }
       r.phase = 1;
       r.learned = true;
@@ -852,27 +852,30 @@ k_secular_guess32(LevelView lv, const double *__restrict__ dl, const float *__re
     j = r - __ldg(lv.rootoff + m);
     K = __ldg(lv.K + m);
     rhoinv_d = 1.0 / __ldg(lv.rho + m);
-    rhoinv = (float)rhoinv_d;
+    rhoinv = f32_of_f64(rhoinv_d);
   }
   const bool active = r < total && K >= 2 && j < K - 1;
   const int n0 = j - GR + 1;  // first near pole
-  // near gaps d_i - d_o from FP64 differences, for the origin o = j or j + 1
-  float gn[2 * GR];
+  // Near gaps d_i - d_o from FP64 differences, for the origin o = j or j + 1: only the
+  // lane's own terms, i = n0 + q0 + t L.  The poles j and j + 1 themselves are 0 and
+  // +-delta (rounding is symmetric).  Every lane took all eight, each a difference and a
+  // conversion on the FP64 pipe, which then bound the whole FP32 iteration.
+  constexpr int NO = L < 2 * GR ? 2 * GR / L : 1;
+  const int q0 = (gl - n0) & (L - 1);
+  float gn[NO];
+  auto near_gap = [&](int o, int i) {
+    const double dorg = __ldg(dl + s + o), di = __ldg(dl + s + i);
+    return f32_of_f64(SQ ? (di - dorg) * (di + dorg) : (di - dorg));
+  };
   auto near_gaps = [&](int o) {
-    const double dorg = active ? __ldg(dl + s + o) : 0.0;
 #pragma unroll
-    for (int q = 0; q < 2 * GR; ++q) {
-      const int i = n0 + q;
-      if (active && i >= 0 && i < K) {
-        const double di = __ldg(dl + s + i);
-        gn[q] = SQ ? (float)((di - dorg) * (di + dorg)) : (float)(di - dorg);
-      } else {
-        gn[q] = 0.f;
-      }
+    for (int t = 0; t < NO; ++t) {
+      const int q = q0 + t * L, i = n0 + q;
+      gn[t] = active && q < 2 * GR && i >= 0 && i < K ? near_gap(o, i) : 0.f;
     }
   };
   near_gaps(j);
-  const float delta = gn[GR];  // d_{j+1} - d_j
+  const float delta = active ? near_gap(j, j + 1) : 0.f;  // d_{j+1} - d_j
   int o = j;
   float do32 = active ? __ldg(d32 + s + j) : 0.f;
   const int Ka = active ? K : 0;
@@ -892,11 +895,11 @@ k_secular_guess32(LevelView lv, const double *__restrict__ dl, const float *__re
         else { b0 = fmaf(zi, t, b0); b1 = fmaf(t, t, b1); }
       }
 #pragma unroll
-      for (int q = 0; q < 2 * GR; ++q) {
-        const int i = n0 + q;
-        if (i < 0 || i >= Ka || (i & (L - 1)) != gl) continue;
+      for (int u = 0; u < NO; ++u) {
+        const int q = q0 + u * L, i = n0 + q;
+        if (q >= 2 * GR || i < 0 || i >= Ka) continue;
         const float zi = __ldg(z32 + s + i);
-        const float t = __fdividef(zi, gn[q] - tau);
+        const float t = __fdividef(zi, gn[u] - tau);
         if (i <= j) { a0 = fmaf(zi, t, a0); a1 = fmaf(t, t, a1); }
         else { b0 = fmaf(zi, t, b0); b1 = fmaf(t, t, b1); }
       }
@@ -909,7 +912,7 @@ k_secular_guess32(LevelView lv, const double *__restrict__ dl, const float *__re
         done = true;
       } else {
         if (w < 0.f) lo = fmaxf(lo, tau); else hi = fminf(hi, tau);
-        const float gL = gn[GR - 1] - tau, gR = gn[GR] - tau;  // the poles j, j + 1
+        const float gL = (o == j ? 0.f : -delta) - tau, gR = (o == j ? delta : 0.f) - tau;  // poles j, j + 1
         const float A = (gL + gR) * w - gL * gR * dw;
         const float B = gL * gR * w;
         const float C = w - gL * a1 - gR * b1;
@@ -973,10 +976,10 @@ k_secular_guess32(LevelView lv, const double *__restrict__ dl, const float *__re
     a1 = group_sum_f<L>(a1);
     b1 = group_sum_f<L>(b1);
     if (go) {
-      const float rh = (float)rhoinv_d, rl = (float)(rhoinv_d - (double)rh);
+      const float rh = f32_of_f64(rhoinv_d), rl = f32_of_f64(rhoinv_d - f64_from(rh));
       ff_add(wh, wl, rh, rl, wh, wl);
       const float w = wh, dw = a1 + b1;
-      const float gL = gn[GR - 1] - tau, gR = gn[GR] - tau;  // the poles j, j + 1
+      const float gL = (o == j ? 0.f : -delta) - tau, gR = (o == j ? delta : 0.f) - tau;  // poles j, j + 1
       const float A = (gL + gR) * w - gL * gR * dw;
       const float B = gL * gR * w;
       const float C = w - gL * a1 - gR * b1;
