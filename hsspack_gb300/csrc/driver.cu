@@ -72,6 +72,9 @@ struct Ctx {
   PackedZ *pz = nullptr;             // packed-output request of the running solve
   double *zstage = nullptr;          // pinned staging of packed eigenvectors
   size_t zstage_cap = 0;
+  std::vector<char> plan;            // host lists kept between calls (hss_finalize frees them)
+  std::vector<GemmDesc> probs;
+  std::vector<double> hd, he;
   long long launches = 0;
   Ctx() {
     hss_default_config(&cfg);
@@ -377,64 +380,80 @@ static void run_merges(Ctx &c, const std::vector<int> &ms, const std::vector<int
   CK(cudaMemcpyAsync((void *)hwin, dwin, (size_t)P * 7 * sizeof(int), cudaMemcpyDeviceToHost, st));
   CK(cudaMemcpyAsync(hrho, drho, (size_t)P * sizeof(double), cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
-  // ---- plan
-  std::vector<int> as, an, aK, aoff(1, 0), gs, gn, gng;
-  std::vector<double> arho;
-  std::vector<int> ds_, dn_, dr_, dK_, doff(1, 0);  // dr_, dn_: row window (first, count)
-  std::vector<double> drho_;
-  std::vector<long long> q2off, soff, toff;
-  std::vector<int> hsel;  // HSS merges (index into active arrays)
-  for (auto *v : {&as, &an, &aK, &aoff, &gs, &gn, &gng, &ds_, &dn_, &dr_, &dK_, &doff}) v->reserve(P + 1);
-  for (auto *v : {&arho, &drho_}) v->reserve(P);
-  for (auto *v : {&q2off, &soff}) v->reserve(P);
-  long long q2tot = 0, stot = 0;
-  int maxn = 0, maxn_g = 0;
+  // ---- plan: counts first, then every array the level's launches read straight into
+  // one kept buffer and up in one copy (lists grown entry by entry and packed afterwards
+  // left the GPU waiting 0.7 ms for the 30016 merges of a batch's bottom level)
+  int PA = 0, PD = 0, PG = 0;
   for (int m = 0; m < P; ++m) {
-    const int K = hout[5 * m], ng = hout[5 * m + 1];
-    c.stats.n_merges++;
-    c.stats.total_k += K;
-    c.stats.max_k = std::max(c.stats.max_k, K);
-    if (ng > 0) { gs.push_back(ms[m]); gn.push_back(mn[m]); gng.push_back(ng); maxn_g = std::max(maxn_g, mn[m]); }
-    if (K == 0) continue;
-    as.push_back(ms[m]); an.push_back(mn[m]); aK.push_back(K); arho.push_back(hrho[m]);
-    aoff.push_back(aoff.back() + K);
-    maxn = std::max(maxn, mn[m]);
-    const bool use_hss = K >= c.cfg.bsmlz;
-    if (use_hss) {
-      hsel.push_back((int)as.size() - 1);
-      c.stats.n_hss_merges++;
-      continue;
-    }
-    c.stats.n_dense_merges++;
-    const int row0 = L.sup ? hwin[m].x : ms[m], rows = L.sup ? hwin[m].y - row0 : mn[m];
-    ds_.push_back(ms[m]); dn_.push_back(rows); dr_.push_back(row0); dK_.push_back(K);
-    drho_.push_back(hrho[m]);
-    doff.push_back(doff.back() + K);
-    q2off.push_back(q2tot);
-    q2tot += (long long)rows * K;
-    soff.push_back(stot);
-    stot += (long long)K * K;
+    const int K = hout[5 * m];
+    PG += hout[5 * m + 1] > 0;
+    PA += K > 0;
+    PD += K > 0 && K < c.cfg.bsmlz;
   }
-  const int PA = (int)as.size();
-  // every array the level's launches read, in one upload
-  std::vector<int> apoff(PA + 1, 0);
-  for (int a = 0; a < PA; ++a) apoff[a + 1] = apoff[a] + an[a];
-  Pack pk;
-  const size_t o_gs = pk.add(gs), o_gn = pk.add(gn), o_gng = pk.add(gng);
-  const size_t o_as = pk.add(as), o_aK = pk.add(aK), o_aoff = pk.add(aoff), o_arho = pk.add(arho),
-               o_apoff = pk.add(apoff);
-  const size_t o_ds = pk.add(ds_), o_dK = pk.add(dK_), o_doff = pk.add(doff), o_drho = pk.add(drho_),
-               o_dn = pk.add(dn_), o_dr = pk.add(dr_), o_q2 = pk.add(q2off), o_so = pk.add(soff);
-  char *dpk = pk.upload(c, "l_pack", st);
+  size_t pbytes = 0;
+  auto room = [&](size_t n, size_t sz) {
+    const size_t o = pbytes;
+    pbytes = (pbytes + n * sz + 15) & ~(size_t)15;
+    return o;
+  };
+  const size_t o_gs = room(PG, 4), o_gn = room(PG, 4), o_gng = room(PG, 4);
+  const size_t o_as = room(PA, 4), o_aK = room(PA, 4), o_aoff = room(PA + 1, 4),
+               o_arho = room(PA, 8), o_apoff = room(PA + 1, 4);
+  const size_t o_ds = room(PD, 4), o_dK = room(PD, 4), o_doff = room(PD + 1, 4),
+               o_drho = room(PD, 8), o_dn = room(PD, 4), o_dr = room(PD, 4), o_q2 = room(PD, 8),
+               o_so = room(PD, 8);
+  if (c.plan.size() < pbytes) c.plan.resize(pbytes);
+  char *pl = c.plan.data();
+  int *gs = (int *)(pl + o_gs), *gn = (int *)(pl + o_gn), *gng = (int *)(pl + o_gng);
+  int *as = (int *)(pl + o_as), *aK = (int *)(pl + o_aK), *aoff = (int *)(pl + o_aoff),
+      *apoff = (int *)(pl + o_apoff);
+  int *ds_ = (int *)(pl + o_ds), *dK_ = (int *)(pl + o_dK), *doff = (int *)(pl + o_doff),
+      *dn_ = (int *)(pl + o_dn), *dr_ = (int *)(pl + o_dr);  // dr_, dn_: row window
+  double *arho = (double *)(pl + o_arho), *drho_ = (double *)(pl + o_drho);
+  long long *q2off = (long long *)(pl + o_q2), *soff = (long long *)(pl + o_so);
+  std::vector<int> hsel;  // HSS merges (index into active arrays)
+  long long q2tot = 0, stot = 0;
+  int maxn_g = 0, maxK = 0, maxKd = 0, maxnd = 0;
+  double k2 = 0.0;
+  aoff[0] = apoff[0] = doff[0] = 0;
+  c.stats.n_merges += P;
+  for (int m = 0, a = 0, g = 0, x = 0; m < P; ++m) {
+    const int K = hout[5 * m], ng = hout[5 * m + 1];
+    c.stats.total_k += K;
+    if (ng > 0) { gs[g] = ms[m]; gn[g] = mn[m]; gng[g++] = ng; maxn_g = std::max(maxn_g, mn[m]); }
+    if (K == 0) continue;
+    as[a] = ms[m]; aK[a] = K; arho[a] = hrho[m];
+    aoff[a + 1] = aoff[a] + K;
+    apoff[a + 1] = apoff[a] + mn[m];
+    maxK = std::max(maxK, K);
+    k2 += (double)K * K;
+    ++a;
+    if (K >= c.cfg.bsmlz) { hsel.push_back(a - 1); continue; }
+    const int row0 = L.sup ? hwin[m].x : ms[m], rows = L.sup ? hwin[m].y - row0 : mn[m];
+    ds_[x] = ms[m]; dn_[x] = rows; dr_[x] = row0; dK_[x] = K; drho_[x] = hrho[m];
+    doff[x + 1] = doff[x] + K;
+    q2off[x] = q2tot;
+    q2tot += (long long)rows * K;
+    soff[x] = stot;
+    stot += (long long)K * K;
+    maxKd = std::max(maxKd, K);
+    maxnd = std::max(maxnd, rows);
+    ++x;
+  }
+  c.stats.max_k = std::max(c.stats.max_k, maxK);
+  c.stats.n_hss_merges += (int)hsel.size();
+  c.stats.n_dense_merges += PD;
+  char *dpk = buf<char>(c, "l_pack", std::max<size_t>(pbytes, 16));
+  stage_h2d(dpk, pl, pbytes, st);
   // ---- Givens rotations of deflation
-  if (!gs.empty()) {
+  if (PG > 0) {
     int *g1 = (int *)(dpk + o_gs), *g2 = (int *)(dpk + o_gn), *g3 = (int *)(dpk + o_gng);
     stage_begin(HSS_ST_GIVENS, st);
-    launch_widen((int)gs.size(), maxn_g, g1, g3, L.w, Q, ldq, L.sup, st);
-    launch_givens((int)gs.size(), maxn_g, g1, g2, g3, L.w, Q, ldq, st, bu ? bu->zrest : nullptr,
+    launch_widen(PG, maxn_g, g1, g3, L.w, Q, ldq, L.sup, st);
+    launch_givens(PG, maxn_g, g1, g2, g3, L.w, Q, ldq, st, bu ? bu->zrest : nullptr,
                   bu ? bu->nrest : 0, bu ? bu->zld : 0, L.sup);
     long long gb = 0;
-    for (size_t i = 0; i < gs.size(); ++i) gb += 32LL * gn[i] * gng[i];
+    for (int i = 0; i < PG; ++i) gb += 32LL * gn[i] * gng[i];
     stage_end(HSS_ST_GIVENS, st, gb, 0.0);
     c.launches++;
   }
@@ -443,12 +462,9 @@ static void run_merges(Ctx &c, const std::vector<int> &ms, const std::vector<int
   int *vs = (int *)(dpk + o_as), *vK = (int *)(dpk + o_aK), *voff = (int *)(dpk + o_aoff);
   double *vrho = (double *)(dpk + o_arho);
   LevelView lv{vs, vK, vrho, voff, PA};
-  const int total = aoff.back();
+  const int total = aoff[PA];
   c.stats.secular_roots += total;
-  double k2 = 0.0;
-  for (int K : aK) k2 += (double)K * K;
   float *guess = nullptr;
-  const int maxK = *std::max_element(aK.begin(), aK.end());
   float4 *gref = nullptr;
   if (c.cfg.predictor >= 2) {
     // starts from an FP32 pre-solve of every root (3: refined by one
@@ -472,7 +488,7 @@ static void run_merges(Ctx &c, const std::vector<int> &ms, const std::vector<int
     float *feat = buf<float>(c, "pred_feat", (size_t)L.n * (mlp_nfeat() + 1));
     guess = buf<float>(c, "guess", L.n);
     stage_begin(HSS_ST_SECULAR, st);
-    launch_secular_mid(lv, total, *std::max_element(aK.begin(), aK.end()), L.w.dl, L.w.zw, feat, st);
+    launch_secular_mid(lv, total, maxK, L.w.dl, L.w.zw, feat, st);
     stage_end(HSS_ST_SECULAR, st, 0, 0.0);
     stage_begin(HSS_ST_PREDICT, st);
     launch_predict(L.n, feat, buf<char>(c, "pred_wb", 0), buf<float>(c, "pred_norm", 0), guess, st);
@@ -486,7 +502,7 @@ static void run_merges(Ctx &c, const std::vector<int> &ms, const std::vector<int
   stage_end(HSS_ST_SECULAR, st, 40LL * total, 0.0);  // flops from the pole-term count
   stage_begin(HSS_ST_LOWNER, st);
   launch_lowner(lv, total, L.w.dl, L.difl, L.difr, L.w.zw, L.zhat, st, false,
-                *std::max_element(aK.begin(), aK.end()));
+                maxK);
   stage_end(HSS_ST_LOWNER, st, 40LL * total, 5.0 * k2);
   c.launches += 2;
   // the remaining Z columns follow the new eigenvectors (mdsbed4.f90:266-268); the
@@ -505,17 +521,15 @@ static void run_merges(Ctx &c, const std::vector<int> &ms, const std::vector<int
     c.launches += 2;
   };
   // ---- dense merges: S, gather, GEMM (block structured), scatter
-  const int PD = (int)ds_.size();
   if (PD > 0) {
     int *xs = (int *)(dpk + o_ds), *xK = (int *)(dpk + o_dK), *xoff = (int *)(dpk + o_doff),
         *xn = (int *)(dpk + o_dn), *xr = (int *)(dpk + o_dr);
     double *xrho = (double *)(dpk + o_drho);
     long long *xq2 = (long long *)(dpk + o_q2), *xso = (long long *)(dpk + o_so);
     LevelView dv{xs, xK, xrho, xoff, PD};
-    const int dtot = doff.back();
+    const int dtot = doff[PD];
     double *Q2 = buf<double>(c, "Q2", q2tot);
     double *S = buf<double>(c, "S", stot);
-    int maxnd = *std::max_element(dn_.begin(), dn_.end());
     stage_begin(HSS_ST_GATHER, st);
     launch_gather(PD, dtot, maxnd, xs, xn, xoff, L.w.ndslot, L.w.grp, xq2, Q, ldq, Q2, st, L.sup, xr);
     stage_end(HSS_ST_GATHER, st, 16LL * q2tot, 0.0);
@@ -523,14 +537,14 @@ static void run_merges(Ctx &c, const std::vector<int> &ms, const std::vector<int
     // (banded updates keep one order of summation: their small z are rounding noise
     // of earlier updates and decide signs of vectors)
     launch_build_S(dv, dtot, L.w.dl, L.difl, L.difr, L.zhat, L.w.grp, xso, S,
-                   *std::max_element(dK_.begin(), dK_.end()), bu != nullptr, st,
+                   maxKd, bu != nullptr, st,
                    zup && hsel.empty() ? L.alpha : nullptr, NewRows{L.sup, xr, xn, L.w.ndslot});
     stage_end(HSS_ST_BUILD_S, st, 8LL * stot * 2, 0.0);
     if (zup) zupdate();
     // GEMM problems: top rows use type 1,2 columns, bottom rows type 2,3; the products
     // go straight into the non-deflated slots' columns (their old ones are in Q2)
-    std::vector<GemmDesc> probs;
-    probs.reserve(2 * (size_t)PD);
+    std::vector<GemmDesc> &probs = c.probs;
+    probs.clear();
     int di = 0;
     for (int m = 0; m < P; ++m) {
       const int K = hout[5 * m];
@@ -562,7 +576,7 @@ static void run_merges(Ctx &c, const std::vector<int> &ms, const std::vector<int
   // ---- HSS merges: one at a time (each has its own HSS tree)
   for (int a : hsel) {
     HssMergeArgs h;
-    h.s = as[a]; h.n = an[a]; h.K = aK[a];
+    h.s = as[a]; h.n = apoff[a + 1] - apoff[a]; h.K = aK[a];
     h.leaf = c.cfg.hss_leaf; h.tol = c.cfg.tol; h.precision = c.cfg.precision;
     h.dl = L.w.dl + h.s; h.difl = L.difl + h.s; h.difr = L.difr + h.s; h.zhat = L.zhat + h.s;
     h.alpha = L.alpha + h.s; h.ndslot = L.w.ndslot + h.s;
@@ -574,11 +588,7 @@ static void run_merges(Ctx &c, const std::vector<int> &ms, const std::vector<int
   // ---- new ascending order and eigenvalues of the rewritten slots
   stage_begin(HSS_ST_FINISH, st);
   launch_merge_finish_grid(PA, apoff[PA], (int *)(dpk + o_apoff), vs, vK, L.lam, L.w, perm, Dp, st);
-  {
-    long long nn = 0;
-    for (int x : an) nn += x;
-    stage_end(HSS_ST_FINISH, st, 24 * nn, 0.0);
-  }
+  stage_end(HSS_ST_FINISH, st, 24LL * apoff[PA], 0.0);
   c.launches++;
 }
 
@@ -594,17 +604,20 @@ static void dc_blocks(Ctx &c, const std::vector<int> &bs, const std::vector<int>
   const int smlsiz = std::max(1, std::min(c.cfg.smlsiz, 32));
   const int nb = (int)bs.size();
   std::vector<std::vector<int>> ends(nb);
-  std::vector<int> ls, lz;
+  std::vector<int> ls, lz, sz, nx;
+  ls.reserve(N / std::max(1, smlsiz / 2) + nb);
+  lz.reserve(N / std::max(1, smlsiz / 2) + nb);
   int mmax = 1;
   double fl = 0.0;
   for (int b = 0; b < nb; ++b) {
-    std::vector<int> sz(1, bm[b]);
-    while (*std::max_element(sz.begin(), sz.end()) > smlsiz) {
-      std::vector<int> nx;
-      for (int x : sz) { nx.push_back(x / 2); nx.push_back((x + 1) / 2); }
+    sz.assign(1, bm[b]);
+    for (int big = bm[b]; big > smlsiz; big = (big + 1) / 2) {  // big: the largest part
+      nx.resize(2 * sz.size());
+      for (size_t i = 0; i < sz.size(); ++i) { nx[2 * i] = sz[i] / 2; nx[2 * i + 1] = (sz[i] + 1) / 2; }
       sz.swap(nx);
     }
     int acc = bs[b];
+    ends[b].reserve(sz.size());
     for (int x : sz) {
       ls.push_back(acc); lz.push_back(x);
       acc += x;
@@ -615,7 +628,8 @@ static void dc_blocks(Ctx &c, const std::vector<int> &bs, const std::vector<int>
   }
   const int nl = (int)ls.size();
   int *dls = buf<int>(c, "leaf_s", nl), *dlz = buf<int>(c, "leaf_z", nl);
-  h2d(dls, ls, st); h2d(dlz, lz, st);
+  stage_h2d(dls, ls.data(), sizeof(int) * nl, st);
+  stage_h2d(dlz, lz.data(), sizeof(int) * nl, st);
   stage_begin(HSS_ST_LEAF, st);
   launch_leaf(nl, dls, dlz, mmax, N, d, e, Q, ldq, Dp, perm, status, st, sup);
   stage_end(HSS_ST_LEAF, st, 8LL * N * smlsiz, fl);
@@ -702,7 +716,9 @@ static int solve_core(Ctx &c, const std::vector<Problem> &pr, cudaStream_t st) {
     h2d(dP, P, st);
   }
   // global d, e with e = 0 at every block end; split and scale per problem
-  std::vector<double> hd(N), he(N, 0.0);
+  // (kept buffers: every entry is written below, he's zeros at the block ends included)
+  if (c.hd.size() < (size_t)N) { c.hd.resize(N); c.he.resize(N); }
+  double *hd = c.hd.data(), *he = c.he.data();
   std::vector<int> bstart, bsize, bprob;
   std::vector<double> bscale;
   std::vector<int> nblocks(np, 0);
@@ -770,8 +786,8 @@ static int solve_core(Ctx &c, const std::vector<Problem> &pr, cudaStream_t st) {
       bprob.insert(bprob.end(), b.prob.begin(), b.prob.end());
     }
   }
-  CK(cudaMemcpyAsync(d, hd.data(), sizeof(double) * N, cudaMemcpyHostToDevice, st));
-  CK(cudaMemcpyAsync(e, he.data(), sizeof(double) * N, cudaMemcpyHostToDevice, st));
+  CK(cudaMemcpyAsync(d, hd, sizeof(double) * N, cudaMemcpyHostToDevice, st));
+  CK(cudaMemcpyAsync(e, he, sizeof(double) * N, cudaMemcpyHostToDevice, st));
   dc_blocks(c, bstart, bsize, N, d, e, Q, L, Dp, perm, status, st, sup);
   {
     std::vector<int> ss, sm;
@@ -1854,6 +1870,10 @@ int hss_finalize(void) {
   if (c.zstage) cudaFreeHost(c.zstage);
   c.zstage = nullptr;
   c.zstage_cap = 0;
+  std::vector<char>().swap(c.plan);
+  std::vector<GemmDesc>().swap(c.probs);
+  std::vector<double>().swap(c.hd);
+  std::vector<double>().swap(c.he);
   return 0;
 }
 
