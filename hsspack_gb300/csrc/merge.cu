@@ -1106,21 +1106,40 @@ __global__ void k_scale_blocks(int nb, const int *__restrict__ bs, const int *__
 // Final ordering of every problem: column j of problem p's output is the
 // global slot perm[P[p] + j]; its eigenvalue is Dp[slot].  Z[p], W[p] are the
 // per-problem output pointers, ldz[p] their leading dimensions.
-__global__ void k_final_gather_batch(int np, const long long *__restrict__ P,
-                                     const int *__restrict__ perm, const double *__restrict__ Dp,
-                                     const double *__restrict__ Q, long long ldq,
-                                     double *const *__restrict__ Z, const long long *__restrict__ ldz,
-                                     double *const *__restrict__ W, const int2 *__restrict__ sup) {
-  const long long c = blockIdx.x;
-  const int p = problem_of(P, np, c);
-  const long long r0 = __ldg(P + p), n = __ldg(P + p + 1) - r0, j = c - r0;
+//
+// Bound by the output's writes.  A warp per column, 16 bytes a lane from the first
+// aligned entry on: the chain before a column's first store (its problem, slot and
+// support) is then hidden by the other warps' columns; a CTA per column, every thread
+// searching the problem by itself, spent as long on it as on the 2000 stores.  512
+// problems of 256 to 4096, 12.2 GB: 2.45 -> 2.15 ms.
+__global__ void __launch_bounds__(256)
+k_final_gather_batch(int np, long long total, const long long *__restrict__ P,
+                     const int *__restrict__ perm, const double *__restrict__ Dp,
+                     const double *__restrict__ Q, long long ldq, double *const *__restrict__ Z,
+                     const long long *__restrict__ ldz, double *const *__restrict__ W,
+                     const int2 *__restrict__ sup) {
+  const long long c = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (c >= total) return;
+  const int p = find_merge_warp(P, np, c);
+  const long long r0 = __ldg(P + p), j = c - r0;
+  const int n = (int)(__ldg(P + p + 1) - r0);
   const long long slot = perm[c];
   const double *src = Q + slot * ldq + r0;
   double *dst = Z[p] + j * ldz[p];
-  long long lo = 0, hi = n;  // rows holding data (global rows sup[slot]) relative to r0
-  if (sup) { const int2 r = sup[slot]; lo = r.x - r0; hi = r.y - r0; }
-  for (long long i = threadIdx.x; i < n; i += blockDim.x) dst[i] = (i >= lo && i < hi) ? src[i] : 0.0;
-  if (threadIdx.x == 0) W[p][j] = Dp[slot];
+  int lo = 0, hi = n;  // rows holding data (global rows sup[slot]) relative to r0
+  if (sup) { const int2 r = sup[slot]; lo = (int)(r.x - r0); hi = (int)(r.y - r0); }
+  auto val = [&](int i) { return i >= lo && i < hi ? src[i] : 0.0; };
+  const int head = min(n, (int)(((uintptr_t)dst >> 3) & 1)), body = (n - head) >> 1;
+  double2 *d2 = reinterpret_cast<double2 *>(dst + head);
+#pragma unroll 4
+  for (int t = lane; t < body; t += 32)
+    d2[t] = make_double2(val(head + 2 * t), val(head + 2 * t + 1));
+  if (lane == 0) {
+    if (head) dst[0] = val(0);
+    if (head + 2 * body < n) dst[n - 1] = val(n - 1);
+    W[p][j] = Dp[slot];
+  }
 }
 
 // ---------------------------------------------------------------- launch --
@@ -1256,7 +1275,7 @@ void launch_final_gather_batch(int np, long long total, const long long *P, cons
                                const long long *ldz, double *const *W, cudaStream_t st,
                                const int2 *sup) {
   if (np > 0 && total > 0)
-    k_final_gather_batch<<<(unsigned)total, 256, 0, st>>>(np, P, perm, Dp, Q, ldq, Z, ldz, W,
+    k_final_gather_batch<<<(unsigned)((total + 7) / 8), 256, 0, st>>>(np, total, P, perm, Dp, Q, ldq, Z, ldz, W,
                                                           sup);
 }
 
