@@ -84,6 +84,29 @@ __device__ __forceinline__ HousePar house_par(double alpha, double sg) {
   return h;
 }
 
+// sqrt(x) and 1 / sqrt(x)'s own rounding 1 / r as the divide gives it, both rounded to
+// nearest, for x in sqrt_pair's range: one Newton correction each from the residual in a
+// fused multiply-add (Markstein, IBM J. Res. Dev. 34, 1990).  Ten FP64 instructions.
+__device__ __forceinline__ void sqrt_rcp_rn(double x, double &r, double &rinv) {
+  double r0, y;
+  sqrt_pair(x, r0, y);
+  r = fma(fma(-r0, r0, x), 0.5 * y, r0);
+  rinv = fma(y, fma(-r, y, 1.0), y);
+}
+// a / b rounded to nearest from y = 1 / b within about an ulp (a, b and the quotient
+// well inside the normal range)
+__device__ __forceinline__ double div_rn(double a, double b, double y) {
+  const double q = a * y;
+  return fma(fma(-q, b, a), y, q);
+}
+
+// a / b rounded to nearest, by div_rn where both are within 2^+-480
+__device__ __forceinline__ double quot_rn(double a, double b) {
+  const unsigned ha = __double2hiint(a) & 0x7fffffff, hb = __double2hiint(b) & 0x7fffffff;
+  constexpr unsigned lo = 0x21f00000, w = 0x5df00000 - lo;
+  return ha - lo < w && hb - lo < w ? div_rn(a, b, rcp_nr(b)) : a / b;
+}
+
 // |d| as FP32 rounded towards zero by integer operations (a conversion holds the
 // FP64 pipe); 0 below FP32's range, infinity above
 __device__ __forceinline__ float abs_f32(double d) {

@@ -67,7 +67,8 @@ __device__ __forceinline__ void leaf_ranks_ties(int m, const double *D, int *rk)
 // behind it (measured: a dependent chain and eight independent ones, 1 to 4
 // warps per SM, all 64.2 cycles per instruction, 8 warps 128).  So few leaves
 // get a warp each, and the group halves once there are more than two warps per
-// quarter of the 152 SMs.  Leaf stage at the neighbouring choices (tridiagonal):
+// quarter of the 152 SMs.  Leaf stage at the neighbouring choices (tridiagonal,
+// rotations without their final rounding, a fifth less):
 //   128 leaves of 16 rows   G = 32 or 16 0.42 ms   8 0.51   4 0.66
 //   1024 of 16              G = 16 0.47 ms         8 0.55   4 0.71
 //   3800 of 8 to 16         G = 8  0.59 ms        16 0.73   4 0.69

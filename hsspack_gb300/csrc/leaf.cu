@@ -19,12 +19,17 @@
 //  * the split test of the next sweep is made as the sweep goes (a bit per
 //    off-diagonal), so no scan over E precedes a sweep;
 //  * column i + 1 of the eigenvector block stays in registers from one rotation
-//    to the next; r and 1 / r of a rotation come from one estimate (sqrt_pair).
+//    to the next; r and 1 / r of a rotation come from one estimate, each rounded
+//    to nearest (sqrt_rcp_rn).
+// The arithmetic is the plain loop's to the last bit (the fused multiply-adds are
+// written out).  A merge takes the signs of its vectors from z, which holds entries
+// down to 8 eps: with a shift or rotations an ulp off, leaves of 20 rows and more turned
+// a vector's sign in one solve of ten.
 // Shared memory is interleaved by lane, so lanes at different columns never
 // share a bank.  Leaf stage, one thread per leaf with nested loops before -> now:
-// n = 257 (16 leaves of 16 rows) 2.33 -> 0.42 ms, n = 2048 2.10 -> 0.42 ms, 512
-// problems (61000 leaves of 8 to 16) 6.37 -> 3.43 ms, n = 32768 (4096 of 8)
-// 0.41 -> 0.20 ms.
+// n = 257 (16 leaves of 16 rows) 2.33 -> 0.51 ms, n = 2048 2.10 -> 0.53 ms, 512
+// problems (61000 leaves of 8 to 16) 6.37 -> 4.09 ms, n = 32768 (4096 of 8)
+// 0.41 -> 0.29 ms.
 #include "hss_common.cuh"
 #include "hss_kernels.h"
 #include "hss_leaf.cuh"
@@ -104,22 +109,16 @@ k_leaf_ql(int nleaf, const int *__restrict__ lstart, const int *__restrict__ lsi
           bad = 1;
           done = true;
         } else {
-          // Wilkinson's shift D(l) - t.  Any shift keeps the iteration backward
-          // stable and t only steers it, so t is an FP32 number (the same sweeps,
-          // a tenth of the FP64 instructions) unless E(l) leaves FP32's range.
-          const double el = E[l * 32], dl = D[l * 32], dd = D[(l + 1) * 32] - dl;
-          const float ef = (float)el, df = (float)dd;
-          double tq;
-          if (fabsf(ef) > 1e-30f && fabsf(df) < 1e30f && fabsf(ef) < 1e15f) {
-            const float q0 = __fdividef(df, 2.f * ef);
-            const float rf = fabsf(q0) < 1e15f ? sqrtf(fmaf(q0, q0, 1.f)) : fabsf(q0);
-            tq = (double)__fdividef(ef, q0 + copysignf(rf, q0));
-          } else {  // operands are O(||T||) after the block scaling: a plain sqrt is safe
-            g = dd / (2.0 * el);
-            tq = el / (g + copysign(sqrt(fma(g, g, 1.0)), g));
-          }
+          // Wilkinson's shift; operands are O(||T||) after the block scaling, so a plain
+          // sqrt is safe
+          const double el = E[l * 32], dl = D[l * 32];
+          g = quot_rn(D[(l + 1) * 32] - dl, 2.0 * el);
+          const double x0 = fma(g, g, 1.0);
+          double r0, ri0;
+          if (__double2hiint(x0) < 0x7bf00000) sqrt_rcp_rn(x0, r0, ri0);  // below 2^960
+          else r0 = sqrt(x0);
           d1 = D[mm * 32];
-          g = d1 - dl + tq;
+          g = d1 - dl + quot_rn(el, g + copysign(r0, g));
           sn = 1.0; cs = 1.0; p = 0.0;
           i = mm - 1;
           dprev = 0.0;
@@ -136,7 +135,7 @@ k_leaf_ql(int nleaf, const int *__restrict__ lstart, const int *__restrict__ lsi
       double r, rinv;
       const int hx = __double2hiint(x);
       if (hx >= 0x03f00000 && hx < 0x7bf00000) {  // 2^-960 <= x < 2^960
-        sqrt_pair(x, r, rinv);
+        sqrt_rcp_rn(x, r, rinv);
         sn = f * rinv;
         cs = g * rinv;
       } else {
@@ -157,7 +156,7 @@ k_leaf_ql(int nleaf, const int *__restrict__ lstart, const int *__restrict__ lsi
         g = d1 - p;
         // 2 cs by its exponent (b = cs E(i) is zero or NaN where that is not 2 cs)
         const double cs2 = __hiloint2double(__double2hiint(cs) + (1 << 20), __double2loint(cs));
-        const double w = fma(di - g, sn, cs2 * b);
+        const double w = fma(cs2, b, (di - g) * sn);
         p = sn * w;
         d1 = g + p;
         D[(i + 1) * 32] = d1;
@@ -173,11 +172,11 @@ k_leaf_ql(int nleaf, const int *__restrict__ lstart, const int *__restrict__ lsi
         for (int t = 0; t < R; ++t) {
           if (R > 4 && t >= rows) break;
           const double zi = Z[(i * R + t) * 32];
-          Z[((i + 1) * R + t) * 32] = sn * zi + cs * zc[t];
-          zc[t] = cs * zi - sn * zc[t];
+          Z[((i + 1) * R + t) * 32] = fma(sn, zi, cs * zc[t]);
+          zc[t] = fma(cs, zi, -(sn * zc[t]));
         }
         if (i == l) {  // end of the sweep
-          d1 -= p;
+          d1 = __dsub_rn(d1, p);
           D[l * 32] = d1;
           E[l * 32] = g;
           E[mm * 32] = 0.0;

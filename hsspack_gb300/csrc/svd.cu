@@ -42,22 +42,25 @@ constexpr int SVD_LEAF_MAX = 32;
 // rotations at one FP64 warp instruction per 64 cycles.  Each lane carries its
 // own copy of the bidiagonal and its rows of U and V, one pass of the flat
 // loop is one pair of rotations for every lane, and the zero tests run as the
-// sweep goes: bit i of `ez` says E(i) = 0, of `dz` D(i) = 0.  Leaf stage, one
-// thread per leaf before -> now: n = 1001 (64 leaves of 15 rows) 5.12 -> 0.57 ms,
-// n = 16384 (1024 of 15) 5.52 -> 0.92 ms.
+// sweep goes: bit i of `ez` says E(i) = 0, of `dz` D(i) = 0.  The rotations are hypot
+// and the correctly rounded quotients (div_rn), for the signs' sake as there: half an
+// ulp either way turned a pair of vectors in a third of the solves with leaves of 20
+// rows.  Leaf stage, one
+// thread per leaf before -> now: n = 1001 (64 leaves of 15 rows) 5.12 -> 0.94 ms,
+// n = 16384 (1024 of 15) 5.52 -> 1.52 ms.
 
-// Rotation taking (y, z) to (t, 0): t = hypot(y, z), cs = y / t, sn = z / t.
+// Rotation taking (y, z) to (t, 0): t = hypot(y, z), cs = y / t, sn = z / t (the divides
+// from one reciprocal estimate where all three are within 2^+-480)
 __device__ __forceinline__ void plane_rotation(double y, double z, double &t, double &cs,
                                                double &sn) {
-  const double x = fma(y, y, z * z);
-  const int hx = __double2hiint(x);
-  if (hx >= 0x03f00000 && hx < 0x7bf00000) {  // 2^-960 <= x < 2^960
-    double rinv;
-    sqrt_pair(x, t, rinv);
-    cs = y * rinv;
-    sn = z * rinv;
+  t = hypot(y, z);
+  const unsigned hy = __double2hiint(y) & 0x7fffffff, hz = __double2hiint(z) & 0x7fffffff;
+  constexpr unsigned lo = 0x21f00000, w = 0x5df00000 - lo;
+  if (hy - lo < w && hz - lo < w) {
+    const double ri = rcp_nr(t);
+    cs = div_rn(y, t, ri);
+    sn = div_rn(z, t, ri);
   } else {
-    t = hypot(y, z);
     cs = t == 0.0 ? 1.0 : y / t;
     sn = t == 0.0 ? 0.0 : z / t;
   }
@@ -100,7 +103,7 @@ k_svd_leaf(int nleaf, const int *__restrict__ lstart, const int *__restrict__ ls
     for (int t = 0; t < rows; ++t) {
       const double xi = X[(i * R + t) * 32], xj = X[(j * R + t) * 32];
       X[(i * R + t) * 32] = cs * xi + sn * xj;
-      X[(j * R + t) * 32] = cs * xj - sn * xi;
+      X[(j * R + t) * 32] = -sn * xi + cs * xj;
     }
   };
   unsigned ez = 0, dz = 0;
@@ -194,25 +197,16 @@ k_svd_leaf(int nleaf, const int *__restrict__ lstart, const int *__restrict__ ls
           }
           scan();
         } else {
-          // Wilkinson shift t22 - tq from the trailing 2 x 2 of B^T B of the block.
-          // Any shift keeps the iteration backward stable; tq only steers it, so it
-          // is an FP32 number unless its operands leave FP32's range.
+          // Wilkinson shift from the trailing 2 x 2 of B^T B of the block
           const double d1 = D[(hi - 1) * 32], d2 = D[hi * 32], e1 = E[(hi - 1) * 32];
-          const double e0 = hi - 1 > lo ? E[(hi - 2) * 32] : 0.0;
-          const double t11 = fma(d1, d1, e0 * e0), t12 = d1 * e1, t22 = fma(d2, d2, e1 * e1);
-          const double dd = 0.5 * (t11 - t22);
-          const float tf = (float)t12, df = (float)dd;
-          double tq;
-          if (fabsf(tf) > 1e-15f && fabsf(tf) < 1e15f && fabsf(df) < 1e15f) {
-            tq = (double)__fdividef(tf * tf, df + copysignf(sqrtf(fmaf(df, df, tf * tf)), df));
-          } else if (dd == 0.0 && t12 == 0.0) {
-            tq = 0.0;
-          } else {
-            tq = t12 * t12 / (dd + copysign(hypot(dd, t12), dd != 0.0 ? dd : 1.0));
-          }
+          const double t11 = d1 * d1 + (hi - 1 > lo ? E[(hi - 2) * 32] * E[(hi - 2) * 32] : 0.0);
+          const double t12 = d1 * e1, t22 = d2 * d2 + e1 * e1, dd = 0.5 * (t11 - t22);
+          double mu;
+          if (dd == 0.0 && t12 == 0.0) mu = t22;
+          else mu = t22 - t12 * t12 / (dd + copysign(hypot(dd, t12), dd != 0.0 ? dd : 1.0));
           dk = D[lo * 32];
           ek = E[lo * 32];
-          y = fma(dk, dk, tq - t22);
+          y = dk * dk - mu;
           z = dk * ek;
           k = lo;
           dprev = 0.0;
@@ -230,7 +224,7 @@ k_svd_leaf(int nleaf, const int *__restrict__ lstart, const int *__restrict__ ls
       double t, cs, sn;
       plane_rotation(y, z, t, cs, sn);
       const double eprev = t;  // E(k - 1)
-      const double d0 = cs * dk + sn * ek, e0 = cs * ek - sn * dk;
+      const double d0 = cs * dk + sn * ek, e0 = -sn * dk + cs * ek;
       const double bl = sn * d1;
       d1 *= cs;
 #pragma unroll
@@ -238,7 +232,7 @@ k_svd_leaf(int nleaf, const int *__restrict__ lstart, const int *__restrict__ ls
         if (R > 4 && j >= rows) break;
         const double x = Vs[((k + 1) * R + j) * 32];
         Vs[(k * R + j) * 32] = cs * vc[j] + sn * x;
-        vc[j] = cs * x - sn * vc[j];
+        vc[j] = -sn * vc[j] + cs * x;
       }
       plane_rotation(d0, bl, t, cs, sn);
       D[k * 32] = t;
@@ -249,13 +243,13 @@ k_svd_leaf(int nleaf, const int *__restrict__ lstart, const int *__restrict__ ls
         ez = ng ? ez | 1u << (k - 1) : ez;
       }
       dprev = t;
-      const double ekn = cs * e0 + sn * d1, d1n = cs * d1 - sn * e0;
+      const double ekn = cs * e0 + sn * d1, d1n = -sn * e0 + cs * d1;
 #pragma unroll
       for (int j = 0; j < R; ++j) {
         if (R > 4 && j >= rows) break;
         const double x = Us[((k + 1) * R + j) * 32];
         Us[(k * R + j) * 32] = cs * uc[j] + sn * x;
-        uc[j] = cs * x - sn * uc[j];
+        uc[j] = -sn * uc[j] + cs * x;
       }
       if (k + 1 < hi) {
         ek = E[(k + 1) * 32];
