@@ -2576,8 +2576,10 @@ int hss_svdhssupdat_dev(int n, double *d, double *f, double *z, double *vt, int 
     CK(cudaMemsetAsync(status, 0, 8 * sizeof(int), st));
     int rank = 0;
     float t2[2] = {0.f, 0.f};
+    gemm_flag_clear(c, st);
     const int K = svd_update_core(n, d, f, z, vt, ldvt, tol, ni, c.cfg.precision, &rank, status,
                                   t2, st);
+    gemm_flag_check(c, st);
     int hst[8];
     CK(cudaMemcpyAsync(hst, status, sizeof hst, cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));

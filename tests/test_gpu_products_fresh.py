@@ -34,7 +34,7 @@ def used_memory():
         assert cu.cuMemFree_v2(p) == 0
 
 
-@pytest.mark.parametrize("entry", ["dhssmm", "cauchyhssmm", "dhssevc"])
+@pytest.mark.parametrize("entry", ["dhssmm", "cauchyhssmm", "dhssevc", "svdhssupdat"])
 def test_products_on_used_memory(entry, used_memory):
     n = 600
     rng = np.random.default_rng(0)
@@ -56,6 +56,17 @@ def test_products_on_used_memory(entry, used_memory):
             b = dev(B.T)
             hp.cauchyhssmm_dev(dev(D), dev(F), dev(u), dev(v), b, 64, 1e-14)
             out, ref = b.cpu().numpy().T, C @ B
+        elif entry == "svdhssupdat":
+            # right singular vectors of [diag(f); z^T], the rows of the result
+            f, z = np.sort(rng.uniform(0.1, 1.0, n)), rng.uniform(0.5, 1.0, n)
+            vt = dev(np.eye(n).ravel())
+            k = hp.svdhssupdat_dev(torch.zeros(n, dtype=torch.float64, device="cuda"), dev(f), dev(z),
+                                   vt, 1e-14, 64)
+            assert k == n
+            V = vt.cpu().numpy().reshape(n, n, order="F")
+            A = np.vstack([np.diag(f), z])
+            G = V @ (A.T @ A) @ V.T
+            out, ref = G, np.diag(np.diag(G))
         else:
             # C(i, j) = u_i v_j / (F_i - lam_j), lam_j = D_j between F_j and F_{j+1}
             dr = np.append(D[:-1] - F[1:], 0.0)
