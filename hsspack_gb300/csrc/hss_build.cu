@@ -198,8 +198,9 @@ __device__ __forceinline__ double pole_dd(bool sq, const Pole &p, const Pole &q)
 //
 // Bound: the latency of a pivot step, a chain of scans and reductions with FP64
 // warp instructions of 64 cycles each (12000 to 14000 cycles per step of a short
-// node, 43000 with FP64 comparisons in the reductions).  HSS stage of Cauchy
-// n = 3000 14.3 -> 5.9 ms, of the disordered chain n = 3000 27.8 -> 12.0 ms.
+// node, 43000 with FP64 comparisons in the reductions).  HSS product of Cauchy
+// n = 3000 (the whole call) 17.0 -> 8.1 ms, of the disordered chain n = 3000 27.8 ->
+// 11.7 ms.
 template <bool ROW>
 __device__ int rrlu_node(const PoleDiff &P, double *F, double *A, double *Z, double *W, int *PL,
                          int *PQ, double *V, int *PU, int M, int N, double tol, int rmax,

@@ -1189,7 +1189,7 @@ void launch_build_S(const LevelView &lv, int total, const double *dl, const doub
   if (total <= 0) return;
   // lanes per column: a group keeps at least two terms per lane, and the level at
   // least 152 x 512 lanes (512 problems, 32 lanes at every level before: 7.2 ms, now
-  // 3.5 ms).  fixed: 32, whatever the level
+  // 2.9 ms).  fixed: 32, whatever the level
   int L = 32;
   while (!fixed && L > 4 && (L * 2 > maxk || (long long)total * (L / 2) >= 152LL * 512)) L /= 2;
   const int tb = root_block((long long)total * L);
