@@ -167,7 +167,10 @@ k_band_leaf(int nleaf, const int *__restrict__ lstart, const int *__restrict__ l
     // - e(a_qq) the squared test's ratio lies in (2^(D-2), 2^(D+2)), so D alone decides
     // all but the close cases
     const int relx = (__double2hiint(rel * rel) >> 20) - 1023;
-    bool conv = false;
+    // a NaN anywhere in the block is one in its norm (the test by bit patterns below takes
+    // it for a large bound and would skip every pair)
+    bool conv = m > 1 && fro != fro;
+    if (conv && lane == 0) atomicMax(status, HSS_LEAF_NOCONV);
     for (int sweep = 0; sweep < JACOBI_SWEEPS && !conv; ++sweep) {
       conv = true;
       for (int p = 0; p < m - 1; ++p)
