@@ -326,7 +326,9 @@ __device__ int rrlu_node(const PoleDiff &P, double *F, double *A, double *Z, dou
       // An upper bound of what is left of the Schur complement first: two FP64
       // differences and FP32 arithmetic per entry.  Where it is below the tolerance
       // too (the usual end of a node), the search below could only confirm that.
-      // (|Z|, |V| rounded up, differences down, none to 0 or infinity.)
+      // (|Z|, |V| rounded up, differences down; no factor, quotient or product below
+      // FP32's normal numbers, where it would lose bits or vanish.  So a tolerance down
+      // there, as with u and v near 1e-17, always leaves it to the search.)
       float *ZF = (float *)(W + k);  // rows k .. M - 1; W(k) and on are not set yet
       auto up_f32 = [](double v) { return fmaxf(abs_f32(v) * 1.000001f, 1.2e-38f); };
       for (int i = k + tid; i < M; i += HT) ZF[i - k] = up_f32(Z[i]);
@@ -342,7 +344,7 @@ __device__ int rrlu_node(const PoleDiff &P, double *F, double *A, double *Z, dou
           const Pole pli = ROW ? Pole{F[i], 0.0, 0.0, 0.0, PL[i]} : pole(PL[i]);
           cm = fmaxf(cm, ZF[i - k] / fminf(abs_f32(den_p(pli, puj)), 3e38f));
         }
-        em = fmaxf(em, cm * vj);
+        em = fmaxf(em, fmaxf(cm * vj, 1.2e-38f));
       }
       KeyIdx e{(unsigned long long)__float_as_uint(em), 0};
       e = cluster_best(block_best(e, red), G, cslot, cphase);
