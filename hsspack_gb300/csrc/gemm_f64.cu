@@ -114,6 +114,8 @@ int gemm_tiles(int M, int N) { return ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
 // of its first output together and the lanes walk on from there: a search of
 // its own by every thread (17 dependent loads with a batch's 88000 problems)
 // took longer than the K <= 32 multiply-adds.
+// Latency bound where the products are few, so eight terms are loaded at a time (one
+// 32^3 product 14.3 -> 9.5 us, 512 problems' products 12.4 -> 12.0 ms).
 // A triangular B (P.tri) ends each sum at the diagonal: 8192 x 8192 by 256 blocks of
 // 32 x 32 at this part's FP64 rate, 3.48 -> 1.82 ms.
 __global__ void __launch_bounds__(256)
@@ -130,8 +132,16 @@ k_gemm_small(int nprob, const GemmDesc *__restrict__ probs, const long long *__r
   const double *a = P.A + i, *b = P.B + (long long)j * P.ldb;
   double acc = 0.0;
   const int K = P.tri ? min(P.K, j + 1) : P.K;
-#pragma unroll 4
-  for (int k = 0; k < K; ++k) acc = fma(__ldg(a + (long long)k * P.lda), __ldg(b + k), acc);
+  int k = 0;
+  for (; k + 8 <= K; k += 8) {
+    double x[8], y[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) { x[u] = __ldg(a + (long long)(k + u) * P.lda); y[u] = __ldg(b + k + u); }
+#pragma unroll
+    for (int u = 0; u < 8; ++u) acc = fma(x[u], y[u], acc);
+  }
+#pragma unroll 1
+  for (; k < K; ++k) acc = fma(__ldg(a + (long long)k * P.lda), __ldg(b + k), acc);
   double *c = P.C + (long long)(P.cmap ? __ldg(P.cmap + j) : j) * P.ldc + i;
   *c = P.beta ? *c + acc : acc;
 }
