@@ -483,8 +483,10 @@ __device__ __forceinline__ void secular_lanes(const LevelView &lv, const double 
 
 // One root per group of L lanes (L = 1..32 chosen from the level's largest
 // K so that each lane sums ~8 pole terms and the group reductions stay cheap).
+// At most 80 registers, so that three CTAs share an SM: at 81 and more two did, and
+// a level of 3000 warps took two waves (hss_secular_dev, K = 3000: 1.23 -> 1.01 ms).
 template <int L, bool SQ>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 3)
 k_secular(LevelView lv, const double *__restrict__ dl, const double *__restrict__ zw,
           double *__restrict__ lam, double *__restrict__ difl, double *__restrict__ difr,
           int *__restrict__ iters, int *__restrict__ status, unsigned long long *__restrict__ itsum,
