@@ -67,7 +67,7 @@ __device__ __forceinline__ double bsvd_at(const double *__restrict__ AB, long lo
 // vanished (rank-deficient blocks).  Results ascending in slots a .. a + r - 1
 // (U, V, Dp, perm), null vectors in V slots a + r .. a + c - 1.
 __global__ void __launch_bounds__(256)
-k_bsvd_leaf(int nleaf, const int *__restrict__ la, const int *__restrict__ lr,
+k_bsvd_leaf(int nleaf, int n, const int *__restrict__ la, const int *__restrict__ lr,
             const int *__restrict__ lc, int sb, const double *__restrict__ AB, long long ldab,
             double *__restrict__ U, long long ldu, double *__restrict__ V, long long ldv,
             double *__restrict__ Dp, int *__restrict__ perm, int *__restrict__ status) {
@@ -84,10 +84,25 @@ k_bsvd_leaf(int nleaf, const int *__restrict__ la, const int *__restrict__ lr,
   const int L = blockIdx.x;
   if (L >= nleaf) return;
   const int a = la[L], r = lr[L], c = lc[L];
+  // NaN and infinity: the ranks below, and the merges' order, need numbers.  Each CTA
+  // looks at the matrix's columns up to the next leaf, so the appended rows are looked at
+  // too; such an entry counts as zero here and the call ends after the leaves.
+  auto finite = [](double x) { return ((__double2hiint(x) >> 20) & 0x7ff) != 0x7ff; };
+  int bad = 0;
   for (int t = tid; t < c * r; t += blockDim.x) {
     const int q = t / r, i = t % r;
-    Bs[q * RP + i] = bsvd_at(AB, ldab, sb, a + i, a + q);
+    const double x = bsvd_at(AB, ldab, sb, a + i, a + q);
+    bad |= !finite(x);
+    Bs[q * RP + i] = finite(x) ? x : 0.0;
   }
+  if (nleaf > 1) {
+    const int j0 = L == 0 ? 0 : a, j1 = L + 1 < nleaf ? la[L + 1] : n;
+    for (int t = tid; t < (j1 - j0) * (sb + 1); t += blockDim.x) {
+      const int j = j0 + t / (sb + 1), i = j - t % (sb + 1);
+      bad |= i >= 0 && !finite(bsvd_at(AB, ldab, sb, i, j));
+    }
+  }
+  if (bad) atomicMax(status, HSS_BAD_INPUT);
   for (int t = tid; t < c * c; t += blockDim.x) {
     const int q = t / c, i = t % c;
     Vs[q * CP + i] = (i == q) ? 1.0 : 0.0;
@@ -174,7 +189,10 @@ k_bsvd_leaf(int nleaf, const int *__restrict__ la, const int *__restrict__ lr,
     double s2 = 0.0;
     for (int i = lane; i < r; i += 32) s2 += Bs[q * RP + i] * Bs[q * RP + i];
     s2 = warp_sum(s2);
-    if (lane == 0) sg[q] = sqrt(s2);
+    if (lane == 0) {
+      sg[q] = sqrt(s2);
+      if (nleaf > 1 && !finite(s2)) atomicMax(status, HSS_BAD_INPUT);  // (an overflow)
+    }
   }
   __syncthreads();
   for (int q = tid; q < c; q += blockDim.x) {
@@ -399,7 +417,7 @@ size_t bsvd_leaf_smem() {
 int bsvd_rows_max() { return BSVD_ROWS_MAX; }
 int bsvd_cols_max() { return BSVD_COLS_MAX; }
 
-void launch_bsvd_leaf(int nleaf, const int *la, const int *lr, const int *lc, int sb,
+void launch_bsvd_leaf(int nleaf, int n, const int *la, const int *lr, const int *lc, int sb,
                       const double *AB, long long ldab, double *U, long long ldu, double *V,
                       long long ldv, double *Dp, int *perm, int *status, cudaStream_t st) {
   if (nleaf <= 0) return;
@@ -409,7 +427,7 @@ void launch_bsvd_leaf(int nleaf, const int *la, const int *lr, const int *lc, in
     cudaFuncSetAttribute(k_bsvd_leaf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     attr = true;
   }
-  k_bsvd_leaf<<<nleaf, 256, smem, st>>>(nleaf, la, lr, lc, sb, AB, ldab, U, ldu, V, ldv, Dp, perm,
+  k_bsvd_leaf<<<nleaf, 256, smem, st>>>(nleaf, n, la, lr, lc, sb, AB, ldab, U, ldu, V, ldv, Dp, perm,
                                         status);
 }
 

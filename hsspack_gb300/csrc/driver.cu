@@ -152,6 +152,21 @@ static void *pinned(Ctx &c, size_t bytes) {
 }
 
 void *pool_get(const char *name, size_t bytes) { return buf<char>(ctx(), name, bytes); }
+// |x| as an integer: orders as magnitudes do, infinity at MAG_INF, NaN above it.
+// Merges order eigenvalues by comparisons and take slot numbers from the positions, which
+// a NaN would leave unset: solvers with merges to run check their inputs with it.
+constexpr unsigned long long MAG_INF = 0x7ff0000000000000ull;
+static inline unsigned long long mag_bits(double x) {
+  unsigned long long b;
+  memcpy(&b, &x, sizeof b);
+  return b & 0x7fffffffffffffffull;
+}
+static const char *const NOT_FINITE = "NaN or infinity in the input";
+// the values of a call that ended there: NaN, not what an earlier call left
+static void no_values(double *w, int n, cudaStream_t st) {
+  CK(cudaMemsetAsync(w, 0xff, sizeof(double) * n, st));
+}
+
 // error word of the tensor-core products (set by a CTA whose bounded wait
 // timed out; reset at the start of every solve, read with its status)
 static int *gemm_flag(Ctx &c) { return buf<int>(c, "gemm_err", 1); }
@@ -726,6 +741,7 @@ static int solve_core(Ctx &c, const std::vector<Problem> &pr, cudaStream_t st) {
   struct Blocks {
     std::vector<int> start, size, prob;
     std::vector<double> scale;
+    bool bad = false;  // an infinity where merges follow (a NaN is always split off)
   };
   // problems p0 .. p1 - 1 into their own block lists (problems touch disjoint
   // ranges of hd, he and nblocks, so ranges of problems run on separate threads)
@@ -739,11 +755,13 @@ static int solve_core(Ctx &c, const std::vector<Problem> &pr, cudaStream_t st) {
         int finish = start;
         while (finish < o + n - 1 && !negligible(he[finish], hd[finish], hd[finish + 1])) ++finish;
         he[finish] = 0.0;
-        double nrm = 0.0;
-        for (int i = start; i <= finish; ++i) nrm = std::max(nrm, std::fabs(hd[i]));
-        for (int i = start; i < finish; ++i) nrm = std::max(nrm, std::fabs(he[i]));
+        unsigned long long top = 0;
+        for (int i = start; i <= finish; ++i) top = std::max(top, mag_bits(hd[i]));
+        for (int i = start; i < finish; ++i) top = std::max(top, mag_bits(he[i]));
         const int m = finish - start + 1;
-        double scl = 1.0;
+        double nrm, scl = 1.0;
+        memcpy(&nrm, &top, sizeof nrm);
+        if (m > smlsiz && top >= MAG_INF) out.bad = true;
         if (m > smlsiz && nrm > 0.0) {
           scl = nrm;
           const double mul = 1.0 / nrm;
@@ -762,6 +780,7 @@ static int solve_core(Ctx &c, const std::vector<Problem> &pr, cudaStream_t st) {
     // whole problems of about N / nt positions; the lists join in problem order
     const int nt = N >= (1 << 17) && np > 1 ? std::min(host_threads(), np) : 1;
     std::vector<Blocks> part(nt);
+    bool bad = false;
     std::vector<int> cut(nt + 1, np);
     cut[0] = 0;
     for (int t = 1, p = 0; t < nt; ++t) {
@@ -780,10 +799,19 @@ static int solve_core(Ctx &c, const std::vector<Problem> &pr, cudaStream_t st) {
     split(cut[0], cut[1], part[0]);
     for (auto &x : th) x.join();
     for (const Blocks &b : part) {
+      bad |= b.bad;
       bstart.insert(bstart.end(), b.start.begin(), b.start.end());
       bsize.insert(bsize.end(), b.size.begin(), b.size.end());
       bscale.insert(bscale.end(), b.scale.begin(), b.scale.end());
       bprob.insert(bprob.end(), b.prob.begin(), b.prob.end());
+    }
+    if (bad) {
+      for (auto &q : pr) no_values(q.w, q.n, st);
+      CK(cudaStreamSynchronize(st));
+      cudaEventDestroy(ev0);
+      cudaEventDestroy(ev1);
+      c.err = NOT_FINITE;
+      return 1;
     }
   }
   CK(cudaMemcpyAsync(d, hd, sizeof(double) * N, cudaMemcpyHostToDevice, st));
@@ -976,16 +1004,21 @@ static int band_core(Ctx &c, int n, int kd, const double *ab, long long ldab, do
     stage_end(HSS_ST_LEAF, st, 8LL * n * (kd + 1), fl);
   }
   c.launches += 2;
+  bool failed = false;  // in a cut or leaf: no merges then
   if (nl > 1) {
     std::vector<double> hS((size_t)ncut * kd);
+    int leaf_status = 0;
     CK(cudaMemcpyAsync(hS.data(), Sc, sizeof(double) * hS.size(), cudaMemcpyDeviceToHost, st));
+    CK(cudaMemcpyAsync(&leaf_status, status, sizeof(int), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
+    failed = leaf_status != 0;
+    for (double x : hS) failed |= mag_bits(x) >= MAG_INF;
     LevelArrays L = level_arrays(c, n);
     L.sup = sup;
     double *Z = buf<double>(c, "band_Z", (size_t)kd * n);
     std::vector<int> lastleaf(nl);
     for (int i = 0; i < nl; ++i) lastleaf[i] = i;
-    while (ends.size() > 1) {
+    while (ends.size() > 1 && !failed) {
       std::vector<int> ms, mn, mn1, mcut, nxe, nxl;
       for (size_t i = 0; i + 1 < ends.size(); i += 2) {
         const int s = i == 0 ? 0 : ends[i - 1];
@@ -1032,6 +1065,7 @@ static int band_core(Ctx &c, int n, int kd, const double *ab, long long ldab, do
   }
   stage_begin(HSS_ST_FINAL, st);
   launch_final_gather(n, perm, Dp, Q, n, z, ldz, w, st, sup);
+  if (failed) no_values(w, n, st);
   stage_end(HSS_ST_FINAL, st, 8LL * n * n + 20LL * n, 0.0);
   c.launches++;
   CK(cudaEventRecord(ev1, st));
@@ -1066,6 +1100,10 @@ static int band_core(Ctx &c, int n, int kd, const double *ab, long long ldab, do
   if (hst[0] != 0) {
     c.err = hst[0] == HSS_SECULAR_NOCONV ? "secular iteration did not converge"
                                           : "leaf Jacobi iteration did not converge";
+    return 1;
+  }
+  if (failed) {
+    c.err = NOT_FINITE;
     return 1;
   }
   return 0;
@@ -1288,6 +1326,9 @@ static void run_svd_merges(Ctx &c, const std::vector<int> &ms, const std::vector
                  perm, L, status, st, &sp);
 }
 
+// largest leaf of the bidiagonal SVD's tree
+static int svd_leaf_rows(const Ctx &c) { return std::max(4, std::min(c.cfg.smlsiz, 32)); }
+
 // MDBDSDC('U', COMPQ) (SRC/mdbdsdc.f90:1) of the upper bidiagonal (d, e) in
 // HBM: singular values into w (descending), U (ldu) and VT (ldvt) when
 // vectors.  Tree as DLASDT: a node of N rows splits into nl = N/2 rows, the
@@ -1301,7 +1342,7 @@ static int svd_core(Ctx &c, int n, const double *d, const double *e, double *Uo,
   CK(cudaEventCreate(&ev0));
   CK(cudaEventCreate(&ev1));
   CK(cudaEventRecord(ev0, st));
-  const int smlsiz = std::max(4, std::min(c.cfg.smlsiz, 32));
+  const int smlsiz = svd_leaf_rows(c);
   // levels of nodes, root first: (start, rows, sqre)
   struct Node { int a, N, sq; };
   std::vector<std::vector<Node>> lv(1, std::vector<Node>{Node{0, n, 0}});
@@ -1418,9 +1459,17 @@ static int svd_solve(Ctx &c, bool lower, int n, std::vector<double> hd, std::vec
       sn[i] = -ss;
     }
   }
-  double nrm = 0.0;
-  for (int i = 0; i < n; ++i) nrm = std::max(nrm, std::fabs(hd[i]));
-  for (int i = 0; i + 1 < n; ++i) nrm = std::max(nrm, std::fabs(he[i]));
+  unsigned long long top = 0;
+  for (int i = 0; i < n; ++i) top = std::max(top, mag_bits(hd[i]));
+  for (int i = 0; i + 1 < n; ++i) top = std::max(top, mag_bits(he[i]));
+  if (n > svd_leaf_rows(c) && top >= MAG_INF) {
+    no_values(dw, n, st);
+    CK(cudaStreamSynchronize(st));
+    c.err = NOT_FINITE;
+    return 1;
+  }
+  double nrm;
+  memcpy(&nrm, &top, sizeof nrm);
   const double scl = nrm > 0.0 ? nrm : 1.0;
   for (int i = 0; i < n; ++i) hd[i] /= scl;
   for (int i = 0; i + 1 < n; ++i) he[i] /= scl;
@@ -1598,11 +1647,14 @@ static int bsvd_core(Ctx &c, int n, int sb, const double *ab, long long ldab, in
     int *dla = buf<int>(c, "bl_a", nl), *dlr = buf<int>(c, "bl_r", nl), *dlc = buf<int>(c, "bl_c", nl);
     h2d(dla, la, st); h2d(dlr, lr, st); h2d(dlc, lc, st);
     stage_begin(HSS_ST_LEAF, st);
-    launch_bsvd_leaf(nl, dla, dlr, dlc, sb, ab, ldab, U, n, V, n, Dp, perm, status, st);
+    launch_bsvd_leaf(nl, n, dla, dlr, dlc, sb, ab, ldab, U, n, V, n, Dp, perm, status, st);
     stage_end(HSS_ST_LEAF, st, 8LL * n * (sb + 1) + 16LL * n * 96, flops);
     c.launches++;
   }
-  if (depth > 0) {
+  int leaf_status = 0;
+  CK(cudaMemcpyAsync(&leaf_status, status, sizeof(int), cudaMemcpyDeviceToHost, st));
+  CK(cudaStreamSynchronize(st));
+  if (depth > 0 && leaf_status == 0) {
     LevelArrays L = level_arrays(c, n);
     for (int d = depth - 1; d >= 0; --d) {  // merges bottom-up
       c.stats.n_levels++;
@@ -1610,10 +1662,14 @@ static int bsvd_core(Ctx &c, int n, int sb, const double *ab, long long ldab, in
         run_bsvd_append(c, lv[d], k, sb, n, ab, ldab, U, V, n, Dp, perm, L, status, st);
     }
   }
-  stage_begin(HSS_ST_FINAL, st);
-  launch_svd_outputs(n, perm, Dp, U, n, V, n, Uo, ldu, VT, ldvt, w, true, st);
-  stage_end(HSS_ST_FINAL, st, 32LL * n * n, 0.0);
-  c.launches += 2;
+  if (leaf_status == 0) {  // (perm is complete once the merges have run)
+    stage_begin(HSS_ST_FINAL, st);
+    launch_svd_outputs(n, perm, Dp, U, n, V, n, Uo, ldu, VT, ldvt, w, true, st);
+    stage_end(HSS_ST_FINAL, st, 32LL * n * n, 0.0);
+    c.launches += 2;
+  } else {
+    no_values(w, n, st);
+  }
   CK(cudaEventRecord(ev1, st));
   int hst[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   CK(cudaMemcpyAsync(hst, status, sizeof hst, cudaMemcpyDeviceToHost, st));
@@ -1637,7 +1693,8 @@ static int bsvd_core(Ctx &c, int n, int sb, const double *ab, long long ldab, in
     return 1;
   }
   if (hst[0] != 0) {
-    c.err = hst[0] == HSS_SECULAR_NOCONV ? "secular iteration did not converge"
+    c.err = hst[0] == HSS_BAD_INPUT          ? NOT_FINITE
+            : hst[0] == HSS_SECULAR_NOCONV ? "secular iteration did not converge"
                                           : "leaf Jacobi iteration did not converge";
     return 1;
   }

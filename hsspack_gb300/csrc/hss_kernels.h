@@ -233,7 +233,7 @@ void launch_rows_rotate_back(int n, int ncols, const double *cs, const double *s
 size_t bsvd_leaf_smem();
 int bsvd_rows_max();
 int bsvd_cols_max();
-void launch_bsvd_leaf(int nleaf, const int *la, const int *lr, const int *lc, int sb,
+void launch_bsvd_leaf(int nleaf, int n, const int *la, const int *lr, const int *lc, int sb,
                       const double *AB, long long ldab, double *U, long long ldu, double *V,
                       long long ldv, double *Dp, int *perm, int *status, cudaStream_t st);
 void launch_bsvd_z(int P, int total, const int *poff, const int *ms, const int *mrow, int sb, int n,
