@@ -473,19 +473,24 @@ __device__ int rrlu_node(const PoleDiff &P, double *F, double *A, double *Z, dou
         double zn[(512 + HT - 1) / HT];
         int cnt = 0;
         for (int j = k + 1 + tid; j < M; j += HT, ++cnt)
-          zn[cnt] = (j != jj) ? Z[j] * (rowdiff(j, jj) / rowdiff(j, ii)) : Z[j];
+          zn[cnt] = (j != jj) ? Z[j] * (rowdiff(j, jj) / rowdiff(j, ii)) : 0.0;
         double wn = 0.0;
         if (tid <= k && tid != ii) wn = W[tid] * (rowdiff(tid, ii) / rowdiff(tid, jj));
         double wn2[(256 + HT - 1) / HT];
         int c2 = 0;
         for (int j = tid + HT; j <= k; j += HT, ++c2)
-          wn2[c2] = (j != ii) ? W[j] * (rowdiff(j, ii) / rowdiff(j, jj)) : W[j];
+          wn2[c2] = (j != ii) ? W[j] * (rowdiff(j, ii) / rowdiff(j, jj)) : 0.0;
         __syncthreads();
         cnt = 0;
-        for (int j = k + 1 + tid; j < M; j += HT, ++cnt) Z[j] = zn[cnt];
+        // (Z[jj] and W[ii] have one writer, thread 0: a second one that put the old value
+        // back could come after it, and the CTAs of a cluster, each with its own copy, then
+        // went apart: one left the kernel while others still read its slots)
+        for (int j = k + 1 + tid; j < M; j += HT, ++cnt)
+          if (j != jj) Z[j] = zn[cnt];
         if (tid <= k && tid != ii) W[tid] = wn;
         c2 = 0;
-        for (int j = tid + HT; j <= k; j += HT, ++c2) W[j] = wn2[c2];
+        for (int j = tid + HT; j <= k; j += HT, ++c2)
+          if (j != ii) W[j] = wn2[c2];
         if (tid == 0) {
           Z[jj] = ujj;
           W[ii] = wii;
