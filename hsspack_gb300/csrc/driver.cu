@@ -1954,6 +1954,9 @@ int hss_mdstedc_dev(int n, double *d, double *e, double *z, int ldz, void *strea
   } catch (CudaError &ex) {
     c.err = ex.msg;
     return 1000000;
+  } catch (HssError &ex) {
+    c.err = ex.msg;
+    return 1000001;
   }
 }
 
@@ -1983,6 +1986,9 @@ int hss_mdstedc_v_dev(int n, double *d, double *e, double *z, int ldz, void *str
   } catch (CudaError &ex) {
     c.err = ex.msg;
     return 1000000;
+  } catch (HssError &ex) {
+    c.err = ex.msg;
+    return 1000001;
   }
 }
 
@@ -2028,6 +2034,9 @@ int hss_mdstedc_batch_dev(int nprob, const int *n, double *d, double *e, double 
   } catch (CudaError &ex) {
     c.err = ex.msg;
     return 1000000;
+  } catch (HssError &ex) {
+    c.err = ex.msg;
+    return 1000001;
   }
 }
 
@@ -2048,6 +2057,9 @@ int hss_mdsbevd_dev(int n, int kd, const double *ab, int ldab, double *w, double
   } catch (CudaError &ex) {
     c.err = ex.msg;
     return 1000000;
+  } catch (HssError &ex) {
+    c.err = ex.msg;
+    return 1000001;
   }
 }
 
@@ -2073,6 +2085,9 @@ int hss_mdbdsdc_dev(int n, double *d, double *e, double *u, int ldu, double *vt,
   } catch (CudaError &ex) {
     c.err = ex.msg;
     return 1000000;
+  } catch (HssError &ex) {
+    c.err = ex.msg;
+    return 1000001;
   }
 }
 
@@ -2127,6 +2142,9 @@ void mdbdsdc_(const char *uplo, const char *compq, const int *n_, double *d, dou
   } catch (CudaError &ex) {
     c.err = ex.msg;
     *info = 1000000;
+  } catch (HssError &ex) {
+    c.err = ex.msg;
+    *info = 1000001;
   }
 }
 
@@ -2286,6 +2304,9 @@ void mdsbevd_(const char *compz, const char *uplo, const int *n_, const int *kd_
   } catch (CudaError &ex) {
     c.err = ex.msg;
     *info = 1000000;
+  } catch (HssError &ex) {
+    c.err = ex.msg;
+    *info = 1000001;
   }
 }
 
@@ -2331,6 +2352,9 @@ void mdsbedc_(const char *jobz, const char *uplo, const int *n_, const int *kd_,
   } catch (CudaError &ex) {
     c.err = ex.msg;
     *info = 1000000;
+  } catch (HssError &ex) {
+    c.err = ex.msg;
+    *info = 1000001;
   }
 }
 
@@ -2425,6 +2449,9 @@ void mdstedc_(const char *compz, const int *n_, double *d, double *e, double *z,
   } catch (CudaError &ex) {
     c.err = ex.msg;
     *info = 1000000;
+  } catch (HssError &ex) {
+    c.err = ex.msg;
+    *info = 1000001;
   }
 }
 
