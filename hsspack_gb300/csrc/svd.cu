@@ -70,6 +70,16 @@ static size_t svd_leaf_smem(int rmax, int R) {
   return (size_t)(2 * rmax + (2 * rmax + 1) * R) * 32 * sizeof(double);
 }
 
+// A rotation's two results with their fused multiply-adds written out: left to the compiler,
+// instances for different G and R fuse different products, and the vectors of leaves of
+// 3 to 7 and of 32 rows differed in the last bit from the plain loop's.
+__device__ __forceinline__ double turn0(double cs, double sn, double x, double y) {
+  return fma(cs, x, sn * y);
+}
+__device__ __forceinline__ double turn1(double cs, double sn, double x, double y) {
+  return fma(cs, y, -(sn * x));
+}
+
 template <int G, int R>
 __global__ void __launch_bounds__(32)
 k_svd_leaf(int nleaf, const int *__restrict__ lstart, const int *__restrict__ lsize,
@@ -102,8 +112,8 @@ k_svd_leaf(int nleaf, const int *__restrict__ lstart, const int *__restrict__ ls
   auto rotate = [&](double *X, int i, int j, double cs, double sn) {
     for (int t = 0; t < rows; ++t) {
       const double xi = X[(i * R + t) * 32], xj = X[(j * R + t) * 32];
-      X[(i * R + t) * 32] = cs * xi + sn * xj;
-      X[(j * R + t) * 32] = -sn * xi + cs * xj;
+      X[(i * R + t) * 32] = turn0(cs, sn, xi, xj);
+      X[(j * R + t) * 32] = turn1(cs, sn, xi, xj);
     }
   };
   unsigned ez = 0, dz = 0;
@@ -199,14 +209,14 @@ k_svd_leaf(int nleaf, const int *__restrict__ lstart, const int *__restrict__ ls
         } else {
           // Wilkinson shift from the trailing 2 x 2 of B^T B of the block
           const double d1 = D[(hi - 1) * 32], d2 = D[hi * 32], e1 = E[(hi - 1) * 32];
-          const double t11 = d1 * d1 + (hi - 1 > lo ? E[(hi - 2) * 32] * E[(hi - 2) * 32] : 0.0);
-          const double t12 = d1 * e1, t22 = d2 * d2 + e1 * e1, dd = 0.5 * (t11 - t22);
+          const double e0 = hi - 1 > lo ? E[(hi - 2) * 32] : 0.0, t11 = fma(d1, d1, e0 * e0);
+          const double t12 = d1 * e1, t22 = fma(d2, d2, e1 * e1), dd = 0.5 * (t11 - t22);
           double mu;
           if (dd == 0.0 && t12 == 0.0) mu = t22;
           else mu = t22 - t12 * t12 / (dd + copysign(hypot(dd, t12), dd != 0.0 ? dd : 1.0));
           dk = D[lo * 32];
           ek = E[lo * 32];
-          y = dk * dk - mu;
+          y = fma(dk, dk, -mu);
           z = dk * ek;
           k = lo;
           dprev = 0.0;
@@ -224,15 +234,15 @@ k_svd_leaf(int nleaf, const int *__restrict__ lstart, const int *__restrict__ ls
       double t, cs, sn;
       plane_rotation(y, z, t, cs, sn);
       const double eprev = t;  // E(k - 1)
-      const double d0 = cs * dk + sn * ek, e0 = -sn * dk + cs * ek;
+      const double d0 = turn0(cs, sn, dk, ek), e0 = turn1(cs, sn, dk, ek);
       const double bl = sn * d1;
       d1 *= cs;
 #pragma unroll
       for (int j = 0; j < R; ++j) {
         if (R > 4 && j >= rows) break;
         const double x = Vs[((k + 1) * R + j) * 32];
-        Vs[(k * R + j) * 32] = cs * vc[j] + sn * x;
-        vc[j] = -sn * vc[j] + cs * x;
+        Vs[(k * R + j) * 32] = turn0(cs, sn, vc[j], x);
+        vc[j] = turn1(cs, sn, vc[j], x);
       }
       plane_rotation(d0, bl, t, cs, sn);
       D[k * 32] = t;
@@ -243,13 +253,13 @@ k_svd_leaf(int nleaf, const int *__restrict__ lstart, const int *__restrict__ ls
         ez = ng ? ez | 1u << (k - 1) : ez;
       }
       dprev = t;
-      const double ekn = cs * e0 + sn * d1, d1n = -sn * e0 + cs * d1;
+      const double ekn = turn0(cs, sn, e0, d1), d1n = turn1(cs, sn, e0, d1);
 #pragma unroll
       for (int j = 0; j < R; ++j) {
         if (R > 4 && j >= rows) break;
         const double x = Us[((k + 1) * R + j) * 32];
-        Us[(k * R + j) * 32] = cs * uc[j] + sn * x;
-        uc[j] = -sn * uc[j] + cs * x;
+        Us[(k * R + j) * 32] = turn0(cs, sn, uc[j], x);
+        uc[j] = turn1(cs, sn, uc[j], x);
       }
       if (k + 1 < hi) {
         ek = E[(k + 1) * 32];
