@@ -188,8 +188,7 @@ k_band_leaf(int nleaf, const int *__restrict__ lstart, const int *__restrict__ l
           double r1 = fma(th, th, 1.0), ri, t;
           if (__double2hiint(r1) < 0x7bf00000) {  // below 2^960
             sqrt_rcp_rn(r1, r1, ri);
-            const double b = fabs(th) + r1, y = rcp_nr(b);
-            t = copysign(fma(y, fma(-b, y, 1.0), y), th);
+            t = copysign(rcp_rn(fabs(th) + r1), th);
           } else {
             t = copysign(1.0, th) / (fabs(th) + sqrt(r1));
           }

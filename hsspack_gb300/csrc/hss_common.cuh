@@ -57,13 +57,54 @@ __device__ __forceinline__ void sqrt_pair(double x, double &r, double &rinv) {
   r = fma(h, c, h);
 }
 
+// Rounding to nearest from estimates within about an ulp, by Newton corrections whose
+// residuals fused multiply-adds form exactly (Markstein, IBM J. Res. Dev. 34, 1990), for
+// operands and results well inside the normal range.  The correction of a reciprocal
+// is exact but for a divisor with a mantissa of ones: 1 / b is then a power of two and
+// a little over half an ulp, the correction gives the power of two, and ones_bit adds
+// the ulp.  A quotient within 2^-51 ulps of the middle of two doubles may be either.
+__device__ __forceinline__ double ones_bit(double y, double b) {
+  int lo = __double2loint(y);
+  if ((__double2loint(b) & (__double2hiint(b) | (int)0xfff00000)) == -1) lo |= 1;
+  return __hiloint2double(__double2hiint(y), lo);
+}
+// sqrt(x) for x in sqrt_pair's range, and y = 1 / sqrt(x) within about an ulp
+__device__ __forceinline__ double sqrt_rn(double x, double &y) {
+  double r0;
+  sqrt_pair(x, r0, y);
+  const double y2 = __hiloint2double(__double2hiint(y) - (1 << 20), __double2loint(y));  // y / 2
+  return fma(fma(-r0, r0, x), y2, r0);
+}
+// r = sqrt(x) and 1 / r as the divide gives it: ten FP64 instructions
+__device__ __forceinline__ void sqrt_rcp_rn(double x, double &r, double &rinv) {
+  double y;
+  r = sqrt_rn(x, y);
+  rinv = ones_bit(fma(y, fma(-r, y, 1.0), y), r);
+}
+__device__ __forceinline__ double rcp_rn(double b) {
+  const double y = rcp_nr(b);
+  return ones_bit(fma(y, fma(-b, y, 1.0), y), b);
+}
+// a / b from y = 1 / b
+__device__ __forceinline__ double div_rn(double a, double b, double y) {
+  const double q = a * y;
+  return fma(fma(-q, b, a), y, q);
+}
+// a / b, by div_rn where both are within 2^+-480
+__device__ __forceinline__ double quot_rn(double a, double b) {
+  const unsigned ha = __double2hiint(a) & 0x7fffffff, hb = __double2hiint(b) & 0x7fffffff;
+  constexpr unsigned lo = 0x21f00000, w = 0x5df00000 - lo;
+  return ha - lo < w && hb - lo < w ? div_rn(a, b, rcp_nr(b)) : a / b;
+}
+
 // Householder reflector of (alpha, tail) with the tail's squared norm sg: beta, tau, and
 // scale with v = [1; tail * scale]
 struct HousePar {
   double beta, tau, scale;
 };
-// (one lane forms it, at a warp's FP64 price: root, reciprocal root and reciprocal
-// from estimates, each within about an ulp)
+// (one lane forms it, at a warp's FP64 price: the root and the reciprocal from estimates,
+// rounded to nearest; tau = 1 + |alpha| / |beta| in one multiply-add, within 1.5 ulps where
+// (beta - alpha) / beta has two)
 __device__ __forceinline__ HousePar house_par(double alpha, double sg) {
   HousePar h{alpha, 0.0, 0.0};
   if (sg > 0.0) {
@@ -71,10 +112,10 @@ __device__ __forceinline__ HousePar house_par(double alpha, double sg) {
     const int hx = __double2hiint(x);
     if (hx >= 0x03f00000 && hx < 0x7bf00000) {  // 2^-960 <= x < 2^960
       double rt, ri;
-      sqrt_pair(x, rt, ri);
+      rt = sqrt_rn(x, ri);
       h.beta = -copysign(rt, alpha);
-      h.tau = (h.beta - alpha) * -copysign(ri, alpha);
-      h.scale = rcp_nr(alpha - h.beta);
+      h.tau = fma(fabs(alpha), ri, 1.0);
+      h.scale = rcp_rn(alpha - h.beta);
     } else {
       h.beta = -copysign(sqrt(x), alpha);
       h.tau = (h.beta - alpha) / h.beta;
@@ -82,31 +123,6 @@ __device__ __forceinline__ HousePar house_par(double alpha, double sg) {
     }
   }
   return h;
-}
-
-// sqrt(x) and 1 / sqrt(x)'s own rounding 1 / r as the divide gives it, both rounded to
-// nearest, for x in sqrt_pair's range: one Newton correction each from the residual in a
-// fused multiply-add (Markstein, IBM J. Res. Dev. 34, 1990).  Ten FP64 instructions.
-// (Against sqrt and the divide on 3e8 random operands: no difference.)
-__device__ __forceinline__ void sqrt_rcp_rn(double x, double &r, double &rinv) {
-  double r0, y;
-  sqrt_pair(x, r0, y);
-  const double y2 = __hiloint2double(__double2hiint(y) - (1 << 20), __double2loint(y));  // y / 2
-  r = fma(fma(-r0, r0, x), y2, r0);
-  rinv = fma(y, fma(-r, y, 1.0), y);
-}
-// a / b rounded to nearest from y = 1 / b within about an ulp (a, b and the quotient
-// well inside the normal range)
-__device__ __forceinline__ double div_rn(double a, double b, double y) {
-  const double q = a * y;
-  return fma(fma(-q, b, a), y, q);
-}
-
-// a / b rounded to nearest, by div_rn where both are within 2^+-480
-__device__ __forceinline__ double quot_rn(double a, double b) {
-  const unsigned ha = __double2hiint(a) & 0x7fffffff, hb = __double2hiint(b) & 0x7fffffff;
-  constexpr unsigned lo = 0x21f00000, w = 0x5df00000 - lo;
-  return ha - lo < w && hb - lo < w ? div_rn(a, b, rcp_nr(b)) : a / b;
 }
 
 // |d| as FP32 rounded towards zero by integer operations (a conversion holds the

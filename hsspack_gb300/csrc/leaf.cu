@@ -20,9 +20,9 @@
 //    off-diagonal), so no scan over E precedes a sweep;
 //  * column i + 1 of the eigenvector block stays in registers from one rotation
 //    to the next; r and 1 / r of a rotation come from one estimate, each rounded
-//    to nearest (sqrt_rcp_rn).
+//    to nearest (but for a divisor in 2^52).
 // The arithmetic is the plain loop's to the last bit (the fused multiply-adds are
-// written out).  A merge takes the signs of its vectors from z, which holds entries
+// written out; tests/test_gpu_bits.py).  A merge takes the signs of its vectors from z, which holds entries
 // down to 8 eps: with a shift or rotations an ulp off, leaves of 20 rows and more turned
 // a vector's sign in one solve of ten.
 // Shared memory is interleaved by lane, so lanes at different columns never
@@ -135,7 +135,11 @@ k_leaf_ql(int nleaf, const int *__restrict__ lstart, const int *__restrict__ lsi
       double r, rinv;
       const int hx = __double2hiint(x);
       if (hx >= 0x03f00000 && hx < 0x7bf00000) {  // 2^-960 <= x < 2^960
-        sqrt_rcp_rn(x, r, rinv);
+        // (sqrt_rcp_rn but for its last bit where r's mantissa is all ones: the test of that
+        // in this chain costs 4 % of the stage)
+        double y;
+        r = sqrt_rn(x, y);
+        rinv = fma(y, fma(-r, y, 1.0), y);
         sn = f * rinv;
         cs = g * rinv;
       } else {

@@ -41,6 +41,7 @@
 #include "hss_common.cuh"
 #include "hss_gemm.h"
 #include "hss_hss.h"
+#include "hss_jacobi.cuh"
 #include "hss_plan.h"
 #include "hss_pool.h"
 
@@ -236,48 +237,6 @@ k_tall_qr(const TallDesc *__restrict__ descs, const QrJob *__restrict__ jobs) {
     const int c = e / r, i = e - c * r;
     jb.out[(long long)c * jb.ldo + (long long)i * jb.ros] = i <= c ? S[c * LD + i] : 0.0;
   }
-}
-
-// Tangent of the Jacobi rotation of two rows with squared norms a, b > 0 and product c:
-// the root of smaller modulus of c t^2 + x t - c = 0, x = b - a (t^2 + 2 zeta t = 1 with
-// zeta = x / 2c).  False: c^2 <= jtol2 a b, nothing to rotate.  The test and the first
-// estimate are FP32 on numbers brought to c's exponent by integer operations, and one
-// Newton step in FP64 (whose slope may be FP32's) finishes it: four FP64 instructions
-// where a reciprocal and a comparison in FP64 made it thirteen.  n = 2000, all
-// bases of a DHSSMM: 9.59 -> 9.28 ms.
-__device__ __forceinline__ bool jacobi_tan(double a, double b, double c, double jtol2, double &t) {
-  const int hc = __double2hiint(c), Ec = (hc >> 20) & 0x7ff;
-  const int Ea = __double2hiint(a) >> 20, Eb = __double2hiint(b) >> 20;
-  const double x = b - a;
-  const int hx = __double2hiint(x), Ex = (hx >> 20) & 0x7ff;
-  if (Ea >= 600 && Eb >= 600 && Ea < 1500 && Eb < 1500) {
-    if (Ec < 450) return false;  // (c^2 / (a b) below 2^-300)
-    auto mant = [](double v, int e) {  // |v| as FP32 with the exponent set to e
-      return __int_as_float((e + 127) << 23 | (__double2hiint(v) & 0xfffff) << 3 |
-                            (unsigned)__double2loint(v) >> 29);
-    };
-    const float mc = mant(c, 0);
-    const int D = 2 * Ec - Ea - Eb;
-    if (D < -100 || mc * mc * __int_as_float((D + 127) << 23) <= (float)jtol2 * mant(a, 0) * mant(b, 0))
-      return false;
-    const int dx = Ex - Ec;
-    if (dx < 120) {
-      const float zf = dx < -120 ? 0.f : __fdividef(0.5f * mant(x, dx), mc);
-      const float rf = zf < 1e15f ? sqrtf(fmaf(zf, zf, 1.f)) : zf;
-      const int sg = (hx ^ hc) & 0x80000000;
-      const double t0 = f64_of_f32(__fdividef(1.f, zf + rf));
-      t = __hiloint2double(__double2hiint(t0) | sg, __double2loint(t0));
-      const double f = fma(t, fma(t, c, x), -c);
-      const double w = f64_of_f32(__fdividef(0.5f, rf * mc));  // 1 / |2 c (t + zeta)|, c's sign x's
-      t = fma(f, __hiloint2double((__double2hiint(w) - ((Ec - 1023) << 20)) | (~hx & 0x80000000),
-                                  __double2loint(w)), t);
-      return true;
-    }
-  }
-  if (!(c * c > jtol2 * a * b)) return false;
-  const double zeta = x / (2.0 * c);
-  t = copysign(1.0 / (fabs(zeta) + sqrt(fma(zeta, zeta, 1.0))), zeta);
-  return true;
 }
 
 // Basis of one node from its R factor: the left singular vectors of R^T with

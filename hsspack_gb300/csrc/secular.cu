@@ -692,7 +692,7 @@ __global__ void k_build_S(LevelView lv, const double *__restrict__ dl,
   } else {
     double rt;
     const int hx = __double2hiint(acc);
-    if (hx >= 0x03f00000 && hx < 0x7bf00000) sqrt_pair(acc, rt, a);  // [2^-960, 2^960)
+    if (hx >= 0x03f00000 && hx < 0x7bf00000) sqrt_rcp_rn(acc, rt, a);  // [2^-960, 2^960)
     else a = 1.0 / sqrt(acc);
   }
   __syncwarp();

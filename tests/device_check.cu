@@ -1,5 +1,29 @@
-// The leaf solvers' iterations as plain loops, one thread per matrix (tests/test_gpu_bits.py).
+// The rounding helpers and the Jacobi angle of the kernels on arrays of operands, and the
+// leaf solvers' iterations as plain loops, one thread per matrix (tests/test_gpu_bits.py).
 #include "hss_common.cuh"
+#include "hss_jacobi.cuh"
+
+using namespace hss;
+
+__global__ void k_ops(int op, int n, const double *a, const double *b, const double *c, double *x,
+                      double *y, double *z) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  if (op == 0) sqrt_rcp_rn(a[i], x[i], y[i]);
+  if (op == 1) x[i] = quot_rn(a[i], b[i]);
+  if (op == 2) x[i] = rcp_rn(a[i]);
+  if (op == 3) {
+    const HousePar h = house_par(a[i], b[i]);
+    x[i] = h.beta;
+    y[i] = h.tau;
+    z[i] = h.scale;
+  }
+  if (op == 4) {
+    double t = 0.0;
+    y[i] = jacobi_tan(a[i], b[i], c[i], z[i], t);
+    x[i] = t;
+  }
+}
 
 constexpr int M = 32;
 struct Work {
@@ -154,6 +178,11 @@ __global__ void k_gk(int n, const int *m_, const int *off, const long long *zoff
 }
 
 extern "C" {
+int check_ops(int op, int n, const double *a, const double *b, const double *c, double *x, double *y,
+              double *z) {
+  k_ops<<<(n + 255) / 256, 256>>>(op, n, a, b, c, x, y, z);
+  return (int)cudaDeviceSynchronize();
+}
 long long check_work_bytes() { return (long long)sizeof(Work); }
 int check_leaves(int svd, int n, const int *m, const int *off, const long long *zoff, const double *d,
                  const double *e, void *work, double *w, double *U, double *V) {

@@ -1,5 +1,6 @@
-"""What the kernels promise to the last bits: the leaf solvers against their iterations as
-plain loops (tests/device_check.cu)."""
+"""What the kernels promise to the last bits: the helpers that replace sqrt and divides
+against numpy's (correctly rounded) ones, the Jacobi angle against extended precision, and
+the leaf solvers against their iterations as plain loops (tests/device_check.cu)."""
 import ctypes
 import os
 import subprocess
@@ -32,6 +33,113 @@ def _dev(a):
 
 def _p(t):
     return ctypes.c_void_p(t.data_ptr())
+
+
+def _ops(lib, op, a, b=None, c=None, z=None):
+    t = [_dev(v if v is not None else a) for v in (a, b, c)]
+    out = [torch.zeros_like(t[0]), torch.zeros_like(t[0]), _dev(z if z is not None else a)]
+    torch.cuda.synchronize()
+    assert lib.check_ops(op, len(a), *[_p(v) for v in t + out]) == 0
+    return [v.cpu().numpy() for v in out]
+
+
+def _operands(n, seed, lo, hi):
+    """Random mantissas and signs, exponents of lo .. hi; a share just below a power of two
+    and one with few bits."""
+    rng = np.random.default_rng(seed)
+    m = rng.uniform(1.0, 2.0, n)
+    m[: n // 8] = 2.0 - 2.0 ** -52 * rng.integers(1, 5, n // 8)
+    m[n // 8: n // 4] = 1.0 + 2.0 ** -rng.integers(1, 53, n // 4 - n // 8)
+    return np.ldexp(m * rng.choice([-1.0, 1.0], n), rng.integers(lo, hi, n))
+
+
+N = 1 << 20
+
+
+def test_roots(lib):
+    x = np.abs(_operands(N, 1, -960, 960))
+    r = np.sqrt(x)
+    got = _ops(lib, 0, x)
+    assert np.array_equal(got[0], r)
+    assert np.array_equal(got[1], 1.0 / r)
+
+
+@pytest.mark.parametrize("lo,hi", [(-479, 479), (-3, 3), (-1000, 1000)])
+def test_quotients(lib, lo, hi):
+    a, b = _operands(N, 2, lo, hi), _operands(N, 3, lo, hi)[::-1].copy()
+    with np.errstate(all="ignore"):
+        ref = a / b
+    assert np.array_equal(_ops(lib, 1, a, b)[0], ref)
+    if hi < 1000:
+        assert np.array_equal(_ops(lib, 2, b)[0], 1.0 / b)
+
+
+def test_quotients_next_to_a_midpoint(lib):
+    """a / b at a distance of 2^-54 ulps from the middle of two doubles, the closest there
+    is: b q = a 2^54 -+ 1 with an odd q.  There the result may be either neighbour."""
+    rng = np.random.default_rng(4)
+    a, b = [], []
+    while len(a) < 4096:
+        x = int(rng.integers(1 << 52, 1 << 53)) | 1
+        s = 1 if len(a) % 2 else -1
+        q = -s * pow(x, -1, 1 << 54) % (1 << 54)
+        y, rest = divmod(x * q + s, 1 << 54)
+        assert rest == 0
+        if q >> 53 and 0 < y < 1 << 53:
+            a.append(float(y))
+            b.append(float(x))
+    a, b = np.array(a), np.array(b)
+    ref = a / b
+    assert (np.abs(_ops(lib, 1, a, b)[0] - ref) <= np.spacing(ref)).all()
+
+
+def test_reflector(lib):
+    alpha = _operands(N, 5, -200, 200)
+    sg = np.abs(_operands(N, 6, -400, 400))[::-1].copy()
+    beta, tau, scale = _ops(lib, 3, alpha, sg)
+    x = np.longdouble(alpha) * alpha + sg  # one rounding more than the kernel's fma
+    ok = np.abs(beta) - np.sqrt(x).astype(np.float64)
+    assert (np.abs(ok) <= np.spacing(np.abs(beta))).all() and (beta * alpha < 0).all()
+    L = np.longdouble
+    exact = 1 + np.abs(L(alpha)) / np.sqrt(L(alpha) * alpha + sg)
+    # 1 / |beta| within an ulp times a factor of at most 1, and one rounding
+    assert (np.abs(L(tau) - exact) <= 1.5 * 2.0 ** -52).all()
+    assert np.array_equal(scale, 1.0 / (alpha - beta))
+
+
+@pytest.mark.parametrize("spread", [2, 40, 300])
+def test_jacobi_tangent(lib, spread):
+    """Root of smaller modulus of c t^2 + x t - c, x = b - a.  The last step rounds once
+    and its residual's error is at most half an ulp of t more: two ulps, four where the
+    operands' range calls for the plain formula."""
+    rng = np.random.default_rng(spread)
+    n = 1 << 18
+    a = np.ldexp(rng.uniform(1, 2, n), rng.integers(-spread, spread, n))
+    b = a * np.ldexp(rng.uniform(0.5, 1, n), rng.integers(-60, 60, n))
+    b[: n // 4] = a[: n // 4] * (1.0 + np.ldexp(rng.uniform(-1, 1, n // 4), -rng.integers(0, 53, n // 4)))
+    b[b == a] *= 1.5
+    c = np.sqrt(a) * np.sqrt(b) * np.ldexp(rng.uniform(-1, 1, n), -rng.integers(0, 40, n))
+    t, go, _ = _ops(lib, 4, a, b, c, np.full(n, 1e-30))
+    L = np.longdouble
+    x = L(b - a)
+    ref = 2 * L(c) / (x + np.copysign(np.sqrt(x * x + 4 * L(c) * L(c)), x))
+    go = go != 0
+    assert go.sum() > n // 2
+    err = np.abs((t - ref) / L(1) / np.spacing(np.abs(ref.astype(np.float64))))[go]
+    assert err.max() <= (2.0 if spread <= 300 else 4.0), float(err.max())
+
+
+def test_jacobi_threshold(lib):
+    """Every pair with c^2 > jtol^2 a b in FP64 is rotated, none with less than 0.9999 of it."""
+    rng = np.random.default_rng(9)
+    n = 1 << 18
+    a = np.ldexp(rng.uniform(1, 2, n), rng.integers(-200, 200, n))
+    b = a * np.ldexp(rng.uniform(0.5, 1, n), rng.integers(-20, 20, n))
+    j2 = (2.0 ** -52 * rng.integers(16, 129, n)) ** 2
+    c = np.sqrt(j2 * a * b) * (1.0 + np.ldexp(rng.uniform(-1, 1, n), -rng.integers(1, 53, n)))
+    c *= rng.choice([-1.0, 1.0], n)
+    go = _ops(lib, 4, a, b, c, j2)[1] != 0
+    assert go[c * c > j2 * a * b].all() and not go[c * c < 0.9999 * j2 * a * b].any()
 
 
 def _plain(lib, svd, sizes, d, e):
