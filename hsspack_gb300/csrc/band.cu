@@ -276,7 +276,7 @@ __global__ void k_band_z(int P, const int *__restrict__ ms, const int *__restric
 // zhat_i alpha_j / (d_i - lam_j) (warp per root, as the alpha kernel).  Bound by the
 // FP64 pipe, where the division is most of a term: it is formed once for up to ZU
 // columns (n = 16384, kd = 4, with the norms taken from the vector blocks instead
-// of a pass of their own: 9.3 -> 4.0 ms).
+// of a pass of their own: 9.6 -> 3.3 ms).
 constexpr int ZU = 8;
 template <int NC>
 __device__ __forceinline__ void band_zupdate_cols(const PoleDiff &P, int j, int s, int K, double aj,

@@ -212,7 +212,7 @@ long long sbr_reflectors(int n, int b, std::vector<long long> *roff) {
 void launch_sbr_load(int n, int kd, int b, const double *AB, long long ldab, double *LB, int ldb,
                      cudaStream_t st) {
   const long long total = (long long)n * ldb;
-  const int grid = (int)std::min<long long>((total + 255) / 256, 152LL * 16);
+  const int grid = (int)std::min<long long>((total + 255) / 256, HSS_SMS * 16LL);
   k_sbr_load<<<grid, 256, 0, st>>>(n, kd, b, AB, ldab, LB, ldb);
 }
 

@@ -535,7 +535,7 @@ static void run_merges(Ctx &c, const std::vector<int> &ms, const std::vector<int
     stage_end(HSS_ST_OTHER, st, 0, (2.0 + 4.0 * bu->nrest) * k2);
     c.launches += 2;
   };
-  // ---- dense merges: S, gather, GEMM (block structured), scatter
+  // ---- dense merges: gather, S, block-structured products into the slots
   if (PD > 0) {
     int *xs = (int *)(dpk + o_ds), *xK = (int *)(dpk + o_dK), *xoff = (int *)(dpk + o_doff),
         *xn = (int *)(dpk + o_dn), *xr = (int *)(dpk + o_dr);
@@ -1246,18 +1246,15 @@ static void svd_merge_tail(Ctx &c, const std::vector<int> &ms, const std::vector
     stage_end(HSS_ST_BUILD_S, st, 16LL * totB, 20.0 * k2);
     // the products go straight into the non-deflated slots' columns
     std::vector<GemmDesc> probs;
-    int tiles = 0;
     double fl = 0.0;
     long long gb = 0;
     for (int m = 0; m < PD; ++m) {
       const int K = dK_[m], N = dN_[m], M = dM_[m];
       const int *slots = L.w.ndslot + ds_[m], ldi = (int)ld;
-      probs.push_back(GemmDesc{U2 + qU[m], Ub + bo[m], U + rU_[m], N, K, ldi, N, K, K, 0, tiles, 0,
+      probs.push_back(GemmDesc{U2 + qU[m], Ub + bo[m], U + rU_[m], N, K, ldi, N, K, K, 0, 0, 0,
                                slots});
-      tiles += gemm_tiles(N, K);
-      probs.push_back(GemmDesc{V2 + qV[m], Vb + bo[m], V + rV_[m], M, K, ldi, M, K, K, 0, tiles, 0,
+      probs.push_back(GemmDesc{V2 + qV[m], Vb + bo[m], V + rV_[m], M, K, ldi, M, K, K, 0, 0, 0,
                                slots});
-      tiles += gemm_tiles(M, K);
       fl += 2.0 * (double)(N + M) * K * K;
       gb += 8LL * ((long long)(N + M) * K * 2 + 2LL * K * K);
     }

@@ -6,6 +6,9 @@
 #define HSS_EPS 1.1102230246251565e-16   /* 2^-53, LAPACK DLAMCH('Epsilon') */
 #define HSS_WARP 32
 #define HSS_FULL 0xffffffffu
+// SMs of a GB300, for the rules that split work by them.  A constant, not the device's count:
+// lanes per column and per leaf fix orders of summation, so results depend on it.
+constexpr int HSS_SMS = 152;
 
 // ---- warp all-reduce (butterfly: every lane ends with the same bits) --------
 __device__ __forceinline__ double warp_sum(double v) {

@@ -128,8 +128,7 @@ void launch_gather(int P, int total, int maxn, const int *ms, const int *mn, con
                    const int *mr = nullptr);
 void launch_scatter(int P, int total, int maxn, const int *ms, const int *mn, const int *rootoff,
                     const int *ndslot, const long long *toff, const double *T, double *Q,
-                    long long ldq, cudaStream_t st, int2 *sup = nullptr,
-                    const int *mr = nullptr);
+                    long long ldq, cudaStream_t st, int2 *sup = nullptr);
 // columns about to be rotated: both of a pair made valid on the union of their
 // supports
 void launch_widen(int P, int maxn, const int *ms, const int *ng,

@@ -67,18 +67,21 @@ __device__ __forceinline__ void leaf_ranks_ties(int m, const double *D, int *rk)
 // behind it (measured: a dependent chain and eight independent ones, 1 to 4
 // warps per SM, all 64.2 cycles per instruction, 8 warps 128).  So few leaves
 // get a warp each, and the group halves once there are more than two warps per
-// quarter of the 152 SMs.  Leaf stage at the neighbouring choices (tridiagonal,
-// rotations without their final rounding, a fifth less):
-//   128 leaves of 16 rows   G = 32 or 16 0.42 ms   8 0.51   4 0.66
-//   1024 of 16              G = 16 0.47 ms         8 0.55   4 0.71
-//   3800 of 8 to 16         G = 8  0.59 ms        16 0.73   4 0.69
-//   15000 of 8 to 16        G = 2  1.22 ms         4 1.36   1 1.52
-//   61000 of 8 to 16        G = 2  3.43 ms         4 4.44   1 4.02
-// Above 12 rows one lane per leaf leaves shared memory for three CTAs on an SM,
-// two lanes for five.
+// quarter of the SMs.  Leaf stage of tridiagonal batches, the rule's choice (*) and its
+// neighbours, ms:
+//   128 leaves of 16 rows   G = 32 0.47   16* 0.50    8 0.62    4 0.79
+//   512 of 25               G = 32* 1.15  16 1.35     8 1.71    4 2.48
+//   1024 of 16              G = 32 0.76   16* 0.57    8 0.66    4 0.82
+//   3800 of 8 to 16         G = 16 1.30    8* 0.92    4 0.83    2 1.11
+//   15000 of 8 to 16        G = 4 2.32     2* 2.17    1 2.90
+//   61000 of 8 to 16        G = 4 7.85     2* 6.21    1 7.38
+//   61000 of 4 to 8         G = 4 2.22     2 1.34     1* 0.97
+// Above 12 rows one lane per leaf leaves shared memory for three CTAs on an SM, two lanes
+// for five.  Many leaves of 24 to 32 rows would want more lanes for the same reason (15000
+// of them: 2* 36.7, 8 16.2).
 inline int leaf_lanes(int nleaf, int mmax) {
   int G = 32;
-  while (G > 1 && (long long)nleaf * G / 32 > 8 * 152) G /= 2;
+  while (G > 1 && (long long)nleaf * G / 32 > 8 * HSS_SMS) G /= 2;
   while (G > 8 && G / 2 >= mmax) G /= 2;
   if (G == 1 && mmax > 12) G = 2;
   while (G < 32 && (mmax + G - 1) / G > 16) G *= 2;

@@ -27,9 +27,9 @@
 // a vector's sign in one solve of ten.
 // Shared memory is interleaved by lane, so lanes at different columns never
 // share a bank.  Leaf stage, one thread per leaf with nested loops before -> now:
-// n = 257 (16 leaves of 16 rows) 2.33 -> 0.51 ms, n = 2048 2.10 -> 0.53 ms, 512
-// problems (61000 leaves of 8 to 16) 6.37 -> 4.09 ms, n = 32768 (4096 of 8)
-// 0.41 -> 0.29 ms.
+// n = 257 (16 leaves of 16 rows) 2.33 -> 0.50 ms, n = 2048 2.10 -> 0.51 ms, 512
+// problems (61000 leaves of 8 to 16) 6.37 -> 3.97 ms, n = 32768 (4096 of 8)
+// 0.41 -> 0.27 ms.
 #include "hss_common.cuh"
 #include "hss_kernels.h"
 #include "hss_leaf.cuh"
@@ -240,7 +240,6 @@ void launch_leaf(int nleaf, const int *lstart, const int *lsize, int mmax, int n
 #define LEAF_TRY(g, r) if (G == g && R <= r) return leaf_launch<g, r>(LEAF_ARGS)
   LEAF_TRY(1, 8);
   LEAF_TRY(1, 12);
-  LEAF_TRY(1, 16);
   LEAF_TRY(2, 4);
   LEAF_TRY(2, 6);
   LEAF_TRY(2, 8);

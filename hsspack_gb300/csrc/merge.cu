@@ -32,9 +32,9 @@ __device__ __forceinline__ double qat(const double *__restrict__ Q, long long ld
 
 // Row windows: the union of the supports of the columns that a merge takes up.
 // Rows outside it are zero in all of them and stay zero in the new ones, so the
-// products of a merge run over its window alone.  (Gather, digit planes, products
-// and scatter scale with the rows: 512 problems 60.8 -> 58.2 ms, n = 32768 7.29 ->
-// 6.73 ms, COMPZ = 'V' n = 2048 6.18 -> 4.79 ms, band n = 16384, kd = 4 65.5 -> 62.0.)
+// products of a merge run over its window alone.  (Gather, digit planes and products scale
+// with the rows: alone it took 4 % off 512 problems and 5 % off the band n = 16384, kd = 4,
+// 8 % off n = 32768, 22 % off COMPZ = 'V' n = 2048.)
 __device__ __forceinline__ void window_add(int2 &w, int2 r) {
   if (r.y > r.x) { w.x = min(w.x, r.x); w.y = max(w.y, r.y); }
 }
@@ -904,7 +904,7 @@ __global__ void k_gather(int P, int nseg, const int *__restrict__ ms, const int 
 
 // Write the new eigenvectors (columns of T, n_m x K) into the non-deflated slots.
 __global__ void k_scatter(int P, int nseg, const int *__restrict__ ms, const int *__restrict__ mn,
-                          const int *__restrict__ mr, const int *__restrict__ rootoff, const int *__restrict__ ndslot,
+                          const int *__restrict__ rootoff, const int *__restrict__ ndslot,
                           const long long *__restrict__ toff, const double *__restrict__ T,
                           double *__restrict__ Q, long long ldq, int2 *__restrict__ sup) {
   const long long wg = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -915,10 +915,9 @@ __global__ void k_scatter(int P, int nseg, const int *__restrict__ ms, const int
   const int s = ms[m], n = mn[m];
   const int i0 = q * GS_SEG, i1 = min(n, i0 + GS_SEG);
   if (i0 >= i1) return;
-  const int row0 = mr ? mr[m] : s;
   const double *src = T + toff[m] + (long long)j * n;
-  double *dst = Q + (long long)ndslot[s + j] * ldq + row0;
-  if (sup && q == 0 && lane == 0) sup[ndslot[s + j]] = make_int2(row0, row0 + n);
+  double *dst = Q + (long long)ndslot[s + j] * ldq + s;
+  if (sup && q == 0 && lane == 0) sup[ndslot[s + j]] = make_int2(s, s + n);
   for (int i = i0 + lane; i < i1; i += 32) dst[i] = src[i];
 }
 
@@ -1214,12 +1213,12 @@ void launch_gather(int P, int total, int maxn, const int *ms, const int *mn, con
 }
 void launch_scatter(int P, int total, int maxn, const int *ms, const int *mn, const int *rootoff,
                     const int *ndslot, const long long *toff, const double *T, double *Q,
-                    long long ldq, cudaStream_t st, int2 *sup, const int *mr) {
+                    long long ldq, cudaStream_t st, int2 *sup) {
   if (total <= 0) return;
   const int nseg = (maxn + GS_SEG - 1) / GS_SEG;
   const long long warps = (long long)total * nseg;
-  k_scatter<<<(unsigned)((warps + 7) / 8), 256, 0, st>>>(P, nseg, ms, mn, mr, rootoff, ndslot, toff,
-                                                         T, Q, ldq, sup);
+  k_scatter<<<(unsigned)((warps + 7) / 8), 256, 0, st>>>(P, nseg, ms, mn, rootoff, ndslot, toff, T,
+                                                         Q, ldq, sup);
 }
 void launch_widen(int P, int maxn, const int *ms, const int *ng,
                   const LevelScratch &w, double *Q, long long ldq, int2 *sup, cudaStream_t st) {

@@ -1068,7 +1068,7 @@ k_secular_mid(LevelView lv, const double *__restrict__ dl, const double *__restr
 // Threads per CTA for the root kernels: 256 when the level fills the GPU
 // several times over, else 64 so that a small level still spreads over all
 // 152 SMs (the kernels use no shared memory and no block barriers).
-static inline int root_block(long long threads) { return threads >= 152LL * 256 * 2 ? 256 : 64; }
+static inline int root_block(long long threads) { return threads >= (long long)HSS_SMS * 256 * 2 ? 256 : 64; }
 
 static inline int warp_grid(int total, int threads) {
   return (int)(((long long)total * 32 + threads - 1) / threads);
@@ -1079,9 +1079,9 @@ static inline int warp_grid(int total, int threads) {
 // no-allocation Loewner entry), hence relaxed atomics.
 static std::atomic<int> g_sec_terms{8};
 void set_secular_terms(int t) { g_sec_terms.store(t > 0 ? t : 8, std::memory_order_relaxed); }
-static std::atomic<long long> g_sec_threads{152LL * 256};
+static std::atomic<long long> g_sec_threads{(long long)HSS_SMS * 256};
 void set_secular_threads(int t) {
-  g_sec_threads.store(t > 0 ? t : 152LL * 256, std::memory_order_relaxed);
+  g_sec_threads.store(t > 0 ? t : (long long)HSS_SMS * 256, std::memory_order_relaxed);
 }
 
 // Lanes per root of a level with `total` roots and largest merge maxk: the
@@ -1110,7 +1110,7 @@ void launch_secular(const LevelView &lv, int total, int maxk, const double *dl, 
   unsigned grid = (unsigned)(((long long)total * L + tb - 1) / tb);
   // wide levels at one root per lane: 152 x 512 lanes, each with a sequence of
   // roots (secular_lanes), once there are at least two roots per lane
-  constexpr long long SEC_LANES = 152LL * 512;
+  constexpr long long SEC_LANES = HSS_SMS * 512LL;
   const bool lanes = L == 1 && total >= 2 * SEC_LANES;
   if (lanes) { tb = 256; grid = (unsigned)(SEC_LANES / tb); }
   switch (L * 2 + (sq ? 1 : 0)) {
@@ -1193,7 +1193,7 @@ void launch_build_S(const LevelView &lv, int total, const double *dl, const doub
   // least 152 x 512 lanes (512 problems, 32 lanes at every level before: 7.2 ms, now
   // 2.9 ms).  fixed: 32, whatever the level
   int L = 32;
-  while (!fixed && L > 4 && (L * 2 > maxk || (long long)total * (L / 2) >= 152LL * 512)) L /= 2;
+  while (!fixed && L > 4 && (L * 2 > maxk || (long long)total * (L / 2) >= HSS_SMS * 512LL)) L /= 2;
   const int tb = root_block((long long)total * L);
   const unsigned grid = (unsigned)(((long long)total * L + tb - 1) / tb);
 #define BS_CASE(n) \

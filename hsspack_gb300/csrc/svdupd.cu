@@ -128,9 +128,7 @@ int svd_update_core(int n, double *d, double *f, double *z, double *vt, long lon
     launch_alpha(lv, K, f, difl, difr, zhat, alpha, st, true);
     k_negate<<<(K + 255) / 256, 256, 0, st>>>(K, alpha);
     if (K >= 2 * ni) {
-      // the HSS product runs in FP64 whatever the configured precision: the
-      // split-BF16 form of this product once ended in a device fault (n = 10000,
-      // V = I) whose cause is not established, so it is not used here
+      // the HSS product runs in FP64 whatever the configured precision
       (void)precision;
       hss_dhssevc_core(K, ni, tol, 0, f, zhat, alpha, difl, difr, W2, n, n, rank, st, times, true,
                        1.1);

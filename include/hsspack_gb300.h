@@ -48,7 +48,8 @@ typedef struct hss_config {
   int reserved[2];
 } hss_config;
 
-/* stages timed when hss_config.profile = 1 */
+/* stages timed when hss_config.profile = 1 (HSS_ST_SCATTER keeps its number and reads 0:
+ * the products write the new vectors in place) */
 enum hss_stage {
   HSS_ST_LEAF = 0, HSS_ST_PREPARE, HSS_ST_GIVENS, HSS_ST_SECULAR, HSS_ST_LOWNER,
   HSS_ST_BUILD_S, HSS_ST_GATHER, HSS_ST_GEMM, HSS_ST_SCATTER, HSS_ST_FINISH,
