@@ -191,3 +191,63 @@ def test_bidiagonal_leaf(lib, n):
             assert torch.equal(vo.view(n, n), v.view(n, n).flip(0).T)
     finally:
         hp.restore_config(old)
+
+
+def _digit_rows(x):
+    """Seven rounded base-256 digits (ties up) of the rows of x scaled to below 2^60 by the
+    exponent of the row's largest entry, and those exponents."""
+    e = np.frexp(np.abs(x).max(axis=1))[1]
+    q = [[int(v) for v in np.ldexp(r, 60 - int(ei))] for r, ei in zip(x, e)]
+    d = []
+    for row in q:
+        digs = []
+        for v in row:
+            ds = []
+            for s in range(7):
+                sh = 53 - 8 * s
+                t = (v + (1 << (sh - 1))) >> sh
+                ds.append(t)
+                v -= t << sh
+            digs.append(ds)
+        d.append(digs)
+    return d, e
+
+
+@pytest.mark.parametrize("k", [8, 127, 128, 129, 300])
+@pytest.mark.parametrize("path", [0, 1])
+def test_split_product_bits(k, path):
+    """The split products' own arithmetic in Python integers: digit products of groups 0 to 6,
+    exact sums, one rounding (path 1: one per window of 128, added up).  Entries of at least
+    2^-7 of their row's largest, so the scaled integers are exact."""
+    rng = np.random.default_rng(k)
+    m, n = 140, 40
+    A, B = (rng.uniform(0.01, 1.0, s) * rng.choice([-1.0, 1.0], s) for s in ((m, k), (k, n)))
+    A *= np.ldexp(1.0, rng.integers(-30, 30, (m, 1)))
+    A[:, 0] = np.abs(A).max(axis=1)
+    B[0] = 1.0
+    dA, dB = (_dev(x.ravel(order="F")) for x in (A, B))
+    dC = torch.empty(m * n, dtype=torch.float64, device="cuda")
+    old = hp.set_config(gemm_path=path, split_min_log2=15)
+    try:
+        hp.gemm_dev(dA, dB, dC, m, n, k, m, k, m, precision=1)
+    finally:
+        hp.restore_config(old)
+    C = dC.cpu().numpy().reshape(m, n, order="F")
+    rows, cols = [0, 31, 32, 127, 128, 139], [0, 15, 16, 31, 32, 39]
+    da, ea = _digit_rows(A[rows])
+    db, eb = _digit_rows(B[:, cols].T)
+    for i, r in enumerate(rows):
+        for j, c in enumerate(cols):
+            parts = []
+            for w0 in range(0, k, 128) if path else [0]:
+                v = 0
+                for t in range(w0, min(k, w0 + 128) if path else k):
+                    for s in range(7):
+                        for p in range(7 - s):
+                            v += (da[i][t][s] * db[j][t][p]) << (8 * (6 - s - p))
+                parts.append(v)
+            # weight of group 6: 2^(e + f - 30 - 32)
+            ref = 0.0
+            for v in parts:
+                ref += np.ldexp(float(v), int(ea[i] + eb[j]) - 62)
+            assert C[r, c] == ref, (r, c, C[r, c], ref)
